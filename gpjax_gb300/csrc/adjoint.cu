@@ -13,6 +13,7 @@
 // go to a workspace array that a single block reduces in a fixed order, so
 // the gradient is deterministic.
 #include "simt_tile.cuh"
+#include "xgemm.cuh"
 
 namespace gpk {
 
@@ -20,7 +21,9 @@ namespace gpk {
 // the variance term and the noise term.
 __host__ __device__ inline int grad_slots(int d) { return d + 2; }
 
-template <typename T, int DMAX>
+// FROM_W: V holds W = Sigma^-1 itself (lower tiles), formed beforehand on the
+// tensor cores; the kernel is then the reduction alone.
+template <typename T, int DMAX, bool FROM_W = false>
 __global__ void __launch_bounds__((GemmCfg<T>::BM / GemmCfg<T>::TM) * (GemmCfg<T>::BN / GemmCfg<T>::TN))
     lauum_grad_kernel(int kind, const T* __restrict__ V, int64_t ldv, int n, int d,
                       const T* __restrict__ xs, const double* __restrict__ alpha,
@@ -46,20 +49,27 @@ __global__ void __launch_bounds__((GemmCfg<T>::BM / GemmCfg<T>::TM) * (GemmCfg<T
   int I, J;
   tri_index(t, I, J);
   const int i0 = I * BM, j0 = J * BN;
-  int klo, khi;
-  tile_krange<BM, BN, BK>(n, TRI_UPPER, TRI_UPPER, i0, j0, klo, khi);
-  T acc[TM][TN];
+  if constexpr (FROM_W) {
+    for (int e = threadIdx.x; e < BM * BN; e += NT) {
+      const int r = e / BN, c = e % BN;
+      Ws[r * WLD + c] = i0 + r < n && j0 + c <= i0 + r ? V[(int64_t)(i0 + r) * ldv + j0 + c] : T(0);
+    }
+  } else {
+    int klo, khi;
+    tile_krange<BM, BN, BK>(n, TRI_UPPER, TRI_UPPER, i0, j0, klo, khi);
+    T acc[TM][TN];
 #pragma unroll
-  for (int a = 0; a < TM; ++a)
+    for (int a = 0; a < TM; ++a)
 #pragma unroll
-    for (int b = 0; b < TN; ++b) acc[a][b] = T(0);
-  simt_tile_mma<T>(V, ldv, n, TRI_UPPER, V, ldv, n, TRI_UPPER, i0, j0, klo, khi, sm, acc);
-  // (simt_tile_mma ends with a barrier, so the staging area can be reused)
-  const int tx = threadIdx.x % NTX, ty = threadIdx.x / NTX;
+      for (int b = 0; b < TN; ++b) acc[a][b] = T(0);
+    simt_tile_mma<T>(V, ldv, n, TRI_UPPER, V, ldv, n, TRI_UPPER, i0, j0, klo, khi, sm, acc);
+    // (simt_tile_mma ends with a barrier, so the staging area can be reused)
+    const int tx = threadIdx.x % NTX, ty = threadIdx.x / NTX;
 #pragma unroll
-  for (int a = 0; a < TM; ++a)
+    for (int a = 0; a < TM; ++a)
 #pragma unroll
-    for (int b = 0; b < TN; ++b) Ws[(ty + a * NTY) * WLD + tx + b * NTX] = acc[a][b];
+      for (int b = 0; b < TN; ++b) Ws[(ty + a * NTY) * WLD + tx + b * NTX] = acc[a][b];
+  }
   for (int e = threadIdx.x; e < BM * DMAX; e += NT) {
     int r = e / DMAX, k = e % DMAX;
     sxi[e] = (i0 + r < n && k < d) ? xs[(int64_t)(i0 + r) * d + k] : T(0);
@@ -131,7 +141,7 @@ __global__ void __launch_bounds__((GemmCfg<T>::BM / GemmCfg<T>::TM) * (GemmCfg<T
   }
 }
 
-template <typename T, int DMAX>
+template <typename T, int DMAX, bool FROM_W = false>
 static cudaError_t launch_lauum_grad(int kind, const T* V, int64_t ldv, int n, int d, const T* xs,
                                      const double* alpha, double* gpart, const double* kaptr,
                                      cudaStream_t s) {
@@ -144,10 +154,10 @@ static cudaError_t launch_lauum_grad(int kind, const T* V, int64_t ldv, int n, i
   const size_t smem = ((front + 15) & ~size_t(15)) + (size_t)(BM + BN) * DMAX * sizeof(T) +
                       (size_t)(BM + BN) * sizeof(T) + 16 +
                       (size_t)(GPK_MAX_D + 2) * (NT / 32) * sizeof(double);
-  cudaFuncSetAttribute(lauum_grad_kernel<T, DMAX>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)smem);
-  lauum_grad_kernel<T, DMAX><<<tiles, NT, smem, s>>>(kind, V, ldv, n, d, xs, alpha, gpart,
-                                                     kaptr);
+  cudaFuncSetAttribute(lauum_grad_kernel<T, DMAX, FROM_W>,
+                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  lauum_grad_kernel<T, DMAX, FROM_W><<<tiles, NT, smem, s>>>(kind, V, ldv, n, d, xs, alpha, gpart,
+                                                             kaptr);
   return launch_status();
 }
 
@@ -168,6 +178,31 @@ cudaError_t lauum_grad(int kind, const T* V, int64_t ldv, int n, int d, const T*
   if (d <= 8) return launch_lauum_grad<T, 8>(kind, V, ldv, n, d, xs, alpha, gpart, ka, s);
   if (d <= 16) return launch_lauum_grad<T, 16>(kind, V, ldv, n, d, xs, alpha, gpart, ka, s);
   if (d <= 32) return launch_lauum_grad<T, 32>(kind, V, ldv, n, d, xs, alpha, gpart, ka, s);
+  return cudaErrorInvalidValue;
+}
+
+cudaError_t lauum_grad_x(int kind, const double* V, int64_t ldv, int n, int d, const double* xs,
+                         const double* theta, int n_ls, const double* alpha, double* gpart,
+                         double* W, int64_t ldw, const XRoom& x, cudaStream_t s) {
+  if (n <= 0) return cudaSuccess;
+  GemmProb<double> p{};
+  p.A = p.B = V;
+  p.lda = p.ldb = ldv;
+  p.a_tri = p.b_tri = TRI_UPPER;
+  p.C = W;
+  p.ldc = ldw;
+  p.M = p.N = p.K = n;
+  p.c_lower = 1;
+  p.alpha = 1.0;
+  cudaError_t e = gemm_nt_x(p, 1, x, s);
+  if (e != cudaSuccess) return e;
+  const double* ka = kind == GPK_RATIONAL_QUADRATIC ? theta + n_ls + 3 : nullptr;
+  if (d <= 8)
+    return launch_lauum_grad<double, 8, true>(kind, W, ldw, n, d, xs, alpha, gpart, ka, s);
+  if (d <= 16)
+    return launch_lauum_grad<double, 16, true>(kind, W, ldw, n, d, xs, alpha, gpart, ka, s);
+  if (d <= 32)
+    return launch_lauum_grad<double, 32, true>(kind, W, ldw, n, d, xs, alpha, gpart, ka, s);
   return cudaErrorInvalidValue;
 }
 

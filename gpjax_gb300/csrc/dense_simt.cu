@@ -8,7 +8,9 @@
 // (gpjax/linalg/operations.py:54-55), jsp.linalg.solve_triangular
 // (operations.py:105-107) and the LU of jnp.linalg.solve / slogdet
 // (operations.py:109-111,163-165).
+#include "fixed64.cuh"
 #include "simt_tile.cuh"
+#include "xgemm.cuh"
 
 namespace gpk {
 
@@ -101,8 +103,7 @@ cudaError_t gemm_nt(const GemmProb<T>& p, int batch, cudaStream_t s) {
 // Diagonal-block Cholesky: one CTA factors the nb x nb block at (k0, k0) in
 // shared memory (unblocked right-looking, two barriers per column).  Each
 // pivot's square root and reciprocal are taken once, by the thread that
-// finishes that diagonal entry (float64 square roots and divisions are slow
-// on this part: one per thread per column dominated the block).
+// finishes that diagonal entry.  Float32 form; the float64 one is below.
 // ---------------------------------------------------------------------------
 template <typename T, int NB>
 __global__ void __launch_bounds__(512) potrf_diag_kernel(T* A, int64_t lda, int n, int k0,
@@ -240,89 +241,292 @@ __global__ void __launch_bounds__(128) trsm_rows_thread_kernel(T* A, int64_t lda
   }
 }
 
-// Panel solve, float64 form: TRSM_ROWS rows per CTA (so that a short panel
-// still spreads over many SMs: float64 throughput per SM is low), eliminated
-// column by column by all threads: after column j is final, every later
-// column c of every row takes x[c] -= (x[j] / L[j, j]) L[c, j].  The columns
-// stay unscaled until the end (one barrier per column).
-constexpr int TRSM_ROWS = 32;
-template <typename T, int NB>
-__global__ void __launch_bounds__(256) trsm_rows_kernel(T* A, int64_t lda, int n, int k0) {
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  constexpr int LD = NB + 1;
-  T* Ls = reinterpret_cast<T*>(smem_raw);
-  T* Xs = Ls + NB * LD;
-  T* rinv = Xs + TRSM_ROWS * LD;
-  const int nb = min(NB, n - k0);
-  const int r0 = k0 + nb + blockIdx.x * TRSM_ROWS;
-  const int rows = min(TRSM_ROWS, n - r0);
-  if (rows <= 0) return;
-  for (int e = threadIdx.x; e < nb * nb; e += blockDim.x) {
-    int i = e / nb, j = e % nb;
-    Ls[i * LD + j] = (j <= i) ? A[(int64_t)(k0 + i) * lda + k0 + j] : T(0);
-  }
-  for (int e = threadIdx.x; e < rows * nb; e += blockDim.x) {
-    int r = e / nb, c = e % nb;
-    Xs[r * LD + c] = A[(int64_t)(r0 + r) * lda + k0 + c];
+// ---------------------------------------------------------------------------
+// Float64 form of both, in fixed point (fixed64.cuh).
+//
+// The diagonal block: thread (row i, column group g), right-looking.  Columns
+// go eight at a time; the columns to the right of a group take its eight
+// together, so that their 64-bit sums are shifted into place once per eight
+// products.  The chain of 64 pivots bounds it (a reciprocal root takes about
+// 310 clocks, a scaled entry 125, a product and its difference 53).
+// ---------------------------------------------------------------------------
+constexpr int FX_NB = 64;
+constexpr int FX_G = 8;  // columns factored between updates of the rest
+__global__ void __launch_bounds__(256)
+    potrf_diag_fixed_kernel(double* A, int64_t lda, int n, int k0, double* logdiag, int* info) {
+  using namespace fx;
+  __shared__ long long S[FX_NB][FX_NB + 1];
+  __shared__ Limbs lim[FX_G][FX_NB];
+  __shared__ int ex[FX_NB], sbad[FX_NB], sdead;
+  const int nb = min(FX_NB, n - k0);
+  const int i = threadIdx.x & 63, g = threadIdx.x >> 6;
+  if (threadIdx.x < FX_NB) {
+    ex[i] = i < nb ? scale_of(A[(int64_t)(k0 + i) * lda + k0 + i]) : 0;
+    sbad[i] = 0;
+    if (i == 0) sdead = 0;
   }
   __syncthreads();
-  for (int j = threadIdx.x; j < nb; j += blockDim.x) rinv[j] = T(1) / Ls[j * LD + j];
+  for (int e = threadIdx.x; e < FX_NB * FX_NB; e += 256) {
+    const int r = e >> 6, c = e & 63;
+    bool bad = false;
+    S[r][c] = r < nb && c <= r
+                  ? to_fixed(A[(int64_t)(k0 + r) * lda + k0 + c], ex[r] + ex[c], bad)
+                  : 0;
+    if (bad) sbad[r] = 1;
+  }
   __syncthreads();
-  for (int j = 0; j + 1 < nb; ++j) {
-    const int w = nb - 1 - j;  // columns j+1 .. nb-1
-    const T rj = rinv[j];
-    for (int e = threadIdx.x; e < rows * w; e += blockDim.x) {
-      const int r = e / w, c = j + 1 + e % w;
-      Xs[r * LD + c] -= (Xs[r * LD + j] * rj) * Ls[c * LD + j];
+  // step j: the first 64 threads bring column j up to date with column j - 1
+  // and scale it by its pivot's reciprocal root (each thread derives the pivot
+  // itself); the others meanwhile apply column j - 1 to the group's columns
+  // after j.  One barrier per column.
+  for (int c0 = 0; c0 < nb; c0 += FX_G) {
+    const int c1 = min(c0 + FX_G, nb);
+    Limbs lv{0, 0};  // this row's entry of the previous column (first 64 threads)
+    for (int j = c0; j < c1; ++j) {
+      if (g == 0) {
+        long long t = S[i][j], d = S[j][j];
+        if (j > c0) {
+          const Limbs w = lim[j - 1 - c0][j];
+          Acc at, ad;
+          at.add(lv, w);
+          ad.add(w, w);
+          t -= at.value();
+          d -= ad.value();
+        }
+        bool bad = false;
+        long long v = 0;
+        if (d > 0 && !sbad[j]) {
+          long long y;
+          int s;
+          rsqrt_fixed(d, y, s);
+          v = i >= j ? times_rsqrt(t, y, s, bad) : 0;
+        } else if (i == j) {
+          atomicMin(info, k0 + j + 1);
+          sdead = 1;
+        }
+        lv = limbs(v);
+        lim[j - c0][i] = lv;
+        if (bad) sbad[i] = 1;
+      } else if (j > c0) {
+        const Limbs mine = lim[j - 1 - c0][i];
+        for (int k = j + g; k < c1; k += 3) {
+          if (i < k) continue;
+          Acc acc;
+          acc.add(mine, lim[j - 1 - c0][k]);
+          S[i][k] -= acc.value();
+        }
+      }
+      __syncthreads();
+      if (sdead) break;
+    }
+    if (sdead) break;
+    if (c1 < nb) {
+      Limbs lq[FX_G];
+#pragma unroll
+      for (int q = 0; q < FX_G; ++q) lq[q] = lim[q][i];
+      for (int k = c1 + g; k < nb; k += 4) {
+        if (i < k) continue;
+        Acc acc;
+#pragma unroll
+        for (int q = 0; q < FX_G; ++q) acc.add(lq[q], lim[q][k]);
+        S[i][k] -= acc.value();
+      }
+    }
+    for (int q = g; q < c1 - c0; q += 4) {
+      const Limbs l = lim[q][i];
+      S[i][c0 + q] = ((long long)l.h << 32) + l.l;
     }
     __syncthreads();
   }
-  for (int e = threadIdx.x; e < rows * nb; e += blockDim.x) {
-    int r = e / nb, c = e % nb;
-    A[(int64_t)(r0 + r) * lda + k0 + c] = Xs[r * LD + c] * rinv[c];
+  const bool dead = sdead != 0;  // a pivot failed
+  const double nan = __longlong_as_double(0x7ff8000000000000ULL);
+  __syncthreads();
+  if (logdiag && threadIdx.x < nb)
+    logdiag[k0 + i] = dead ? nan : log(to_double(S[i][i], ex[i]));
+  for (int e = threadIdx.x; e < nb * nb; e += 256) {
+    const int r = e / nb, c = e % nb;
+    A[(int64_t)(k0 + r) * lda + k0 + c] =
+        c > r ? 0.0 : dead ? nan : to_double(S[r][c], ex[r]);
   }
+}
+
+// Panel solve X L^T = A for 32 rows per CTA: lane = row; one warp substitutes
+// a group of eight columns, then the eight warps split the columns to the
+// right.  A row's scale comes from its own
+// diagonal entry, which bounds every entry of the factor's row; a column's
+// from the norm of that row of L.
+constexpr int FX_ROWS = 32;
+constexpr int FX_XLD = FX_NB + 1;
+constexpr size_t FX_TRSM_SMEM = (size_t)FX_NB * FX_NB * sizeof(fx::Limbs) +
+                                (size_t)FX_ROWS * FX_XLD * 8 + (size_t)FX_NB * 16 +
+                                FX_ROWS * 8 + (size_t)FX_G * FX_ROWS * sizeof(fx::Limbs);
+__global__ void __launch_bounds__(256)
+    trsm_rows_fixed_kernel(double* A, int64_t lda, int n, int k0) {
+  using namespace fx;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  Limbs* L = reinterpret_cast<Limbs*>(smem_raw);                   // [64][64], row j of L
+  long long* X = reinterpret_cast<long long*>(L + FX_NB * FX_NB);  // [32][65]
+  long long* ry = X + FX_ROWS * FX_XLD;                            // 1 / L_jj: mantissa
+  int* rs = reinterpret_cast<int*>(ry + FX_NB);                    // and shift
+  int* ej = rs + FX_NB;
+  int* ei = ej + FX_NB;
+  int* sbad = ei + FX_ROWS;
+  Limbs* LX = reinterpret_cast<Limbs*>(sbad + FX_ROWS);            // [8][32], current group
+  const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
+  const int r0 = k0 + FX_NB + blockIdx.x * FX_ROWS, rows = min(FX_ROWS, n - r0);
+  for (int j = g; j < FX_NB; j += 8) {
+    const double* row = A + (int64_t)(k0 + j) * lda + k0;
+    double a[2];
+    int xb[2], xm = 1;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int k = lane + 32 * h;
+      a[h] = k <= j ? row[k] : 0.0;
+      xb[h] = (int)((__double_as_longlong(a[h]) >> 52) & 0x7ff);
+      xm = max(xm, xb[h]);
+    }
+    xm = __reduce_max_sync(0xffffffffu, xm);
+    // squared norm over 2^(2 (xm - 1022)) from the leading bits, rounded up
+    float nsq = 0.f;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const unsigned top = (unsigned)(__double_as_longlong(a[h]) >> 29) & 0x7fffffu;
+      const float f = xm - xb[h] < 100
+                          ? __uint_as_float(((unsigned)(126 - (xm - xb[h])) << 23) | top)
+                          : 0.f;
+      nsq = fmaf(f, f, nsq);
+    }
+    nsq = warp_sum(nsq) * 1.00001f;  // below 64
+    const int x2 = (int)((__float_as_uint(nsq) >> 23) & 0xff) - 126;  // nsq < 2^x2
+    const int e = xm - 1022 + ((x2 + 1) >> 1);
+    bool bad = false;  // a NaN of a failed block: its rows' results are not read
+#pragma unroll
+    for (int h = 0; h < 2; ++h) L[j * FX_NB + lane + 32 * h] = limbs(to_fixed(a[h], e, bad));
+    if (lane == 0) ej[j] = e;
+  }
+  if (threadIdx.x < FX_ROWS) {
+    const int r = r0 + threadIdx.x;
+    ei[threadIdx.x] = threadIdx.x < rows ? scale_of(A[(int64_t)r * lda + r]) : 0;
+    sbad[threadIdx.x] = 0;
+  }
+  __syncthreads();
+  if (threadIdx.x < FX_NB) {
+    const int j = threadIdx.x;
+    const unsigned long long b = (unsigned long long)__double_as_longlong(
+        1.0 / A[(int64_t)(k0 + j) * lda + k0 + j]);
+    ry[j] = (long long)((b & 0xfffffffffffffULL) | (1ULL << 52)) << 9;  // [1, 2) 2^61
+    rs[j] = -((int)((b >> 52) & 0x7ff) - 1023 + ej[j]);
+    if (((b >> 52) & 0x7ff) == 0x7ff || ((b >> 52) & 0x7ff) == 0) {
+      ry[j] = 0;
+      rs[j] = 0;
+    }
+  }
+  for (int e = threadIdx.x; e < FX_ROWS * FX_NB; e += 256) {
+    const int r = e >> 6, c = e & 63;
+    bool bad = false;
+    X[r * FX_XLD + c] =
+        r < rows ? to_fixed(A[(int64_t)(r0 + r) * lda + k0 + c], ei[r] + ej[c], bad) : 0;
+    if (bad) sbad[r] = 1;
+  }
+  __syncthreads();
+  long long* x = X + lane * FX_XLD;
+  for (int c0 = 0; c0 < FX_NB; c0 += FX_G) {
+    if (g == 0) {
+      long long t[FX_G];
+      bool bad = false;
+#pragma unroll
+      for (int q = 0; q < FX_G; ++q) t[q] = x[c0 + q];
+#pragma unroll
+      for (int q = 0; q < FX_G; ++q) {
+        t[q] = times_rsqrt(t[q], ry[c0 + q], rs[c0 + q], bad);
+        const Limbs l = limbs(t[q]);
+        LX[q * FX_ROWS + lane] = l;
+#pragma unroll
+        for (int u = q + 1; u < FX_G; ++u) {
+          Acc acc;
+          acc.add(l, L[(c0 + u) * FX_NB + c0 + q]);
+          t[u] -= acc.value();
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < FX_G; ++q) x[c0 + q] = t[q];
+      if (bad) sbad[lane] = 1;
+    }
+    __syncthreads();
+    if (c0 + FX_G == FX_NB) break;
+    Limbs lx[FX_G];
+#pragma unroll
+    for (int q = 0; q < FX_G; ++q) lx[q] = LX[q * FX_ROWS + lane];
+    for (int k = c0 + FX_G + g; k < FX_NB; k += 8) {
+      Acc acc;
+#pragma unroll
+      for (int q = 0; q < FX_G; ++q) acc.add(lx[q], L[k * FX_NB + c0 + q]);
+      x[k] -= acc.value();
+    }
+    __syncthreads();
+  }
+  const double nan = __longlong_as_double(0x7ff8000000000000ULL);
+  for (int e = threadIdx.x; e < FX_ROWS * FX_NB; e += 256) {
+    const int r = e >> 6, c = e & 63;
+    if (r < rows)
+      A[(int64_t)(r0 + r) * lda + k0 + c] =
+          sbad[r] ? nan : to_double(X[r * FX_XLD + c], ei[r]);
+  }
+}
+
+// Factor the 64 columns at o and the rows below.
+static cudaError_t potrf_block64(double* A, int64_t lda, int n, int o, double* logdiag, int* info,
+                                 cudaStream_t s) {
+  potrf_diag_fixed_kernel<<<1, 256, 0, s>>>(A, lda, n, o, logdiag, info);
+  cudaError_t e = launch_status();
+  const int rest = n - o - FX_NB;
+  if (e != cudaSuccess || rest <= 0) return e;
+  cudaFuncSetAttribute(trsm_rows_fixed_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)FX_TRSM_SMEM);
+  trsm_rows_fixed_kernel<<<(rest + FX_ROWS - 1) / FX_ROWS, 256, FX_TRSM_SMEM, s>>>(A, lda, n, o);
+  return launch_status();
 }
 
 template <typename T>
 cudaError_t potrf_lower(T* A, int64_t lda, int n, double* logdiag, int* info, double* dtrack,
                         bool zero_upper, cudaStream_t s) {
   constexpr int NB = Blk<T>::NB;
-  const size_t smem_diag = (size_t)(NB * (NB + 1) + 3 * NB) * sizeof(T) + 2 * NB * sizeof(double);
   constexpr bool f64 = sizeof(T) == 8;
-  const size_t smem_trsm =
-      (size_t)(NB * (NB + 1) + (f64 ? TRSM_ROWS : 128) * (NB + 1) + NB) * sizeof(T);
-  cudaFuncSetAttribute(potrf_diag_kernel<T, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)smem_diag);
-  if (f64)
-    cudaFuncSetAttribute(trsm_rows_kernel<T, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                         (int)smem_trsm);
-  else
+  const size_t smem_diag = (size_t)(NB * (NB + 1) + 3 * NB) * sizeof(T) + 2 * NB * sizeof(double);
+  const size_t smem_trsm = (size_t)(NB * (NB + 1) + 128 * (NB + 1) + NB) * sizeof(T);
+  if constexpr (!f64) {
+    cudaFuncSetAttribute(potrf_diag_kernel<T, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)smem_diag);
     cudaFuncSetAttribute(trsm_rows_thread_kernel<T, NB>,
                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_trsm);
+  }
   if (zero_upper && n > NB) {
     zero_upper_kernel<T><<<(int)cdiv((int64_t)n * n, 256), 256, 0, s>>>(A, lda, n, NB);
     cudaError_t e0 = launch_status();
     if (e0 != cudaSuccess) return e0;
   }
   for (int k0 = 0; k0 < n; k0 += NB) {
-    const int nb = min(NB, n - k0);
-    potrf_diag_kernel<T, NB><<<1, 512, smem_diag, s>>>(A, lda, n, k0, logdiag, info, dtrack);
-    cudaError_t e = launch_status();
-    if (e != cudaSuccess) return e;
-    const int rest = n - k0 - nb;
-    if (rest <= 0) break;
-    if (f64)
-      trsm_rows_kernel<T, NB><<<(rest + TRSM_ROWS - 1) / TRSM_ROWS, 256, smem_trsm, s>>>(A, lda, n,
-                                                                                       k0);
-    else
-      trsm_rows_thread_kernel<T, NB><<<(rest + 127) / 128, 128, smem_trsm, s>>>(A, lda, n, k0);
-    e = launch_status();
-    if (e != cudaSuccess) return e;
-    if (dtrack) {
-      diag_track_kernel<T><<<(int)cdiv((int64_t)rest * 32, 256), 256, 0, s>>>(A, lda, n, k0 + nb,
-                                                                           k0, nb, dtrack);
+    const int nb = min(NB, n - k0), rest = n - k0 - nb;
+    cudaError_t e;
+    if constexpr (f64) {
+      // its own diagonal supplies the pivots: no float64 track beside it
+      e = potrf_block64(A, lda, n, k0, logdiag, info, s);
+      if (e != cudaSuccess) return e;
+      if (rest <= 0) break;
+    } else {
+      potrf_diag_kernel<T, NB><<<1, 512, smem_diag, s>>>(A, lda, n, k0, logdiag, info, dtrack);
       e = launch_status();
       if (e != cudaSuccess) return e;
+      if (rest <= 0) break;
+      trsm_rows_thread_kernel<T, NB><<<(rest + 127) / 128, 128, smem_trsm, s>>>(A, lda, n, k0);
+      e = launch_status();
+      if (e != cudaSuccess) return e;
+      if (dtrack) {
+        diag_track_kernel<T><<<(int)cdiv((int64_t)rest * 32, 256), 256, 0, s>>>(
+            A, lda, n, k0 + nb, k0, nb, dtrack);
+        e = launch_status();
+        if (e != cudaSuccess) return e;
+      }
     }
     GemmProb<T> p{};
     p.A = A + (int64_t)(k0 + nb) * lda + k0;
@@ -338,6 +542,47 @@ cudaError_t potrf_lower(T* A, int64_t lda, int n, double* logdiag, int* info, do
     if (e != cudaSuccess) return e;
   }
   return cudaSuccess;
+}
+
+// Columns [o, o + w) of the float64 factor, all rows below included: the left
+// half, one product that brings the right half up to date, the right half.
+// The products grow with the recursion (K up to n / 2), which is what their
+// tensor-core form wants; the right-looking order above rewrites the whole
+// trailing matrix once per 64 columns.
+static cudaError_t potrf_rec(double* A, int64_t lda, int n, int o, int w, double* logdiag,
+                             int* info, const XRoom& x, cudaStream_t s) {
+  constexpr int NB = Blk<double>::NB;
+  if (w <= NB) return potrf_block64(A, lda, n, o, logdiag, info, s);
+  int h = NB;
+  while (2 * h < w) h *= 2;
+  cudaError_t e = potrf_rec(A, lda, n, o, h, logdiag, info, x, s);
+  if (e != cudaSuccess) return e;
+  GemmProb<double> p{};
+  p.A = p.B = A + (int64_t)(o + h) * lda + o;
+  p.C = A + (int64_t)(o + h) * lda + o + h;
+  p.lda = p.ldb = p.ldc = lda;
+  p.M = n - o - h;
+  p.N = w - h;
+  p.K = h;
+  p.c_lower = 1;
+  p.alpha = -1.0;
+  p.beta = 1.0;
+  e = gemm_nt_x(p, 1, x, s);
+  if (e != cudaSuccess) return e;
+  return potrf_rec(A, lda, n, o + h, w - h, logdiag, info, x, s);
+}
+
+cudaError_t potrf_lower_x(double* A, int64_t lda, int n, double* logdiag, int* info,
+                          bool zero_upper, const XRoom& x, cudaStream_t s) {
+  // without room for digit planes every product is a CUDA-core one
+  if (!x.bytes) return potrf_lower<double>(A, lda, n, logdiag, info, nullptr, zero_upper, s);
+  constexpr int NB = Blk<double>::NB;
+  if (zero_upper && n > NB) {
+    zero_upper_kernel<double><<<(int)cdiv((int64_t)n * n, 256), 256, 0, s>>>(A, lda, n, NB);
+    cudaError_t e = launch_status();
+    if (e != cudaSuccess) return e;
+  }
+  return potrf_rec(A, lda, n, 0, n, logdiag, info, x, s);
 }
 
 // ---------------------------------------------------------------------------
@@ -391,7 +636,8 @@ __global__ void __launch_bounds__(NB) trtri_diag_kernel(const T* L, int64_t ldl,
 
 template <typename T>
 static cudaError_t trtri_merge(const T* L, int64_t ldl, T* M, int64_t ldm, T* V, int64_t ldv,
-                               T* scratch, int o, int b, int b2, int count, cudaStream_t s) {
+                               T* scratch, int o, int b, int b2, int count, const XRoom& x,
+                               cudaStream_t s) {
   // count pairs starting at offset o, each [b | b2], pair stride 2b.
   const int64_t step = 2 * (int64_t)b;
   GemmProb<T> p{};
@@ -412,7 +658,7 @@ static cudaError_t trtri_merge(const T* L, int64_t ldl, T* M, int64_t ldm, T* V,
   p.K = b;
   p.alpha = T(1);
   p.beta = T(0);
-  cudaError_t e = gemm_nt<T>(p, count, s);
+  cudaError_t e = gemm_nt_room<T>(p, count, x, s);
   if (e != cudaSuccess) return e;
   // M21 = -M22 T ; M21[i,j] = sum_c M22[i,c] TT[j,c]; also V12 = M21^T
   GemmProb<T> q{};
@@ -434,12 +680,12 @@ static cudaError_t trtri_merge(const T* L, int64_t ldl, T* M, int64_t ldm, T* V,
   q.K = b2;
   q.alpha = T(-1);
   q.beta = T(0);
-  return gemm_nt<T>(q, count, s);
+  return gemm_nt_room<T>(q, count, x, s);
 }
 
 template <typename T>
 cudaError_t trtri_lower(const T* L, int64_t ldl, int n, T* M, int64_t ldm, T* V, int64_t ldv,
-                        T* scratch, cudaStream_t s) {
+                        T* scratch, const XRoom& x, cudaStream_t s) {
   constexpr int NB = Blk<T>::NB;
   const size_t smem = (size_t)(2 * NB * (NB + 1) + NB) * sizeof(T);
   cudaFuncSetAttribute(trtri_diag_kernel<T, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -455,13 +701,14 @@ cudaError_t trtri_lower(const T* L, int64_t ldl, int n, T* M, int64_t ldm, T* V,
     for (int q = 0; q < npairs; ++q)
       if ((int64_t)q * 2 * b + 2 * b <= n) ++full;
     if (full > 0) {
-      e = trtri_merge<T>(L, ldl, M, ldm, V, ldv, scratch, 0, b, b, full, s);
+      e = trtri_merge<T>(L, ldl, M, ldm, V, ldv, scratch, 0, b, b, full, x, s);
       if (e != cudaSuccess) return e;
     }
     if (full < npairs) {
       const int o = full * 2 * b;
       const int b2 = n - o - b;
-      e = trtri_merge<T>(L, ldl, M, ldm, V, ldv, scratch + (int64_t)full * b * b, o, b, b2, 1, s);
+      e = trtri_merge<T>(L, ldl, M, ldm, V, ldv, scratch + (int64_t)full * b * b, o, b, b2, 1, x,
+                         s);
       if (e != cudaSuccess) return e;
     }
   }
@@ -524,7 +771,7 @@ cudaError_t gemv_dense(const T* A, int64_t ld, int rows, int cols, const double*
   template cudaError_t potrf_lower<T>(T*, int64_t, int, double*, int*, double*, bool,          \
                                       cudaStream_t);                                            \
   template cudaError_t trtri_lower<T>(const T*, int64_t, int, T*, int64_t, T*, int64_t, T*,     \
-                                      cudaStream_t);                                            \
+                                      const XRoom&, cudaStream_t);                                            \
   template cudaError_t gemv_tri<T>(const T*, int64_t, int, bool, const double*, double*, double, \
                                    bool, cudaStream_t);                                         \
   template cudaError_t gemv_dense<T>(const T*, int64_t, int, int, const double*, double*,      \

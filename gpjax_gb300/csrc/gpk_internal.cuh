@@ -35,19 +35,31 @@ cudaError_t gemm_nt(const GemmProb<T>& p, int batch, cudaStream_t s);
 
 // Lower Cholesky in place (row-major, lda).  logdiag[n] (may be null)
 // receives log(L_ii) in float64; info gets the first failing order.
-// dtrack (may be null): float64 copy of diag(A) that is kept up to date
-// through the factorisation and supplies the pivots, so the diagonal never
-// accumulates rounding of the working precision.  zero_upper clears the
+// dtrack (may be null; float32 only): float64 copy of diag(A) that is kept up
+// to date through the factorisation and supplies the pivots, so the diagonal
+// never accumulates rounding of the working precision.  zero_upper clears the
 // strict upper triangle outside the diagonal blocks first.
 template <typename T>
 cudaError_t potrf_lower(T* A, int64_t lda, int n, double* logdiag, int* info, double* dtrack,
                         bool zero_upper, cudaStream_t s);
 
+// Workspace for the digit planes of float64 products on the tensor cores
+// (xgemm.cuh); bytes = 0: none, every float64 product runs on the CUDA cores.
+struct XRoom {
+  void* mem = nullptr;
+  size_t bytes = 0;
+};
+
+// The float64 factor with products on the tensor cores where x has room
+// (potrf_lower<double> otherwise).
+cudaError_t potrf_lower_x(double* A, int64_t lda, int n, double* logdiag, int* info,
+                          bool zero_upper, const XRoom& x, cudaStream_t s);
+
 // M = L^-1 (lower, row-major) and V = L^-T (upper, row-major) from the factor L.
 // scratch: n*n/2 elements of T.
 template <typename T>
 cudaError_t trtri_lower(const T* L, int64_t ldl, int n, T* M, int64_t ldm, T* V, int64_t ldv,
-                        T* scratch, cudaStream_t s);
+                        T* scratch, const XRoom& x, cudaStream_t s);
 
 // y = op(Tri) x in float64 accumulation, Tri [n, n] row-major;
 // lower: y_i = sum_{c<=i} Tri[i,c] x_c ; upper: y_i = sum_{c>=i} Tri[i,c] x_c.
@@ -85,6 +97,12 @@ cudaError_t lauum_grad(int kind, const T* V, int64_t ldv, int n, int d, const T*
                        cudaStream_t s);
 template <typename T>
 int lauum_grad_tiles(int n);
+
+// The same sums from V through W = V V^T stored in `W` (n x ldw, lower tiles),
+// formed on the tensor cores with x's room.
+cudaError_t lauum_grad_x(int kind, const double* V, int64_t ldv, int n, int d, const double* xs,
+                         const double* theta, int n_ls, const double* alpha, double* gpart,
+                         double* W, int64_t ldw, const XRoom& x, cudaStream_t s);
 
 // r = diff - (K(xs, xs) + (jitter + obs_stddev^2) I) alpha, K regenerated in T,
 // float64 accumulation; rpart holds residual_scratch_doubles(n) doubles.

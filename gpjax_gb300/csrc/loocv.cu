@@ -14,8 +14,10 @@
 // noise gradient 2 obs_stddev tr(G).  Everything is float64: Sigma's Cholesky
 // factor, its triangular inverse, W = L^-T L^-1 and W diag(a) W as SIMT GEMMs,
 // alpha refined once against a float64 residual.
+#include <algorithm>
 #include <climits>
 #include "gpk_internal.cuh"
+#include "xgemm.cuh"
 
 extern "C" size_t gpk_cross_covariance_vjp_workspace_bytes(int64_t n, int64_t m, int d);
 extern "C" gpk_status gpk_cross_covariance_vjp(int kind, int64_t n, int64_t m, int d,
@@ -34,6 +36,7 @@ struct LoocvBuffers {
   double *diff, *z, *alpha, *r, *logdiag, *dtrack, *rpart, *a, *sa, *b, *u, *red, *gth;
   void* vjp_ws;
   size_t vjp_bytes;
+  XRoom x;  // digit planes
 };
 
 size_t loocv_layout(int64_t n, int d, void* ws, LoocvBuffers& b) {
@@ -60,6 +63,8 @@ size_t loocv_layout(int64_t n, int d, void* ws, LoocvBuffers& b) {
   b.gth = (double*)take((size_t)(GPK_MAX_D + 8) * 8);
   b.vjp_bytes = gpk_cross_covariance_vjp_workspace_bytes(n, n, d);
   b.vjp_ws = take(b.vjp_bytes);
+  b.x.bytes = xroom_fit(off, n <= 512 ? 0 : std::max(xroom_factor_bytes(n), xsplit_bytes(n, n)));
+  b.x.mem = take(b.x.bytes);
   return off + 256;
 }
 
@@ -185,8 +190,8 @@ extern "C" gpk_status gpk_conjugate_loocv(int kind, int64_t n, int d, const doub
   GPK_CUDA_TRY(cross_cov_scaled<double, double>(kind, nn, nn, d, b.xs, b.xs, theta, n_ls, 1,
                                                 jitter, b.A, ld, s));
   GPK_CUDA_TRY(sigma_diag_init(kind, nn, theta, n_ls, jitter, b.dtrack, s));
-  GPK_CUDA_TRY(potrf_lower<double>(b.A, ld, nn, b.logdiag, info, b.dtrack, false, s));
-  GPK_CUDA_TRY(trtri_lower<double>(b.A, ld, nn, b.M, ld, b.V, ld, b.scratch, s));
+  GPK_CUDA_TRY(potrf_lower_x(b.A, ld, nn, b.logdiag, info, false, b.x, s));
+  GPK_CUDA_TRY(trtri_lower<double>(b.A, ld, nn, b.M, ld, b.V, ld, b.scratch, b.x, s));
   // alpha = Sigma^-1 (y - m) (objectives.py:167), refined once
   GPK_CUDA_TRY(gemv_tri<double>(b.M, ld, nn, true, b.diff, b.z, 1.0, false, s));
   GPK_CUDA_TRY(gemv_tri<double>(b.V, ld, nn, false, b.z, b.alpha, 1.0, false, s));
@@ -205,7 +210,7 @@ extern "C" gpk_status gpk_conjugate_loocv(int kind, int64_t n, int d, const doub
     p.a_tri = p.b_tri = TRI_UPPER;
     p.alpha = 1.0;
     p.beta = 0.0;
-    GPK_CUDA_TRY(gemm_nt<double>(p, 1, s));
+    GPK_CUDA_TRY(gemm_nt_x(p, 1, b.x, s));
   }
   loocv_point_kernel<<<g1, 256, 0, s>>>(nn, b.W, ld, b.alpha, b.a, b.sa, b.b, b.red);
   GPK_LAUNCH_CHECK();
@@ -222,7 +227,7 @@ extern "C" gpk_status gpk_conjugate_loocv(int kind, int64_t n, int d, const doub
     p.c_lower = 1;
     p.alpha = 1.0;
     p.beta = 0.0;
-    GPK_CUDA_TRY(gemm_nt<double>(p, 1, s));
+    GPK_CUDA_TRY(gemm_nt_x(p, 1, b.x, s));
     loocv_cotangent_kernel<<<g2, 256, 0, s>>>(nn, b.A, ld, b.u, b.alpha, b.red);
     GPK_LAUNCH_CHECK();
     loocv_mirror_kernel<<<g2, 256, 0, s>>>(nn, b.A, ld);

@@ -18,6 +18,7 @@
 #include <mutex>
 #include <vector>
 #include "gpk_internal.cuh"
+#include "xgemm.cuh"
 
 namespace gpk {
 
@@ -61,6 +62,7 @@ struct MllBuffers {
   int64_t ld;
   T *A, *M, *V, *scratch, *xs;
   double *diff, *z, *alpha, *r, *logdiag, *rpart, *gpart, *dtrack, *fin;
+  XRoom x;  // float64: digit planes, right after scratch (both hold W in the adjoint)
 };
 
 template <typename T>
@@ -72,6 +74,8 @@ static size_t mll_layout(int64_t n, int d, void* ws, MllBuffers<T>& b) {
   b.M = a.take<T>(nn);
   b.V = a.take<T>(nn);
   b.scratch = a.take<T>((size_t)n * n / 2 + 64);
+  b.x.bytes = sizeof(T) == 8 ? xroom_fit(nn * sizeof(T) * 4, xroom_factor_bytes(n)) : 0;
+  b.x.mem = a.take<char>(b.x.bytes);
   b.xs = a.take<T>((size_t)n * d);
   b.diff = a.take<double>(n);
   b.z = a.take<double>(n);
@@ -236,9 +240,12 @@ static gpk_status mll_run(int kind, int n, int d, const double* x, int64_t ldx, 
                                       b.ld, s));
   GPK_CUDA_TRY(sigma_diag_init(kind, n, theta, n_ls, jitter, b.dtrack, s));
   prof_mark(1, s);
-  GPK_CUDA_TRY(potrf_lower<T>(b.A, b.ld, n, b.logdiag, info, b.dtrack, false, s));
+  if constexpr (sizeof(T) == 8)
+    GPK_CUDA_TRY(potrf_lower_x(b.A, b.ld, n, b.logdiag, info, false, b.x, s));
+  else
+    GPK_CUDA_TRY(potrf_lower<T>(b.A, b.ld, n, b.logdiag, info, b.dtrack, false, s));
   prof_mark(2, s);
-  GPK_CUDA_TRY(trtri_lower<T>(b.A, b.ld, n, b.M, b.ld, b.V, b.ld, b.scratch, s));
+  GPK_CUDA_TRY(trtri_lower<T>(b.A, b.ld, n, b.M, b.ld, b.V, b.ld, b.scratch, b.x, s));
   prof_mark(3, s);
   GPK_CUDA_TRY(gemv_tri<T>(b.M, b.ld, n, true, b.diff, b.z, 1.0, false, s));
   GPK_CUDA_TRY(gemv_tri<T>(b.V, b.ld, n, false, b.z, b.alpha, 1.0, false, s));
@@ -249,7 +256,15 @@ static gpk_status mll_run(int kind, int n, int d, const double* x, int64_t ldx, 
     GPK_CUDA_TRY(gemv_tri<T>(b.V, b.ld, n, false, b.z, b.alpha, 1.0, true, s));
   }
   prof_mark(4, s);
-  if (want_grad)
+  if (want_grad && b.x.bytes) {
+    // the factor and M are done with: their arrays (adjacent) take V's digit
+    // planes, scratch and the room after it W
+    if constexpr (sizeof(T) == 8) {
+      const XRoom planes{b.A, (size_t)(reinterpret_cast<char*>(b.V) - reinterpret_cast<char*>(b.A))};
+      GPK_CUDA_TRY(lauum_grad_x(kind, b.V, b.ld, n, d, b.xs, theta, n_ls, b.alpha, b.gpart,
+                                b.scratch, b.ld, planes, s));
+    }
+  } else if (want_grad)
     GPK_CUDA_TRY(lauum_grad<T>(kind, b.V, b.ld, n, d, b.xs, theta, n_ls, b.alpha, b.gpart, s));
   prof_mark(5, s);
   GPK_CUDA_TRY(mll_finalize_launch(n, d, theta, n_ls, b.logdiag, b.diff, b.alpha, b.gpart,
@@ -480,7 +495,7 @@ __global__ void transpose_kernel(int rows, int cols, const T* __restrict__ src, 
 
 template <typename T>
 static size_t solve_layout(int64_t n, int64_t nrhs, bool upper, void* ws, T** M, T** V, T** scr,
-                           T** BT, T** LT, int64_t* ld) {
+                           T** BT, T** LT, int64_t* ld, XRoom* x) {
   Arena a(ws);
   *ld = pad_ld(n);
   *M = a.take<T>((size_t)n * *ld);
@@ -488,17 +503,22 @@ static size_t solve_layout(int64_t n, int64_t nrhs, bool upper, void* ws, T** M,
   *scr = a.take<T>((size_t)n * n / 2 + 64);
   *BT = a.take<T>((size_t)nrhs * *ld);
   *LT = upper ? a.take<T>((size_t)n * *ld) : nullptr;  // lower copy U^T of an upper input
+  if (sizeof(T) == 8)  // digit planes: the inverse's products; then B^T beside it
+    x->bytes = xroom_fit(a.off, n <= 512 ? 0 : std::max(xroom_factor_bytes(n),
+                                                       xsplit_bytes(nrhs, n) + xsplit_bytes(n, n)));
+  x->mem = a.take<char>(x->bytes);
   return a.off + 256;
 }
 
 static size_t solve_ws(int64_t n, int64_t nrhs, int dtype, bool upper) {
   int64_t ld;
+  XRoom x;
   if (dtype == GPK_F64) {
     double *M, *V, *S, *B, *LT;
-    return solve_layout<double>(n, nrhs, upper, nullptr, &M, &V, &S, &B, &LT, &ld);
+    return solve_layout<double>(n, nrhs, upper, nullptr, &M, &V, &S, &B, &LT, &ld, &x);
   }
   float *M, *V, *S, *B, *LT;
-  return solve_layout<float>(n, nrhs, upper, nullptr, &M, &V, &S, &B, &LT, &ld);
+  return solve_layout<float>(n, nrhs, upper, nullptr, &M, &V, &S, &B, &LT, &ld, &x);
 }
 
 extern "C" size_t gpk_solve_triangular_workspace_bytes(int64_t n, int64_t nrhs, int dtype) {
@@ -519,7 +539,8 @@ static gpk_status solve_run(int n, int nrhs, const T* L, int64_t lda, bool upper
                             T* B, int64_t ldb, void* ws, cudaStream_t s) {
   T *M, *V, *scr, *BT, *LT;
   int64_t ld;
-  solve_layout<T>(n, nrhs, upper, ws, &M, &V, &scr, &BT, &LT, &ld);
+  XRoom x;
+  solve_layout<T>(n, nrhs, upper, ws, &M, &V, &scr, &BT, &LT, &ld, &x);
   dim3 tb(32, 8);
   if (upper) {
     transpose_kernel<T><<<dim3((unsigned)cdiv(n, 32), (unsigned)cdiv(n, 32)), tb, 0, s>>>(
@@ -528,7 +549,7 @@ static gpk_status solve_run(int n, int nrhs, const T* L, int64_t lda, bool upper
     L = LT;
     lda = ld;
   }
-  GPK_CUDA_TRY(trtri_lower<T>(L, lda, n, M, ld, V, ld, scr, s));
+  GPK_CUDA_TRY(trtri_lower<T>(L, lda, n, M, ld, V, ld, scr, x, s));
   // lower: T^-1 = M, T^-T = V ; upper (T = L^T): T^-1 = V, T^-T = M
   const bool use_v = upper != trans;
   transpose_kernel<T><<<dim3((unsigned)cdiv(nrhs, 32), (unsigned)cdiv(n, 32)), tb, 0, s>>>(
@@ -548,7 +569,7 @@ static gpk_status solve_run(int n, int nrhs, const T* L, int64_t lda, bool upper
   p.ldct = ldb;
   p.alpha = T(1);
   p.beta = T(0);
-  GPK_CUDA_TRY(gemm_nt<T>(p, 1, s));
+  GPK_CUDA_TRY(gemm_nt_room<T>(p, 1, x, s));
   return GPK_OK;
 }
 
@@ -588,12 +609,15 @@ extern "C" gpk_status gpk_solve_triangular_ex(int64_t n, int64_t nrhs, int dtype
 // workspace first.
 // ---------------------------------------------------------------------------
 static size_t gemm64_layout(int64_t M, int64_t N, int64_t K, int transa, int transb, void* ws,
-                            double** At, double** Bt, int64_t* lda_t, int64_t* ldb_t) {
+                            double** At, double** Bt, int64_t* lda_t, int64_t* ldb_t,
+                            char** xs, size_t* xs_bytes) {
   Arena a(ws);
   *lda_t = pad_ld(K);
   *ldb_t = pad_ld(K);
   *At = transa ? a.take<double>((size_t)M * *lda_t) : nullptr;  // op(A) = A^T: A^T copy [M, K]
   *Bt = transb ? nullptr : a.take<double>((size_t)N * *ldb_t);  // op(B) = B: B^T copy [N, K]
+  *xs_bytes = xsplit_bytes(M, K) + xsplit_bytes(N, K);  // digit planes of the split form
+  *xs = a.take<char>(*xs_bytes);
   return a.off + 256;
 }
 
@@ -601,7 +625,9 @@ extern "C" size_t gpk_gemm_f64_workspace_bytes(int transa, int transb, int64_t M
                                                int64_t K) {
   double *a, *b;
   int64_t la, lb;
-  return gemm64_layout(M, N, K, transa, transb, nullptr, &a, &b, &la, &lb);
+  char* xs;
+  size_t nx;
+  return gemm64_layout(M, N, K, transa, transb, nullptr, &a, &b, &la, &lb, &xs, &nx);
 }
 
 extern "C" gpk_status gpk_gemm_f64(int transa, int transb, int64_t M, int64_t N, int64_t K,
@@ -617,7 +643,9 @@ extern "C" gpk_status gpk_gemm_f64(int transa, int transb, int64_t M, int64_t N,
     return GPK_ERR_WORKSPACE;
   double *At, *Bt;
   int64_t la, lb;
-  gemm64_layout(M, N, K, transa, transb, workspace, &At, &Bt, &la, &lb);
+  char* xs;
+  size_t nx;
+  gemm64_layout(M, N, K, transa, transb, workspace, &At, &Bt, &la, &lb, &xs, &nx);
   dim3 tb(32, 8);
   const double* An = A;
   int64_t ldan = lda;
@@ -649,7 +677,7 @@ extern "C" gpk_status gpk_gemm_f64(int transa, int transb, int64_t M, int64_t N,
   p.K = (int)K;
   p.alpha = alpha;
   p.beta = beta;
-  GPK_CUDA_TRY(gemm_nt<double>(p, 1, s));
+  GPK_CUDA_TRY(gemm_nt_x(p, 1, XRoom{xs, nx}, s));
   return GPK_OK;
 }
 

@@ -9,6 +9,7 @@
 #include <algorithm>
 #include <climits>
 #include "gpk_internal.cuh"
+#include "xgemm.cuh"
 
 namespace gpk {
 
@@ -42,6 +43,7 @@ struct PredBuffers {
   int64_t ld, ldt;
   T *A, *M, *V, *scratch, *xs, *ts, *Ktx, *QT, *QQ;
   double *tsd, *diff, *z, *alpha, *r, *rpart, *logdiag, *dtrack;
+  XRoom x;  // float64: digit planes
 };
 
 template <typename T>
@@ -66,6 +68,14 @@ size_t pred_layout(int64_t n, int64_t t, int d, bool want_cov, void* ws, PredBuf
   b.logdiag = a.take<double>(n);
   b.dtrack = a.take<double>(n);
   b.rpart = a.take<double>(residual_scratch_doubles((int)n));
+  if (sizeof(T) == 8) {
+    // the factor's products; then Ktx beside M, and Q^T alone
+    const size_t want = n <= 512 && t <= 512 ? 0
+                                             : std::max(xroom_factor_bytes(n),
+                                                        xsplit_bytes(t, n) + xsplit_bytes(n, n));
+    b.x.bytes = xroom_fit(a.off, want);
+  }
+  b.x.mem = a.take<char>(b.x.bytes);
   return a.off + 256;
 }
 
@@ -153,8 +163,11 @@ gpk_status predict_run(int kind, int n, int t, int d, const double* x, int64_t l
   GPK_CUDA_TRY(cross_cov_scaled<T, T>(kind, n, n, d, b.xs, b.xs, theta, n_ls, 1, jitter, b.A,
                                       b.ld, s));
   GPK_CUDA_TRY(sigma_diag_init(kind, n, theta, n_ls, jitter, b.dtrack, s));
-  GPK_CUDA_TRY(potrf_lower<T>(b.A, b.ld, n, b.logdiag, info, b.dtrack, false, s));
-  GPK_CUDA_TRY(trtri_lower<T>(b.A, b.ld, n, b.M, b.ld, b.V, b.ld, b.scratch, s));
+  if constexpr (sizeof(T) == 8)
+    GPK_CUDA_TRY(potrf_lower_x(b.A, b.ld, n, b.logdiag, info, false, b.x, s));
+  else
+    GPK_CUDA_TRY(potrf_lower<T>(b.A, b.ld, n, b.logdiag, info, b.dtrack, false, s));
+  GPK_CUDA_TRY(trtri_lower<T>(b.A, b.ld, n, b.M, b.ld, b.V, b.ld, b.scratch, b.x, s));
   GPK_CUDA_TRY(gemv_tri<T>(b.M, b.ld, n, true, b.diff, b.z, 1.0, false, s));
   GPK_CUDA_TRY(gemv_tri<T>(b.V, b.ld, n, false, b.z, b.alpha, 1.0, false, s));
   for (int it = 0; it < refine; ++it) {
@@ -178,7 +191,7 @@ gpk_status predict_run(int kind, int n, int t, int d, const double* x, int64_t l
   p.ldc = b.ld;
   p.alpha = T(1);
   p.beta = T(0);
-  GPK_CUDA_TRY(gemm_nt<T>(p, 1, s));
+  GPK_CUDA_TRY(gemm_nt_room<T>(p, 1, b.x, s));
   pred_mean_var_kernel<T><<<(int)cdiv((int64_t)t * 32, 256), 256, 0, s>>>(
       n, t, b.Ktx, b.QT, b.ld, b.alpha, theta, n_ls, kind, prior_jitter, info, mean, var);
   GPK_LAUNCH_CHECK();
@@ -196,7 +209,7 @@ gpk_status predict_run(int kind, int n, int t, int d, const double* x, int64_t l
     q.ldc = b.ldt;
     q.alpha = T(1);
     q.beta = T(0);
-    GPK_CUDA_TRY(gemm_nt<T>(q, 1, s));
+    GPK_CUDA_TRY(gemm_nt_room<T>(q, 1, b.x, s));
     pred_cov_kernel<T><<<(int)cdiv((int64_t)t * t, 256), 256, 0, s>>>(
         t, d, kind, b.tsd, b.QQ, b.ldt, theta, n_ls, prior_jitter, info, cov, ldcov);
     GPK_LAUNCH_CHECK();

@@ -22,11 +22,13 @@
 // the GEMM epilogue; c = Phi d and Phi 1 are summed in float-float during
 // generation.  The m x m algebra always runs in float64.  Reductions go
 // through per-block partials summed in a fixed order.
+#include <algorithm>
 #include <climits>
 #include <mutex>
 #include <type_traits>
 #include "gpk_internal.cuh"
 #include "tc_gemm.cuh"
+#include "xgemm.cuh"
 
 namespace gpk {
 namespace {
@@ -45,8 +47,9 @@ struct Arena {
 };
 
 constexpr int KCHUNK = 8192;    // P = sum over n-chunks of Phi_k Phi_k^T (float64 sum of chunks)
-constexpr int AB = 64;          // fused adjoint tile
-constexpr int ASPLIT = 64;      // column (n) split of the fused adjoint
+constexpr int AB = 64;          // plain adjoint: inducing points per block
+constexpr int ASPLIT = 64;      // and splits of the data points
+constexpr int ABLK = 65536;     // data points whose Phi^T and G^T are held at a time
 constexpr int DMAXS = 16;       // input dimension limit of the SGPR path
 
 inline int64_t pad64(int64_t n) { return ((n + 63) / 64) * 64; }
@@ -66,17 +69,29 @@ inline tc::TcParams sg_adj_params(int64_t n, int64_t m, int d) {
   return q;
 }
 
+// Plain form: columns per partial of P.  Short enough that the lower 128 x 64
+// tiles of all partials fill the chip twice, within [1024, KCHUNK].
+inline int plain_kchunk(int64_t n, int64_t m) {
+  const int64_t tm = (m + 127) / 128, tiles = tm * (tm + 1);
+  const int64_t parts = (2 * 152 + tiles - 1) / tiles;
+  const int64_t k = ((n + parts - 1) / parts + 63) / 64 * 64;
+  return (int)std::min<int64_t>(KCHUNK, std::max<int64_t>(1024, k));
+}
+
 template <typename T>
 struct SgprBuf {
   static constexpr bool kMixed = std::is_same<T, float>::value;
   int64_t ldn, ldm;
   int nchunks, nb, nxb, gtiles, gcols;
+  int kchunk, pgroup;                             // columns per P partial; partials per product
   T *zs, *xs, *Phi, *Pparts, *Ht;                 // Phi, Ht: plain form only
+  T *PhiT, *GT;                                   // plain form: ABLK rows of Phi^T and G^T
   float *Phh, *Phl, *PTh, *PTl, *Hh, *Hl;         // mixed form only
   double *zs64, *Kf, *Lz, *Mz, *Vz, *Kinv, *Su, *Mu, *Vu, *Suinv, *P64, *T1, *KPK, *GK, *scr;
   double *dv, *cv, *phi1, *gam, *gams, *pgam, *ldK, *ldU, *red, *thK, *dzK, *thP, *dzP;
   double *ddpart, *cpart, *colpart, *sth, *gzs, *ddds;
   int* err;
+  XRoom xk, xu;  // digit planes of the Kzz chain (side stream) and of the rest
 };
 
 template <typename T>
@@ -85,7 +100,8 @@ size_t sgpr_layout(int64_t n, int64_t m, int d, void* ws, SgprBuf<T>& b) {
   Arena a(ws);
   b.ldn = pad64(n);
   b.ldm = pad64(m);
-  b.nchunks = (int)((n + KCHUNK - 1) / KCHUNK);
+  b.kchunk = mixed ? KCHUNK : plain_kchunk(n, m);
+  b.nchunks = (int)((n + b.kchunk - 1) / b.kchunk);
   b.nb = (int)((n + 255) / 256);
   // Phi generation blocks: the chunk-blocked P operand is written (zeros past
   // n) up to nchunks * KCHUNK columns
@@ -100,6 +116,9 @@ size_t sgpr_layout(int64_t n, int64_t m, int d, void* ws, SgprBuf<T>& b) {
   b.Phi = mixed ? nullptr : a.take<T>((size_t)m * b.ldn);
   b.Pparts = a.take<T>((size_t)b.nchunks * m * m);
   b.Ht = mixed ? nullptr : a.take<T>(mm);
+  const int64_t ablk = std::min<int64_t>(n, ABLK);
+  b.PhiT = mixed ? nullptr : a.take<T>((size_t)ablk * b.ldm);
+  b.GT = mixed ? nullptr : a.take<T>((size_t)ablk * b.ldm);
   b.Phh = b.Phl = b.PTh = b.PTl = b.Hh = b.Hl = nullptr;
   if (mixed) {
     // chunk-blocked: Phh[c][i][k] = hi(Phi[i][c * KCHUNK + k]), so that one
@@ -155,6 +174,19 @@ size_t sgpr_layout(int64_t n, int64_t m, int d, void* ws, SgprBuf<T>& b) {
   b.gzs = a.take<double>((size_t)m * d);
   b.ddds = a.take<double>(2);
   b.err = a.take<int>(1);
+  const size_t small = m <= 512 ? 0 : std::max(xroom_factor_bytes(m), 2 * xsplit_bytes(m, m));
+  size_t want = small;
+  if (!mixed) {
+    // P's partials go through the room in groups of at most 2 GB of digits
+    const int64_t per = (int64_t)xsplit_bytes(m, b.kchunk);
+    b.pgroup = (int)std::max<int64_t>(1, std::min<int64_t>(b.nchunks, ((int64_t)2 << 30) / per));
+    want = std::max({want, xsplit_bytes(b.pgroup * m, b.kchunk),
+                     xsplit_bytes(ablk, m) + xsplit_bytes(m, m)});
+  }
+  b.xk.bytes = xroom_fit(a.off, small);
+  b.xk.mem = a.take<char>(b.xk.bytes);
+  b.xu.bytes = xroom_fit(a.off, want);
+  b.xu.mem = a.take<char>(b.xu.bytes);
   return a.off + 256;
 }
 
@@ -489,150 +521,79 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// Fused Phi adjoint: for row tile I (AB rows of Z) and column tiles j = s, s+S, ...
-//   G = H Phi + gamma d^T / s^2   (tile by tile, never stored)
+// Plain form's Phi adjoint over one block of data points:
+//   G^T + d gamma^T / s^2  (rows: data points, columns: inducing points)
 // reduced against dPhi/dtheta and dPhi/dZ regenerated from the scaled inputs.
-template <typename T>
+// Block (I, split): AB inducing points (one per lane pair of warps, rows read
+// coalesced) and every ASPLIT-th group of four data points; the four row
+// phases of a block are summed in a fixed order, and later blocks of data
+// points add to the first's partials.
+template <int D>
 __global__ void __launch_bounds__(256)
-    sg_phi_adjoint(int kind, int m, int n, int d, const T* __restrict__ Ht, int64_t ldm,
-                   const T* __restrict__ Phi, int64_t ldn, const T* __restrict__ zs,
-                   const T* __restrict__ xs, const double* __restrict__ gam,
-                   const double* __restrict__ dv, const double* __restrict__ theta, int n_ls,
-                   double* __restrict__ thP, double* __restrict__ dzP) {
-  constexpr int BKc = 16;
-  extern __shared__ __align__(16) unsigned char sg_smem[];
-  typedef T Row64[AB + 1];
-  typedef T RowD[DMAXS + 1];
-  typedef double RowDd[DMAXS + 1];
-  Row64* As = reinterpret_cast<Row64*>(sg_smem);     // [BKc]
-  Row64* Bs = As + BKc;                              // [BKc]
-  Row64* Gs = Bs + BKc;                              // [AB]
-  RowD* szi = reinterpret_cast<RowD*>(Gs + AB);      // [AB]
-  RowD* sxj = szi + AB;                              // [AB]
-  RowDd* sdz = reinterpret_cast<RowDd*>(
-      (reinterpret_cast<uintptr_t>(sxj + AB) + 15) & ~static_cast<uintptr_t>(15));  // [AB]
-  RowDd* sred = sdz + AB;                            // [8]
-  const int I = blockIdx.x, split = blockIdx.y;
-  const int i0 = I * AB;
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const double sd = theta[n_ls + 1], s = sd * sd;
-  for (int e = threadIdx.x; e < AB * DMAXS; e += 256) {
-    const int r = e / DMAXS, k = e % DMAXS;
-    szi[r][k] = (i0 + r < m && k < d) ? zs[(int64_t)(i0 + r) * d + k] : T(0);
-    sdz[r][k] = 0.0;
+    sg_phi_reduce(int kind, int m, int rows, int d, const double* __restrict__ GT,
+                  const double* __restrict__ PhiT, int64_t ldm, const double* __restrict__ zs,
+                  const double* __restrict__ xs, const double* __restrict__ gams,
+                  const double* __restrict__ dv, const double* __restrict__ theta, int n_ls,
+                  int first, double* __restrict__ thP, double* __restrict__ dzP) {
+  __shared__ double red[4][AB][D + 1];
+  const int il = threadIdx.x & (AB - 1), ph = threadIdx.x >> 6;
+  const int i = blockIdx.x * AB + il, split = blockIdx.y;
+  const double inv = 1.0 / theta[n_ls], ka = kshape<double>(kind, theta, n_ls);
+  double zi[D], al[D], az[D], av = 0.0;
+#pragma unroll
+  for (int k = 0; k < D; ++k) {
+    zi[k] = i < m && k < d ? zs[(int64_t)i * d + k] : 0.0;
+    al[k] = az[k] = 0.0;
   }
-  double al[DMAXS], av = 0.0;
+  const double gi = i < m ? gams[i] : 0.0;
+  if (i < m) {
+    for (int j = 4 * split + ph; j < rows; j += 4 * ASPLIT) {
+      const double g = fma(gi, dv[j], GT[(int64_t)j * ldm + i]);
+      double dz[D], sq = 0.0;
 #pragma unroll
-  for (int k = 0; k < DMAXS; ++k) al[k] = 0.0;
-  const int ntile = (n + AB - 1) / AB;
-  // element ownership in the reduction: 4 threads per row, 16 columns each
-  const int er = threadIdx.x >> 2, ec = (threadIdx.x & 3) * 16;
-  for (int J = split; J < ntile; J += ASPLIT) {
-    const int j0 = J * AB;
-    T acc[4][4];
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-      for (int b = 0; b < 4; ++b) acc[a][b] = T(0);
-    for (int c0 = 0; c0 < m; c0 += BKc) {
-      __syncthreads();
-      for (int e = threadIdx.x; e < AB * BKc; e += 256) {
-        const int r = e / BKc, kk = e % BKc;
-        As[kk][r] = (i0 + r < m && c0 + kk < m) ? Ht[(int64_t)(i0 + r) * ldm + c0 + kk] : T(0);
+      for (int k = 0; k < D; ++k) {
+        dz[k] = k < d ? zi[k] - xs[(int64_t)j * d + k] : 0.0;
+        sq = fma(dz[k], dz[k], sq);
       }
-      for (int e = threadIdx.x; e < AB * BKc; e += 256) {
-        const int kk = e / AB, cc = e % AB;
-        Bs[kk][cc] = (c0 + kk < m && j0 + cc < n) ? Phi[(int64_t)(c0 + kk) * ldn + j0 + cc] : T(0);
+      double k1, c1;
+      if (kind == GPK_RBF)
+        k1 = c1 = PhiT[(int64_t)j * ldm + i] * inv;  // the value is its own coefficient
+      else
+        kval_dcoef<double>(kind, sq, 1.0, k1, c1, ka);
+      av = fma(g, k1, av);
+      const double gc = g * c1;
+#pragma unroll
+      for (int k = 0; k < D; ++k) {
+        const double t = gc * dz[k];
+        az[k] += t;
+        al[k] = fma(t, dz[k], al[k]);
       }
-      __syncthreads();
-#pragma unroll
-      for (int kk = 0; kk < BKc; ++kk) {
-        T av4[4], bv4[4];
-#pragma unroll
-        for (int a = 0; a < 4; ++a) av4[a] = As[kk][ty + 16 * a];
-#pragma unroll
-        for (int b = 0; b < 4; ++b) bv4[b] = Bs[kk][tx + 16 * b];
-#pragma unroll
-        for (int a = 0; a < 4; ++a)
-#pragma unroll
-          for (int b = 0; b < 4; ++b) acc[a][b] = fma(av4[a], bv4[b], acc[a][b]);
-      }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int a = 0; a < 4; ++a)
-#pragma unroll
-      for (int b = 0; b < 4; ++b) Gs[ty + 16 * a][tx + 16 * b] = acc[a][b];
-    for (int e = threadIdx.x; e < AB * DMAXS; e += 256) {
-      const int r = e / DMAXS, k = e % DMAXS;
-      sxj[r][k] = (j0 + r < n && k < d) ? xs[(int64_t)(j0 + r) * d + k] : T(0);
-    }
-    __syncthreads();
-    const int gi = i0 + er;
-    double zacc[DMAXS];
-#pragma unroll
-    for (int k = 0; k < DMAXS; ++k) zacc[k] = 0.0;
-    {
-      const double gami = gi < m ? gam[gi] / (s * s) : 0.0;
-      for (int cc = ec; cc < ec + 16 && gi < m; ++cc) {
-        const int gj = j0 + cc;
-        if (gj >= n) break;
-        const T g = (T)((double)Gs[er][cc] + gami * dv[gj]);
-        T dz[DMAXS], sq = T(0);
-#pragma unroll
-        for (int k = 0; k < DMAXS; ++k) {
-          dz[k] = szi[er][k] - sxj[cc][k];
-          sq += dz[k] * dz[k];
-        }
-        T k1, c1;
-        kval_dcoef<T>(kind, sq, T(1), k1, c1, kshape<T>(kind, theta, n_ls));
-        av += (double)(g * k1);
-        const T gc = g * c1;
-#pragma unroll
-        for (int k = 0; k < DMAXS; ++k) {
-          al[k] += (double)(gc * dz[k] * dz[k]);
-          zacc[k] += (double)(gc * dz[k]);
-        }
-      }
-    }
-    // 4 consecutive lanes share a row: combine (whole warp), one lane adds
-#pragma unroll
-    for (int k = 0; k < DMAXS; ++k) {
-      double v = zacc[k];
-      v += __shfl_xor_sync(0xffffffffu, v, 1);
-      v += __shfl_xor_sync(0xffffffffu, v, 2);
-      zacc[k] = v;
-    }
-    if ((threadIdx.x & 3) == 0 && gi < m) {
-#pragma unroll
-      for (int k = 0; k < DMAXS; ++k) sdz[er][k] += zacc[k];
     }
   }
+  auto put = [&](double v, double* out) { *out = first ? v : *out + v; };
+#pragma unroll
+  for (int k = 0; k < D; ++k) red[ph][il][k] = az[k];
   __syncthreads();
-  // theta partials of this block
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  for (int k = 0; k <= d; ++k) {
-    // slot k: [0, d) lengthscale terms, d variance term
-    double v = av;
-    if (k < d) {
-      v = 0.0;
-#pragma unroll
-      for (int q = 0; q < DMAXS; ++q)
-        if (q == k) v = al[q];
-    }
-    v = warp_sum(v);
-    if (l == 0) sred[w][k] = v;
-  }
-  __syncthreads();
-  const int mt = gridDim.x;
-  if (threadIdx.x <= d) {
-    double t = 0.0;
-    for (int q = 0; q < 8; ++q) t += sred[q][threadIdx.x];
-    thP[((int64_t)split * mt + I) * (d + 1) + threadIdx.x] = t;
-  }
   for (int e = threadIdx.x; e < AB * d; e += 256) {
     const int r = e / d, k = e % d;
-    if (i0 + r < m) dzP[((int64_t)split * m + i0 + r) * d + k] = sdz[r][k];
+    if (blockIdx.x * AB + r < m)
+      put((red[0][r][k] + red[1][r][k]) + (red[2][r][k] + red[3][r][k]),
+          dzP + ((int64_t)split * m + blockIdx.x * AB + r) * d + k);
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < D; ++k) {
+    const double v = warp_sum(al[k]);
+    if ((threadIdx.x & 31) == 0) red[0][threadIdx.x >> 5][k] = v;
+  }
+  const double v = warp_sum(av);
+  if ((threadIdx.x & 31) == 0) red[0][threadIdx.x >> 5][D] = v;
+  __syncthreads();
+  if (threadIdx.x <= d) {
+    const int k = threadIdx.x < d ? threadIdx.x : D;
+    double t = 0.0;
+    for (int w = 0; w < 8; ++w) t += red[0][w][k];
+    put(t, thP + ((int64_t)split * gridDim.x + blockIdx.x) * (d + 1) + threadIdx.x);
   }
 }
 
@@ -809,8 +770,8 @@ gpk_status sgpr_run(int kind, int n, int m, int d, const double* x, int64_t ldx,
                                                 b.Kf, ldm, ss));
   GPK_CUDA_TRY(cross_cov_scaled<double, double>(kind, m, m, d, b.zs64, b.zs64, theta, n_ls, 2,
                                                 jitter, b.Lz, ldm, ss));
-  GPK_CUDA_TRY(potrf_lower<double>(b.Lz, ldm, m, b.ldK, info, nullptr, false, ss));
-  GPK_CUDA_TRY(trtri_lower<double>(b.Lz, ldm, m, b.Mz, ldm, b.Vz, ldm, b.scr, ss));
+  GPK_CUDA_TRY(potrf_lower_x(b.Lz, ldm, m, b.ldK, info, false, b.xk, ss));
+  GPK_CUDA_TRY(trtri_lower<double>(b.Lz, ldm, m, b.Mz, ldm, b.Vz, ldm, b.scr, b.xk, ss));
   {
     GemmProb<double> p{};
     p.A = b.Vz;
@@ -823,7 +784,7 @@ gpk_status sgpr_run(int kind, int n, int m, int d, const double* x, int64_t ldx,
     p.c_lower = 1;
     p.alpha = 1.0;
     p.beta = 0.0;
-    GPK_CUDA_TRY(gemm_nt<double>(p, 1, ss));
+    GPK_CUDA_TRY(gemm_nt_x(p, 1, b.xk, ss));
     sg_mirror<<<mgrid, 256, 0, ss>>>(m, ldm, b.Kinv);
     GPK_LAUNCH_CHECK();
   }
@@ -869,28 +830,28 @@ gpk_status sgpr_run(int kind, int n, int m, int d, const double* x, int64_t ldx,
                                                                      b.cv, b.phi1);
     GPK_LAUNCH_CHECK();
     // P: lower triangles of Phi_k Phi_k^T per n-chunk, summed in float64
-    const int full = n / KCHUNK;
+    const int full = n / b.kchunk;
     GemmProb<T> p{};
-    p.A = b.Phi;
-    p.B = b.Phi;
     p.lda = p.ldb = b.ldn;
-    p.sA = p.sB = KCHUNK;
-    p.C = b.Pparts;
+    p.sA = p.sB = b.kchunk;
     p.ldc = m;
     p.sC = (int64_t)m * m;
     p.M = p.N = m;
-    p.K = KCHUNK;
+    p.K = b.kchunk;
     p.c_lower = 1;
     p.alpha = T(1);
     p.beta = T(0);
-    if (full > 0) GPK_CUDA_TRY(gemm_nt<T>(p, full, s));
-    const int rest = n - full * KCHUNK;
+    for (int c = 0; c < full; c += b.pgroup) {
+      p.A = p.B = b.Phi + (int64_t)c * b.kchunk;
+      p.C = b.Pparts + (int64_t)c * m * m;
+      GPK_CUDA_TRY(gemm_nt_room<T>(p, std::min(b.pgroup, full - c), b.xu, s));
+    }
+    const int rest = n - full * b.kchunk;
     if (rest > 0) {
-      p.A = b.Phi + (int64_t)full * KCHUNK;
-      p.B = p.A;
+      p.A = p.B = b.Phi + (int64_t)full * b.kchunk;
       p.C = b.Pparts + (int64_t)full * m * m;
       p.K = rest;
-      GPK_CUDA_TRY(gemm_nt<T>(p, 1, s));
+      GPK_CUDA_TRY(gemm_nt_room<T>(p, 1, b.xu, s));
     }
   }
   GPK_CUDA_TRY(cudaStreamWaitEvent(s, side->join, 0));
@@ -910,8 +871,8 @@ gpk_status sgpr_run(int kind, int n, int m, int d, const double* x, int64_t ldx,
                                                          b.Su);
     GPK_LAUNCH_CHECK();
   }
-  GPK_CUDA_TRY(potrf_lower<double>(b.Su, ldm, m, b.ldU, info, nullptr, true, s));
-  GPK_CUDA_TRY(trtri_lower<double>(b.Su, ldm, m, b.Mu, ldm, b.Vu, ldm, b.scr, s));
+  GPK_CUDA_TRY(potrf_lower_x(b.Su, ldm, m, b.ldU, info, true, b.xu, s));
+  GPK_CUDA_TRY(trtri_lower<double>(b.Su, ldm, m, b.Mu, ldm, b.Vu, ldm, b.scr, b.xu, s));
   {  // Su^-1 = Vu Vu^T (lower triangle, then mirrored)
     GemmProb<double> p{};
     p.A = b.Vu;
@@ -924,7 +885,7 @@ gpk_status sgpr_run(int kind, int n, int m, int d, const double* x, int64_t ldx,
     p.c_lower = 1;
     p.alpha = 1.0;
     p.beta = 0.0;
-    GPK_CUDA_TRY(gemm_nt<double>(p, 1, s));
+    GPK_CUDA_TRY(gemm_nt_x(p, 1, b.xu, s));
     sg_mirror<<<mgrid, 256, 0, s>>>(m, ldm, b.Suinv);
     GPK_LAUNCH_CHECK();
     // T1 = K^-1 P ; KPK = T1 K^-1 (symmetric operands: NT form; KPK is
@@ -938,12 +899,12 @@ gpk_status sgpr_run(int kind, int n, int m, int d, const double* x, int64_t ldx,
     q.M = q.N = q.K = m;
     q.alpha = 1.0;
     q.beta = 0.0;
-    GPK_CUDA_TRY(gemm_nt<double>(q, 1, s));
+    GPK_CUDA_TRY(gemm_nt_x(q, 1, b.xu, s));
     q.A = b.T1;
     q.B = b.Kinv;
     q.C = b.KPK;
     q.c_lower = 1;
-    GPK_CUDA_TRY(gemm_nt<double>(q, 1, s));
+    GPK_CUDA_TRY(gemm_nt_x(q, 1, b.xu, s));
     sg_mirror<<<mgrid, 256, 0, s>>>(m, ldm, b.KPK);
     GPK_LAUNCH_CHECK();
   }
@@ -972,16 +933,27 @@ gpk_status sgpr_run(int kind, int n, int m, int d, const double* x, int64_t ldx,
       GPK_CUDA_TRY(colsum(b.thP, b.gtiles, d + 1, b.sth, false, b.colpart, s));
       GPK_CUDA_TRY(colsum(b.dzP, b.gcols, (int64_t)m * d, b.gzs, false, b.colpart, s));
     } else {
+      // G^T = Phi^T H (H symmetric) a block of data points at a time
       const int mt = (m + AB - 1) / AB;
-      dim3 grid(mt, ASPLIT);
-      const size_t smem = (size_t)(2 * 16 + AB) * (AB + 1) * sizeof(T) +
-                          (size_t)2 * AB * (DMAXS + 1) * sizeof(T) + 16 +
-                          (size_t)(AB + 8) * (DMAXS + 1) * sizeof(double);
-      cudaFuncSetAttribute(sg_phi_adjoint<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)smem);
-      sg_phi_adjoint<T><<<grid, 256, smem, s>>>(kind, m, n, d, b.Ht, ldm, b.Phi, b.ldn, b.zs,
-                                                b.xs, b.gam, b.dv, theta, n_ls, b.thP, b.dzP);
-      GPK_LAUNCH_CHECK();
+      for (int r0 = 0; r0 < n; r0 += ABLK) {
+        const int rows = std::min(ABLK, n - r0);
+        GPK_CUDA_TRY(cross_cov_scaled<T, T>(kind, rows, m, d, b.xs + (int64_t)r0 * d, b.zs, theta,
+                                            n_ls, 0, 0.0, b.PhiT, ldm, s));
+        GemmProb<T> q{};
+        q.A = b.PhiT;
+        q.B = b.Ht;
+        q.C = b.GT;
+        q.lda = q.ldb = q.ldc = ldm;
+        q.M = rows;
+        q.N = q.K = m;
+        q.alpha = T(1);
+        GPK_CUDA_TRY(gemm_nt_room<T>(q, 1, b.xu, s));
+        auto* reduce = d <= 8 ? sg_phi_reduce<8> : sg_phi_reduce<DMAXS>;
+        reduce<<<dim3(mt, ASPLIT), 256, 0, s>>>(kind, m, rows, d, b.GT, b.PhiT, ldm, b.zs,
+                                                b.xs + (int64_t)r0 * d, b.gams, b.dv + r0, theta,
+                                                n_ls, r0 == 0, b.thP, b.dzP);
+        GPK_LAUNCH_CHECK();
+      }
       GPK_CUDA_TRY(colsum(b.thP, (int64_t)ASPLIT * mt, d + 1, b.sth, false, b.colpart, s));
       GPK_CUDA_TRY(colsum(b.dzP, ASPLIT, (int64_t)m * d, b.gzs, false, b.colpart, s));
     }

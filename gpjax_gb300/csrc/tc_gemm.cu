@@ -91,63 +91,6 @@ struct SmemCtl {
 constexpr int EPI_WARPS = 8;   // epilogue warps: two per TMEM lane quarter
 constexpr int EPI_THREADS = EPI_WARPS * 32;
 
-// Launch index -> output tile (I, J), grouped so that the CTAs resident at
-// one time share operand panels in L2: groups of TILE_GROUP tile rows, walked
-// column by column (consecutive CTAs take consecutive rows of one column).
-// Row tiles are BM high, column tiles bn wide; for c_lower only tiles holding
-// elements on or below the diagonal exist: row tile I reaches column tiles
-// J < ncols(I), and column tile J starts at row tile imin(J).
-constexpr int TILE_GROUP = 8;
-__host__ __device__ inline int lower_ncols(int I, int tiles_n, int bn) {
-  return min(tiles_n, (I * BM + BM - 1) / bn + 1);
-}
-__host__ __device__ inline void tile_of(int t, int c_lower, int tiles_m, int tiles_n, int bn,
-                                        int& I, int& J) {
-  constexpr int G = TILE_GROUP;
-  if (!c_lower) {
-    const int g = t / (G * tiles_n), l = t % (G * tiles_n);
-    const int rows = min(G, tiles_m - g * G);
-    J = l / rows;
-    I = g * G + l % rows;
-    return;
-  }
-  int g = 0, base = 0, rows = 0;
-  for (;; ++g) {
-    rows = min(G, tiles_m - g * G);
-    int cnt = 0;
-    for (int r = 0; r < rows; ++r) cnt += lower_ncols(g * G + r, tiles_n, bn);
-    if (t < base + cnt) break;
-    base += cnt;
-  }
-  int l = t - base;
-  const int full_cols = lower_ncols(g * G, tiles_n, bn);  // every row of the group reaches these
-  if (l < full_cols * rows) {
-    J = l / rows;
-    I = g * G + l % rows;
-    return;
-  }
-  l -= full_cols * rows;
-  for (J = full_cols;; ++J) {
-    const int num = J * bn - BM + 1;
-    const int imin = num > 0 ? (num + BM - 1) / BM : 0;
-    const int r0 = max(g * G, imin);
-    const int cnt = g * G + rows - r0;
-    if (l < cnt) {
-      I = r0 + l;
-      return;
-    }
-    l -= cnt;
-  }
-}
-
-// Number of launch indices tile_of maps (the grid of one GEMM).
-__host__ __device__ inline int tile_count(int c_lower, int tiles_m, int tiles_n, int bn) {
-  if (!c_lower) return tiles_m * tiles_n;
-  int cnt = 0;
-  for (int I = 0; I < tiles_m; ++I) cnt += lower_ncols(I, tiles_n, bn);
-  return cnt;
-}
-
 // MODE: epilogue.  TS: tile shape (Tile<TS>).  DM: bound on the input
 // dimension of the MODE_GRAD epilogue (registers scale with it).
 template <int MODE, int TS, int DM>
@@ -782,24 +725,32 @@ static EncodeTiledFn encode_fn() {
   return fn;
 }
 
+bool tc_encode_map(CUtensorMap* m, CUtensorMapDataType type, int rank, const void* base,
+                   const cuuint64_t* dims, const cuuint64_t* strides, const cuuint32_t* box,
+                   CUtensorMapSwizzle swizzle) {
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) return false;
+  if ((reinterpret_cast<uintptr_t>(base) & 15u) != 0) return false;
+  for (int k = 0; k + 1 < rank; ++k)
+    if (strides[k] & 15) return false;
+  const cuuint32_t estr[5] = {1, 1, 1, 1, 1};
+  return fn(m, type, rank, const_cast<void*>(base), dims, strides, box, estr,
+            CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+            CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 // float32 row-major [rows, cols] with leading dimension ld; box bk x box_rows
 // (bk = 32: 128B swizzle, bk = 16: 64B swizzle; one K slice row per box row)
 static bool make_map(CUtensorMap* m, const void* base, int64_t rows, int64_t cols, int64_t ld,
                      int bk, int box_rows, int elem = 4) {
-  EncodeTiledFn fn = encode_fn();
-  if (!fn) return false;
-  if ((reinterpret_cast<uintptr_t>(base) & 15u) != 0 || ((ld * elem) & 15) != 0) return false;
-  cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-  cuuint64_t strides[1] = {(cuuint64_t)(ld * elem)};
-  cuuint32_t box[2] = {(cuuint32_t)bk, (cuuint32_t)box_rows};
-  cuuint32_t estr[2] = {1, 1};
+  const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
+  const cuuint64_t strides[1] = {(cuuint64_t)(ld * elem)};
+  const cuuint32_t box[2] = {(cuuint32_t)bk, (cuuint32_t)box_rows};
   const int row_bytes = bk * elem;  // 128 -> 128B swizzle, 64 -> 64B swizzle
-  CUresult r = fn(m, elem == 2 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32,
-                  2, const_cast<void*>(base), dims, strides, box, estr,
-                  CU_TENSOR_MAP_INTERLEAVE_NONE,
-                  row_bytes == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
-                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  return r == CUDA_SUCCESS;
+  return tc_encode_map(m, elem == 2 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16
+                                    : CU_TENSOR_MAP_DATA_TYPE_FLOAT32,
+                       2, base, dims, strides, box,
+                       row_bytes == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B);
 }
 
 template <int TS>

@@ -20,11 +20,11 @@
 #pragma once
 #include <cuda.h>
 #include "gpk_internal.cuh"
+#include "tile_order.cuh"
 
 namespace gpk {
 namespace tc {
 
-constexpr int BM = 128;                        // output tile rows (TMEM lanes)
 constexpr int NUM_THREADS = 320;               // w0 TMA, w1 MMA + TMEM, w2..w9 epilogue
 constexpr int GRAD_DMAX = 16;                  // largest input dimension of the adjoint epilogue
 

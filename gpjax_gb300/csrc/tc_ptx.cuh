@@ -131,6 +131,17 @@ __device__ __forceinline__ void mma_f16(uint32_t tmem_d, uint64_t a, uint64_t b,
       : "memory");
 }
 
+// True on one lane of a converged warp.
+__device__ __forceinline__ bool elect_one() {
+  uint32_t leader;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}\n"
+      : "=r"(leader));
+  return leader != 0;
+}
+
 __device__ __forceinline__ void mma_commit(uint64_t* bar) {
   asm volatile(
       "tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
@@ -181,4 +192,11 @@ __device__ __forceinline__ void tmem_ld32_nowait(uint32_t taddr, uint32_t (&r)[3
 }
 
 }  // namespace tc
+
+// cuTensorMapEncodeTiled with unit element strides and zero fill (tc_gemm.cu);
+// false where the driver entry point, the base or a stride will not do.
+bool tc_encode_map(CUtensorMap* m, CUtensorMapDataType type, int rank, const void* base,
+                   const cuuint64_t* dims, const cuuint64_t* strides, const cuuint32_t* box,
+                   CUtensorMapSwizzle swizzle);
+
 }  // namespace gpk
