@@ -35,6 +35,7 @@ __global__ void __launch_bounds__((Cfg::BM / Cfg::TM) * (Cfg::BN / Cfg::TN))
   if (p.c_lower) {
     if (t >= tilesM * (tilesM + 1) / 2) return;
     tri_index(t, I, J);
+    if (J >= tilesN) return;  // a tall product's tiles right of its columns
   } else {
     if (t >= tilesM * tilesN) return;
     I = t / tilesN;
@@ -260,18 +261,23 @@ __global__ void __launch_bounds__(256)
   __shared__ int ex[FX_NB], sbad[FX_NB], sdead;
   const int nb = min(FX_NB, n - k0);
   const int i = threadIdx.x & 63, g = threadIdx.x >> 6;
+  double av[FX_NB * FX_NB / 256];  // every load in flight at once
+#pragma unroll
+  for (int u = 0; u < FX_NB * FX_NB / 256; ++u) {
+    const int e = threadIdx.x + u * 256, r = e >> 6, c = e & 63;
+    av[u] = r < nb && c <= r ? A[(int64_t)(k0 + r) * lda + k0 + c] : 0.0;
+  }
   if (threadIdx.x < FX_NB) {
     ex[i] = i < nb ? scale_of(A[(int64_t)(k0 + i) * lda + k0 + i]) : 0;
     sbad[i] = 0;
     if (i == 0) sdead = 0;
   }
   __syncthreads();
-  for (int e = threadIdx.x; e < FX_NB * FX_NB; e += 256) {
-    const int r = e >> 6, c = e & 63;
+#pragma unroll
+  for (int u = 0; u < FX_NB * FX_NB / 256; ++u) {
+    const int e = threadIdx.x + u * 256, r = e >> 6, c = e & 63;
     bool bad = false;
-    S[r][c] = r < nb && c <= r
-                  ? to_fixed(A[(int64_t)(k0 + r) * lda + k0 + c], ex[r] + ex[c], bad)
-                  : 0;
+    S[r][c] = r < nb || r != c ? to_fixed(av[u], ex[r] + ex[c], bad) : ONE;  // identity past nb
     if (bad) sbad[r] = 1;
   }
   __syncthreads();
@@ -279,52 +285,54 @@ __global__ void __launch_bounds__(256)
   // and scale it by its pivot's reciprocal root (each thread derives the pivot
   // itself); the others meanwhile apply column j - 1 to the group's columns
   // after j.  One barrier per column.
-  for (int c0 = 0; c0 < nb; c0 += FX_G) {
-    const int c1 = min(c0 + FX_G, nb);
+  for (int c0 = 0; c0 < FX_NB; c0 += FX_G) {
     Limbs lv{0, 0};  // this row's entry of the previous column (first 64 threads)
-    for (int j = c0; j < c1; ++j) {
+#pragma unroll
+    for (int q = 0; q < FX_G; ++q) {
+      const int j = c0 + q;
       if (g == 0) {
         long long t = S[i][j], d = S[j][j];
-        if (j > c0) {
-          const Limbs w = lim[j - 1 - c0][j];
+        const int jbad = sbad[j];
+        if (q > 0) {
+          const Limbs w = lim[q - 1][j];
           Acc at, ad;
           at.add(lv, w);
           ad.add(w, w);
           t -= at.value();
           d -= ad.value();
         }
+        const bool good = d > 0 && !jbad;
+        long long y;
+        int s;
+        rsqrt_fixed(good ? d : ONE, y, s);
         bool bad = false;
-        long long v = 0;
-        if (d > 0 && !sbad[j]) {
-          long long y;
-          int s;
-          rsqrt_fixed(d, y, s);
-          v = i >= j ? times_rsqrt(t, y, s, bad) : 0;
-        } else if (i == j) {
+        const long long v = times_rsqrt(i >= j ? t : 0, y, s, bad);
+        lv = limbs(v);
+        lim[q][i] = lv;
+        if (bad) sbad[i] = 1;
+        if (!good && i == j) {  // the rest of this group's columns mean nothing
           atomicMin(info, k0 + j + 1);
           sdead = 1;
         }
-        lv = limbs(v);
-        lim[j - c0][i] = lv;
-        if (bad) sbad[i] = 1;
-      } else if (j > c0) {
-        const Limbs mine = lim[j - 1 - c0][i];
-        for (int k = j + g; k < c1; k += 3) {
-          if (i < k) continue;
+      } else if (q > 0) {
+        const Limbs mine = lim[q - 1][i];
+#pragma unroll
+        for (int h = 0; h < (FX_G - q + 1) / 3; ++h) {
+          const int k = j + g + 3 * h;
+          if (k >= c0 + FX_G || i < k) continue;
           Acc acc;
-          acc.add(mine, lim[j - 1 - c0][k]);
+          acc.add(mine, lim[q - 1][k]);
           S[i][k] -= acc.value();
         }
       }
       __syncthreads();
-      if (sdead) break;
     }
     if (sdead) break;
-    if (c1 < nb) {
+    if (c0 + FX_G < nb) {
       Limbs lq[FX_G];
 #pragma unroll
       for (int q = 0; q < FX_G; ++q) lq[q] = lim[q][i];
-      for (int k = c1 + g; k < nb; k += 4) {
+      for (int k = c0 + FX_G + g; k < nb; k += 4) {
         if (i < k) continue;
         Acc acc;
 #pragma unroll
@@ -332,9 +340,10 @@ __global__ void __launch_bounds__(256)
         S[i][k] -= acc.value();
       }
     }
-    for (int q = g; q < c1 - c0; q += 4) {
-      const Limbs l = lim[q][i];
-      S[i][c0 + q] = ((long long)l.h << 32) + l.l;
+#pragma unroll
+    for (int h = 0; h < FX_G / 4; ++h) {
+      const Limbs l = lim[g + 4 * h][i];
+      S[i][c0 + g + 4 * h] = ((long long)l.h << 32) + l.l;
     }
     __syncthreads();
   }
@@ -343,23 +352,26 @@ __global__ void __launch_bounds__(256)
   __syncthreads();
   if (logdiag && threadIdx.x < nb)
     logdiag[k0 + i] = dead ? nan : log(to_double(S[i][i], ex[i]));
-  for (int e = threadIdx.x; e < nb * nb; e += 256) {
-    const int r = e / nb, c = e % nb;
-    A[(int64_t)(k0 + r) * lda + k0 + c] =
-        c > r ? 0.0 : dead ? nan : to_double(S[r][c], ex[r]);
+#pragma unroll 4
+  for (int u = 0; u < FX_NB * FX_NB / 256; ++u) {
+    const int e = threadIdx.x + u * 256, r = e >> 6, c = e & 63;
+    if (r < nb && c < nb)
+      A[(int64_t)(k0 + r) * lda + k0 + c] =
+          c > r ? 0.0 : dead ? nan : to_double(S[r][c], ex[r]);
   }
 }
 
 // Panel solve X L^T = A for 32 rows per CTA: lane = row; one warp substitutes
-// a group of eight columns, then the eight warps split the columns to the
+// a group of four columns, then the eight warps split the columns to the
 // right.  A row's scale comes from its own
 // diagonal entry, which bounds every entry of the factor's row; a column's
 // from the norm of that row of L.
 constexpr int FX_ROWS = 32;
 constexpr int FX_XLD = FX_NB + 1;
+constexpr int FX_TG = 4;  // columns substituted between updates of the rest
 constexpr size_t FX_TRSM_SMEM = (size_t)FX_NB * FX_NB * sizeof(fx::Limbs) +
                                 (size_t)FX_ROWS * FX_XLD * 8 + (size_t)FX_NB * 16 +
-                                FX_ROWS * 8 + (size_t)FX_G * FX_ROWS * sizeof(fx::Limbs);
+                                FX_ROWS * 8 + (size_t)FX_TG * FX_ROWS * sizeof(fx::Limbs);
 __global__ void __launch_bounds__(256)
     trsm_rows_fixed_kernel(double* A, int64_t lda, int n, int k0) {
   using namespace fx;
@@ -371,17 +383,29 @@ __global__ void __launch_bounds__(256)
   int* ej = rs + FX_NB;
   int* ei = ej + FX_NB;
   int* sbad = ei + FX_ROWS;
-  Limbs* LX = reinterpret_cast<Limbs*>(sbad + FX_ROWS);            // [8][32], current group
+  Limbs* LX = reinterpret_cast<Limbs*>(sbad + FX_ROWS);            // [FX_TG][32]
   const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
   const int r0 = k0 + FX_NB + blockIdx.x * FX_ROWS, rows = min(FX_ROWS, n - r0);
-  for (int j = g; j < FX_NB; j += 8) {
-    const double* row = A + (int64_t)(k0 + j) * lda + k0;
-    double a[2];
+  double av[FX_ROWS * FX_NB / 256], lv[2 * FX_NB / 8];  // every load in flight at once
+#pragma unroll
+  for (int u = 0; u < FX_NB / 8; ++u)
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int j = g + 8 * u, k = lane + 32 * h;
+      lv[2 * u + h] = k <= j ? A[(int64_t)(k0 + j) * lda + k0 + k] : 0.0;
+    }
+#pragma unroll
+  for (int u = 0; u < FX_ROWS * FX_NB / 256; ++u) {
+    const int e = threadIdx.x + u * 256, r = e >> 6, c = e & 63;
+    av[u] = r < rows ? A[(int64_t)(r0 + r) * lda + k0 + c] : 0.0;
+  }
+#pragma unroll
+  for (int u = 0; u < FX_NB / 8; ++u) {
+    const int j = g + 8 * u;
+    const double* a = lv + 2 * u;
     int xb[2], xm = 1;
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      const int k = lane + 32 * h;
-      a[h] = k <= j ? row[k] : 0.0;
       xb[h] = (int)((__double_as_longlong(a[h]) >> 52) & 0x7ff);
       xm = max(xm, xb[h]);
     }
@@ -416,51 +440,51 @@ __global__ void __launch_bounds__(256)
         1.0 / A[(int64_t)(k0 + j) * lda + k0 + j]);
     ry[j] = (long long)((b & 0xfffffffffffffULL) | (1ULL << 52)) << 9;  // [1, 2) 2^61
     rs[j] = -((int)((b >> 52) & 0x7ff) - 1023 + ej[j]);
-    if (((b >> 52) & 0x7ff) == 0x7ff || ((b >> 52) & 0x7ff) == 0) {
+    if (((b >> 52) & 0x7ff) == 0x7ff || rs[j] < -58 || rs[j] > 1) {  // a failed block
       ry[j] = 0;
       rs[j] = 0;
     }
   }
-  for (int e = threadIdx.x; e < FX_ROWS * FX_NB; e += 256) {
-    const int r = e >> 6, c = e & 63;
+#pragma unroll
+  for (int u = 0; u < FX_ROWS * FX_NB / 256; ++u) {
+    const int e = threadIdx.x + u * 256, r = e >> 6, c = e & 63;
     bool bad = false;
-    X[r * FX_XLD + c] =
-        r < rows ? to_fixed(A[(int64_t)(r0 + r) * lda + k0 + c], ei[r] + ej[c], bad) : 0;
+    X[r * FX_XLD + c] = to_fixed(av[u], ei[r] + ej[c], bad);
     if (bad) sbad[r] = 1;
   }
   __syncthreads();
   long long* x = X + lane * FX_XLD;
-  for (int c0 = 0; c0 < FX_NB; c0 += FX_G) {
+  for (int c0 = 0; c0 < FX_NB; c0 += FX_TG) {
     if (g == 0) {
-      long long t[FX_G];
+      long long t[FX_TG];
       bool bad = false;
 #pragma unroll
-      for (int q = 0; q < FX_G; ++q) t[q] = x[c0 + q];
+      for (int q = 0; q < FX_TG; ++q) t[q] = x[c0 + q];
 #pragma unroll
-      for (int q = 0; q < FX_G; ++q) {
+      for (int q = 0; q < FX_TG; ++q) {
         t[q] = times_rsqrt(t[q], ry[c0 + q], rs[c0 + q], bad);
         const Limbs l = limbs(t[q]);
         LX[q * FX_ROWS + lane] = l;
 #pragma unroll
-        for (int u = q + 1; u < FX_G; ++u) {
+        for (int u = q + 1; u < FX_TG; ++u) {
           Acc acc;
           acc.add(l, L[(c0 + u) * FX_NB + c0 + q]);
           t[u] -= acc.value();
         }
       }
 #pragma unroll
-      for (int q = 0; q < FX_G; ++q) x[c0 + q] = t[q];
+      for (int q = 0; q < FX_TG; ++q) x[c0 + q] = t[q];
       if (bad) sbad[lane] = 1;
     }
     __syncthreads();
-    if (c0 + FX_G == FX_NB) break;
-    Limbs lx[FX_G];
+    if (c0 + FX_TG == FX_NB) break;
+    Limbs lx[FX_TG];
 #pragma unroll
-    for (int q = 0; q < FX_G; ++q) lx[q] = LX[q * FX_ROWS + lane];
-    for (int k = c0 + FX_G + g; k < FX_NB; k += 8) {
+    for (int q = 0; q < FX_TG; ++q) lx[q] = LX[q * FX_ROWS + lane];
+    for (int k = c0 + FX_TG + g; k < FX_NB; k += 8) {
       Acc acc;
 #pragma unroll
-      for (int q = 0; q < FX_G; ++q) acc.add(lx[q], L[k * FX_NB + c0 + q]);
+      for (int q = 0; q < FX_TG; ++q) acc.add(lx[q], L[k * FX_NB + c0 + q]);
       x[k] -= acc.value();
     }
     __syncthreads();

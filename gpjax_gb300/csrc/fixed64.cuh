@@ -95,32 +95,31 @@ __device__ __forceinline__ void rsqrt_fixed(long long d, long long& y, int& s) {
     m >>= 1;
     ++ex;
   }
-  const float f = rsqrtf((float)(unsigned)(m >> 32) * 2.3283064365386963e-10f);
+  float f = (float)(unsigned)(m >> 32) * 2.3283064365386963e-10f;
+  asm("rsqrt.approx.ftz.f32 %0, %0;" : "+f"(f));
   const unsigned y0 = (unsigned)(f * 1073741824.f);
   const unsigned long long yy = (unsigned long long)y0 * y0;              // 2^-60
-  const long long e = (1LL << 60) - (long long)__umul64hi(m, yy);
-  const long long e2 = ((e >> 10) * (e >> 10)) >> 40;
-  const long long corr = (e >> 1) + ((3 * e2) >> 3);
-  const long long b = (long long)y0 << 31;                               // 2^-61
-  y = b + (__mul64hi(b, corr << 20) >> 16);
+  const long long e = (1LL << 60) - (long long)__umul64hi(m, yy);         // |e| < 2^40
+  const int eh = (int)(e >> 10);
+  const long long corr = (e >> 1) + ((3 * (((long long)eh * eh) >> 40)) >> 3);
+  // y0 (1 + corr) at 2^-61, corr in two parts so that 32-bit multiplies do
+  const int ch = (int)(corr >> 20), cl = (int)(corr & 0xfffff);
+  const long long dy = (long long)((unsigned long long)y0 * (unsigned)cl >> 20) +
+                       (long long)(int)(y0 >> 1) * ch * 2 + (long long)(int)(y0 & 1) * ch;
+  y = ((long long)y0 << 31) + (dy >> 9);
   s = ex / 2;  // ex is even
 }
 
-// a / sqrt(d) in fixed point from rsqrt_fixed's y and s; *bad when it leaves
-// the range of a definite matrix.
+// a / sqrt(d) in fixed point from rsqrt_fixed's y and s (-58 <= s <= 1); *bad
+// is set when it leaves the range of a definite matrix.  No branches: these
+// sit on the chain of pivots.
 __device__ __forceinline__ long long times_rsqrt(long long a, long long y, int s, bool& bad) {
   const long long mag = a < 0 ? -a : a;
-  const int cap = FRAC + 1 + s;  // |a| < 2^cap keeps the shifted operand in range
-  if (cap < 0 || (mag >> cap) != 0) {
-    bad = true;
-    return 0;
-  }
+  const bool over = (mag >> (FRAC + 1 + s)) != 0;  // the shifted operand would wrap
   const long long v = __mul64hi(a << (2 - s), y) << 1;
-  if (v > LIMIT || v < -LIMIT) {
-    bad = true;
-    return 0;
-  }
-  return v;
+  const bool out = over || v > LIMIT || v < -LIMIT;
+  bad = bad || out;
+  return out ? 0 : v;
 }
 
 }  // namespace fx

@@ -63,7 +63,7 @@ size_t loocv_layout(int64_t n, int d, void* ws, LoocvBuffers& b) {
   b.gth = (double*)take((size_t)(GPK_MAX_D + 8) * 8);
   b.vjp_bytes = gpk_cross_covariance_vjp_workspace_bytes(n, n, d);
   b.vjp_ws = take(b.vjp_bytes);
-  b.x.bytes = xroom_fit(off, n <= 512 ? 0 : std::max(xroom_factor_bytes(n), xsplit_bytes(n, n)));
+  b.x.bytes = xroom_fit(off, n <= 128 ? 0 : std::max(xroom_factor_bytes(n), xsplit_bytes(n, n)));
   b.x.mem = take(b.x.bytes);
   return off + 256;
 }

@@ -66,7 +66,7 @@ struct MllBuffers {
 };
 
 template <typename T>
-static size_t mll_layout(int64_t n, int d, void* ws, MllBuffers<T>& b) {
+static size_t mll_layout(int64_t n, int d, void* ws, MllBuffers<T>& b, bool room = true) {
   Arena a(ws);
   b.ld = pad_ld(n);
   const size_t nn = (size_t)n * b.ld;
@@ -74,7 +74,7 @@ static size_t mll_layout(int64_t n, int d, void* ws, MllBuffers<T>& b) {
   b.M = a.take<T>(nn);
   b.V = a.take<T>(nn);
   b.scratch = a.take<T>((size_t)n * n / 2 + 64);
-  b.x.bytes = sizeof(T) == 8 ? xroom_fit(nn * sizeof(T) * 4, xroom_factor_bytes(n)) : 0;
+  b.x.bytes = sizeof(T) == 8 && room ? xroom_fit(nn * sizeof(T) * 4, xroom_factor_bytes(n)) : 0;
   b.x.mem = a.take<char>(b.x.bytes);
   b.xs = a.take<T>((size_t)n * d);
   b.diff = a.take<double>(n);
@@ -227,9 +227,9 @@ template <typename T>
 static gpk_status mll_run(int kind, int n, int d, const double* x, int64_t ldx, const double* y,
                           const double* theta, int n_ls, double jitter, int refine, int want_grad,
                           double* out_mll, double* out_grad, int* info, void* ws,
-                          cudaStream_t s) {
+                          cudaStream_t s, bool room = true) {
   MllBuffers<T> b;
-  mll_layout<T>(n, d, ws, b);
+  mll_layout<T>(n, d, ws, b, room);
   prof_mark(0, s);
   init_info_kernel<<<1, 1, 0, s>>>(info);
   GPK_LAUNCH_CHECK();
@@ -504,7 +504,7 @@ static size_t solve_layout(int64_t n, int64_t nrhs, bool upper, void* ws, T** M,
   *BT = a.take<T>((size_t)nrhs * *ld);
   *LT = upper ? a.take<T>((size_t)n * *ld) : nullptr;  // lower copy U^T of an upper input
   if (sizeof(T) == 8)  // digit planes: the inverse's products; then B^T beside it
-    x->bytes = xroom_fit(a.off, n <= 512 ? 0 : std::max(xroom_factor_bytes(n),
+    x->bytes = xroom_fit(a.off, n <= 128 ? 0 : std::max(xroom_factor_bytes(n),
                                                        xsplit_bytes(nrhs, n) + xsplit_bytes(n, n)));
   x->mem = a.take<char>(x->bytes);
   return a.off + 256;
@@ -764,7 +764,7 @@ extern "C" gpk_status gpk_conjugate_mll_noalloc(int kind, int64_t n, int d, cons
   }
   if (!x || !y) return GPK_ERR_BAD_ARG;
   MllBuffers<double> b;
-  if (mll_layout<double>(n, d, nullptr, b) > kNoallocBytes) return GPK_ERR_UNSUPPORTED;
+  if (mll_layout<double>(n, d, nullptr, b, false) > kNoallocBytes) return GPK_ERR_UNSUPPORTED;
   void* ws = nullptr;
   const gpk_status st = noalloc_scratch(&ws);
   if (st != GPK_OK) return st;
@@ -772,5 +772,5 @@ extern "C" gpk_status gpk_conjugate_mll_noalloc(int kind, int64_t n, int d, cons
   // call (Gram, factor, inverse, solves, per-tile partials), so nothing left
   // by an earlier call has to be cleared.
   return mll_run<double>(kind, (int)n, d, x, ldx, y, theta, n_ls, jitter, 1, want_grad, out_mll,
-                         out_grad, info, ws, stream);
+                         out_grad, info, ws, stream, false);
 }

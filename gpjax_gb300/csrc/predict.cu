@@ -70,7 +70,7 @@ size_t pred_layout(int64_t n, int64_t t, int d, bool want_cov, void* ws, PredBuf
   b.rpart = a.take<double>(residual_scratch_doubles((int)n));
   if (sizeof(T) == 8) {
     // the factor's products; then Ktx beside M, and Q^T alone
-    const size_t want = n <= 512 && t <= 512 ? 0
+    const size_t want = n <= 128 && t <= 128 ? 0
                                              : std::max(xroom_factor_bytes(n),
                                                         xsplit_bytes(t, n) + xsplit_bytes(n, n));
     b.x.bytes = xroom_fit(a.off, want);

@@ -174,7 +174,7 @@ size_t sgpr_layout(int64_t n, int64_t m, int d, void* ws, SgprBuf<T>& b) {
   b.gzs = a.take<double>((size_t)m * d);
   b.ddds = a.take<double>(2);
   b.err = a.take<int>(1);
-  const size_t small = m <= 512 ? 0 : std::max(xroom_factor_bytes(m), 2 * xsplit_bytes(m, m));
+  const size_t small = m <= 128 ? 0 : std::max(xroom_factor_bytes(m), 2 * xsplit_bytes(m, m));
   size_t want = small;
   if (!mixed) {
     // P's partials go through the room in groups of at most 2 GB of digits

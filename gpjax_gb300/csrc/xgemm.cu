@@ -22,7 +22,7 @@ constexpr int XEPI_WARPS = 8, XEPI_THREADS = XEPI_WARPS * 32;
 constexpr int XHC = XN / 2;       // accumulator columns of one epilogue thread
 constexpr int XTLD = XN + 1;      // staged tile row stride (doubles)
 constexpr int XNAN = 0x7ff;       // row exponent of a row with a NaN or an infinity
-constexpr double XMIN_MULTS = 4e6;  // below this the CUDA cores finish before the split would
+constexpr double XMIN_MULTS = 5e5;  // below, a CUDA-core product is as quick as the split
 constexpr int XMAX_K = 1 << 18;   // the drained 64-bit sums stay below K * 2^41
 
 // K slices summed by one accumulator before it is drained: a group holds up to
@@ -200,6 +200,7 @@ __global__ void __launch_bounds__(XTHREADS, 1)
       }
       if (leader) mma_commit(&ctl->empty[s]);
     };
+    static_assert(XSTAGES * XSTAGE_BYTES >= BM * (XTLD + XN) * 8, "both output tiles fit the ring");
     static_assert(XSTAGES == 2, "the stage is a compile-time constant of each call below");
     for (int kc = 0; kc < nk && ok; kc += 2) {
       chunk(kc, 0);
@@ -257,19 +258,38 @@ __global__ void __launch_bounds__(XTHREADS, 1)
       }
     }
     const double nan = __longlong_as_double(0x7ff8000000000000ULL);
+    const double beta = p.beta;
+    const int am = p.alpha_mode, bm = p.beta_mode;
+    double* C = p.C ? p.C + (int64_t)z * p.sC : nullptr;
+    double* Ct = p.Ct ? p.Ct + (int64_t)z * p.sCt : nullptr;
+    auto inside = [&](int rr, int cc) {
+      const int gi = i0 + rr, gj = j0 + cc;
+      return gi < p.M && gj < p.N && !(p.c_lower && gj > gi);
+    };
     asm volatile("bar.sync 1, %0;" ::"r"(XEPI_THREADS) : "memory");  // ring free, eb staged
+    // the old C tile comes into the other half of the ring while the sums are
+    // rounded (2.5 us of loads otherwise)
+    double* ctile = otile + BM * XTLD;
+    if (C && bm != 1) {
+#pragma unroll 4
+      for (int e = et; e < BM * XN; e += XEPI_THREADS) {
+        const int rr = e / XN, cc = e % XN;
+        if (inside(rr, cc))
+          asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(ctile + e)),
+                       "l"(C + (int64_t)(i0 + rr) * p.ldc + j0 + cc)
+                       : "memory");
+      }
+    }
 #pragma unroll
     for (int c = 0; c < XHC; ++c) {
       const int eb = ctl->eb[hcol + c];
       const bool bad = !have || ea == XNAN || eb == XNAN;
       otile[r * XTLD + hcol + c] = bad ? nan : x_round(hi[c], lo[c], ea + eb - 2 * 1022 - 70);
     }
+    asm volatile("cp.async.wait_all;" ::: "memory");
     asm volatile("bar.sync 1, %0;" ::"r"(XEPI_THREADS) : "memory");
-    const double alpha = p.alpha, beta = p.beta;
-    double* C = p.C ? p.C + (int64_t)z * p.sC : nullptr;
-    double* Ct = p.Ct ? p.Ct + (int64_t)z * p.sCt : nullptr;
-    // on integer modes: a float64 comparison per element runs at the float64 rate
-    const int am = p.alpha_mode, bm = p.beta_mode;
+    // integer modes: a float64 comparison per element runs at the float64 rate
+    const double alpha = p.alpha;
     auto scaled = [&](double v) {
       if (am == 1) return v;
       if (am == 2)
@@ -277,36 +297,22 @@ __global__ void __launch_bounds__(XTHREADS, 1)
       return alpha * v;
     };
     if (C) {
-      constexpr int RB = 8;  // elements in flight per thread
-      for (int e0 = et; e0 < BM * XN; e0 += XEPI_THREADS * RB) {
-        double cv[RB];
-        bool in[RB];
-#pragma unroll
-        for (int u = 0; u < RB; ++u) {
-          const int e = e0 + u * XEPI_THREADS, rr = e / XN, cc = e % XN;
-          const int gi = i0 + rr, gj = j0 + cc;
-          in[u] = gi < p.M && gj < p.N && !(p.c_lower && gj > gi);
-          cv[u] = in[u] && bm != 1 ? C[(int64_t)gi * p.ldc + gj] : 0.0;
-        }
-#pragma unroll
-        for (int u = 0; u < RB; ++u) {
-          const int e = e0 + u * XEPI_THREADS, rr = e / XN, cc = e % XN;
-          if (!in[u]) continue;
-          double v = scaled(otile[rr * XTLD + cc]);
-          if (bm == 2)
-            v += cv[u];
-          else if (bm == 0)
-            v = fma(beta, cv[u], v);
-          C[(int64_t)(i0 + rr) * p.ldc + j0 + cc] = v;
-        }
+#pragma unroll 8
+      for (int e = et; e < BM * XN; e += XEPI_THREADS) {
+        const int rr = e / XN, cc = e % XN;
+        if (!inside(rr, cc)) continue;
+        double v = scaled(otile[rr * XTLD + cc]);
+        if (bm == 2)
+          v += ctile[e];
+        else if (bm == 0)
+          v = fma(beta, ctile[e], v);
+        C[(int64_t)(i0 + rr) * p.ldc + j0 + cc] = v;
       }
     }
     if (Ct) {
       for (int e = et; e < BM * XN; e += XEPI_THREADS) {
         const int cc = e / BM, rr = e % BM;
-        const int gi = i0 + rr, gj = j0 + cc;
-        if (gi >= p.M || gj >= p.N || (p.c_lower && gj > gi)) continue;
-        Ct[(int64_t)gj * p.ldct + gi] = scaled(otile[rr * XTLD + cc]);
+        if (inside(rr, cc)) Ct[(int64_t)(j0 + cc) * p.ldct + i0 + rr] = scaled(otile[rr * XTLD + cc]);
       }
     }
   }
@@ -509,7 +515,8 @@ cudaError_t gemm_nt_x(const GemmProb<double>& p, int batch, const XRoom& x, cuda
                      (batch == 1 || (p.N == p.M && p.sA == p.sB));
   const size_t na = xsplit_bytes((int64_t)p.M * batch, p.K);
   const size_t nb = front ? 0 : xsplit_bytes((int64_t)p.N * batch, p.K);
-  const double mults = (double)p.M * p.N * p.K * batch * (p.c_lower ? 0.5 : 1.0);
+  const double outs = (double)p.M * p.N - (p.c_lower ? 0.5 * p.N * p.N : 0.0);
+  const double mults = outs * p.K * batch;
   if (!x.mem || na + nb > x.bytes || p.K > XMAX_K || p.K < XK || mults < XMIN_MULTS ||
       (int64_t)p.M * batch > INT_MAX / 2 || (int64_t)p.N * batch > INT_MAX / 2)
     return gemm_nt<double>(p, batch, s);
@@ -526,7 +533,7 @@ cudaError_t gemm_nt_x(const GemmProb<double>& p, int batch, const XRoom& x, cuda
 }
 
 size_t xroom_factor_bytes(int64_t n) {
-  if (n <= 512) return 0;
+  if (n <= 128) return 0;  // at most two blocks
   int64_t b = 64;
   while (2 * b < n) b *= 2;
   // a product of the factor or of a merge level reads at most n rows in all, of
