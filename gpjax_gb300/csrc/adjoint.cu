@@ -23,21 +23,22 @@ __host__ __device__ inline int grad_slots(int d) { return d + 2; }
 
 // FROM_W: V holds W = Sigma^-1 itself (lower tiles), formed beforehand on the
 // tensor cores; the kernel is then the reduction alone.
-template <typename T, int DMAX, bool FROM_W = false>
-__global__ void __launch_bounds__((GemmCfg<T>::BM / GemmCfg<T>::TM) * (GemmCfg<T>::BN / GemmCfg<T>::TN))
+template <typename T, int DMAX, typename Cfg = GemmCfg<T>, bool FROM_W = false>
+__global__ void __launch_bounds__((Cfg::BM / Cfg::TM) * (Cfg::BN / Cfg::TN))
     lauum_grad_kernel(int kind, const T* __restrict__ V, int64_t ldv, int n, int d,
                       const T* __restrict__ xs, const double* __restrict__ alpha,
                       double* __restrict__ gpart, const double* __restrict__ kaptr) {
-  constexpr int BM = GemmCfg<T>::BM, BN = GemmCfg<T>::BN, BK = GemmCfg<T>::BK;
-  constexpr int TM = GemmCfg<T>::TM, TN = GemmCfg<T>::TN;
+  constexpr int BM = Cfg::BM, BN = Cfg::BN, BK = Cfg::BK;
+  constexpr int TM = Cfg::TM, TN = Cfg::TN;
   constexpr int NTX = BN / TN, NTY = BM / TM, NT = NTX * NTY;
   constexpr int WLD = BN + 1;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   // main-loop staging and the W tile share the front of shared memory
-  SimtSmem<T>& sm = *reinterpret_cast<SimtSmem<T>*>(smem_raw);
+  SimtSmem<T, Cfg>& sm = *reinterpret_cast<SimtSmem<T, Cfg>*>(smem_raw);
   T* Ws = reinterpret_cast<T*>(smem_raw);
-  constexpr size_t front = sizeof(SimtSmem<T>) > sizeof(T) * BM * WLD ? sizeof(SimtSmem<T>)
-                                                                       : sizeof(T) * BM * WLD;
+  constexpr size_t front = sizeof(SimtSmem<T, Cfg>) > sizeof(T) * BM * WLD
+                               ? sizeof(SimtSmem<T, Cfg>)
+                               : sizeof(T) * BM * WLD;
   T* sxi = reinterpret_cast<T*>(smem_raw + ((front + 15) & ~size_t(15)));
   T* sxj = sxi + BM * DMAX;
   T* sai = sxj + BN * DMAX;
@@ -62,7 +63,7 @@ __global__ void __launch_bounds__((GemmCfg<T>::BM / GemmCfg<T>::TM) * (GemmCfg<T
     for (int a = 0; a < TM; ++a)
 #pragma unroll
       for (int b = 0; b < TN; ++b) acc[a][b] = T(0);
-    simt_tile_mma<T>(V, ldv, n, TRI_UPPER, V, ldv, n, TRI_UPPER, i0, j0, klo, khi, sm, acc);
+    simt_tile_mma<T, Cfg>(V, ldv, n, TRI_UPPER, V, ldv, n, TRI_UPPER, i0, j0, klo, khi, sm, acc);
     // (simt_tile_mma ends with a barrier, so the staging area can be reused)
     const int tx = threadIdx.x % NTX, ty = threadIdx.x / NTX;
 #pragma unroll
@@ -141,44 +142,77 @@ __global__ void __launch_bounds__((GemmCfg<T>::BM / GemmCfg<T>::TM) * (GemmCfg<T
   }
 }
 
-template <typename T, int DMAX, bool FROM_W = false>
+template <typename T, int DMAX, typename Cfg, bool FROM_W>
 static cudaError_t launch_lauum_grad(int kind, const T* V, int64_t ldv, int n, int d, const T* xs,
                                      const double* alpha, double* gpart, const double* kaptr,
                                      cudaStream_t s) {
-  constexpr int BM = GemmCfg<T>::BM, BN = GemmCfg<T>::BN;
-  constexpr int NT = (GemmCfg<T>::BM / GemmCfg<T>::TM) * (GemmCfg<T>::BN / GemmCfg<T>::TN);
+  constexpr int BM = Cfg::BM, BN = Cfg::BN;
+  constexpr int NT = (Cfg::BM / Cfg::TM) * (Cfg::BN / Cfg::TN);
   const int tiles_m = (n + BM - 1) / BM;
   const int tiles = tiles_m * (tiles_m + 1) / 2;
-  const size_t front = sizeof(SimtSmem<T>) > sizeof(T) * BM * (BN + 1) ? sizeof(SimtSmem<T>)
-                                                                          : sizeof(T) * BM * (BN + 1);
+  const size_t front = sizeof(SimtSmem<T, Cfg>) > sizeof(T) * BM * (BN + 1)
+                           ? sizeof(SimtSmem<T, Cfg>)
+                           : sizeof(T) * BM * (BN + 1);
   const size_t smem = ((front + 15) & ~size_t(15)) + (size_t)(BM + BN) * DMAX * sizeof(T) +
                       (size_t)(BM + BN) * sizeof(T) + 16 +
                       (size_t)(GPK_MAX_D + 2) * (NT / 32) * sizeof(double);
-  cudaFuncSetAttribute(lauum_grad_kernel<T, DMAX, FROM_W>,
+  cudaFuncSetAttribute(lauum_grad_kernel<T, DMAX, Cfg, FROM_W>,
                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  lauum_grad_kernel<T, DMAX, FROM_W><<<tiles, NT, smem, s>>>(kind, V, ldv, n, d, xs, alpha, gpart,
-                                                             kaptr);
+  lauum_grad_kernel<T, DMAX, Cfg, FROM_W><<<tiles, NT, smem, s>>>(kind, V, ldv, n, d, xs, alpha,
+                                                                  gpart, kaptr);
   return launch_status();
+}
+
+// Tile edge of the float64 form: 16 while those tiles fit about two waves of
+// the chip (n <= 384), 32 up to n = 1536, 64 above (each block's float64 work
+// runs at 1.7 operations per clock, so too few blocks is what a small n pays
+// for: n = 100 took 172 us in three 64 x 64 tiles).
+template <typename T>
+static int lauum_edge(int n) {
+  if (sizeof(T) == 4) return GemmCfg<float>::BM;
+  return n <= 384 ? 16 : n <= 1536 ? 32 : 64;
 }
 
 template <typename T>
 int lauum_grad_tiles(int n) {
-  const int tm = (n + GemmCfg<T>::BM - 1) / GemmCfg<T>::BM;
+  const int e = lauum_edge<T>(n), tm = (n + e - 1) / e;
   return tm * (tm + 1) / 2;
 }
 template int lauum_grad_tiles<double>(int);
 template int lauum_grad_tiles<float>(int);
+
+template <typename T, bool FROM_W>
+static cudaError_t lauum_dispatch(int kind, const T* V, int64_t ldv, int n, int d, const T* xs,
+                                  const double* theta, int n_ls, const double* alpha,
+                                  double* gpart, cudaStream_t s) {
+  const double* ka = kind == GPK_RATIONAL_QUADRATIC ? theta + n_ls + 3 : nullptr;
+  auto by_tile = [&](auto dmax) {
+    constexpr int D = decltype(dmax)::value;
+    if constexpr (sizeof(T) == 8) {
+      const int e = lauum_edge<T>(n);
+      if (e == 16)
+        return launch_lauum_grad<T, D, GemmCfgTiny<T>, FROM_W>(kind, V, ldv, n, d, xs, alpha,
+                                                               gpart, ka, s);
+      if (e == 32)
+        return launch_lauum_grad<T, D, GemmCfgSmall<T>, FROM_W>(kind, V, ldv, n, d, xs, alpha,
+                                                                gpart, ka, s);
+    }
+    return launch_lauum_grad<T, D, GemmCfg<T>, FROM_W>(kind, V, ldv, n, d, xs, alpha, gpart, ka,
+                                                       s);
+  };
+  if (sizeof(T) == 8 && d <= 4) return by_tile(std::integral_constant<int, sizeof(T) == 8 ? 4 : 8>{});
+  if (d <= 8) return by_tile(std::integral_constant<int, 8>{});
+  if (d <= 16) return by_tile(std::integral_constant<int, 16>{});
+  if (d <= 32) return by_tile(std::integral_constant<int, 32>{});
+  return cudaErrorInvalidValue;
+}
 
 template <typename T>
 cudaError_t lauum_grad(int kind, const T* V, int64_t ldv, int n, int d, const T* xs,
                        const double* theta, int n_ls, const double* alpha, double* gpart,
                        cudaStream_t s) {
   if (n <= 0) return cudaSuccess;
-  const double* ka = kind == GPK_RATIONAL_QUADRATIC ? theta + n_ls + 3 : nullptr;
-  if (d <= 8) return launch_lauum_grad<T, 8>(kind, V, ldv, n, d, xs, alpha, gpart, ka, s);
-  if (d <= 16) return launch_lauum_grad<T, 16>(kind, V, ldv, n, d, xs, alpha, gpart, ka, s);
-  if (d <= 32) return launch_lauum_grad<T, 32>(kind, V, ldv, n, d, xs, alpha, gpart, ka, s);
-  return cudaErrorInvalidValue;
+  return lauum_dispatch<T, false>(kind, V, ldv, n, d, xs, theta, n_ls, alpha, gpart, s);
 }
 
 cudaError_t lauum_grad_x(int kind, const double* V, int64_t ldv, int n, int d, const double* xs,
@@ -196,14 +230,7 @@ cudaError_t lauum_grad_x(int kind, const double* V, int64_t ldv, int n, int d, c
   p.alpha = 1.0;
   cudaError_t e = gemm_nt_x(p, 1, x, s);
   if (e != cudaSuccess) return e;
-  const double* ka = kind == GPK_RATIONAL_QUADRATIC ? theta + n_ls + 3 : nullptr;
-  if (d <= 8)
-    return launch_lauum_grad<double, 8, true>(kind, W, ldw, n, d, xs, alpha, gpart, ka, s);
-  if (d <= 16)
-    return launch_lauum_grad<double, 16, true>(kind, W, ldw, n, d, xs, alpha, gpart, ka, s);
-  if (d <= 32)
-    return launch_lauum_grad<double, 32, true>(kind, W, ldw, n, d, xs, alpha, gpart, ka, s);
-  return cudaErrorInvalidValue;
+  return lauum_dispatch<double, true>(kind, W, ldw, n, d, xs, theta, n_ls, alpha, gpart, s);
 }
 
 // ---------------------------------------------------------------------------
@@ -294,13 +321,89 @@ cudaError_t residual(int kind, int n, int d, const T* xs, const double* theta, i
   return launch_status();
 }
 
+// The residual from stored kernel values: one 64 x 64 tile (I <= J) of the
+// upper triangle per block, its row sums against alpha_J and column sums
+// against alpha_I: two multiply-adds an element instead of a kernel
+// evaluation.  part[t][i] receives what tile row/column t contributes to row i,
+// summed in order by the finishing kernel.
+constexpr int RS_T = 64;
+__global__ void __launch_bounds__(256)
+    residual_stored_kernel(int n, const double* __restrict__ A, int64_t lda,
+                           const double* __restrict__ alpha, double* __restrict__ part) {
+  __shared__ double tile[RS_T][RS_T + 1];
+  __shared__ double ai[RS_T], aj[RS_T], red[2][4][RS_T];
+  int I, J;
+  tri_index(blockIdx.x, J, I);  // I <= J
+  const int i0 = I * RS_T, j0 = J * RS_T;
+  const int c = threadIdx.x & 63, q = threadIdx.x >> 6;
+#pragma unroll
+  for (int u = 0; u < RS_T / 4; ++u) {
+    const int r = q + 4 * u, gi = i0 + r, gj = j0 + c;
+    tile[r][c] = gi < n && gj < n && gj > gi ? A[(int64_t)gi * lda + gj] : 0.0;
+  }
+  if (q == 0) ai[c] = i0 + c < n ? alpha[i0 + c] : 0.0;
+  if (q == 1) aj[c] = j0 + c < n ? alpha[j0 + c] : 0.0;
+  __syncthreads();
+  double cs = 0.0, rs = 0.0;
+#pragma unroll
+  for (int u = 0; u < RS_T / 4; ++u) {
+    const int k = q * (RS_T / 4) + u;
+    cs = fma(tile[k][c], ai[k], cs);  // column c, rows of this quarter
+    rs = fma(tile[c][k], aj[k], rs);  // row c, columns of this quarter
+  }
+  red[0][q][c] = cs;
+  red[1][q][c] = rs;
+  __syncthreads();
+  if (q >= 2) return;
+  const double v = (red[q][0][c] + red[q][1][c]) + (red[q][2][c] + red[q][3][c]);
+  if (I == J) {
+    red[q][0][c] = v;  // own slots only
+    asm volatile("bar.sync 1, 128;" ::: "memory");
+    if (q == 0 && j0 + c < n) part[(int64_t)I * n + j0 + c] = v + red[1][0][c];
+  } else if (q == 0) {
+    if (j0 + c < n) part[(int64_t)I * n + j0 + c] = v;
+  } else if (i0 + c < n) {
+    part[(int64_t)J * n + i0 + c] = v;
+  }
+}
+
+__global__ void residual_stored_finish(int kind, int n, int nt, const double* __restrict__ theta,
+                                       int n_ls, double jitter, const double* __restrict__ diff,
+                                       const double* __restrict__ alpha,
+                                       const double* __restrict__ part, double* __restrict__ r) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const double sd = theta[n_ls + 1];
+  const double kd =
+      (kval<double>(kind, 0.0, theta[n_ls], kshape<double>(kind, theta, n_ls)) + jitter) + sd * sd;
+  double s0 = 0.0, s1 = 0.0;
+  int t = 0;
+#pragma unroll 4
+  for (; t + 1 < nt; t += 2) {
+    s0 += part[(int64_t)t * n + i];
+    s1 += part[(int64_t)(t + 1) * n + i];
+  }
+  if (t < nt) s0 += part[(int64_t)t * n + i];
+  r[i] = diff[i] - fma(kd, alpha[i], s0 + s1);
+}
+
+cudaError_t residual_stored(int kind, int n, const double* A, int64_t lda, const double* theta,
+                            int n_ls, double jitter, const double* diff, const double* alpha,
+                            double* r, double* part, cudaStream_t s) {
+  if (n <= 0) return cudaSuccess;
+  const int nt = (n + RS_T - 1) / RS_T;
+  residual_stored_kernel<<<nt * (nt + 1) / 2, 256, 0, s>>>(n, A, lda, alpha, part);
+  cudaError_t e = launch_status();
+  if (e != cudaSuccess) return e;
+  residual_stored_finish<<<(int)cdiv(n, 64), 64, 0, s>>>(kind, n, nt, theta, n_ls, jitter, diff,
+                                                         alpha, part, r);
+  return launch_status();
+}
+
 template cudaError_t lauum_grad<double>(int, const double*, int64_t, int, int, const double*,
                                         const double*, int, const double*, double*, cudaStream_t);
 template cudaError_t lauum_grad<float>(int, const float*, int64_t, int, int, const float*,
                                        const double*, int, const double*, double*, cudaStream_t);
-template cudaError_t residual<double>(int, int, int, const double*, const double*, int, double,
-                                      const double*, const double*, double*, double*,
-                                      cudaStream_t);
 template cudaError_t residual<float>(int, int, int, const float*, const double*, int, double,
                                      const double*, const double*, double*, double*, cudaStream_t);
 

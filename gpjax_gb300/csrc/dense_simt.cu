@@ -95,8 +95,13 @@ cudaError_t gemm_nt(const GemmProb<T>& p, int batch, cudaStream_t s) {
   if (p.M <= 0 || p.N <= 0 || batch <= 0) return cudaSuccess;
   // float64 only: the float32 form runs many independent GPs side by side
   // (batched MLL), where total work rather than one launch's latency counts
-  if (sizeof(T) == 8 && (int64_t)gemm_tiles<T, GemmCfg<T>>(p) * batch < SIMT_SMALL_BELOW)
+  if (sizeof(T) == 8 && (int64_t)gemm_tiles<T, GemmCfg<T>>(p) * batch < SIMT_SMALL_BELOW) {
+    // tiles of 16 once four times as many 32 x 32 tiles still fit one wave (a
+    // 36 x 36 x 64 update: 27 us with 32 x 32 tiles, 9 with 16 x 16)
+    if ((int64_t)gemm_tiles<T, GemmCfgSmall<T>>(p) * batch * 4 <= SIMT_SMALL_BELOW)
+      return gemm_nt_cfg<T, GemmCfgTiny<T>>(p, batch, s);
     return gemm_nt_cfg<T, GemmCfgSmall<T>>(p, batch, s);
+  }
   return gemm_nt_cfg<T, GemmCfg<T>>(p, batch, s);
 }
 
@@ -254,7 +259,8 @@ __global__ void __launch_bounds__(128) trsm_rows_thread_kernel(T* A, int64_t lda
 constexpr int FX_NB = 64;
 constexpr int FX_G = 8;  // columns factored between updates of the rest
 __global__ void __launch_bounds__(256)
-    potrf_diag_fixed_kernel(double* A, int64_t lda, int n, int k0, double* logdiag, int* info) {
+    potrf_diag_fixed_kernel(double* A, int64_t lda, int n, int k0, double* logdiag, int* info,
+                            int keep_upper) {
   using namespace fx;
   __shared__ long long S[FX_NB][FX_NB + 1];
   __shared__ Limbs lim[FX_G][FX_NB];
@@ -355,7 +361,7 @@ __global__ void __launch_bounds__(256)
 #pragma unroll 4
   for (int u = 0; u < FX_NB * FX_NB / 256; ++u) {
     const int e = threadIdx.x + u * 256, r = e >> 6, c = e & 63;
-    if (r < nb && c < nb)
+    if (r < nb && c < nb && !(keep_upper && c > r))
       A[(int64_t)(k0 + r) * lda + k0 + c] =
           c > r ? 0.0 : dead ? nan : to_double(S[r][c], ex[r]);
   }
@@ -500,8 +506,8 @@ __global__ void __launch_bounds__(256)
 
 // Factor the 64 columns at o and the rows below.
 static cudaError_t potrf_block64(double* A, int64_t lda, int n, int o, double* logdiag, int* info,
-                                 cudaStream_t s) {
-  potrf_diag_fixed_kernel<<<1, 256, 0, s>>>(A, lda, n, o, logdiag, info);
+                                 bool keep_upper, cudaStream_t s) {
+  potrf_diag_fixed_kernel<<<1, 256, 0, s>>>(A, lda, n, o, logdiag, info, keep_upper);
   cudaError_t e = launch_status();
   const int rest = n - o - FX_NB;
   if (e != cudaSuccess || rest <= 0) return e;
@@ -513,7 +519,7 @@ static cudaError_t potrf_block64(double* A, int64_t lda, int n, int o, double* l
 
 template <typename T>
 cudaError_t potrf_lower(T* A, int64_t lda, int n, double* logdiag, int* info, double* dtrack,
-                        bool zero_upper, cudaStream_t s) {
+                        bool zero_upper, cudaStream_t s, bool keep_upper) {
   constexpr int NB = Blk<T>::NB;
   constexpr bool f64 = sizeof(T) == 8;
   const size_t smem_diag = (size_t)(NB * (NB + 1) + 3 * NB) * sizeof(T) + 2 * NB * sizeof(double);
@@ -534,7 +540,7 @@ cudaError_t potrf_lower(T* A, int64_t lda, int n, double* logdiag, int* info, do
     cudaError_t e;
     if constexpr (f64) {
       // its own diagonal supplies the pivots: no float64 track beside it
-      e = potrf_block64(A, lda, n, k0, logdiag, info, s);
+      e = potrf_block64(A, lda, n, k0, logdiag, info, keep_upper, s);
       if (e != cudaSuccess) return e;
       if (rest <= 0) break;
     } else {
@@ -574,12 +580,12 @@ cudaError_t potrf_lower(T* A, int64_t lda, int n, double* logdiag, int* info, do
 // tensor-core form wants; the right-looking order above rewrites the whole
 // trailing matrix once per 64 columns.
 static cudaError_t potrf_rec(double* A, int64_t lda, int n, int o, int w, double* logdiag,
-                             int* info, const XRoom& x, cudaStream_t s) {
+                             int* info, bool keep_upper, const XRoom& x, cudaStream_t s) {
   constexpr int NB = Blk<double>::NB;
-  if (w <= NB) return potrf_block64(A, lda, n, o, logdiag, info, s);
+  if (w <= NB) return potrf_block64(A, lda, n, o, logdiag, info, keep_upper, s);
   int h = NB;
   while (2 * h < w) h *= 2;
-  cudaError_t e = potrf_rec(A, lda, n, o, h, logdiag, info, x, s);
+  cudaError_t e = potrf_rec(A, lda, n, o, h, logdiag, info, keep_upper, x, s);
   if (e != cudaSuccess) return e;
   GemmProb<double> p{};
   p.A = p.B = A + (int64_t)(o + h) * lda + o;
@@ -593,20 +599,20 @@ static cudaError_t potrf_rec(double* A, int64_t lda, int n, int o, int w, double
   p.beta = 1.0;
   e = gemm_nt_x(p, 1, x, s);
   if (e != cudaSuccess) return e;
-  return potrf_rec(A, lda, n, o + h, w - h, logdiag, info, x, s);
+  return potrf_rec(A, lda, n, o + h, w - h, logdiag, info, keep_upper, x, s);
 }
 
 cudaError_t potrf_lower_x(double* A, int64_t lda, int n, double* logdiag, int* info,
-                          bool zero_upper, const XRoom& x, cudaStream_t s) {
+                          bool zero_upper, const XRoom& x, cudaStream_t s, bool keep_upper) {
   // without room for digit planes every product is a CUDA-core one
-  if (!x.bytes) return potrf_lower<double>(A, lda, n, logdiag, info, nullptr, zero_upper, s);
+  if (!x.bytes) return potrf_lower<double>(A, lda, n, logdiag, info, nullptr, zero_upper, s, keep_upper);
   constexpr int NB = Blk<double>::NB;
   if (zero_upper && n > NB) {
     zero_upper_kernel<double><<<(int)cdiv((int64_t)n * n, 256), 256, 0, s>>>(A, lda, n, NB);
     cudaError_t e = launch_status();
     if (e != cudaSuccess) return e;
   }
-  return potrf_rec(A, lda, n, 0, n, logdiag, info, x, s);
+  return potrf_rec(A, lda, n, 0, n, logdiag, info, keep_upper, x, s);
 }
 
 // ---------------------------------------------------------------------------
@@ -655,6 +661,54 @@ __global__ void __launch_bounds__(NB) trtri_diag_kernel(const T* L, int64_t ldl,
     int i = e / nb, j = e % nb;
     M[(int64_t)(k0 + i) * ldm + k0 + j] = Ms[i * LD + j];
     V[(int64_t)(k0 + i) * ldv + k0 + j] = Ms[j * LD + i];
+  }
+}
+
+// The float64 leaf: right-looking forward substitution on the identity, all
+// threads on every step (row k final, the rows below lose L[i, k] / L[k, k]
+// times it).  One thread per column, as above, is a chain of dependent
+// products: 130 us; this one issues each product once: TRTRI64_US.
+template <int NB>
+__global__ void __launch_bounds__(256)
+    trtri_diag64_kernel(const double* L, int64_t ldl, int n, double* M, int64_t ldm, double* V,
+                        int64_t ldv) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  constexpr int LD = NB + 1;
+  double* Ls = reinterpret_cast<double*>(smem_raw);
+  double* Ms = Ls + NB * LD;
+  double* ri = Ms + NB * LD;  // 1 / L[i, i]
+  const int k0 = blockIdx.x * NB;
+  const int nb = min(NB, n - k0);
+#pragma unroll 8
+  for (int u = 0; u < NB * NB / 256; ++u) {
+    const int e = threadIdx.x + u * 256, i = e / NB, j = e % NB;
+    Ls[i * LD + j] = (i < nb && j <= i) ? L[(int64_t)(k0 + i) * ldl + k0 + j] : 0.0;
+    Ms[i * LD + j] = i == j ? 1.0 : 0.0;
+  }
+  __syncthreads();
+  if (threadIdx.x < nb) ri[threadIdx.x] = 1.0 / Ls[threadIdx.x * LD + threadIdx.x];
+  __syncthreads();
+  for (int e = threadIdx.x; e < NB * NB; e += 256) {
+    const int i = e / NB, j = e % NB;
+    if (j < i && i < nb) Ls[i * LD + j] *= ri[j];
+  }
+  __syncthreads();
+  for (int k = 0; k + 1 < nb; ++k) {
+    const int w = k + 1, total = (nb - w) * w;
+    const float inv = 1.f / (float)w;
+    for (int e = threadIdx.x; e < total; e += 256) {
+      const int r = (int)(((float)e + 0.5f) * inv);  // e / w
+      const int i = w + r, c = e - r * w;
+      Ms[i * LD + c] = fma(-Ls[i * LD + k], Ms[k * LD + c], Ms[i * LD + c]);
+    }
+    __syncthreads();
+  }
+#pragma unroll 4
+  for (int u = 0; u < NB * NB / 256; ++u) {
+    const int e = threadIdx.x + u * 256, i = e / NB, j = e % NB;
+    if (i >= nb || j >= nb) continue;
+    M[(int64_t)(k0 + i) * ldm + k0 + j] = Ms[i * LD + j] * ri[i];
+    V[(int64_t)(k0 + i) * ldv + k0 + j] = Ms[j * LD + i] * ri[j];
   }
 }
 
@@ -712,10 +766,16 @@ cudaError_t trtri_lower(const T* L, int64_t ldl, int n, T* M, int64_t ldm, T* V,
                         T* scratch, const XRoom& x, cudaStream_t s) {
   constexpr int NB = Blk<T>::NB;
   const size_t smem = (size_t)(2 * NB * (NB + 1) + NB) * sizeof(T);
-  cudaFuncSetAttribute(trtri_diag_kernel<T, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)smem);
   const int nblk = (n + NB - 1) / NB;
-  trtri_diag_kernel<T, NB><<<nblk, NB, smem, s>>>(L, ldl, n, M, ldm, V, ldv);
+  if constexpr (sizeof(T) == 8) {
+    cudaFuncSetAttribute(trtri_diag64_kernel<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)smem);
+    trtri_diag64_kernel<NB><<<nblk, 256, smem, s>>>(L, ldl, n, M, ldm, V, ldv);
+  } else {
+    cudaFuncSetAttribute(trtri_diag_kernel<T, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)smem);
+    trtri_diag_kernel<T, NB><<<nblk, NB, smem, s>>>(L, ldl, n, M, ldm, V, ldv);
+  }
   cudaError_t e = launch_status();
   if (e != cudaSuccess) return e;
   for (int b = NB; b < n; b *= 2) {
@@ -793,7 +853,7 @@ cudaError_t gemv_dense(const T* A, int64_t ld, int rows, int cols, const double*
 #define GPK_INST(T)                                                                             \
   template cudaError_t gemm_nt<T>(const GemmProb<T>&, int, cudaStream_t);                       \
   template cudaError_t potrf_lower<T>(T*, int64_t, int, double*, int*, double*, bool,          \
-                                      cudaStream_t);                                            \
+                                      cudaStream_t, bool);                                           \
   template cudaError_t trtri_lower<T>(const T*, int64_t, int, T*, int64_t, T*, int64_t, T*,     \
                                       const XRoom&, cudaStream_t);                                            \
   template cudaError_t gemv_tri<T>(const T*, int64_t, int, bool, const double*, double*, double, \

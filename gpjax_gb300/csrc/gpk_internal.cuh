@@ -38,10 +38,12 @@ cudaError_t gemm_nt(const GemmProb<T>& p, int batch, cudaStream_t s);
 // dtrack (may be null; float32 only): float64 copy of diag(A) that is kept up
 // to date through the factorisation and supplies the pivots, so the diagonal
 // never accumulates rounding of the working precision.  zero_upper clears the
-// strict upper triangle outside the diagonal blocks first.
+// strict upper triangle outside the diagonal blocks first; keep_upper
+// (float64) leaves the diagonal blocks' own upper triangles as they are instead
+// of zeroing them.
 template <typename T>
 cudaError_t potrf_lower(T* A, int64_t lda, int n, double* logdiag, int* info, double* dtrack,
-                        bool zero_upper, cudaStream_t s);
+                        bool zero_upper, cudaStream_t s, bool keep_upper = false);
 
 // Workspace for the digit planes of float64 products on the tensor cores
 // (xgemm.cuh); bytes = 0: none, every float64 product runs on the CUDA cores.
@@ -53,7 +55,8 @@ struct XRoom {
 // The float64 factor with products on the tensor cores where x has room
 // (potrf_lower<double> otherwise).
 cudaError_t potrf_lower_x(double* A, int64_t lda, int n, double* logdiag, int* info,
-                          bool zero_upper, const XRoom& x, cudaStream_t s);
+                          bool zero_upper, const XRoom& x, cudaStream_t s,
+                          bool keep_upper = false);
 
 // M = L^-1 (lower, row-major) and V = L^-T (upper, row-major) from the factor L.
 // scratch: n*n/2 elements of T.
@@ -80,7 +83,8 @@ cudaError_t scale_inputs(const double* x, int64_t ldx, int n, int d, const doubl
 
 // Gram/cross-covariance from scaled inputs.  mode 0: out = K(xs, ys) full;
 // mode 1: lower triangle of (K(xs, xs) + jitter I) + obs_stddev^2 I with zeros
-// above the diagonal; mode 2: the same without the noise term.
+// above the diagonal; mode 2: the same without the noise term; mode 3: mode 1
+// with the kernel values above the diagonal (for residual_stored).
 template <typename T, typename TO>
 cudaError_t cross_cov_scaled(int kind, int n, int m, int d, const T* xs, const T* ys,
                              const double* theta, int n_ls, int mode, double diag_add, TO* out,
@@ -111,6 +115,11 @@ cudaError_t residual(int kind, int n, int d, const T* xs, const double* theta, i
                      double jitter, const double* diff, const double* alpha, double* r,
                      double* rpart, cudaStream_t s);
 size_t residual_scratch_doubles(int n);
+// The same from the kernel values of mode 3 that the factorisation left above
+// A's diagonal; part holds n * ceil(n / 64) doubles (trtri_lower's scratch does).
+cudaError_t residual_stored(int kind, int n, const double* A, int64_t lda, const double* theta,
+                            int n_ls, double jitter, const double* diff, const double* alpha,
+                            double* r, double* part, cudaStream_t s);
 // Scratch (doubles) of the multi-block MLL finalisation.
 size_t mll_finalize_scratch_doubles(int d);
 

@@ -10,6 +10,7 @@
 // 64-row panel of each side in shared memory and every thread produces a
 // column strip of the output tile.
 #include "gpk_internal.cuh"
+#include "simt_tile.cuh"
 
 namespace gpk {
 
@@ -34,13 +35,14 @@ cudaError_t scale_inputs(const double* x, int64_t ldx, int n, int d, const doubl
 
 constexpr int GT = 64;  // output tile edge
 
-template <typename T, typename TO>
+// D bounds the input dimension (coordinates past d are zero and add nothing).
+template <typename T, typename TO, int D>
 __global__ void __launch_bounds__(256)
     cross_cov_kernel(int kind, int n, int m, int d, const T* __restrict__ xs,
                      const T* __restrict__ ys, const double* __restrict__ theta, int n_ls, int mode,
                      double jitter, TO* __restrict__ out, int64_t ldo) {
-  __shared__ T sx[GT][GPK_MAX_D + 1];
-  __shared__ T sy[GT][GPK_MAX_D + 1];
+  __shared__ T sx[GT][D + 1];
+  __shared__ T sy[GT][D + 1];
   const int i0 = blockIdx.y * GT, j0 = blockIdx.x * GT;
   const T s2 = (T)theta[n_ls];
   const double sd = theta[n_ls + 1];
@@ -52,19 +54,19 @@ __global__ void __launch_bounds__(256)
     }
     return;
   }
-  for (int e = threadIdx.x; e < GT * d; e += blockDim.x) {
-    int r = e / d, k = e % d;
-    sx[r][k] = (i0 + r < n) ? xs[(int64_t)(i0 + r) * d + k] : T(0);
-    sy[r][k] = (j0 + r < m) ? ys[(int64_t)(j0 + r) * d + k] : T(0);
+  for (int e = threadIdx.x; e < GT * D; e += blockDim.x) {
+    int r = e / D, k = e % D;
+    sx[r][k] = (i0 + r < n && k < d) ? xs[(int64_t)(i0 + r) * d + k] : T(0);
+    sy[r][k] = (j0 + r < m && k < d) ? ys[(int64_t)(j0 + r) * d + k] : T(0);
   }
   __syncthreads();
   const int c = threadIdx.x % GT;
   const int rbase = threadIdx.x / GT;  // 0..3
   const int gj = j0 + c;
   if (gj >= m) return;
-  T yv[GPK_MAX_D];
+  T yv[D];
 #pragma unroll
-  for (int k = 0; k < GPK_MAX_D; ++k) yv[k] = (k < d) ? sy[c][k] : T(0);
+  for (int k = 0; k < D; ++k) yv[k] = sy[c][k];
   for (int r = rbase; r < GT; r += 4) {
     const int gi = i0 + r;
     if (gi >= n) break;
@@ -74,11 +76,9 @@ __global__ void __launch_bounds__(256)
     } else {
       T sq = T(0);
 #pragma unroll
-      for (int k = 0; k < GPK_MAX_D; ++k) {
-        if (k < d) {
-          T df = sx[r][k] - yv[k];
-          sq = fma(df, df, sq);
-        }
+      for (int k = 0; k < D; ++k) {
+        T df = sx[r][k] - yv[k];
+        sq = fma(df, df, sq);
       }
       T kv = kval<T>(kind, sq, s2, kshape<T>(kind, theta, n_ls));
       if (mode == 1 && gi == gj) {
@@ -95,15 +95,88 @@ __global__ void __launch_bounds__(256)
   }
 }
 
+// Mode 3, float64: Sigma's lower triangle and the kernel values above it, one
+// TE x TE tile (I >= J) per block, evaluated once and stored twice (the second
+// time transposed through shared memory).  TE = 32 below n = 1536: with 64 the
+// float64 work of a small matrix sits in too few blocks.
+template <int D, int TE>
+__global__ void __launch_bounds__(256)
+    gram_sym_kernel(int kind, int n, int d, const double* __restrict__ xs,
+                    const double* __restrict__ theta, int n_ls, double jitter,
+                    double* __restrict__ out, int64_t ldo) {
+  __shared__ double sx[TE][D + 1], sy[TE][D + 1];
+  __shared__ double st[TE][TE + 1];
+  int I, J;
+  tri_index(blockIdx.x, I, J);
+  const int i0 = I * TE, j0 = J * TE;
+  const double s2 = theta[n_ls], sd = theta[n_ls + 1], ka = kshape<double>(kind, theta, n_ls);
+  for (int e = threadIdx.x; e < TE * D; e += 256) {
+    const int r = e / D, k = e % D;
+    sx[r][k] = (i0 + r < n && k < d) ? xs[(int64_t)(i0 + r) * d + k] : 0.0;
+    sy[r][k] = (j0 + r < n && k < d) ? xs[(int64_t)(j0 + r) * d + k] : 0.0;
+  }
+  __syncthreads();
+  const int c = threadIdx.x % TE, gj = j0 + c;
+  double yv[D];
+#pragma unroll
+  for (int k = 0; k < D; ++k) yv[k] = sy[c][k];
+  for (int r = threadIdx.x / TE; r < TE; r += 256 / TE) {
+    const int gi = i0 + r;
+    if (gi >= n || gj > gi) continue;
+    double sq = 0.0;
+#pragma unroll
+    for (int k = 0; k < D; ++k) {
+      const double df = sx[r][k] - yv[k];
+      sq = fma(df, df, sq);
+    }
+    const double kv = kval<double>(kind, sq, s2, ka);
+    st[r][c] = kv;
+    out[(int64_t)gi * ldo + gj] = gi == gj ? (kv + jitter) + sd * sd : kv;
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < TE * TE; e += 256) {
+    const int rr = e / TE, cc = e % TE;  // element (i0 + cc, j0 + rr) at (j0 + rr, i0 + cc)
+    if (i0 + cc < n && j0 + rr < i0 + cc) out[(int64_t)(j0 + rr) * ldo + i0 + cc] = st[cc][rr];
+  }
+}
+
 template <typename T, typename TO>
 cudaError_t cross_cov_scaled(int kind, int n, int m, int d, const T* xs, const T* ys,
                              const double* theta, int n_ls, int mode, double jitter, TO* out,
                              int64_t ldo, cudaStream_t s) {
   if (n <= 0 || m <= 0) return cudaSuccess;
   if (d > GPK_MAX_D) return cudaErrorInvalidValue;
+  if constexpr (sizeof(T) == 8) {
+    if (mode == 3) {
+      auto sym = [&](auto dim) {
+        constexpr int D = decltype(dim)::value;
+        constexpr int BIG = D <= 8 ? 64 : 32;  // 64 with D > 8 exceeds static shared memory
+        const int te = n < 1536 ? 32 : BIG, nt = (n + te - 1) / te;
+        auto* k = te == 32 ? gram_sym_kernel<D, 32> : gram_sym_kernel<D, BIG>;
+        k<<<nt * (nt + 1) / 2, 256, 0, s>>>(kind, n, d, xs, theta, n_ls, jitter, out, ldo);
+      };
+      if (d <= 4)
+        sym(std::integral_constant<int, 4>{});
+      else if (d <= 8)
+        sym(std::integral_constant<int, 8>{});
+      else if (d <= 16)
+        sym(std::integral_constant<int, 16>{});
+      else
+        sym(std::integral_constant<int, 32>{});
+      return launch_status();
+    }
+  }
   dim3 grid((unsigned)cdiv(m, GT), (unsigned)cdiv(n, GT));
-  cross_cov_kernel<T, TO><<<grid, 256, 0, s>>>(kind, n, m, d, xs, ys, theta, n_ls, mode, jitter,
-                                               out, ldo);
+  auto run = [&](auto dim) {
+    cross_cov_kernel<T, TO, decltype(dim)::value><<<grid, 256, 0, s>>>(
+        kind, n, m, d, xs, ys, theta, n_ls, mode, jitter, out, ldo);
+  };
+  if (d <= 8)
+    run(std::integral_constant<int, 8>{});
+  else if (d <= 16)
+    run(std::integral_constant<int, 16>{});
+  else
+    run(std::integral_constant<int, 32>{});
   return launch_status();
 }
 

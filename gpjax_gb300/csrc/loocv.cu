@@ -33,7 +33,7 @@ namespace {
 struct LoocvBuffers {
   int64_t ld;
   double *A, *M, *V, *W, *scratch, *xs;
-  double *diff, *z, *alpha, *r, *logdiag, *dtrack, *rpart, *a, *sa, *b, *u, *red, *gth;
+  double *diff, *z, *alpha, *r, *logdiag, *a, *sa, *b, *u, *red, *gth;
   void* vjp_ws;
   size_t vjp_bytes;
   XRoom x;  // digit planes
@@ -56,9 +56,8 @@ size_t loocv_layout(int64_t n, int d, void* ws, LoocvBuffers& b) {
   b.W = (double*)take(nn);  // Sigma^-1
   b.scratch = (double*)take(((size_t)n * n / 2 + 64) * 8);
   b.xs = (double*)take((size_t)n * d * 8);
-  double** vecs[] = {&b.diff, &b.z, &b.alpha, &b.r, &b.logdiag, &b.dtrack, &b.a, &b.sa, &b.b, &b.u};
+  double** vecs[] = {&b.diff, &b.z, &b.alpha, &b.r, &b.logdiag, &b.a, &b.sa, &b.b, &b.u};
   for (double** v : vecs) *v = (double*)take((size_t)n * 8);
-  b.rpart = (double*)take(residual_scratch_doubles((int)n) * 8);
   b.red = (double*)take(8 * 8);
   b.gth = (double*)take((size_t)(GPK_MAX_D + 8) * 8);
   b.vjp_bytes = gpk_cross_covariance_vjp_workspace_bytes(n, n, d);
@@ -187,16 +186,15 @@ extern "C" gpk_status gpk_conjugate_loocv(int kind, int64_t n, int d, const doub
   loocv_diff_kernel<<<g1, 256, 0, s>>>(nn, y, theta, n_ls, b.diff);
   GPK_LAUNCH_CHECK();
   // Sigma = K + (jitter + obs_stddev^2) I (objectives.py:160-165), its factor and inverse
-  GPK_CUDA_TRY(cross_cov_scaled<double, double>(kind, nn, nn, d, b.xs, b.xs, theta, n_ls, 1,
+  GPK_CUDA_TRY(cross_cov_scaled<double, double>(kind, nn, nn, d, b.xs, b.xs, theta, n_ls, 3,
                                                 jitter, b.A, ld, s));
-  GPK_CUDA_TRY(sigma_diag_init(kind, nn, theta, n_ls, jitter, b.dtrack, s));
-  GPK_CUDA_TRY(potrf_lower_x(b.A, ld, nn, b.logdiag, info, false, b.x, s));
+  GPK_CUDA_TRY(potrf_lower_x(b.A, ld, nn, b.logdiag, info, false, b.x, s, true));
   GPK_CUDA_TRY(trtri_lower<double>(b.A, ld, nn, b.M, ld, b.V, ld, b.scratch, b.x, s));
   // alpha = Sigma^-1 (y - m) (objectives.py:167), refined once
   GPK_CUDA_TRY(gemv_tri<double>(b.M, ld, nn, true, b.diff, b.z, 1.0, false, s));
   GPK_CUDA_TRY(gemv_tri<double>(b.V, ld, nn, false, b.z, b.alpha, 1.0, false, s));
-  GPK_CUDA_TRY(residual<double>(kind, nn, d, b.xs, theta, n_ls, jitter, b.diff, b.alpha, b.r,
-                                b.rpart, s));
+  GPK_CUDA_TRY(residual_stored(kind, nn, b.A, ld, theta, n_ls, jitter, b.diff, b.alpha, b.r,
+                               b.scratch, s));
   GPK_CUDA_TRY(gemv_tri<double>(b.M, ld, nn, true, b.r, b.z, 1.0, false, s));
   GPK_CUDA_TRY(gemv_tri<double>(b.V, ld, nn, false, b.z, b.alpha, 1.0, true, s));
   // W = Sigma^-1 = L^-T L^-1 = V V^T (objectives.py:168)

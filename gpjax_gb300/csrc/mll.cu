@@ -161,34 +161,43 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-__global__ void mll_finalize_combine_kernel(int n, int d, const double* __restrict__ theta,
-                                            int n_ls, const double* __restrict__ part,
-                                            int want_grad, double jitter, int* __restrict__ info,
-                                            double* __restrict__ out_mll,
-                                            double* __restrict__ out_grad) {
-  if (threadIdx.x != 0) return;
-  const int stride = 6 + d + 2;
-  double tot[3], comp[3];
-  for (int q = 0; q < 3; ++q) {
-    tot[q] = 0.0;
-    comp[q] = 0.0;
-    for (int b = 0; b < FIN_BLOCKS; ++b) {
-      const double v = part[(int64_t)b * stride + 2 * q];
-      const double t = tot[q] + v;
-      comp[q] += part[(int64_t)b * stride + 2 * q + 1] +
-                 ((fabs(tot[q]) >= fabs(v)) ? (tot[q] - t) + v : (v - t) + tot[q]);
-      tot[q] = t;
+// One warp per quantity: the three compensated sums and the gradient slots
+// over the FIN_BLOCKS partials (one thread adding them all in turn took 77 us
+// of float64 latency).
+__global__ void __launch_bounds__(256)
+    mll_finalize_combine_kernel(int n, int d, const double* __restrict__ theta, int n_ls,
+                                const double* __restrict__ part, int want_grad, double jitter,
+                                int* __restrict__ info, double* __restrict__ out_mll,
+                                double* __restrict__ out_grad) {
+  const int stride = 6 + d + 2, w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  __shared__ double tot[3], sg[GPK_MAX_D + 2];
+  for (int q = w; q < 3 + (want_grad ? d + 2 : 0); q += 8) {
+    if (q < 3) {
+      double sum = 0.0, c = 0.0;
+      auto add = [&](double v, double vc) {
+        const double t = sum + v;
+        c += vc + ((fabs(sum) >= fabs(v)) ? (sum - t) + v : (v - t) + sum);
+        sum = t;
+      };
+      for (int b = l; b < FIN_BLOCKS; b += 32)
+        add(part[(int64_t)b * stride + 2 * q], part[(int64_t)b * stride + 2 * q + 1]);
+      for (int o = 16; o > 0; o >>= 1) {
+        const double os = __shfl_xor_sync(0xffffffffu, sum, o);
+        const double oc = __shfl_xor_sync(0xffffffffu, c, o);
+        add(os, oc);
+      }
+      if (l == 0) tot[q] = sum + c;
+    } else {
+      double acc = 0.0;
+      for (int b = l; b < FIN_BLOCKS; b += 32) acc += part[(int64_t)b * stride + 6 + q - 3];
+      acc = warp_sum(acc);
+      if (l == 0) sg[q - 3] = acc;
     }
   }
-  double sg[GPK_MAX_D + 2];
-  for (int sl = 0; sl < d + 2; ++sl) {
-    double acc = 0.0;
-    if (want_grad)
-      for (int b = 0; b < FIN_BLOCKS; ++b) acc += part[(int64_t)b * stride + 6 + sl];
-    sg[sl] = acc;
-  }
-  finalize_outputs(n, d, theta, n_ls, jitter, 2.0 * (tot[0] + comp[0]), tot[1] + comp[1],
-                   tot[2] + comp[2], sg, want_grad, info, out_mll, out_grad);
+  __syncthreads();
+  if (threadIdx.x != 0) return;
+  finalize_outputs(n, d, theta, n_ls, jitter, 2.0 * tot[0], tot[1], tot[2], sg, want_grad, info,
+                   out_mll, out_grad);
 }
 
 size_t mll_finalize_scratch_doubles(int d) { return (size_t)FIN_BLOCKS * (6 + d + 2); }
@@ -207,7 +216,7 @@ cudaError_t mll_finalize_launch(int n, int d, const double* theta, int n_ls, con
                                                          want_grad, scratch);
   cudaError_t e = launch_status();
   if (e != cudaSuccess) return e;
-  mll_finalize_combine_kernel<<<1, 32, 0, s>>>(n, d, theta, n_ls, scratch, want_grad, jitter, info,
+  mll_finalize_combine_kernel<<<1, 256, 0, s>>>(n, d, theta, n_ls, scratch, want_grad, jitter, info,
                                                out_mll, out_grad);
   return launch_status();
 }
@@ -236,12 +245,13 @@ static gpk_status mll_run(int kind, int n, int d, const double* x, int64_t ldx, 
   GPK_CUDA_TRY(scale_inputs<T>(x, ldx, n, d, theta, n_ls, b.xs, s));
   diff_kernel<<<(int)cdiv(n, 256), 256, 0, s>>>(n, y, theta, n_ls, b.diff);
   GPK_LAUNCH_CHECK();
-  GPK_CUDA_TRY(cross_cov_scaled<T, T>(kind, n, n, d, b.xs, b.xs, theta, n_ls, 1, jitter, b.A,
-                                      b.ld, s));
-  GPK_CUDA_TRY(sigma_diag_init(kind, n, theta, n_ls, jitter, b.dtrack, s));
+  constexpr bool f64 = sizeof(T) == 8;
+  GPK_CUDA_TRY(cross_cov_scaled<T, T>(kind, n, n, d, b.xs, b.xs, theta, n_ls, f64 ? 3 : 1, jitter,
+                                      b.A, b.ld, s));
+  if (!f64) GPK_CUDA_TRY(sigma_diag_init(kind, n, theta, n_ls, jitter, b.dtrack, s));
   prof_mark(1, s);
-  if constexpr (sizeof(T) == 8)
-    GPK_CUDA_TRY(potrf_lower_x(b.A, b.ld, n, b.logdiag, info, false, b.x, s));
+  if constexpr (f64)
+    GPK_CUDA_TRY(potrf_lower_x(b.A, b.ld, n, b.logdiag, info, false, b.x, s, true));
   else
     GPK_CUDA_TRY(potrf_lower<T>(b.A, b.ld, n, b.logdiag, info, b.dtrack, false, s));
   prof_mark(2, s);
@@ -250,8 +260,12 @@ static gpk_status mll_run(int kind, int n, int d, const double* x, int64_t ldx, 
   GPK_CUDA_TRY(gemv_tri<T>(b.M, b.ld, n, true, b.diff, b.z, 1.0, false, s));
   GPK_CUDA_TRY(gemv_tri<T>(b.V, b.ld, n, false, b.z, b.alpha, 1.0, false, s));
   for (int it = 0; it < refine; ++it) {
-    GPK_CUDA_TRY(residual<T>(kind, n, d, b.xs, theta, n_ls, jitter, b.diff, b.alpha, b.r, b.rpart,
-                             s));
+    if constexpr (f64)
+      GPK_CUDA_TRY(residual_stored(kind, n, b.A, b.ld, theta, n_ls, jitter, b.diff, b.alpha, b.r,
+                                   b.scratch, s));
+    else
+      GPK_CUDA_TRY(residual<T>(kind, n, d, b.xs, theta, n_ls, jitter, b.diff, b.alpha, b.r,
+                               b.rpart, s));
     GPK_CUDA_TRY(gemv_tri<T>(b.M, b.ld, n, true, b.r, b.z, 1.0, false, s));
     GPK_CUDA_TRY(gemv_tri<T>(b.V, b.ld, n, false, b.z, b.alpha, 1.0, true, s));
   }
@@ -259,7 +273,7 @@ static gpk_status mll_run(int kind, int n, int d, const double* x, int64_t ldx, 
   if (want_grad && b.x.bytes) {
     // the factor and M are done with: their arrays (adjacent) take V's digit
     // planes, scratch and the room after it W
-    if constexpr (sizeof(T) == 8) {
+    if constexpr (f64) {
       const XRoom planes{b.A, (size_t)(reinterpret_cast<char*>(b.V) - reinterpret_cast<char*>(b.A))};
       GPK_CUDA_TRY(lauum_grad_x(kind, b.V, b.ld, n, d, b.xs, theta, n_ls, b.alpha, b.gpart,
                                 b.scratch, b.ld, planes, s));

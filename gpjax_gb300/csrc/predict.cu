@@ -160,19 +160,24 @@ gpk_status predict_run(int kind, int n, int t, int d, const double* x, int64_t l
   GPK_CUDA_TRY(scale_inputs<double>(xt, ldxt, t, d, theta, n_ls, b.tsd, s));
   pred_diff_kernel<<<(int)cdiv(n, 256), 256, 0, s>>>(n, y, theta, n_ls, b.diff);
   GPK_LAUNCH_CHECK();
-  GPK_CUDA_TRY(cross_cov_scaled<T, T>(kind, n, n, d, b.xs, b.xs, theta, n_ls, 1, jitter, b.A,
-                                      b.ld, s));
-  GPK_CUDA_TRY(sigma_diag_init(kind, n, theta, n_ls, jitter, b.dtrack, s));
-  if constexpr (sizeof(T) == 8)
-    GPK_CUDA_TRY(potrf_lower_x(b.A, b.ld, n, b.logdiag, info, false, b.x, s));
+  constexpr bool f64 = sizeof(T) == 8;
+  GPK_CUDA_TRY(cross_cov_scaled<T, T>(kind, n, n, d, b.xs, b.xs, theta, n_ls, f64 ? 3 : 1, jitter,
+                                      b.A, b.ld, s));
+  if (!f64) GPK_CUDA_TRY(sigma_diag_init(kind, n, theta, n_ls, jitter, b.dtrack, s));
+  if constexpr (f64)
+    GPK_CUDA_TRY(potrf_lower_x(b.A, b.ld, n, b.logdiag, info, false, b.x, s, true));
   else
     GPK_CUDA_TRY(potrf_lower<T>(b.A, b.ld, n, b.logdiag, info, b.dtrack, false, s));
   GPK_CUDA_TRY(trtri_lower<T>(b.A, b.ld, n, b.M, b.ld, b.V, b.ld, b.scratch, b.x, s));
   GPK_CUDA_TRY(gemv_tri<T>(b.M, b.ld, n, true, b.diff, b.z, 1.0, false, s));
   GPK_CUDA_TRY(gemv_tri<T>(b.V, b.ld, n, false, b.z, b.alpha, 1.0, false, s));
   for (int it = 0; it < refine; ++it) {
-    GPK_CUDA_TRY(residual<T>(kind, n, d, b.xs, theta, n_ls, jitter, b.diff, b.alpha, b.r, b.rpart,
-                             s));
+    if constexpr (f64)
+      GPK_CUDA_TRY(residual_stored(kind, n, b.A, b.ld, theta, n_ls, jitter, b.diff, b.alpha, b.r,
+                                   b.scratch, s));
+    else
+      GPK_CUDA_TRY(residual<T>(kind, n, d, b.xs, theta, n_ls, jitter, b.diff, b.alpha, b.r,
+                               b.rpart, s));
     GPK_CUDA_TRY(gemv_tri<T>(b.M, b.ld, n, true, b.r, b.z, 1.0, false, s));
     GPK_CUDA_TRY(gemv_tri<T>(b.V, b.ld, n, false, b.z, b.alpha, 1.0, true, s));
   }

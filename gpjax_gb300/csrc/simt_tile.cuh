@@ -19,6 +19,11 @@ template <typename T> struct GemmCfgSmall;
 template <> struct GemmCfgSmall<double> {
   static constexpr int BM = 32, BN = 32, BK = 16, TM = 2, TN = 2;
 };
+// One output per thread: problems of a few blocks (n <= 128), where even the
+// 32 x 32 tiles leave most SMs idle.
+template <typename T> struct GemmCfgTiny {
+  static constexpr int BM = 16, BN = 16, BK = 32, TM = 1, TN = 1;
+};
 template <> struct GemmCfgSmall<float> {
   static constexpr int BM = 64, BN = 64, BK = 16, TM = 4, TN = 4;
 };
