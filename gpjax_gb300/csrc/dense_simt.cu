@@ -250,27 +250,35 @@ __global__ void __launch_bounds__(128) trsm_rows_thread_kernel(T* A, int64_t lda
 // ---------------------------------------------------------------------------
 // Float64 form of both, in fixed point (fixed64.cuh).
 //
-// The diagonal block: thread (row i, column group g), right-looking.  Columns
-// go eight at a time; the columns to the right of a group take its eight
-// together, so that their 64-bit sums are shifted into place once per eight
-// products.  The chain of 64 pivots bounds it (a reciprocal root takes about
-// 310 clocks, a scaled entry 125, a product and its difference 53).
+// The diagonal block: thread (row i, column group g), right-looking, in groups
+// of eight columns.  The chain of 64 pivots bounds it (a reciprocal root takes
+// about 290 clocks, a scaled entry 145, a product and its difference 110, a
+// barrier 50): one group of threads runs the chain, the other seven apply each
+// column to the rest of its group and, one column a step, the group before to
+// the columns further right, so that nothing but the next group's own columns
+// is waited for between groups.  (A single warp holding a whole group in
+// registers needs no barriers but then issues every product itself: 65 us
+// against 40.)
 // ---------------------------------------------------------------------------
 constexpr int FX_NB = 64;
-constexpr int FX_G = 8;  // columns factored between updates of the rest
-__global__ void __launch_bounds__(256)
+constexpr int FX_G = 8;     // columns of a group, and groups of threads
+constexpr int FX_NT = 512;  // threads: 64 rows x 8
+constexpr int FX_EL = FX_NB * FX_NB / FX_NT;
+__global__ void __launch_bounds__(FX_NT)
     potrf_diag_fixed_kernel(double* A, int64_t lda, int n, int k0, double* logdiag, int* info,
                             int keep_upper) {
   using namespace fx;
+  pdl_wait();
+  pdl_trigger();
   __shared__ long long S[FX_NB][FX_NB + 1];
-  __shared__ Limbs lim[FX_G][FX_NB];
+  __shared__ Limbs lim[2][FX_G][FX_NB];  // this group's columns and the last one's
   __shared__ int ex[FX_NB], sbad[FX_NB], sdead;
   const int nb = min(FX_NB, n - k0);
   const int i = threadIdx.x & 63, g = threadIdx.x >> 6;
-  double av[FX_NB * FX_NB / 256];  // every load in flight at once
+  double av[FX_EL];  // every load in flight at once
 #pragma unroll
-  for (int u = 0; u < FX_NB * FX_NB / 256; ++u) {
-    const int e = threadIdx.x + u * 256, r = e >> 6, c = e & 63;
+  for (int u = 0; u < FX_EL; ++u) {
+    const int e = threadIdx.x + u * FX_NT, r = e >> 6, c = e & 63;
     av[u] = r < nb && c <= r ? A[(int64_t)(k0 + r) * lda + k0 + c] : 0.0;
   }
   if (threadIdx.x < FX_NB) {
@@ -280,18 +288,27 @@ __global__ void __launch_bounds__(256)
   }
   __syncthreads();
 #pragma unroll
-  for (int u = 0; u < FX_NB * FX_NB / 256; ++u) {
-    const int e = threadIdx.x + u * 256, r = e >> 6, c = e & 63;
+  for (int u = 0; u < FX_EL; ++u) {
+    const int e = threadIdx.x + u * FX_NT, r = e >> 6, c = e & 63;
     bool bad = false;
     S[r][c] = r < nb || r != c ? to_fixed(av[u], ex[r] + ex[c], bad) : ONE;  // identity past nb
     if (bad) sbad[r] = 1;
   }
   __syncthreads();
-  // step j: the first 64 threads bring column j up to date with column j - 1
-  // and scale it by its pivot's reciprocal root (each thread derives the pivot
-  // itself); the others meanwhile apply column j - 1 to the group's columns
-  // after j.  One barrier per column.
-  for (int c0 = 0; c0 < FX_NB; c0 += FX_G) {
+  // column k loses the eight columns of a group
+  auto update = [&](const Limbs (&l)[FX_G][FX_NB], int k) {
+    if (k >= nb || i < k) return;
+    Acc a0, a1;
+#pragma unroll
+    for (int q = 0; q < FX_G; q += 2) {
+      a0.add(l[q][i], l[q][k]);
+      a1.add(l[q + 1][i], l[q + 1][k]);
+    }
+    S[i][k] -= a0.value() + a1.value();
+  };
+  for (int c0 = 0; c0 < nb; c0 += FX_G) {
+    Limbs(&cur)[FX_G][FX_NB] = lim[(c0 / FX_G) & 1];
+    Limbs(&prev)[FX_G][FX_NB] = lim[((c0 / FX_G) & 1) ^ 1];
     Limbs lv{0, 0};  // this row's entry of the previous column (first 64 threads)
 #pragma unroll
     for (int q = 0; q < FX_G; ++q) {
@@ -300,7 +317,7 @@ __global__ void __launch_bounds__(256)
         long long t = S[i][j], d = S[j][j];
         const int jbad = sbad[j];
         if (q > 0) {
-          const Limbs w = lim[q - 1][j];
+          const Limbs w = cur[q - 1][j];
           Acc at, ad;
           at.add(lv, w);
           ad.add(w, w);
@@ -314,73 +331,62 @@ __global__ void __launch_bounds__(256)
         bool bad = false;
         const long long v = times_rsqrt(i >= j ? t : 0, y, s, bad);
         lv = limbs(v);
-        lim[q][i] = lv;
+        cur[q][i] = lv;
         if (bad) sbad[i] = 1;
         if (!good && i == j) {  // the rest of this group's columns mean nothing
           atomicMin(info, k0 + j + 1);
           sdead = 1;
         }
-      } else if (q > 0) {
-        const Limbs mine = lim[q - 1][i];
-#pragma unroll
-        for (int h = 0; h < (FX_G - q + 1) / 3; ++h) {
-          const int k = j + g + 3 * h;
-          if (k >= c0 + FX_G || i < k) continue;
-          Acc acc;
-          acc.add(mine, lim[q - 1][k]);
-          S[i][k] -= acc.value();
+      } else {
+        if (q > 0) {
+          const int k = j + g;  // the group's columns after j
+          if (k < c0 + FX_G && i >= k) {
+            Acc acc;
+            acc.add(cur[q - 1][i], cur[q - 1][k]);
+            S[i][k] -= acc.value();
+          }
         }
+        if (c0 > 0) update(prev, c0 + FX_G + q * (FX_G - 1) + g - 1);
       }
       __syncthreads();
     }
     if (sdead) break;
-    if (c0 + FX_G < nb) {
-      Limbs lq[FX_G];
-#pragma unroll
-      for (int q = 0; q < FX_G; ++q) lq[q] = lim[q][i];
-      for (int k = c0 + FX_G + g; k < nb; k += 4) {
-        if (i < k) continue;
-        Acc acc;
-#pragma unroll
-        for (int q = 0; q < FX_G; ++q) acc.add(lq[q], lim[q][k]);
-        S[i][k] -= acc.value();
-      }
-    }
-#pragma unroll
-    for (int h = 0; h < FX_G / 4; ++h) {
-      const Limbs l = lim[g + 4 * h][i];
-      S[i][c0 + g + 4 * h] = ((long long)l.h << 32) + l.l;
-    }
+    update(cur, c0 + FX_G + g);  // the next group's columns
+    const Limbs l = cur[g][i];
+    S[i][c0 + g] = ((long long)l.h << 32) + l.l;
     __syncthreads();
   }
   const bool dead = sdead != 0;  // a pivot failed
   const double nan = __longlong_as_double(0x7ff8000000000000ULL);
-  __syncthreads();
-  if (logdiag && threadIdx.x < nb)
-    logdiag[k0 + i] = dead ? nan : log(to_double(S[i][i], ex[i]));
 #pragma unroll 4
-  for (int u = 0; u < FX_NB * FX_NB / 256; ++u) {
-    const int e = threadIdx.x + u * 256, r = e >> 6, c = e & 63;
+  for (int u = 0; u < FX_EL; ++u) {
+    const int e = threadIdx.x + u * FX_NT, r = e >> 6, c = e & 63;
     if (r < nb && c < nb && !(keep_upper && c > r))
       A[(int64_t)(k0 + r) * lda + k0 + c] =
           c > r ? 0.0 : dead ? nan : to_double(S[r][c], ex[r]);
   }
+  if (logdiag && threadIdx.x < nb)
+    logdiag[k0 + i] = dead ? nan : log(to_double(S[i][i], ex[i]));
 }
 
-// Panel solve X L^T = A for 32 rows per CTA: lane = row; one warp substitutes
-// a group of four columns, then the eight warps split the columns to the
-// right.  A row's scale comes from its own
-// diagonal entry, which bounds every entry of the factor's row; a column's
-// from the norm of that row of L.
+// Panel solve X L^T = A for 32 rows per CTA: lane = row.  One warp substitutes
+// a group of four columns while the others apply the group before it to the
+// columns further right; only the next group's four columns are brought up to
+// date in between.  A row's scale comes from its own diagonal entry, which
+// bounds every entry of the factor's row; a column's from the norm of that row
+// of L.
 constexpr int FX_ROWS = 32;
 constexpr int FX_XLD = FX_NB + 1;
-constexpr int FX_TG = 4;  // columns substituted between updates of the rest
+constexpr int FX_TG = 4;  // columns of a group
+constexpr int FX_TW = FX_NT / 32;
 constexpr size_t FX_TRSM_SMEM = (size_t)FX_NB * FX_NB * sizeof(fx::Limbs) +
                                 (size_t)FX_ROWS * FX_XLD * 8 + (size_t)FX_NB * 16 +
-                                FX_ROWS * 8 + (size_t)FX_TG * FX_ROWS * sizeof(fx::Limbs);
-__global__ void __launch_bounds__(256)
-    trsm_rows_fixed_kernel(double* A, int64_t lda, int n, int k0) {
+                                FX_ROWS * 8 + (size_t)2 * FX_TG * FX_ROWS * sizeof(fx::Limbs);
+__global__ void __launch_bounds__(FX_NT)
+    trsm_rows_fixed_kernel(double* A, int64_t lda, int n, int k0, XSplit planes) {
   using namespace fx;
+  pdl_wait();
+  pdl_trigger();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   Limbs* L = reinterpret_cast<Limbs*>(smem_raw);                   // [64][64], row j of L
   long long* X = reinterpret_cast<long long*>(L + FX_NB * FX_NB);  // [32][65]
@@ -389,25 +395,31 @@ __global__ void __launch_bounds__(256)
   int* ej = rs + FX_NB;
   int* ei = ej + FX_NB;
   int* sbad = ei + FX_ROWS;
-  Limbs* LX = reinterpret_cast<Limbs*>(sbad + FX_ROWS);            // [FX_TG][32]
+  Limbs* LX = reinterpret_cast<Limbs*>(sbad + FX_ROWS);            // [2][FX_TG][32]
   const int lane = threadIdx.x & 31, g = threadIdx.x >> 5;
   const int r0 = k0 + FX_NB + blockIdx.x * FX_ROWS, rows = min(FX_ROWS, n - r0);
-  double av[FX_ROWS * FX_NB / 256], lv[2 * FX_NB / 8];  // every load in flight at once
+  constexpr int XE = FX_ROWS * FX_NB / FX_NT, LE = FX_NB / FX_TW;
+  double av[XE], lv[2 * LE];  // every load in flight at once
 #pragma unroll
-  for (int u = 0; u < FX_NB / 8; ++u)
+  for (int u = 0; u < LE; ++u)
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      const int j = g + 8 * u, k = lane + 32 * h;
+      const int j = g + FX_TW * u, k = lane + 32 * h;
       lv[2 * u + h] = k <= j ? A[(int64_t)(k0 + j) * lda + k0 + k] : 0.0;
     }
 #pragma unroll
-  for (int u = 0; u < FX_ROWS * FX_NB / 256; ++u) {
-    const int e = threadIdx.x + u * 256, r = e >> 6, c = e & 63;
+  for (int u = 0; u < XE; ++u) {
+    const int e = threadIdx.x + u * FX_NT, r = e >> 6, c = e & 63;
     av[u] = r < rows ? A[(int64_t)(r0 + r) * lda + k0 + c] : 0.0;
   }
+  if (threadIdx.x < FX_ROWS) {
+    const int r = r0 + threadIdx.x;
+    ei[threadIdx.x] = threadIdx.x < rows ? scale_of(A[(int64_t)r * lda + r]) : 0;
+    sbad[threadIdx.x] = 0;
+  }
 #pragma unroll
-  for (int u = 0; u < FX_NB / 8; ++u) {
-    const int j = g + 8 * u;
+  for (int u = 0; u < LE; ++u) {
+    const int j = g + FX_TW * u;
     const double* a = lv + 2 * u;
     int xb[2], xm = 1;
 #pragma unroll
@@ -431,89 +443,126 @@ __global__ void __launch_bounds__(256)
     const int e = xm - 1022 + ((x2 + 1) >> 1);
     bool bad = false;  // a NaN of a failed block: its rows' results are not read
 #pragma unroll
-    for (int h = 0; h < 2; ++h) L[j * FX_NB + lane + 32 * h] = limbs(to_fixed(a[h], e, bad));
+    for (int h = 0; h < 2; ++h) {
+      L[j * FX_NB + lane + 32 * h] = limbs(to_fixed(a[h], e, bad));
+      if (lane + 32 * h == j) ry[j] = __double_as_longlong(a[h]);
+    }
     if (lane == 0) ej[j] = e;
-  }
-  if (threadIdx.x < FX_ROWS) {
-    const int r = r0 + threadIdx.x;
-    ei[threadIdx.x] = threadIdx.x < rows ? scale_of(A[(int64_t)r * lda + r]) : 0;
-    sbad[threadIdx.x] = 0;
   }
   __syncthreads();
   if (threadIdx.x < FX_NB) {
     const int j = threadIdx.x;
-    const unsigned long long b = (unsigned long long)__double_as_longlong(
-        1.0 / A[(int64_t)(k0 + j) * lda + k0 + j]);
-    ry[j] = (long long)((b & 0xfffffffffffffULL) | (1ULL << 52)) << 9;  // [1, 2) 2^61
-    rs[j] = -((int)((b >> 52) & 0x7ff) - 1023 + ej[j]);
-    if (((b >> 52) & 0x7ff) == 0x7ff || rs[j] < -58 || rs[j] > 1) {  // a failed block
-      ry[j] = 0;
-      rs[j] = 0;
-    }
+    const unsigned long long b =
+        (unsigned long long)__double_as_longlong(1.0 / __longlong_as_double(ry[j]));
+    const int x = (int)((b >> 52) & 0x7ff), s = -(x - 1023 + ej[j]);
+    const bool ok = x != 0x7ff && s >= -58 && s <= 1;  // not a failed block
+    ry[j] = ok ? (long long)((b & 0xfffffffffffffULL) | (1ULL << 52)) << 9 : 0;
+    rs[j] = ok ? s : 0;  // [1, 2) 2^61 and its shift
   }
 #pragma unroll
-  for (int u = 0; u < FX_ROWS * FX_NB / 256; ++u) {
-    const int e = threadIdx.x + u * 256, r = e >> 6, c = e & 63;
+  for (int u = 0; u < XE; ++u) {
+    const int e = threadIdx.x + u * FX_NT, r = e >> 6, c = e & 63;
     bool bad = false;
     X[r * FX_XLD + c] = to_fixed(av[u], ei[r] + ej[c], bad);
     if (bad) sbad[r] = 1;
   }
   __syncthreads();
   long long* x = X + lane * FX_XLD;
-  for (int c0 = 0; c0 < FX_NB; c0 += FX_TG) {
-    if (g == 0) {
-      long long t[FX_TG];
-      bool bad = false;
+  auto solve = [&](int c0) {  // one warp: the group's four columns
+    Limbs* out = LX + ((c0 / FX_TG) & 1) * FX_TG * FX_ROWS;
+    long long t[FX_TG];
+    bool bad = false;
 #pragma unroll
-      for (int q = 0; q < FX_TG; ++q) t[q] = x[c0 + q];
+    for (int q = 0; q < FX_TG; ++q) t[q] = x[c0 + q];
 #pragma unroll
-      for (int q = 0; q < FX_TG; ++q) {
-        t[q] = times_rsqrt(t[q], ry[c0 + q], rs[c0 + q], bad);
-        const Limbs l = limbs(t[q]);
-        LX[q * FX_ROWS + lane] = l;
+    for (int q = 0; q < FX_TG; ++q) {
+      t[q] = times_rsqrt(t[q], ry[c0 + q], rs[c0 + q], bad);
+      const Limbs l = limbs(t[q]);
+      out[q * FX_ROWS + lane] = l;
 #pragma unroll
-        for (int u = q + 1; u < FX_TG; ++u) {
-          Acc acc;
-          acc.add(l, L[(c0 + u) * FX_NB + c0 + q]);
-          t[u] -= acc.value();
-        }
+      for (int u = q + 1; u < FX_TG; ++u) {
+        Acc acc;
+        acc.add(l, L[(c0 + u) * FX_NB + c0 + q]);
+        t[u] -= acc.value();
       }
-#pragma unroll
-      for (int q = 0; q < FX_TG; ++q) x[c0 + q] = t[q];
-      if (bad) sbad[lane] = 1;
     }
-    __syncthreads();
-    if (c0 + FX_TG == FX_NB) break;
+#pragma unroll
+    for (int q = 0; q < FX_TG; ++q) x[c0 + q] = t[q];
+    if (bad) sbad[lane] = 1;
+  };
+  auto update = [&](const Limbs (&lx)[FX_TG], int c0, int k) {  // column k loses the group at c0
+    Acc acc;
+#pragma unroll
+    for (int q = 0; q < FX_TG; ++q) acc.add(lx[q], L[k * FX_NB + c0 + q]);
+    x[k] -= acc.value();
+  };
+  if (g == 0) solve(0);
+  __syncthreads();
+  for (int c0 = 0; c0 + FX_TG < FX_NB; c0 += FX_TG) {
+    const Limbs* in = LX + ((c0 / FX_TG) & 1) * FX_TG * FX_ROWS;
     Limbs lx[FX_TG];
 #pragma unroll
-    for (int q = 0; q < FX_TG; ++q) lx[q] = LX[q * FX_ROWS + lane];
-    for (int k = c0 + FX_TG + g; k < FX_NB; k += 8) {
-      Acc acc;
-#pragma unroll
-      for (int q = 0; q < FX_TG; ++q) acc.add(lx[q], L[k * FX_NB + c0 + q]);
-      x[k] -= acc.value();
-    }
+    for (int q = 0; q < FX_TG; ++q) lx[q] = in[q * FX_ROWS + lane];
+    if (g < FX_TG) update(lx, c0, c0 + FX_TG + g);  // the next group's columns
+    __syncthreads();
+    if (g == 0)
+      solve(c0 + FX_TG);
+    else
+      for (int k = c0 + 2 * FX_TG + g - 1; k < FX_NB; k += FX_TW - 1) update(lx, c0, k);
     __syncthreads();
   }
   const double nan = __longlong_as_double(0x7ff8000000000000ULL);
-  for (int e = threadIdx.x; e < FX_ROWS * FX_NB; e += 256) {
-    const int r = e >> 6, c = e & 63;
+#pragma unroll
+  for (int u = 0; u < XE; ++u) {
+    const int e = threadIdx.x + u * FX_NT, r = e >> 6, c = e & 63;
     if (r < rows)
       A[(int64_t)(r0 + r) * lda + k0 + c] =
           sbad[r] ? nan : to_double(X[r * FX_XLD + c], ei[r]);
   }
+  // the panel's digit planes for the products that read it, at the row scale of
+  // the first panel (updates only lower a diagonal entry and with it the scale)
+  if (planes.planes) {
+    const int r = threadIdx.x >> 4, c = (threadIdx.x & 15) * 4;
+    if (r < rows) {
+      int* expo = planes.expo + r0 + r;
+      const int e0 = k0 == 0 ? ei[r] : *expo - 1022;
+      const bool ok = !sbad[r] && ei[r] <= e0;
+      const int sh = min(62, FRAC - 55 + (ok ? e0 - ei[r] : 0));
+      long long q[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) q[u] = (X[r * FX_XLD + c + u] + (1LL << (sh - 1))) >> sh;
+      x_store_digits4(q,
+                      static_cast<__half*>(planes.planes) + (int64_t)(r0 + r) * planes.ldk + k0 + c,
+                      (int64_t)planes.rows * planes.ldk);
+      __syncwarp();  // the row's 16 lanes have read its exponent
+      if (c == 0 && (k0 == 0 || !ok)) *expo = ok ? e0 + 1022 : XNAN;
+    }
+  }
 }
 
-// Factor the 64 columns at o and the rows below.
+// Factor the 64 columns at o and the rows below (and the rows' digit planes,
+// where there are any).  The kernels start while their predecessor drains.
 static cudaError_t potrf_block64(double* A, int64_t lda, int n, int o, double* logdiag, int* info,
-                                 bool keep_upper, cudaStream_t s) {
-  potrf_diag_fixed_kernel<<<1, 256, 0, s>>>(A, lda, n, o, logdiag, info, keep_upper);
+                                 bool keep_upper, const XSplit& planes, cudaStream_t s) {
+  const PdlAttr attr(o > 0);  // the first follows whatever the caller did before
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(1);
+  cfg.blockDim = dim3(FX_NT);
+  cfg.stream = s;
+  cfg.attrs = const_cast<cudaLaunchAttribute*>(attr.a);
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, potrf_diag_fixed_kernel, A, lda, n, o, logdiag, info,
+                     (int)keep_upper);
   cudaError_t e = launch_status();
   const int rest = n - o - FX_NB;
   if (e != cudaSuccess || rest <= 0) return e;
   cudaFuncSetAttribute(trsm_rows_fixed_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)FX_TRSM_SMEM);
-  trsm_rows_fixed_kernel<<<(rest + FX_ROWS - 1) / FX_ROWS, 256, FX_TRSM_SMEM, s>>>(A, lda, n, o);
+  const PdlAttr pdl(true);
+  cfg.gridDim = dim3((rest + FX_ROWS - 1) / FX_ROWS);
+  cfg.dynamicSmemBytes = FX_TRSM_SMEM;
+  cfg.attrs = const_cast<cudaLaunchAttribute*>(pdl.a);
+  cudaLaunchKernelEx(&cfg, trsm_rows_fixed_kernel, A, lda, n, o, planes);
   return launch_status();
 }
 
@@ -540,7 +589,7 @@ cudaError_t potrf_lower(T* A, int64_t lda, int n, double* logdiag, int* info, do
     cudaError_t e;
     if constexpr (f64) {
       // its own diagonal supplies the pivots: no float64 track beside it
-      e = potrf_block64(A, lda, n, k0, logdiag, info, keep_upper, s);
+      e = potrf_block64(A, lda, n, k0, logdiag, info, keep_upper, XSplit{}, s);
       if (e != cudaSuccess) return e;
       if (rest <= 0) break;
     } else {
@@ -578,41 +627,45 @@ cudaError_t potrf_lower(T* A, int64_t lda, int n, double* logdiag, int* info, do
 // half, one product that brings the right half up to date, the right half.
 // The products grow with the recursion (K up to n / 2), which is what their
 // tensor-core form wants; the right-looking order above rewrites the whole
-// trailing matrix once per 64 columns.
+// trailing matrix once per 64 columns.  They read the digit planes that the
+// panel solves wrote: splitting the operands anew cost 5 to 13 us a product.
 static cudaError_t potrf_rec(double* A, int64_t lda, int n, int o, int w, double* logdiag,
-                             int* info, bool keep_upper, const XRoom& x, cudaStream_t s) {
+                             int* info, bool keep_upper, const XSplit& planes, cudaStream_t s) {
   constexpr int NB = Blk<double>::NB;
-  if (w <= NB) return potrf_block64(A, lda, n, o, logdiag, info, keep_upper, s);
+  if (w <= NB) return potrf_block64(A, lda, n, o, logdiag, info, keep_upper, planes, s);
   int h = NB;
   while (2 * h < w) h *= 2;
-  cudaError_t e = potrf_rec(A, lda, n, o, h, logdiag, info, keep_upper, x, s);
+  cudaError_t e = potrf_rec(A, lda, n, o, h, logdiag, info, keep_upper, planes, s);
   if (e != cudaSuccess) return e;
   GemmProb<double> p{};
-  p.A = p.B = A + (int64_t)(o + h) * lda + o;
   p.C = A + (int64_t)(o + h) * lda + o + h;
-  p.lda = p.ldb = p.ldc = lda;
+  p.ldc = lda;
   p.M = n - o - h;
   p.N = w - h;
   p.K = h;
   p.c_lower = 1;
   p.alpha = -1.0;
   p.beta = 1.0;
-  e = gemm_nt_x(p, 1, x, s);
+  XSplit x = planes;
+  x.row0 = o + h;
+  x.col0 = o;
+  e = xgemm_run(p, x, x, 1, s, true);
   if (e != cudaSuccess) return e;
-  return potrf_rec(A, lda, n, o + h, w - h, logdiag, info, keep_upper, x, s);
+  return potrf_rec(A, lda, n, o + h, w - h, logdiag, info, keep_upper, planes, s);
 }
 
 cudaError_t potrf_lower_x(double* A, int64_t lda, int n, double* logdiag, int* info,
-                          bool zero_upper, const XRoom& x, cudaStream_t s, bool keep_upper) {
+                          bool zero_upper, const XRoom& planes, cudaStream_t s, bool keep_upper) {
   // without room for digit planes every product is a CUDA-core one
-  if (!x.bytes) return potrf_lower<double>(A, lda, n, logdiag, info, nullptr, zero_upper, s, keep_upper);
+  if (planes.bytes < xsplit_bytes(n, n))
+    return potrf_lower<double>(A, lda, n, logdiag, info, nullptr, zero_upper, s, keep_upper);
   constexpr int NB = Blk<double>::NB;
   if (zero_upper && n > NB) {
     zero_upper_kernel<double><<<(int)cdiv((int64_t)n * n, 256), 256, 0, s>>>(A, lda, n, NB);
     cudaError_t e = launch_status();
     if (e != cudaSuccess) return e;
   }
-  return potrf_rec(A, lda, n, 0, n, logdiag, info, keep_upper, x, s);
+  return potrf_rec(A, lda, n, 0, n, logdiag, info, keep_upper, xsplit_at(planes.mem, n, n), s);
 }
 
 // ---------------------------------------------------------------------------

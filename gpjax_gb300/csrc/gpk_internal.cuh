@@ -52,11 +52,18 @@ struct XRoom {
   size_t bytes = 0;
 };
 
-// The float64 factor with products on the tensor cores where x has room
-// (potrf_lower<double> otherwise).
+// The float64 factor with products on the tensor cores where `planes` holds the
+// digit planes of an n x n operand (potrf_lower<double> otherwise).
 cudaError_t potrf_lower_x(double* A, int64_t lda, int n, double* logdiag, int* info,
-                          bool zero_upper, const XRoom& x, cudaStream_t s,
+                          bool zero_upper, const XRoom& planes, cudaStream_t s,
                           bool keep_upper = false);
+// The arrays [from, to) as room for the factor's planes: M and V, adjacent in
+// every layout, are written only after it.  None where the size runs on the
+// CUDA cores.
+inline XRoom planes_in(const XRoom& x, double* from, double* to) {
+  if (!x.bytes) return XRoom();
+  return XRoom{from, (size_t)(reinterpret_cast<char*>(to) - reinterpret_cast<char*>(from))};
+}
 
 // M = L^-1 (lower, row-major) and V = L^-T (upper, row-major) from the factor L.
 // scratch: n*n/2 elements of T.

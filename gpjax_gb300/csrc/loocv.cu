@@ -188,7 +188,8 @@ extern "C" gpk_status gpk_conjugate_loocv(int kind, int64_t n, int d, const doub
   // Sigma = K + (jitter + obs_stddev^2) I (objectives.py:160-165), its factor and inverse
   GPK_CUDA_TRY(cross_cov_scaled<double, double>(kind, nn, nn, d, b.xs, b.xs, theta, n_ls, 3,
                                                 jitter, b.A, ld, s));
-  GPK_CUDA_TRY(potrf_lower_x(b.A, ld, nn, b.logdiag, info, false, b.x, s, true));
+  GPK_CUDA_TRY(potrf_lower_x(b.A, ld, nn, b.logdiag, info, false, planes_in(b.x, b.M, b.W),
+                             s, true));
   GPK_CUDA_TRY(trtri_lower<double>(b.A, ld, nn, b.M, ld, b.V, ld, b.scratch, b.x, s));
   // alpha = Sigma^-1 (y - m) (objectives.py:167), refined once
   GPK_CUDA_TRY(gemv_tri<double>(b.M, ld, nn, true, b.diff, b.z, 1.0, false, s));

@@ -251,7 +251,8 @@ static gpk_status mll_run(int kind, int n, int d, const double* x, int64_t ldx, 
   if (!f64) GPK_CUDA_TRY(sigma_diag_init(kind, n, theta, n_ls, jitter, b.dtrack, s));
   prof_mark(1, s);
   if constexpr (f64)
-    GPK_CUDA_TRY(potrf_lower_x(b.A, b.ld, n, b.logdiag, info, false, b.x, s, true));
+    GPK_CUDA_TRY(potrf_lower_x(b.A, b.ld, n, b.logdiag, info, false,
+                               planes_in(b.x, b.M, b.scratch), s, true));
   else
     GPK_CUDA_TRY(potrf_lower<T>(b.A, b.ld, n, b.logdiag, info, b.dtrack, false, s));
   prof_mark(2, s);
@@ -274,7 +275,7 @@ static gpk_status mll_run(int kind, int n, int d, const double* x, int64_t ldx, 
     // the factor and M are done with: their arrays (adjacent) take V's digit
     // planes, scratch and the room after it W
     if constexpr (f64) {
-      const XRoom planes{b.A, (size_t)(reinterpret_cast<char*>(b.V) - reinterpret_cast<char*>(b.A))};
+      const XRoom planes = planes_in(b.x, b.A, b.V);
       GPK_CUDA_TRY(lauum_grad_x(kind, b.V, b.ld, n, d, b.xs, theta, n_ls, b.alpha, b.gpart,
                                 b.scratch, b.ld, planes, s));
     }

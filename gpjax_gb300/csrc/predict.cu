@@ -165,7 +165,8 @@ gpk_status predict_run(int kind, int n, int t, int d, const double* x, int64_t l
                                       b.A, b.ld, s));
   if (!f64) GPK_CUDA_TRY(sigma_diag_init(kind, n, theta, n_ls, jitter, b.dtrack, s));
   if constexpr (f64)
-    GPK_CUDA_TRY(potrf_lower_x(b.A, b.ld, n, b.logdiag, info, false, b.x, s, true));
+    GPK_CUDA_TRY(potrf_lower_x(b.A, b.ld, n, b.logdiag, info, false,
+                               planes_in(b.x, b.M, b.scratch), s, true));
   else
     GPK_CUDA_TRY(potrf_lower<T>(b.A, b.ld, n, b.logdiag, info, b.dtrack, false, s));
   GPK_CUDA_TRY(trtri_lower<T>(b.A, b.ld, n, b.M, b.ld, b.V, b.ld, b.scratch, b.x, s));

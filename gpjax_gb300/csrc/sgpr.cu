@@ -770,7 +770,8 @@ gpk_status sgpr_run(int kind, int n, int m, int d, const double* x, int64_t ldx,
                                                 b.Kf, ldm, ss));
   GPK_CUDA_TRY(cross_cov_scaled<double, double>(kind, m, m, d, b.zs64, b.zs64, theta, n_ls, 2,
                                                 jitter, b.Lz, ldm, ss));
-  GPK_CUDA_TRY(potrf_lower_x(b.Lz, ldm, m, b.ldK, info, false, b.xk, ss));
+  GPK_CUDA_TRY(potrf_lower_x(b.Lz, ldm, m, b.ldK, info, false,
+                             planes_in(b.xk, b.Mz, b.Kinv), ss));
   GPK_CUDA_TRY(trtri_lower<double>(b.Lz, ldm, m, b.Mz, ldm, b.Vz, ldm, b.scr, b.xk, ss));
   {
     GemmProb<double> p{};
@@ -871,7 +872,8 @@ gpk_status sgpr_run(int kind, int n, int m, int d, const double* x, int64_t ldx,
                                                          b.Su);
     GPK_LAUNCH_CHECK();
   }
-  GPK_CUDA_TRY(potrf_lower_x(b.Su, ldm, m, b.ldU, info, true, b.xu, s));
+  GPK_CUDA_TRY(potrf_lower_x(b.Su, ldm, m, b.ldU, info, true, planes_in(b.xu, b.Mu, b.Suinv),
+                             s));
   GPK_CUDA_TRY(trtri_lower<double>(b.Su, ldm, m, b.Mu, ldm, b.Vu, ldm, b.scr, b.xu, s));
   {  // Su^-1 = Vu Vu^T (lower triangle, then mirrored)
     GemmProb<double> p{};

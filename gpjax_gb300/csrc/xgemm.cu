@@ -10,7 +10,6 @@ namespace {
 
 using namespace tc;
 
-constexpr int XP = 7;             // digit planes
 constexpr int XG = 8;             // digit-sum groups p + q = 2 .. 9
 constexpr int XN = 64;            // output tile columns
 constexpr int XK = 32;            // K elements per stage (64-byte rows, 64B swizzle)
@@ -21,7 +20,6 @@ constexpr int XTHREADS = 320;     // w0 TMA, w1 MMA + TMEM, w2..w9 epilogue
 constexpr int XEPI_WARPS = 8, XEPI_THREADS = XEPI_WARPS * 32;
 constexpr int XHC = XN / 2;       // accumulator columns of one epilogue thread
 constexpr int XTLD = XN + 1;      // staged tile row stride (doubles)
-constexpr int XNAN = 0x7ff;       // row exponent of a row with a NaN or an infinity
 constexpr double XMIN_MULTS = 5e5;  // below, a CUDA-core product is as quick as the split
 constexpr int XMAX_K = 1 << 18;   // the drained 64-bit sums stay below K * 2^41
 
@@ -40,6 +38,7 @@ struct XCtl {
 
 struct XParams {
   int M, N, K, a_tri, b_tri, c_lower, tiles_m, tiles_n;
+  int a_row0, a_col0, b_row0, b_col0;  // origins inside the tensor maps
   const int* ea;
   const int* eb;
   double *C, *Ct;
@@ -142,8 +141,9 @@ __global__ void __launch_bounds__(XTHREADS, 1)
           break;
         uint8_t* st = ring + s * XSTAGE_BYTES;
         mbar_expect_tx(&ctl->full[s], XSTAGE_BYTES);
-        tma_load_3d(st, &ta, klo + kc * XK, z * p.M + i0, 0, &ctl->full[s]);
-        tma_load_3d(st + XP * XA_PLANE, &tb, klo + kc * XK, z * p.N + j0, 0, &ctl->full[s]);
+        tma_load_3d(st, &ta, p.a_col0 + klo + kc * XK, p.a_row0 + z * p.M + i0, 0, &ctl->full[s]);
+        tma_load_3d(st + XP * XA_PLANE, &tb, p.b_col0 + klo + kc * XK, p.b_row0 + z * p.N + j0, 0,
+                    &ctl->full[s]);
         ++issued;
       }
       for (int kc = max(0, issued - XSTAGES); kc < issued; ++kc)
@@ -336,9 +336,7 @@ __device__ __forceinline__ int x_expo(double a) {
   return x > 1 ? x : 1;
 }
 
-// The digits of four elements, one 8-byte store of float16s per plane.  An
-// integer d in [-128, 128] becomes a float16 through the bit pattern of 1536 +
-// d (unit spacing there), less 1536: no conversion instruction.
+// The digits of four float64 elements at row exponent X.
 __device__ __forceinline__ void x_digits4(const double (&a)[4], int X, __half* dst, int64_t plane) {
   long long q[4];
 #pragma unroll
@@ -350,24 +348,7 @@ __device__ __forceinline__ void x_digits4(const double (&a)[4], int X, __half* d
                                : (s < 57 ? (long long)((m + (1ULL << (s - 3))) >> (s - 2)) : 0LL);
     q[u] = (long long)b < 0 ? -v : v;
   }
-  const __half2 base = __halves2half2(__ushort_as_half(0x6600), __ushort_as_half(0x6600));
-#pragma unroll
-  for (int p = XP - 1; p >= 0; --p) {
-    int d[4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      d[u] = p ? (int)((q[u] + 128) & 255) - 128 : (int)q[u];
-      q[u] = (q[u] - d[u]) >> 8;
-    }
-    uint32_t w[2];
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const uint32_t bits = (uint32_t)(0x6600 + d[2 * h]) | ((uint32_t)(0x6600 + d[2 * h + 1]) << 16);
-      const __half2 v = __hsub2(*reinterpret_cast<const __half2*>(&bits), base);
-      w[h] = *reinterpret_cast<const uint32_t*>(&v);
-    }
-    *reinterpret_cast<uint2*>(dst + p * plane) = make_uint2(w[0], w[1]);
-  }
+  x_store_digits4(q, dst, plane);
 }
 
 // One warp per row (and, CHUNKED, per XCHUNK columns of it): the row's largest
@@ -475,7 +456,7 @@ cudaError_t xsplit_run(const double* src, int64_t ld, int64_t stride, int rows, 
 }
 
 cudaError_t xgemm_run(const GemmProb<double>& p, const XSplit& A, const XSplit& B, int batch,
-                      cudaStream_t s) {
+                      cudaStream_t s, bool pdl) {
   if (p.M <= 0 || p.N <= 0 || batch <= 0) return cudaSuccess;
   if (p.K > XMAX_K) return cudaErrorInvalidValue;
   CUtensorMap ma, mb;
@@ -489,8 +470,12 @@ cudaError_t xgemm_run(const GemmProb<double>& p, const XSplit& A, const XSplit& 
   q.c_lower = p.c_lower;
   q.tiles_m = (p.M + BM - 1) / BM;
   q.tiles_n = (p.N + XN - 1) / XN;
-  q.ea = A.expo;
-  q.eb = B.expo;
+  q.a_row0 = A.row0;
+  q.a_col0 = A.col0;
+  q.b_row0 = B.row0;
+  q.b_col0 = B.col0;
+  q.ea = A.expo + A.row0;
+  q.eb = B.expo + B.row0;
   q.C = p.C;
   q.Ct = p.Ct;
   q.ldc = p.ldc;
@@ -503,8 +488,15 @@ cudaError_t xgemm_run(const GemmProb<double>& p, const XSplit& A, const XSplit& 
   q.beta_mode = p.beta == 0.0 ? 1 : p.beta == 1.0 ? 2 : 0;
   const size_t smem = 1024 + (size_t)XSTAGES * XSTAGE_BYTES + sizeof(XCtl);
   cudaFuncSetAttribute(xgemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  const dim3 grid(tile_count(q.c_lower, q.tiles_m, q.tiles_n, XN), 1, batch);
-  xgemm_kernel<<<grid, XTHREADS, smem, s>>>(ma, mb, q);
+  const PdlAttr attr(pdl);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(tile_count(q.c_lower, q.tiles_m, q.tiles_n, XN), 1, batch);
+  cfg.blockDim = dim3(XTHREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cfg.attrs = const_cast<cudaLaunchAttribute*>(attr.a);
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, xgemm_kernel, ma, mb, q);
   return launch_status();
 }
 
@@ -529,7 +521,7 @@ cudaError_t gemm_nt_x(const GemmProb<double>& p, int batch, const XRoom& x, cuda
     e = xsplit_run(p.B, p.ldb, p.sB, p.N, p.K, p.b_tri, batch, B, s);
     if (e != cudaSuccess) return e;
   }
-  return xgemm_run(p, A, B, batch, s);
+  return xgemm_run(p, A, B, batch, s, true);  // follows a split kernel
 }
 
 size_t xroom_factor_bytes(int64_t n) {

@@ -22,6 +22,7 @@
 // instruction every 19 clocks); the 34 float16 products this takes run at
 // 4096.
 #pragma once
+#include <cuda_fp16.h>
 #include "gpk_internal.cuh"
 
 namespace gpk {
@@ -33,7 +34,35 @@ struct XSplit {
   void* planes;
   int* expo;
   int rows, K, ldk;
+  int row0 = 0, col0 = 0;  // origin of the operand inside the planes (col0 a multiple of 8)
 };
+constexpr int XP = 7;        // digit planes
+constexpr int XNAN = 0x7ff;  // row exponent of a row with a NaN or an infinity
+
+// The digits of four elements (integers of 55 fraction bits at the row's
+// scale), one 8-byte store of float16s per plane.  An integer d in [-128, 128]
+// becomes a float16 through the bit pattern of 1536 + d (unit spacing there),
+// less 1536: no conversion instruction.
+__device__ __forceinline__ void x_store_digits4(long long (&q)[4], __half* dst, int64_t plane) {
+  const __half2 base = __halves2half2(__ushort_as_half(0x6600), __ushort_as_half(0x6600));
+#pragma unroll
+  for (int p = XP - 1; p >= 0; --p) {
+    int d[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      d[u] = p ? (int)((q[u] + 128) & 255) - 128 : (int)q[u];
+      q[u] = (q[u] - d[u]) >> 8;
+    }
+    uint32_t w[2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const uint32_t bits = (uint32_t)(0x6600 + d[2 * h]) | ((uint32_t)(0x6600 + d[2 * h + 1]) << 16);
+      const __half2 v = __hsub2(*reinterpret_cast<const __half2*>(&bits), base);
+      w[h] = *reinterpret_cast<const uint32_t*>(&v);
+    }
+    *reinterpret_cast<uint2*>(dst + p * plane) = make_uint2(w[0], w[1]);
+  }
+}
 
 // Bytes of the planes and exponents of `rows` rows of K elements.
 size_t xsplit_bytes(int64_t rows, int64_t K);
@@ -48,9 +77,10 @@ cudaError_t xsplit_run(const double* src, int64_t ld, int64_t stride, int rows, 
 
 // The product of two split operands with p's shape, triangles, outputs, alpha
 // and beta (p.A, p.B and their strides are not read).  Operand rows of batch z
-// start at z * p.M in A and z * p.N in B.
+// start at z * p.M in A and z * p.N in B.  pdl: launched as a programmatic
+// dependent of the kernel before it in the stream.
 cudaError_t xgemm_run(const GemmProb<double>& p, const XSplit& A, const XSplit& B, int batch,
-                      cudaStream_t s);
+                      cudaStream_t s, bool pdl = false);
 
 // gemm_nt<double> with room for the split form: splits A and B (once when B is
 // the front of A's rows) and multiplies on the tensor cores where that is the
@@ -66,8 +96,8 @@ cudaError_t gemm_nt_room(const GemmProb<T>& p, int batch, const XRoom& x, cudaSt
     return gemm_nt<T>(p, batch, s);
 }
 
-// Room for every product of an n x n factorisation and inverse (potrf_lower_x,
-// trtri_lower), 0 for sizes whose products all run on the CUDA cores.
+// Room for every product of an n x n triangular inverse (trtri_lower), 0 for
+// sizes whose products all run on the CUDA cores.
 size_t xroom_factor_bytes(int64_t n);
 // `want` bytes of room, or 0 where a workspace of `base` bytes would grow past
 // what the card can hold beside the caller's data.
