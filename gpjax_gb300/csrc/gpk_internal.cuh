@@ -130,6 +130,14 @@ cudaError_t residual_stored(int kind, int n, const double* A, int64_t lda, const
 // Scratch (doubles) of the multi-block MLL finalisation.
 size_t mll_finalize_scratch_doubles(int d);
 
+// The cotangents of K(x, y) for G (gpk_cross_covariance_vjp); gx and gy may be
+// null, which the workspace size takes into account.
+size_t cross_cov_vjp_bytes(int64_t n, int64_t m, int d, bool need_x, bool need_y);
+cudaError_t cross_cov_vjp(int kind, int n, int m, int d, const double* x, int64_t ldx,
+                          const double* y, int64_t ldy, const double* theta, int n_ls,
+                          const double* G, int64_t ldg, double* gtheta, double* gx, double* gy,
+                          void* ws, cudaStream_t stream);
+
 // dtrack[i] = (k(x_i, x_i) + jitter) + obs_stddev^2 in float64.
 cudaError_t sigma_diag_init(int kind, int n, const double* theta, int n_ls, double jitter,
                             double* dtrack, cudaStream_t s);

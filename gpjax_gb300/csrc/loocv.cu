@@ -19,14 +19,6 @@
 #include "gpk_internal.cuh"
 #include "xgemm.cuh"
 
-extern "C" size_t gpk_cross_covariance_vjp_workspace_bytes(int64_t n, int64_t m, int d);
-extern "C" gpk_status gpk_cross_covariance_vjp(int kind, int64_t n, int64_t m, int d,
-                                               const double* x, int64_t ldx, const double* y,
-                                               int64_t ldy, const double* theta, int n_ls,
-                                               const double* G, int64_t ldg, double* grad_theta,
-                                               double* grad_x, double* grad_y, void* workspace,
-                                               size_t workspace_bytes, cudaStream_t stream);
-
 namespace gpk {
 namespace {
 
@@ -60,7 +52,7 @@ size_t loocv_layout(int64_t n, int d, void* ws, LoocvBuffers& b) {
   for (double** v : vecs) *v = (double*)take((size_t)n * 8);
   b.red = (double*)take(8 * 8);
   b.gth = (double*)take((size_t)(GPK_MAX_D + 8) * 8);
-  b.vjp_bytes = gpk_cross_covariance_vjp_workspace_bytes(n, n, d);
+  b.vjp_bytes = cross_cov_vjp_bytes(n, n, d, false, false);
   b.vjp_ws = take(b.vjp_bytes);
   b.x.bytes = xroom_fit(off, n <= 128 ? 0 : std::max(xroom_factor_bytes(n), xsplit_bytes(n, n)));
   b.x.mem = take(b.x.bytes);
@@ -231,10 +223,8 @@ extern "C" gpk_status gpk_conjugate_loocv(int kind, int64_t n, int d, const doub
     GPK_LAUNCH_CHECK();
     loocv_mirror_kernel<<<g2, 256, 0, s>>>(nn, b.A, ld);
     GPK_LAUNCH_CHECK();
-    const gpk_status st = gpk_cross_covariance_vjp(kind, n, n, d, x, ldx, x, ldx, theta, n_ls,
-                                                   b.A, ld, b.gth, nullptr, nullptr, b.vjp_ws,
-                                                   b.vjp_bytes, s);
-    if (st != GPK_OK) return st;
+    GPK_CUDA_TRY(cross_cov_vjp(kind, nn, nn, d, x, ldx, x, ldx, theta, n_ls, b.A, ld, b.gth, nullptr,
+                               nullptr, b.vjp_ws, s));
   }
   loocv_finalize_kernel<<<1, 1, 0, s>>>(n_ls, theta, b.red, b.gth, want_grad, info, out_loocv,
                                         out_grad);
