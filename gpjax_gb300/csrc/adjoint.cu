@@ -105,6 +105,7 @@ __global__ void __launch_bounds__((Cfg::BM / Cfg::TM) * (Cfg::BN / Cfg::TN))
     T sq = T(0);
 #pragma unroll
     for (int k = 0; k < DMAX; ++k) {
+      if (sizeof(T) == 8 && k >= d) continue;  // uniform: padding costs no float64 work
       const T df = sxi[r * DMAX + k] - sxj[c * DMAX + k];
       dsq[k] = df * df;
       sq += dsq[k];
@@ -114,7 +115,8 @@ __global__ void __launch_bounds__((Cfg::BM / Cfg::TM) * (Cfg::BN / Cfg::TN))
     gvar += (double)(coef * k1);
     const T cc = coef * c1;
 #pragma unroll
-    for (int k = 0; k < DMAX; ++k) gl[k] += (double)(cc * dsq[k]);
+    for (int k = 0; k < DMAX; ++k)
+      if (sizeof(T) == 4 || k < d) gl[k] += (double)(cc * dsq[k]);
     if (gi == gj) gnoise += (double)ai * (double)ai - (double)w;
   }
   // block reduction in float64, fixed order

@@ -84,29 +84,16 @@ __device__ __forceinline__ double to_double(long long v, int e) {
   return v < 0 ? -x : x;
 }
 
-// 1 / sqrt(d) of a fixed-point 0 < d as y 2^(-s - 61): a float32 seed, then
-// one correction y (1 + e/2 + 3 e^2/8) with e = 1 - d y^2 in integers (the
-// seed is good to 2^-21, what is left out is below 2^-62).
+// 1 / sqrt(d) of a fixed-point 0 < d as y 2^(-s - 61).
 __device__ __forceinline__ void rsqrt_fixed(long long d, long long& y, int& s) {
   const int lz = __clzll(d);
   unsigned long long m = (unsigned long long)d << lz;
-  int ex = 64 - FRAC - lz;  // d 2^-59 = (m / 2^64) 2^ex
+  int ex = 64 - FRAC - lz;  // d 2^-FRAC = (m / 2^64) 2^ex
   if (ex & 1) {
     m >>= 1;
     ++ex;
   }
-  float f = (float)(unsigned)(m >> 32) * 2.3283064365386963e-10f;
-  asm("rsqrt.approx.ftz.f32 %0, %0;" : "+f"(f));
-  const unsigned y0 = (unsigned)(f * 1073741824.f);
-  const unsigned long long yy = (unsigned long long)y0 * y0;              // 2^-60
-  const long long e = (1LL << 60) - (long long)__umul64hi(m, yy);         // |e| < 2^40
-  const int eh = (int)(e >> 10);
-  const long long corr = (e >> 1) + ((3 * (((long long)eh * eh) >> 40)) >> 3);
-  // y0 (1 + corr) at 2^-61, corr in two parts so that 32-bit multiplies do
-  const int ch = (int)(corr >> 20), cl = (int)(corr & 0xfffff);
-  const long long dy = (long long)((unsigned long long)y0 * (unsigned)cl >> 20) +
-                       (long long)(int)(y0 >> 1) * ch * 2 + (long long)(int)(y0 & 1) * ch;
-  y = ((long long)y0 << 31) + (dy >> 9);
+  y = (long long)rsqrt_unit(m);
   s = ex / 2;  // ex is even
 }
 

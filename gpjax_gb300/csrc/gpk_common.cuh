@@ -6,6 +6,7 @@
 #include <stdint.h>
 #include <math.h>
 #include "gpk.h"
+#include "fixed_math.cuh"
 
 #define GPK_MAX_D 32  // largest input dimension handled by the register paths
 
@@ -34,9 +35,11 @@ template <> struct Consts<float> {
   static __device__ __forceinline__ float floor_() { return 1e-36f; }
 };
 
-__device__ __forceinline__ double d_exp(double x) { return exp(x); }
+// exp of a non-positive number (every kernel's argument)
+__device__ __forceinline__ double d_exp(double x) { return fx::exp_neg(-x); }
 __device__ __forceinline__ float d_exp(float x) { return expf(x); }
-__device__ __forceinline__ double d_sqrt(double x) { return sqrt(x); }
+// sqrt of a number at or above the kernels' 1e-36 floor
+__device__ __forceinline__ double d_sqrt(double x) { return fx::sqrt_pos(x); }
 __device__ __forceinline__ float d_sqrt(float x) { return sqrtf(x); }
 __device__ __forceinline__ double d_log(double x) { return log(x); }
 __device__ __forceinline__ float d_log(float x) { return logf(x); }

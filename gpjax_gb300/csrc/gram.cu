@@ -77,6 +77,7 @@ __global__ void __launch_bounds__(256)
       T sq = T(0);
 #pragma unroll
       for (int k = 0; k < D; ++k) {
+        if (k >= d) continue;  // uniform: padding coordinates cost no float64 work
         T df = sx[r][k] - yv[k];
         sq = fma(df, df, sq);
       }
@@ -126,6 +127,7 @@ __global__ void __launch_bounds__(256)
     double sq = 0.0;
 #pragma unroll
     for (int k = 0; k < D; ++k) {
+      if (k >= d) continue;
       const double df = sx[r][k] - yv[k];
       sq = fma(df, df, sq);
     }
@@ -246,6 +248,7 @@ __global__ void __launch_bounds__(256)
     T sq = T(0);
 #pragma unroll
     for (int k = 0; k < D; ++k) {
+      if (k >= d) continue;
       const T df = sx[r][k] - yv[k];
       sq = fma(df, df, sq);
     }

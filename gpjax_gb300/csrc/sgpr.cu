@@ -552,7 +552,8 @@ __global__ void __launch_bounds__(256)
       double dz[D], sq = 0.0;
 #pragma unroll
       for (int k = 0; k < D; ++k) {
-        dz[k] = k < d ? zi[k] - xs[(int64_t)j * d + k] : 0.0;
+        if (k >= d) continue;  // uniform: padding coordinates cost no float64 work
+        dz[k] = zi[k] - xs[(int64_t)j * d + k];
         sq = fma(dz[k], dz[k], sq);
       }
       double k1, c1;
@@ -564,6 +565,7 @@ __global__ void __launch_bounds__(256)
       const double gc = g * c1;
 #pragma unroll
       for (int k = 0; k < D; ++k) {
+        if (k >= d) continue;
         const double t = gc * dz[k];
         az[k] += t;
         al[k] = fma(t, dz[k], al[k]);

@@ -106,6 +106,7 @@ __global__ void __launch_bounds__(256)
         double df[D], sq = 0.0;
 #pragma unroll
         for (int k = 0; k < D; ++k) {
+          if (k >= d) continue;  // uniform: padding coordinates cost no float64 work
           df[k] = sx[r * (D + 1) + k] - yv[k];
           sq = fma(df[k], df[k], sq);
         }
@@ -115,6 +116,7 @@ __global__ void __launch_bounds__(256)
         coef = g * c1;
 #pragma unroll
         for (int k = 0; k < D; ++k) {
+          if (k >= d) continue;
           const double v = coef * df[k];
           az[k] += v;
           al[k] = fma(v, df[k], al[k]);
@@ -134,10 +136,12 @@ __global__ void __launch_bounds__(256)
       for (int cc = sub; cc < TE; cc += PH) {
         const double coef = st[r * (TE + 4) + cc];
 #pragma unroll
-        for (int k = 0; k < D; ++k) ar[k] = fma(coef, xv[k] - sy[cc * (D + 1) + k], ar[k]);
+        for (int k = 0; k < D; ++k)
+          if (k < d) ar[k] = fma(coef, xv[k] - sy[cc * (D + 1) + k], ar[k]);
       }
 #pragma unroll
       for (int k = 0; k < D; ++k) {
+        if (k >= d) continue;
 #pragma unroll
         for (int o = 1; o < PH; o *= 2) ar[k] += __shfl_xor_sync(0xffffffffu, ar[k], o);
         if (sub == 0 && gi < n && k < d) rpart[((int64_t)J * n + gi) * d + k] = ar[k];
