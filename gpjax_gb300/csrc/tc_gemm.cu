@@ -181,56 +181,70 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
         mbar_wait_own(&ctl->full[kc % STAGES], (kc / STAGES) & 1, wlim);
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = TL::F16 ? idesc_f16(BM, BN) : idesc_tf32(BM, BN);
-      constexpr int KS = TL::KS, KP = TL::KPSEG;
-      const int nks = nk * KS;  // MMA K steps of this tile
-      bool ok = true, issued_mma = false;
-      if (p.test_stall)  // self-test: wait on a barrier nothing arrives at
-        ok = mbar_wait(&ctl->mdone, 0, abort_flag, p.err, wlim);
-      for (int kc = 0; kc < nk && ok; ++kc) {
-        const int s = kc % STAGES;
-        ok = mbar_wait(&ctl->full[s], (kc / STAGES) & 1, abort_flag, p.err, wlim);
-        if (!ok) break;
-        tc_fence_after();
-        const uint32_t sb = smem_u32(tiles + s * STAGE_BYTES);
-        const uint64_t ahi = sdesc<TL::SWZ>(sb), alo = sdesc<TL::SWZ>(sb + A_BYTES);
-        const uint64_t bhi = sdesc<TL::SWZ>(sb + 2 * A_BYTES);
-        const uint64_t blo = sdesc<TL::SWZ>(sb + 2 * A_BYTES + B_BYTES);
+    // The whole warp runs this loop and an elected lane issues: with the stage
+    // (and with it the accumulator buffer) unrolled and the tensor memory base
+    // broadcast, descriptors stay in uniform registers.  Issued from a one-lane
+    // branch, moving them there took about 80 clocks per MMA, more than the MMA
+    // itself in the narrow and half tiles (65 and 48).
+    constexpr uint32_t idesc = TL::F16 ? idesc_f16(BM, BN) : idesc_tf32(BM, BN);
+    constexpr int KS = TL::KS, KP = TL::KPSEG;
+    static_assert(KP == 1 ? KS == NBUF : STAGES * KS == NBUF * KP,
+                  "the accumulator buffer follows from the stage and K step");
+    const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
+    const bool leader = elect_one();
+    const int nks = nk * KS;  // MMA K steps of this tile
+    bool ok = true, issued_mma = false;
+    if (p.test_stall)  // self-test: wait on a barrier nothing arrives at
+      ok = __all_sync(0xffffffffu, mbar_wait(&ctl->mdone, 0, abort_flag, p.err, wlim));
+    auto slice = [&](int kc, const int s) {
+      ok = __all_sync(0xffffffffu,
+                      mbar_wait(&ctl->full[s], (kc / STAGES) & 1, abort_flag, p.err, wlim));
+      if (!ok) return;
+      tc_fence_after();
+      const uint32_t sb = smem_u32(tiles) + (uint32_t)(s * STAGE_BYTES);
+      const uint64_t ahi = sdesc<TL::SWZ>(sb), alo = sdesc<TL::SWZ>(sb + A_BYTES);
+      const uint64_t bhi = sdesc<TL::SWZ>(sb + 2 * A_BYTES);
+      const uint64_t blo = sdesc<TL::SWZ>(sb + 2 * A_BYTES + B_BYTES);
 #pragma unroll
-        for (int k4 = 0; k4 < KS; ++k4) {
-          // segment of KP K steps per TMEM accumulator buffer
-          const int ks = kc * KS + k4, seg = ks / KP, b = seg % NBUF;
-          const uint32_t tacc = tmem + (uint32_t)(b * BN);
-          const bool first = (ks % KP) == 0;
-          if (first && seg >= NBUF) {
-            ok = mbar_wait(&ctl->tempty[b], ((seg / NBUF) - 1) & 1, abort_flag, p.err, wlim);
-            if (!ok) break;
-            tc_fence_after();
-          }
-          issued_mma = true;
-          // the two cross products (about 2^-11 of the result) before the
-          // hi*hi product, so the running sum carrying them is small
-          const uint64_t off = (uint64_t)((k4 * 32) >> 4);  // 32 bytes per MMA K step
-          if (TL::F16) {
-            mma_f16(tacc, alo + off, bhi + off, idesc, first ? 0u : 1u);
-            mma_f16(tacc, ahi + off, blo + off, idesc, 1u);
-            mma_f16(tacc, ahi + off, bhi + off, idesc, 1u);
-          } else {
-            mma_tf32(tacc, alo + off, bhi + off, idesc, first ? 0u : 1u);
-            mma_tf32(tacc, ahi + off, blo + off, idesc, 1u);
-            mma_tf32(tacc, ahi + off, bhi + off, idesc, 1u);
-          }
-          if ((ks % KP) == KP - 1 || ks == nks - 1) mma_commit(&ctl->tfull[b]);
+      for (int k4 = 0; k4 < KS; ++k4) {
+        // segment of KP K steps per TMEM accumulator buffer
+        const int ks = kc * KS + k4, seg = ks / KP;
+        const int b = KP == 1 ? k4 : (s * KS + k4) / KP % NBUF;
+        const uint32_t tacc = tm + (uint32_t)(b * BN);
+        const bool first = KP == 1 || (s * KS + k4) % KP == 0;
+        if (first && seg >= NBUF) {
+          ok = __all_sync(0xffffffffu, mbar_wait(&ctl->tempty[b], ((seg / NBUF) - 1) & 1,
+                                                 abort_flag, p.err, wlim));
+          if (!ok) return;
+          tc_fence_after();
         }
-        if (!ok) break;
-        mma_commit(&ctl->empty[s]);
+        issued_mma = true;
+        if (!leader) continue;
+        // the two cross products (about 2^-11 of the result) before the
+        // hi*hi product, so the running sum carrying them is small
+        const uint64_t off = (uint64_t)((k4 * 32) >> 4);  // 32 bytes per MMA K step
+        if (TL::F16) {
+          mma_f16(tacc, alo + off, bhi + off, idesc, first ? 0u : 1u);
+          mma_f16(tacc, ahi + off, blo + off, idesc, 1u);
+          mma_f16(tacc, ahi + off, bhi + off, idesc, 1u);
+        } else {
+          mma_tf32(tacc, alo + off, bhi + off, idesc, first ? 0u : 1u);
+          mma_tf32(tacc, ahi + off, blo + off, idesc, 1u);
+          mma_tf32(tacc, ahi + off, bhi + off, idesc, 1u);
+        }
+        if (KP == 1 || (s * KS + k4) % KP == KP - 1 || ks == nks - 1) mma_commit(&ctl->tfull[b]);
       }
-      if (!ok && issued_mma) {
-        // after an abort, the MMAs already issued finish before TMEM is freed
-        mma_commit(&ctl->mdone);
-        mbar_wait_own(&ctl->mdone, 0, wlim);
-      }
+      if (leader) mma_commit(&ctl->empty[s]);
+    };
+    for (int kc0 = 0; kc0 < nk && ok; kc0 += STAGES) {
+#pragma unroll
+      for (int s = 0; s < STAGES; ++s)
+        if (ok && kc0 + s < nk) slice(kc0 + s, s);
+    }
+    if (!ok && issued_mma) {
+      // after an abort, the MMAs already issued finish before TMEM is freed
+      if (leader) mma_commit(&ctl->mdone);
+      mbar_wait_own(&ctl->mdone, 0, wlim);
     }
     __syncwarp();
   } else {
