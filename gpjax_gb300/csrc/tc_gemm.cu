@@ -423,6 +423,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
           }
         }
         if (MODE == MODE_STORE_SPLIT && p.c0) {
+#pragma unroll 4
           for (int rc = ew; rc < BM * BN / 128; rc += EPI_WARPS) {
             const int g = rc * 32 + lane, rr = g / (BN / 4), c4 = (g % (BN / 4)) * 4;
             const int grow = i0 + rr;
@@ -455,15 +456,22 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
           // transposed: output row = tile column j, lanes over tile rows i
           const int64_t trow0 = p.t_row0 + (int64_t)z * p.t_zrow + j0;
           const int64_t tcol = p.t_col0 + (int64_t)z * p.t_zcol + i0;
-          for (int cc = ew; cc < BN; cc += EPI_WARPS) {
-            if (j0 + cc >= p.N) break;
-            const int64_t base = (trow0 + cc) * p.ldt + tcol;
+          // (four columns a warp at a time: float4 reads down the rows are free
+          // of bank conflicts, single columns were read four ways into each)
+#pragma unroll 2
+          for (int cc = 4 * ew; cc < BN; cc += 4 * EPI_WARPS) {
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
               const int ii = lane + 32 * k;  // 32 consecutive rows -> one coalesced line
-              if (i0 + ii < p.M) {
+              const float4 w4 = *reinterpret_cast<const float4*>(&otile[ii * TLD + cc]);
+              const float wv[4] = {w4.x, w4.y, w4.z, w4.w};
+              if (i0 + ii >= p.M) continue;
+#pragma unroll
+              for (int c = 0; c < 4; ++c) {
+                if (j0 + cc + c >= p.N) break;
+                const int64_t base = (trow0 + cc + c) * p.ldt + tcol;
                 float hv, lv;
-                split_tf32(otile[ii * TLD + cc], hv, lv);
+                split_tf32(wv[c], hv, lv);
                 p.t0[base + ii] = hv;
                 p.t1[base + ii] = lv;
               }

@@ -42,6 +42,7 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
 // timeout / abort; a timeout sets the abort flag and *err.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag,
                                           int* err, long long limit) {
+  if (mbar_try_wait(bar, parity)) return true;  // most waits end here, without a clock read
   const long long t0 = clock64();
   for (uint32_t it = 0;; ++it) {
     if (mbar_try_wait(bar, parity)) return true;
