@@ -66,7 +66,8 @@ class ConjugatePosterior(AbstractPosterior):
         mean = torch.empty(m, dtype=torch.float64, device=dev)
         var = torch.empty(m, dtype=torch.float64, device=dev)
         cov = torch.empty((m, m), dtype=torch.float64, device=dev) if full_covariance else None
-        info = torch.zeros(1, dtype=torch.int32, device=dev)
+        info = torch.empty(1, dtype=torch.int32, device=dev) if m else \
+            torch.zeros(1, dtype=torch.int32, device=dev)  # written by the library
         xc, tc, yc = x.detach().contiguous(), t.detach().contiguous(), y.detach().contiguous()
         nbytes = _lib.lib().gpk_predict_workspace_bytes(n, m, d, prec)
         ws = _lib.workspace(nbytes, dev)

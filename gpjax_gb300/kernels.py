@@ -71,14 +71,17 @@ class StationaryKernel(AbstractKernel):
     def n_ls(self) -> int:
         return int(self.lengthscale.value.numel())
 
+    def theta_parts(self, device, obs_stddev=None, constant=None) -> list[torch.Tensor]:
+        """The tensors of :meth:`theta_vector` in order, not yet flattened or moved."""
+        z = torch.zeros(1, dtype=torch.float64, device=device) \
+            if obs_stddev is None or constant is None else None
+        return [self.lengthscale.value, self.variance.value,
+                z if obs_stddev is None else obs_stddev, z if constant is None else constant]
+
     def theta_vector(self, device, obs_stddev=None, constant=None) -> torch.Tensor:
         """[lengthscale..., variance, obs_stddev, constant] as one float64 device vector."""
-        z = torch.zeros(1, dtype=torch.float64, device=device)
-        parts = [self.lengthscale.value.reshape(-1).to(device),
-                 self.variance.value.reshape(1).to(device),
-                 z if obs_stddev is None else obs_stddev.reshape(1).to(device),
-                 z if constant is None else constant.reshape(1).to(device)]
-        return torch.cat(parts)
+        return torch.cat([p.reshape(-1).to(device)
+                          for p in self.theta_parts(device, obs_stddev, constant)])
 
     def __call__(self, x: torch.Tensor, y: torch.Tensor) -> torch.Tensor:
         """k(x, y) for a pair of points."""
@@ -123,7 +126,6 @@ class RationalQuadratic(StationaryKernel):
         self.alpha = a
         super().__init__(active_dims, lengthscale, variance, n_dims, compute_engine)
 
-    def theta_vector(self, device, obs_stddev=None, constant=None) -> torch.Tensor:
-        base = super().theta_vector(device, obs_stddev, constant)
-        return torch.cat([base, torch.full((1,), self.alpha, dtype=torch.float64,
-                                           device=base.device)])
+    def theta_parts(self, device, obs_stddev=None, constant=None) -> list[torch.Tensor]:
+        return super().theta_parts(device, obs_stddev, constant) + [
+            torch.full((1,), self.alpha, dtype=torch.float64, device=device)]

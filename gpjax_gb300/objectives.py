@@ -15,32 +15,77 @@ import torch
 from . import _lib
 from .config import precision_code
 from .gps import _mean_constant
+from .kernels import StationaryKernel
+
+
+def _theta_parts(kernel, dev, likelihood, mean_function) -> list[torch.Tensor]:
+    """The kernel's theta as separate tensors, which the objectives below take as
+    their inputs: the concatenation and its derivative are then one step inside
+    the autograd function instead of a chain of graph nodes on every call."""
+    const = _mean_constant(mean_function, dev)
+    sd = likelihood.obs_stddev.value
+    if type(kernel).theta_vector is not StationaryKernel.theta_vector:
+        return [kernel.theta_vector(dev, sd, const)]
+    return kernel.theta_parts(dev, sd, const)
+
+
+def _like(t: torch.Tensor, device, dtype) -> torch.Tensor:
+    return t if t.device == device and t.dtype == dtype else t.to(device, dtype)
+
+
+def _pack(parts, dev) -> torch.Tensor:
+    """One float64 device vector (called inside an autograd function: no graph)."""
+    return torch.cat([_like(p if p.ndim == 1 else p.reshape(-1), dev, torch.float64)
+                      for p in parts])
+
+
+def _unpack(flat: torch.Tensor, parts_meta, needed) -> list:
+    """The pieces of a gradient in the theta layout, each like its input."""
+    pieces = flat.split([m[0].numel() for m in parts_meta])
+    out = []
+    for piece, (shape, device, dtype), need in zip(pieces, parts_meta, needed):
+        if not need:
+            out.append(None)
+            continue
+        if piece.shape != shape:
+            piece = piece.reshape(shape)
+        out.append(_like(piece, device, dtype))
+    return out
+
+
+def _grad_buffer(th: torch.Tensor, n_ls: int, want_grad: bool) -> torch.Tensor:
+    """The library writes n_ls + 3 entries; a longer theta (the rational
+    quadratic's alpha) keeps zeros past them, and so does one without a gradient."""
+    if want_grad and th.numel() == n_ls + 3:
+        return torch.empty_like(th)
+    return torch.zeros_like(th)
 
 
 class _ConjugateMLL(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, theta, x, y, kind, n_ls, jitter, prec):
-        dev = _lib.require_cuda(x, y, theta)
+    def forward(ctx, x, y, kind, n_ls, jitter, prec, *parts):
+        dev = _lib.require_cuda(x, y)
         n, d = x.shape
-        want_grad = bool(ctx.needs_input_grad[0])
-        th = theta.detach().contiguous()
-        xc, yc = x.detach().contiguous(), y.detach().reshape(-1).contiguous()
-        out = torch.empty(1, dtype=torch.float64, device=dev)
-        grad = torch.zeros(th.numel(), dtype=torch.float64, device=dev)  # n_ls + 3 (+ RQ alpha)
-        info = torch.zeros(1, dtype=torch.int32, device=dev)
+        want_grad = any(ctx.needs_input_grad[6:])
+        th = _pack(parts, dev)
+        xc, yc = x.contiguous(), y.reshape(-1).contiguous()
+        out = torch.empty((), dtype=torch.float64, device=dev)
+        grad = _grad_buffer(th, n_ls, want_grad)
+        info = torch.empty(1, dtype=torch.int32, device=dev)  # written by the library
         nbytes = _lib.lib().gpk_conjugate_mll_workspace_bytes(n, d, prec)
         ws = _lib.workspace(nbytes, dev)
         _lib.call("gpk_conjugate_mll", kind, n, d, xc.data_ptr(), d, yc.data_ptr(), th.data_ptr(),
                   n_ls, float(jitter), prec, int(want_grad), out.data_ptr(), grad.data_ptr(),
                   info.data_ptr(), ws.data_ptr(), ws.numel(), _lib.stream_ptr(dev))
         ctx.save_for_backward(grad)
+        ctx.parts = [(p.shape, p.device, p.dtype) for p in parts]
         ctx.info = info
-        return out[0]
+        return out
 
     @staticmethod
     def backward(ctx, g):
         (grad,) = ctx.saved_tensors
-        return g * grad, None, None, None, None, None, None
+        return (None,) * 6 + tuple(_unpack(g * grad, ctx.parts, ctx.needs_input_grad[6:]))
 
 
 def conjugate_mll(posterior, data, precision: str | None = None) -> torch.Tensor:
@@ -53,36 +98,36 @@ def conjugate_mll(posterior, data, precision: str | None = None) -> torch.Tensor
     kernel = posterior.prior.kernel
     x = kernel.slice_input(data.X)
     dev = _lib.require_cuda(x)
-    const = _mean_constant(posterior.prior.mean_function, dev)
-    theta = kernel.theta_vector(dev, posterior.likelihood.obs_stddev.value, const)
-    return _ConjugateMLL.apply(theta, x, data.y, kernel.kind, kernel.n_ls,
-                               float(posterior.prior.jitter), precision_code(precision))
+    parts = _theta_parts(kernel, dev, posterior.likelihood, posterior.prior.mean_function)
+    return _ConjugateMLL.apply(x, data.y, kernel.kind, kernel.n_ls,
+                               float(posterior.prior.jitter), precision_code(precision), *parts)
 
 
 class _ConjugateLOOCV(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, theta, x, y, kind, n_ls, jitter):
-        dev = _lib.require_cuda(x, y, theta)
+    def forward(ctx, x, y, kind, n_ls, jitter, *parts):
+        dev = _lib.require_cuda(x, y)
         n, d = x.shape
-        want_grad = bool(ctx.needs_input_grad[0])
-        th = theta.detach().contiguous()
-        xc, yc = x.detach().contiguous(), y.detach().reshape(-1).contiguous()
-        out = torch.empty(1, dtype=torch.float64, device=dev)
-        grad = torch.zeros(th.numel(), dtype=torch.float64, device=dev)  # n_ls + 3 (+ RQ alpha)
-        info = torch.zeros(1, dtype=torch.int32, device=dev)
+        want_grad = any(ctx.needs_input_grad[5:])
+        th = _pack(parts, dev)
+        xc, yc = x.contiguous(), y.reshape(-1).contiguous()
+        out = torch.empty((), dtype=torch.float64, device=dev)
+        grad = _grad_buffer(th, n_ls, want_grad)
+        info = torch.empty(1, dtype=torch.int32, device=dev)  # written by the library
         ws = _lib.workspace(_lib.lib().gpk_conjugate_loocv_workspace_bytes(n, d), dev)
         _lib.call("gpk_conjugate_loocv", kind, n, d, xc.data_ptr(), d, yc.data_ptr(),
                   th.data_ptr(), n_ls, float(jitter), int(want_grad), out.data_ptr(),
                   grad.data_ptr(), info.data_ptr(), ws.data_ptr(), ws.numel(),
                   _lib.stream_ptr(dev))
         ctx.save_for_backward(grad)
+        ctx.parts = [(p.shape, p.device, p.dtype) for p in parts]
         ctx.info = info
-        return out[0]
+        return out
 
     @staticmethod
     def backward(ctx, g):
         (grad,) = ctx.saved_tensors
-        return g * grad, None, None, None, None, None
+        return (None,) * 5 + tuple(_unpack(g * grad, ctx.parts, ctx.needs_input_grad[5:]))
 
 
 def conjugate_loocv(posterior, data) -> torch.Tensor:
@@ -93,10 +138,9 @@ def conjugate_loocv(posterior, data) -> torch.Tensor:
     kernel = posterior.prior.kernel
     x = kernel.slice_input(data.X)
     dev = _lib.require_cuda(x)
-    const = _mean_constant(posterior.prior.mean_function, dev)
-    theta = kernel.theta_vector(dev, posterior.likelihood.obs_stddev.value, const)
-    return _ConjugateLOOCV.apply(theta, x, data.y, kernel.kind, kernel.n_ls,
-                                 float(posterior.prior.jitter))
+    parts = _theta_parts(kernel, dev, posterior.likelihood, posterior.prior.mean_function)
+    return _ConjugateLOOCV.apply(x, data.y, kernel.kind, kernel.n_ls,
+                                 float(posterior.prior.jitter), *parts)
 
 
 def value_and_grad(objective, model, data, **kw):
@@ -104,7 +148,8 @@ def value_and_grad(objective, model, data, **kw):
     model's parameters (fit.py:160)."""
     params = named_parameters(model)
     for p in params.values():
-        p.requires_grad_(True)
+        if not (p.value.is_leaf and p.value.requires_grad):
+            p.requires_grad_(True)
     val = objective(model, data, **kw)
     grads = torch.autograd.grad(val, [p.value for p in params.values()], allow_unused=True)
     out = {k: (g if g is not None else torch.zeros_like(p.value))
@@ -199,18 +244,19 @@ def allreduce_callback(workspace: torch.Tensor, group=None):
 
 class _CollapsedELBO(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, theta, z, x, y, kind, n_ls, jitter, prec, group=None):
-        dev = _lib.require_cuda(x, y, theta, z)
+    def forward(ctx, z, x, y, kind, n_ls, jitter, prec, group, *parts):
+        dev = _lib.require_cuda(x, y, z)
         n, d = x.shape
         m = z.shape[0]
-        want = bool(ctx.needs_input_grad[0] or ctx.needs_input_grad[1])
-        th = theta.detach().contiguous()
+        want = bool(ctx.needs_input_grad[0]) or any(ctx.needs_input_grad[8:])
+        th = _pack(parts, dev)
         xc, yc = x.detach().contiguous(), y.detach().reshape(-1).contiguous()
         zc = z.detach().to(torch.float64).contiguous()
-        out = torch.empty(1, dtype=torch.float64, device=dev)
-        grad = torch.zeros(th.numel(), dtype=torch.float64, device=dev)  # n_ls + 3 (+ RQ alpha)
-        gz = torch.zeros((m, d), dtype=torch.float64, device=dev)
-        info = torch.zeros(1, dtype=torch.int32, device=dev)
+        out = torch.empty((), dtype=torch.float64, device=dev)
+        grad = _grad_buffer(th, n_ls, want)
+        gz = torch.empty((m, d), dtype=torch.float64, device=dev) if want else \
+            torch.zeros((m, d), dtype=torch.float64, device=dev)
+        info = torch.empty(1, dtype=torch.int32, device=dev)  # written by the library
         nbytes = _lib.lib().gpk_collapsed_elbo_workspace_bytes(n, m, d, prec)
         ws = _lib.workspace(nbytes, dev)
         if group is None:
@@ -229,13 +275,15 @@ class _CollapsedELBO(torch.autograd.Function):
                       gz.data_ptr(), info.data_ptr(), ws.data_ptr(), ws.numel(),
                       _lib.stream_ptr(dev), cb, None)
         ctx.save_for_backward(grad, gz)
+        ctx.parts = [(p.shape, p.device, p.dtype) for p in parts]
         ctx.info = info
-        return out[0]
+        return out
 
     @staticmethod
     def backward(ctx, g):
         grad, gz = ctx.saved_tensors
-        return g * grad, g * gz, None, None, None, None, None, None, None
+        return (g * gz if ctx.needs_input_grad[0] else None, *(None,) * 7,
+                *_unpack(g * grad, ctx.parts, ctx.needs_input_grad[8:]))
 
 
 def collapsed_elbo(variational_family, data, precision: str | None = None,
@@ -253,10 +301,9 @@ def collapsed_elbo(variational_family, data, precision: str | None = None,
     x = kernel.slice_input(data.X)
     dev = _lib.require_cuda(x)
     z = kernel.slice_input(q.inducing_inputs.value.to(dev))
-    const = _mean_constant(post.prior.mean_function, dev)
-    theta = kernel.theta_vector(dev, post.likelihood.obs_stddev.value, const)
-    return _CollapsedELBO.apply(theta, z, x, data.y, kernel.kind, kernel.n_ls, float(q.jitter),
-                                precision_code(precision), process_group)
+    parts = _theta_parts(kernel, dev, post.likelihood, post.prior.mean_function)
+    return _CollapsedELBO.apply(z, x, data.y, kernel.kind, kernel.n_ls, float(q.jitter),
+                                precision_code(precision), process_group, *parts)
 
 
 def cross_covariance_vjp(kind, n_ls, theta, x, y, G, need_x=False, need_y=False):
@@ -264,8 +311,9 @@ def cross_covariance_vjp(kind, n_ls, theta, x, y, G, need_x=False, need_y=False)
     dev = _lib.require_cuda(x, y, G)
     n, m, d = x.shape[0], y.shape[0], x.shape[1]
     gth = torch.zeros(theta.numel(), dtype=torch.float64, device=dev)  # n_ls + 3 (+ RQ alpha)
-    gx = torch.zeros((n, d), dtype=torch.float64, device=dev) if need_x else None
-    gy = torch.zeros((m, d), dtype=torch.float64, device=dev) if need_y else None
+    make = torch.empty if n and m else torch.zeros  # the library writes all of them
+    gx = make((n, d), dtype=torch.float64, device=dev) if need_x else None
+    gy = make((m, d), dtype=torch.float64, device=dev) if need_y else None
     Gc = G.detach().to(torch.float64).contiguous()
     nbytes = _lib.lib().gpk_cross_covariance_vjp_workspace_bytes(n, m, d)
     ws = _lib.workspace(nbytes, dev)
