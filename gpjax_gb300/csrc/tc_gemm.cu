@@ -35,7 +35,7 @@ __device__ __forceinline__ void split_tf32(float x, float& hi, float& lo) {
 // columns.  Wide (1, large GEMMs): 128 x 256 outputs, 16-wide K slices in 64B
 // swizzle, 4 stages of 48 KB, 2 buffers of 256 columns: a quarter fewer
 // operand bytes, from L2 and from shared memory, per multiply-add.  Half (2,
-// small GEMMs): 128 x 64 outputs, 32-wide slices, 4 stages of 48 KB, 4 buffers
+// small GEMMs): 128 x 64 outputs, 32-wide slices, 4 stages of 48 KB, 8 buffers
 // of 64 columns: twice the CTAs of the narrow tile where that leaves SMs idle.
 // Wide float16 (3): the wide tile's byte geometry (64-byte K slice rows, 64B
 // swizzle, 4 stages of 48 KB) holding 32 float16 K elements per slice, two
@@ -52,7 +52,7 @@ struct Tile {
   static constexpr int A_BYTES = BM * BK * ELEM;
   static constexpr int B_BYTES = BN * BK * ELEM;
   static constexpr int STAGE_BYTES = 2 * (A_BYTES + B_BYTES);  // A_hi, A_lo, B_hi, B_lo
-  static constexpr int NBUF = BN >= 128 ? 512 / BN : 4;        // TMEM accumulator buffers
+  static constexpr int NBUF = 512 / BN;                        // TMEM accumulator buffers
   static constexpr int TMEM_COLS = NBUF * BN;                  // a power of two >= 32
   static constexpr int HC = BN / 2;  // accumulator columns owned by one epilogue thread
   static constexpr int TLD = BN + 4; // staged output tile row stride (floats)
@@ -68,14 +68,20 @@ struct Tile {
   // ~4e3); the wide tiles of the large products drain every 4 steps, which
   // their epilogue keeps up with.
   static constexpr int KPSEG = (TS == 0 || TS == 2) ? 1 : 4;
+  // Buffers handed over at a time, half of them: a handover (barrier waits,
+  // commit, fences on both sides) takes about as long as the MMAs of one K
+  // step, so single-step segments go in groups (half tile, one K step each:
+  // 306 clocks a step, 144 of them MMAs).
+  static constexpr int NGRP = 2;
+  static constexpr int GRP = NBUF / NGRP;
 };
 
 template <int STAGES_>
 struct SmemCtl {
   uint64_t full[STAGES_];
   uint64_t empty[STAGES_];
-  uint64_t tfull[4];   // accumulator segment ready (MMA -> epilogue)
-  uint64_t tempty[4];  // accumulator segment drained (epilogue -> MMA)
+  uint64_t tfull[2];   // accumulator group ready (MMA -> epilogue)
+  uint64_t tempty[2];  // accumulator group drained (epilogue -> MMA)
   uint64_t mdone;      // MMAs issued before an abort have completed
   uint32_t tmem;
   int abort_flag;
@@ -131,7 +137,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
       mbar_init(&ctl->full[s], 1);
       mbar_init(&ctl->empty[s], 1);
     }
-    for (int b = 0; b < NBUF; ++b) {
+    for (int b = 0; b < TL::NGRP; ++b) {
       mbar_init(&ctl->tfull[b], 1);
       mbar_init(&ctl->tempty[b], EPI_WARPS);  // one arrival per epilogue warp
     }
@@ -188,8 +194,10 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
     // itself in the narrow and half tiles (65 and 48).
     constexpr uint32_t idesc = TL::F16 ? idesc_f16(BM, BN) : idesc_tf32(BM, BN);
     constexpr int KS = TL::KS, KP = TL::KPSEG;
-    static_assert(KP == 1 ? KS == NBUF : STAGES * KS == NBUF * KP,
-                  "the accumulator buffer follows from the stage and K step");
+    constexpr int GK = TL::GRP * KP;      // K steps of one group
+    constexpr int IL = KP == 1 ? TL::GRP : KS;  // K steps whose MMAs are issued together
+    static_assert(STAGES * KS % (2 * GK) == 0 && KS % IL == 0 && GK % IL == 0,
+                  "buffers and groups follow from the stage and K step");
     const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
     const bool leader = elect_one();
     const int nks = nk * KS;  // MMA K steps of this tile
@@ -206,33 +214,33 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
       const uint64_t bhi = sdesc<TL::SWZ>(sb + 2 * A_BYTES);
       const uint64_t blo = sdesc<TL::SWZ>(sb + 2 * A_BYTES + B_BYTES);
 #pragma unroll
-      for (int k4 = 0; k4 < KS; ++k4) {
-        // segment of KP K steps per TMEM accumulator buffer
-        const int ks = kc * KS + k4, seg = ks / KP;
-        const int b = KP == 1 ? k4 : (s * KS + k4) / KP % NBUF;
-        const uint32_t tacc = tm + (uint32_t)(b * BN);
-        const bool first = KP == 1 || (s * KS + k4) % KP == 0;
-        if (first && seg >= NBUF) {
-          ok = __all_sync(0xffffffffu, mbar_wait(&ctl->tempty[b], ((seg / NBUF) - 1) & 1,
+      for (int k0 = 0; k0 < KS; k0 += IL) {
+        const int grp = (kc * KS + k0) / GK, gb = (s * KS + k0) / GK % TL::NGRP;
+        if ((s * KS + k0) % GK == 0 && grp >= TL::NGRP) {
+          ok = __all_sync(0xffffffffu, mbar_wait(&ctl->tempty[gb], ((grp / TL::NGRP) - 1) & 1,
                                                  abort_flag, p.err, wlim));
           if (!ok) return;
           tc_fence_after();
         }
         issued_mma = true;
         if (!leader) continue;
-        // the two cross products (about 2^-11 of the result) before the
-        // hi*hi product, so the running sum carrying them is small
-        const uint64_t off = (uint64_t)((k4 * 32) >> 4);  // 32 bytes per MMA K step
-        if (TL::F16) {
-          mma_f16(tacc, alo + off, bhi + off, idesc, first ? 0u : 1u);
-          mma_f16(tacc, ahi + off, blo + off, idesc, 1u);
-          mma_f16(tacc, ahi + off, bhi + off, idesc, 1u);
-        } else {
-          mma_tf32(tacc, alo + off, bhi + off, idesc, first ? 0u : 1u);
-          mma_tf32(tacc, ahi + off, blo + off, idesc, 1u);
-          mma_tf32(tacc, ahi + off, bhi + off, idesc, 1u);
+        // Within an accumulator the two cross products (about 2^-11 of the
+        // result) before the hi*hi product, so the running sum carrying them
+        // is small.  Single-step accumulators take turns (an MMA that adds to
+        // the accumulator of the one before it waits for it).
+#pragma unroll
+        for (int t = 0; t < 3 * IL; ++t) {
+          const int u = KP == 1 ? t % IL : t / 3, m = KP == 1 ? t / IL : t % 3, k4 = k0 + u;
+          const uint32_t tacc = tm + (uint32_t)((s * KS + k4) / KP % NBUF * BN);
+          const uint64_t off = (uint64_t)((k4 * 32) >> 4);  // 32 bytes per MMA K step
+          const uint64_t da = (m == 0 ? alo : ahi) + off, db = (m == 1 ? blo : bhi) + off;
+          const uint32_t add = m == 0 && (s * KS + k4) % KP == 0 ? 0u : 1u;
+          if (TL::F16)
+            mma_f16(tacc, da, db, idesc, add);
+          else
+            mma_tf32(tacc, da, db, idesc, add);
         }
-        if (KP == 1 || (s * KS + k4) % KP == KP - 1 || ks == nks - 1) mma_commit(&ctl->tfull[b]);
+        if ((s * KS + k0) % GK == GK - IL || kc * KS + k0 + IL >= nks) mma_commit(&ctl->tfull[gb]);
       }
       if (leader) mma_commit(&ctl->empty[s]);
     };
@@ -278,59 +286,65 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
 #pragma unroll
     for (int c = 0; c < HC; ++c) acc[c] = 0.f;
     bool have = true;
-    // single-step segments of the half tile are drained two per round trip
-    constexpr int DR = (TL::KPSEG == 1 && HC == 32) ? 2 : 1;
-    for (int seg = 0; seg < nseg; seg += DR) {
-      const int b = seg % NBUF;
-      const bool two = DR == 2 && seg + 1 < nseg;
-      const int b1 = (seg + 1) % NBUF;
-      bool ready = mbar_wait(&ctl->tfull[b], (seg / NBUF) & 1, abort_flag, p.err, wlim);
-      if (two && ready)
-        ready = mbar_wait(&ctl->tfull[b1], ((seg + 1) / NBUF) & 1, abort_flag, p.err, wlim);
-      have = __all_sync(0xffffffffu, ready);
+    const uint32_t tcol0 = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)hcol;
+    const int ngrp = (nseg + TL::GRP - 1) / TL::GRP;
+    for (int grp = 0; grp < ngrp; ++grp) {
+      const int gb = grp % TL::NGRP;
+      have = __all_sync(0xffffffffu, mbar_wait(&ctl->tfull[gb], (grp / TL::NGRP) & 1, abort_flag,
+                                               p.err, wlim));
       if (!have) break;
       tc_fence_after();
-      const uint32_t tb = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b * BN + hcol);
-      if (HC == 32) {
-        uint32_t v0[32], v1[32];
-        tmem_ld32_nowait(tb, v0);
-        if (two) tmem_ld32_nowait(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(b1 * BN + hcol), v1);
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      const uint32_t tg = tcol0 + (uint32_t)(gb * TL::GRP * BN);
+      const int cnt = min(TL::GRP, nseg - grp * TL::GRP);
+      if constexpr (HC == 32) {
 #pragma unroll
-        for (int k = 0; k < 32; ++k) acc[k] += __uint_as_float(v0[k]);
-        if (two) {
-#pragma unroll
-          for (int k = 0; k < 32; ++k) acc[k] += __uint_as_float(v1[k]);
-        }
-      } else if (HC == 64) {
-        uint32_t v0[32], v1[32];
-        tmem_ld32_nowait(tb, v0);
-        tmem_ld32_nowait(tb + 32, v1);
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-        for (int k = 0; k < 32; ++k) {
-          acc[k] += __uint_as_float(v0[k]);
-          acc[32 + k] += __uint_as_float(v1[k]);
-        }
-      } else {
-#pragma unroll
-        for (int cc = 0; cc < HC; cc += 16) {
-          uint32_t v0[16];
-          tmem_ld16_nowait(tb + cc, v0);
+        for (int u = 0; u < TL::GRP; u += 2) {
+          if (u >= cnt) break;
+          const bool two = u + 1 < cnt;
+          uint32_t v0[32], v1[32];
+          tmem_ld32_nowait(tg + (uint32_t)(u * BN), v0);
+          if (two) tmem_ld32_nowait(tg + (uint32_t)((u + 1) * BN), v1);
           asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-          for (int k = 0; k < 16; ++k) acc[cc + k] += __uint_as_float(v0[k]);
+          for (int k = 0; k < 32; ++k) acc[k] += __uint_as_float(v0[k]);
+          if (two) {
+#pragma unroll
+            for (int k = 0; k < 32; ++k) acc[k] += __uint_as_float(v1[k]);
+          }
+        }
+      } else {
+        // 64 columns in one round trip, 128 in eight (fewer live registers)
+        constexpr int W = HC == 64 ? 32 : 16;
+#pragma unroll
+        for (int u = 0; u < TL::GRP; ++u) {
+          if (u >= cnt) break;
+          if constexpr (HC == 64) {
+            uint32_t v0[W], v1[W];
+            tmem_ld32_nowait(tg + (uint32_t)(u * BN), v0);
+            tmem_ld32_nowait(tg + (uint32_t)(u * BN + 32), v1);
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+            for (int k = 0; k < 32; ++k) {
+              acc[k] += __uint_as_float(v0[k]);
+              acc[32 + k] += __uint_as_float(v1[k]);
+            }
+          } else {
+#pragma unroll
+            for (int cc = 0; cc < HC; cc += W) {
+              uint32_t v0[W];
+              tmem_ld16_nowait(tg + (uint32_t)(u * BN + cc), v0);
+              asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+              for (int k = 0; k < W; ++k) acc[cc + k] += __uint_as_float(v0[k]);
+            }
+          }
         }
       }
       tc_fence_before();
       __syncwarp();
-      if (lane == 0) {
-        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&ctl->tempty[b]))
+      if (lane == 0)
+        asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&ctl->tempty[gb]))
                      : "memory");
-        if (two)
-          asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&ctl->tempty[b1]))
-                       : "memory");
-      }
     }
     if (p.ra) {
       // undo the float16 operands' power-of-two row scales (exact)
