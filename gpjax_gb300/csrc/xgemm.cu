@@ -48,25 +48,39 @@ struct XParams {
 };
 
 // (hi * 2^32 + lo) * 2^e rounded to float64, in integer arithmetic (this
-// part's float64 units would take longer than the products of a short K).
+// part's float64 units would take longer than the products of a short K): a
+// 64-bit head and a 32-bit tail, |hi| < 2^58.
 __device__ __forceinline__ double x_round(long long hi, long long lo, int e) {
-  const __int128 T = ((__int128)hi << 32) + lo;
-  unsigned __int128 m = T < 0 ? -(unsigned __int128)T : (unsigned __int128)T;
-  if (m == 0) return 0.0;
-  const unsigned long long mh = (unsigned long long)(m >> 64);
-  const int lz = mh ? __clzll(mh) : 64 + __clzll((unsigned long long)m);
-  m <<= lz;
-  const unsigned long long top = (unsigned long long)(m >> 64);
-  const unsigned long long rest = (unsigned long long)m;
+  long long h = hi + (lo >> 32);
+  unsigned t = (unsigned)lo;
+  const unsigned long long sign = (unsigned long long)h & 0x8000000000000000ULL;
+  if (h < 0) {  // negate the pair
+    h = ~h + (t == 0);
+    t = 0u - t;
+  }
+  if (h == 0) {  // below 2^32 units: the tail is the head
+    if (t == 0) return 0.0;
+    h = t;
+    t = 0;
+    e -= 32;
+  }
+  const int lz = __clzll(h);
+  unsigned long long top = (unsigned long long)h << lz;
+  unsigned rest = 0;
+  if (lz >= 32) {
+    top |= (unsigned long long)t << (lz - 32);
+  } else {
+    top |= ((unsigned long long)t << lz) >> 32;
+    rest = t << lz;
+  }
   unsigned long long r = top >> 11;
-  const unsigned long long rem = top & 0x7ff;
+  const unsigned rem = (unsigned)top & 0x7ff;
   if (rem > 0x400 || (rem == 0x400 && (rest != 0 || (r & 1)))) ++r;
-  const unsigned long long sign = T < 0 ? 0x8000000000000000ULL : 0ULL;
-  const int biased = 127 - lz + e + 1023;
+  const int biased = 63 + 32 - lz + e + 1023;
   if (biased >= 1 && biased <= 2046)
     return __longlong_as_double((long long)(sign | (((unsigned long long)(biased - 1) << 52) + r)));
-  const double v = scalbn((double)r, 127 - lz + e - 52);
-  return T < 0 ? -v : v;
+  const double v = scalbn((double)r, 63 + 32 - lz + e - 52);
+  return sign ? -v : v;
 }
 
 __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, int x, int y, int w,
