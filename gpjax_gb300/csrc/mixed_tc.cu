@@ -370,62 +370,108 @@ __global__ void residual_upper_finish(int kind, int n, const double* __restrict_
 // float16 row scaling: each row's largest magnitude lands in [2^13, 2^14)
 constexpr int V16_TARGET_EXP = 14;
 
-// Rows [0, rows) of the rows x cols block at (row0, col0) of a TF32 pair
-// (hi + lo, leading dimension ld) to compact float16 hi/lo [rows][cols] with
-// the power-of-two row scales of v16_convert_kernel (rinv[r] = 1 / scale).
-// tri = TRI_LOWER / TRI_UPPER keeps the block's lower / upper triangle and
-// writes zeros elsewhere (so nothing outside the operand reaches a scale or
-// a product), TRI_NONE the whole row.  One warp per row; cols % 4 == 0,
-// col0 % 4 == 0.
-__global__ void __launch_bounds__(256)
-    split16_block_kernel(const float* __restrict__ hi, const float* __restrict__ lo, int64_t ld,
-                         int row0, int col0, int rows, int cols, int tri, __half* __restrict__ dh,
-                         __half* __restrict__ dl, float* __restrict__ rinv) {
-  const int r = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  const int lane = threadIdx.x & 31;
-  if (r >= rows) return;
-  const int cb = tri == TRI_UPPER ? r : 0;
-  const int ce = tri == TRI_LOWER ? min(cols, r + 1) : cols;  // exclusive
-  const int64_t o = (int64_t)(row0 + r) * ld + col0;
+// One row (hi + lo, columns [c0, cols), zeros outside [cb, ce)) to float16
+// hi/lo under a power-of-two scale; returns 1 / scale.  One block of 256 threads
+// per row, U * 1024 of its columns kept in registers between the search for the
+// largest magnitude and the conversion, so that they are read once, all loads
+// in flight together; columns past those are read twice.  (One warp a row, two
+// loads in flight and two reads, took twice as long as the bytes.)
+template <int U>
+__device__ __forceinline__ float row_to_f16(const float* __restrict__ hi,
+                                            const float* __restrict__ lo, int c0, int cols, int cb,
+                                            int ce, __half* __restrict__ dh,
+                                            __half* __restrict__ dl) {
+  __shared__ float wmax[8];
+  auto load = [&](int c) {
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (c < cols && c + 3 >= cb && c < ce) {
+      const float4 h = *reinterpret_cast<const float4*>(hi + c);
+      const float4 l = *reinterpret_cast<const float4*>(lo + c);
+      v = make_float4(h.x + l.x, h.y + l.y, h.z + l.z, h.w + l.w);
+      if (c < cb || c + 3 >= ce) {
+        if (c < cb || c >= ce) v.x = 0.f;
+        if (c + 1 < cb || c + 1 >= ce) v.y = 0.f;
+        if (c + 2 < cb || c + 2 >= ce) v.z = 0.f;
+        if (c + 3 < cb || c + 3 >= ce) v.w = 0.f;
+      }
+    }
+    return v;
+  };
+  auto amax = [](float m, const float4& v) {
+    return fmaxf(m, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
+  };
+  const int first = c0 + 4 * (int)threadIdx.x, past = first + U * 1024;
+  float4 keep[U];
   float mx = 0.f;
-  for (int c = (cb & ~3) + lane * 4; c < ce; c += 128) {
-    const float4 h = *reinterpret_cast<const float4*>(hi + o + c);
-    const float4 l = *reinterpret_cast<const float4*>(lo + o + c);
-    const float v[4] = {h.x + l.x, h.y + l.y, h.z + l.z, h.w + l.w};
 #pragma unroll
-    for (int k = 0; k < 4; ++k)
-      if (c + k >= cb && c + k < ce) mx = fmaxf(mx, fabsf(v[k]));
-  }
+  for (int u = 0; u < U; ++u) keep[u] = load(first + u * 1024);
+#pragma unroll
+  for (int u = 0; u < U; ++u) mx = amax(mx, keep[u]);
+#pragma unroll 4
+  for (int c = past; c < cols; c += 1024) mx = amax(mx, load(c));
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
-  int e = 0;
-  if (mx > 0.f && isfinite(mx)) frexpf(mx, &e);
-  e = max(e, -100);
-  const float sc = ldexpf(1.f, V16_TARGET_EXP - e);
-  const int64_t d0 = (int64_t)r * cols;
-  for (int c = lane * 4; c < cols; c += 128) {
-    float v[4] = {0.f, 0.f, 0.f, 0.f};
-    if (c + 3 >= cb && c < ce) {
-      const float4 h = *reinterpret_cast<const float4*>(hi + o + c);
-      const float4 l = *reinterpret_cast<const float4*>(lo + o + c);
-      const float w[4] = {h.x + l.x, h.y + l.y, h.z + l.z, h.w + l.w};
+  if ((threadIdx.x & 31) == 0) wmax[threadIdx.x >> 5] = mx;
+  __syncthreads();
 #pragma unroll
-      for (int k = 0; k < 4; ++k) v[k] = (c + k >= cb && c + k < ce) ? w[k] * sc : 0.f;
-    }
+  for (int w = 0; w < 8; ++w) mx = fmaxf(mx, wmax[w]);
+  int e = 0;
+  if (mx > 0.f && isfinite(mx)) frexpf(mx, &e);  // mx = f * 2^e, f in [0.5, 1)
+  e = max(e, -100);  // keeps both scales finite
+  const float sc = ldexpf(1.f, V16_TARGET_EXP - e);
+  auto put = [&](int c, const float4& w) {
+    if (c >= cols) return;
+    const float v[4] = {w.x * sc, w.y * sc, w.z * sc, w.w * sc};
     __half hv[4], lv[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
       hv[k] = __float2half_rn(v[k]);
       lv[k] = __float2half_rn(v[k] - __half2float(hv[k]));
     }
-    *reinterpret_cast<uint2*>(dh + d0 + c) = make_uint2(
+    *reinterpret_cast<uint2*>(dh + c) = make_uint2(
         (uint32_t)__half_as_ushort(hv[0]) | ((uint32_t)__half_as_ushort(hv[1]) << 16),
         (uint32_t)__half_as_ushort(hv[2]) | ((uint32_t)__half_as_ushort(hv[3]) << 16));
-    *reinterpret_cast<uint2*>(dl + d0 + c) = make_uint2(
+    *reinterpret_cast<uint2*>(dl + c) = make_uint2(
         (uint32_t)__half_as_ushort(lv[0]) | ((uint32_t)__half_as_ushort(lv[1]) << 16),
         (uint32_t)__half_as_ushort(lv[2]) | ((uint32_t)__half_as_ushort(lv[3]) << 16));
-  }
-  if (lane == 0) rinv[r] = ldexpf(1.f, e - V16_TARGET_EXP);
+  };
+#pragma unroll
+  for (int u = 0; u < U; ++u) put(first + u * 1024, keep[u]);
+#pragma unroll 4
+  for (int c = past; c < cols; c += 1024) put(c, load(c));
+  return ldexpf(1.f, e - V16_TARGET_EXP);
+}
+
+// Calls f with the register bound for rows of `cols` columns.
+template <typename F>
+void row16_dispatch(int cols, F&& f) {
+  if (cols <= 2048)
+    f(std::integral_constant<int, 2>{});
+  else if (cols <= 4096)
+    f(std::integral_constant<int, 4>{});
+  else if (cols <= 8192)
+    f(std::integral_constant<int, 8>{});
+  else
+    f(std::integral_constant<int, 16>{});
+}
+
+// Rows [0, rows) of the rows x cols block at (row0, col0) of a TF32 pair
+// (hi + lo, leading dimension ld) to compact float16 hi/lo [rows][cols] with
+// the power-of-two row scales of v16_convert_kernel (rinv[r] = 1 / scale).
+// tri = TRI_LOWER / TRI_UPPER keeps the block's lower / upper triangle and
+// writes zeros elsewhere (so nothing outside the operand reaches a scale or
+// a product), TRI_NONE the whole row.  cols % 4 == 0, col0 % 4 == 0.
+template <int U>
+__global__ void __launch_bounds__(256)
+    split16_block_kernel(const float* __restrict__ hi, const float* __restrict__ lo, int64_t ld,
+                         int row0, int col0, int cols, int tri, __half* __restrict__ dh,
+                         __half* __restrict__ dl, float* __restrict__ rinv) {
+  const int r = blockIdx.x;
+  const int cb = tri == TRI_UPPER ? r : 0;
+  const int ce = tri == TRI_LOWER ? min(cols, r + 1) : cols;  // exclusive
+  const int64_t o = (int64_t)(row0 + r) * ld + col0, d0 = (int64_t)r * cols;
+  const float inv = row_to_f16<U>(hi + o, lo + o, 0, cols, cb, ce, dh + d0, dl + d0);
+  if (threadIdx.x == 0) rinv[r] = inv;
 }
 
 constexpr int kMaxDepth = 24;  // recursion depth bound (n_pad < 128 * 2^23)
@@ -443,8 +489,10 @@ struct F16Set {
 
 cudaError_t to16(const float* hi, const float* lo, int64_t ld, int row0, int col0, int rows,
                  int cols, int tri, __half* dh, __half* dl, float* rinv, cudaStream_t s) {
-  split16_block_kernel<<<(unsigned)cdiv((int64_t)rows * 32, 256), 256, 0, s>>>(
-      hi, lo, ld, row0, col0, rows, cols, tri, dh, dl, rinv);
+  row16_dispatch(cols, [&](auto u) {
+    split16_block_kernel<decltype(u)::value>
+        <<<(unsigned)rows, 256, 0, s>>>(hi, lo, ld, row0, col0, cols, tri, dh, dl, rinv);
+  });
   return launch_status();
 }
 
@@ -758,49 +806,18 @@ cudaError_t chol_inv_rec(TcChol& c, int o, int sz, int depth, cudaEvent_t join =
 // scale per row that brings the row's largest magnitude into [2^13, 2^14):
 // float16 then keeps an 11-bit significand for every entry down to ~2^-17 of
 // the row maximum (smaller ones lose relative precision but not absolute), and
-// the split pair carries ~22 bits like the TF32 split.  One warp per row; row r
-// is converted from column 128 * (r / 128) on, the part the adjoint reads for
-// outputs it keeps.  vscale[r] = 1 / scale (the epilogue's exact undo).
+// the split pair carries ~22 bits like the TF32 split.  Row r is converted from
+// column 128 * (r / 128) on, the part the adjoint reads for outputs it keeps.
+// vscale[r] = 1 / scale (the epilogue's exact undo).
+template <int U>
 __global__ void __launch_bounds__(256)
     v16_convert_kernel(int np, const float* __restrict__ Vh, const float* __restrict__ Vl,
                        int64_t ld, __half* __restrict__ Hh, __half* __restrict__ Hl,
                        float* __restrict__ vscale) {
-  const int r = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  const int lane = threadIdx.x & 31;
-  if (r >= np) return;
-  const int c0 = (r / LEAF) * LEAF;
+  const int r = blockIdx.x, c0 = (r / LEAF) * LEAF;
   const int64_t o = (int64_t)r * ld;
-  float mx = 0.f;
-  for (int c = c0 + lane * 4; c < np; c += 128) {
-    const float4 h = *reinterpret_cast<const float4*>(Vh + o + c);
-    const float4 l = *reinterpret_cast<const float4*>(Vl + o + c);
-    mx = fmaxf(mx, fmaxf(fmaxf(fabsf(h.x + l.x), fabsf(h.y + l.y)),
-                         fmaxf(fabsf(h.z + l.z), fabsf(h.w + l.w))));
-  }
-#pragma unroll
-  for (int off = 16; off > 0; off >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
-  int e = 0;
-  if (mx > 0.f && isfinite(mx)) frexpf(mx, &e);  // mx = f * 2^e, f in [0.5, 1)
-  e = max(e, -100);  // keeps both scales finite
-  const float sc = ldexpf(1.f, V16_TARGET_EXP - e), inv = ldexpf(1.f, e - V16_TARGET_EXP);
-  for (int c = c0 + lane * 4; c < np; c += 128) {
-    const float4 h = *reinterpret_cast<const float4*>(Vh + o + c);
-    const float4 l = *reinterpret_cast<const float4*>(Vl + o + c);
-    const float v[4] = {(h.x + l.x) * sc, (h.y + l.y) * sc, (h.z + l.z) * sc, (h.w + l.w) * sc};
-    __half hv[4], lv[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      hv[k] = __float2half_rn(v[k]);
-      lv[k] = __float2half_rn(v[k] - __half2float(hv[k]));
-    }
-    *reinterpret_cast<uint2*>(Hh + o + c) = make_uint2(
-        (uint32_t)__half_as_ushort(hv[0]) | ((uint32_t)__half_as_ushort(hv[1]) << 16),
-        (uint32_t)__half_as_ushort(hv[2]) | ((uint32_t)__half_as_ushort(hv[3]) << 16));
-    *reinterpret_cast<uint2*>(Hl + o + c) = make_uint2(
-        (uint32_t)__half_as_ushort(lv[0]) | ((uint32_t)__half_as_ushort(lv[1]) << 16),
-        (uint32_t)__half_as_ushort(lv[2]) | ((uint32_t)__half_as_ushort(lv[3]) << 16));
-  }
-  if (lane == 0) vscale[r] = inv;
+  const float inv = row_to_f16<U>(Vh + o, Vl + o, c0, np, c0, np, Hh + o, Hl + o);
+  if (threadIdx.x == 0) vscale[r] = inv;
 }
 
 struct TcBuffers {
@@ -1191,8 +1208,10 @@ gpk_status mll_run_tc(int kind, int n, int d, const double* x, int64_t ldx, cons
   const int ntiles_adj = tc_gemm_tiles(tc::MODE_GRAD, pg);  // gpart rows of the adjoint
   if (want_grad && f16adj) {
     if (!tc_make_map_f16(&mV16, b.V16h, b.V16l, np, np, b.ld)) return GPK_ERR_CUDA;
-    v16_convert_kernel<<<(unsigned)cdiv((int64_t)np * 32, 256), 256, 0, hs>>>(
-        np, b.Vh, b.Vl, b.ld, b.V16h, b.V16l, b.vscale);
+    row16_dispatch(np, [&](auto u) {
+      v16_convert_kernel<decltype(u)::value>
+          <<<(unsigned)np, 256, 0, hs>>>(np, b.Vh, b.Vl, b.ld, b.V16h, b.V16l, b.vscale);
+    });
     GPK_LAUNCH_CHECK();
     GPK_CUDA_TRY(tc_gemm_run(tc::MODE_GRAD, mV16, mV16, pg, 1, hs, true));
   } else if (want_grad) {
