@@ -623,23 +623,55 @@ struct LeafOutPlain {
   __device__ void put_v(const float*, int, int, int, int, int, int) const {}
 };
 
-// dtrack[o + r] -= sum_k L[o + r][c0 + k]^2 (k < w) for rows r < rows: one
-// warp per row, float-float squares, float64 total.
-__device__ __noinline__ void track_rows(const float* L, int ld, int o, int rows, int c0, int w,
-                           double* dtrack) {
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int r = warp; r < rows; r += BNT / 32) {
-    const float* row = L + (int64_t)(o + r) * ld + c0;
-    float hi = 0.f, lo = 0.f;
-    for (int k = lane * 4; k < w; k += 128) {
-      const float4 v = *reinterpret_cast<const float4*>(row + k);
-      ff_sub_sq(hi, lo, v.x);
-      ff_sub_sq(hi, lo, v.y);
-      ff_sub_sq(hi, lo, v.z);
-      ff_sub_sq(hi, lo, v.w);
+// V values per lane summed over the warp at once: lane l returns the sum of
+// value l / (32 / V).  At offset 16 the halves of the warp exchange halves of
+// the values, and so on: V - 1 additions and then log2(32 / V) instead of
+// 5 V, in the pairing of warp_sum (x + y and y + x round alike), so each sum
+// is the one warp_sum gives.  The float64 pipe takes 19 clocks a warp
+// instruction, which is what the row tracks and the adjoint's sums wait for.
+template <int V>
+__device__ __forceinline__ double warp_sums(double (&v)[V], int lane) {
+  static_assert(V >= 2 && V <= 32 && (V & (V - 1)) == 0, "a power of two");
+  int off = 16;
+#pragma unroll
+  for (int h = V / 2; h > 0; h /= 2, off /= 2) {
+    const bool up = lane & off;
+#pragma unroll
+    for (int q = 0; q < h; ++q) {
+      const double send = up ? v[q] : v[q + h];
+      const double keep = up ? v[q + h] : v[q];
+      v[q] = keep + __shfl_xor_sync(0xffffffffu, send, off);
     }
-    const double s = warp_sum((double)hi + (double)lo);
-    if (lane == 0) dtrack[o + r] += s;
+  }
+#pragma unroll
+  for (int o = 16 / V; o > 0; o /= 2) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+  return v[0];
+}
+
+// dtrack[o + r] -= sum_k L[o + r][c0 + k]^2 (k < TT) for rows r < rows (a
+// multiple of TT): float-float squares, float64 totals, eight rows of a warp
+// summed together.
+__device__ __noinline__ void track_rows(const float* L, int ld, int o, int rows, int c0,
+                                        double* dtrack) {
+  constexpr int TR = 8;  // rows of a warp at a time
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  for (int r0 = warp * TR; r0 < rows; r0 += (BNT / 32) * TR) {  // rows: a multiple of TT
+    double v[TR];
+    float4 x[TR];
+#pragma unroll
+    for (int q = 0; q < TR; ++q)
+      x[q] = *reinterpret_cast<const float4*>(L + (int64_t)(o + r0 + q) * ld + c0 + 4 * lane);
+#pragma unroll
+    for (int q = 0; q < TR; ++q) {
+      float hi = 0.f, lo = 0.f;
+      ff_sub_sq(hi, lo, x[q].x);
+      ff_sub_sq(hi, lo, x[q].y);
+      ff_sub_sq(hi, lo, x[q].z);
+      ff_sub_sq(hi, lo, x[q].w);
+      v[q] = (double)hi + (double)lo;
+    }
+    const double s = warp_sums<TR>(v, lane);
+    if ((lane & (32 / TR - 1)) == 0) dtrack[o + r0 + lane / (32 / TR)] += s;
   }
 }
 
@@ -681,8 +713,12 @@ __device__ void node_up(const Slot& S, int ld, int o, int h, int h2, float* smem
 }
 
 // X L_kk^T = A_panel for the R rows below a diagonal block: forward
-// substitution, one thread per row, 32 columns at a time in registers (the
-// solved columns of the row are read back from X).  L_kk comes from the
+// substitution, one thread per row, 32 columns at a time in registers.  The
+// solved columns of the row are read back from X 16 at a time, four float4
+// loads ahead of their use: lanes hold different rows, so every load is a
+// round trip to L2, and one load a column made the solve wait for 192 of
+// them (10% of the kernel; with the row sums of track_rows and the adjoint
+// below, the 512-instance batch went from 36.5 to 33.4 ms).  L_kk comes from the
 // leaf's shared memory, still in place: LT[k][i] = L[i][k] below the
 // diagonal (zeros on and above it) and Rl[i] = 1 / L[i][i].  Substitution is
 // backward stable; X = A_panel M_kk^T with the leaf's inverse is not, and on
@@ -691,6 +727,7 @@ __device__ void node_up(const Slot& S, int ld, int o, int h, int h2, float* smem
 __device__ __noinline__ void panel_solve(const float* __restrict__ Ap, float* __restrict__ Xp, int ld, int R,
                             const float* leaf_smem) {
   constexpr int LDT = LEAF_LDT, PB = 32;
+  constexpr int XV = 4;  // float4 loads of the row's solved columns in flight
   const float* LT = leaf_smem;
   const float* Rl = leaf_smem + 2 * LEAF * LEAF_LDT + 64 * LEAF_TLD + 4 * LEAF;
   for (int row = threadIdx.x; row < R; row += BNT) {
@@ -707,15 +744,36 @@ __device__ __noinline__ void panel_solve(const float* __restrict__ Ap, float* __
         a[4 * g + 2] = v.z;
         a[4 * g + 3] = v.w;
       }
-      for (int m = 0; m < c0; ++m) {  // the solved columns
-        const float xm = xr[m];
+      float4 xn[XV];
 #pragma unroll
-        for (int g = 0; g < PB / 4; ++g) {
-          const float4 l = *reinterpret_cast<const float4*>(LT + m * LDT + c0 + 4 * g);
-          a[4 * g] = fmaf(-xm, l.x, a[4 * g]);
-          a[4 * g + 1] = fmaf(-xm, l.y, a[4 * g + 1]);
-          a[4 * g + 2] = fmaf(-xm, l.z, a[4 * g + 2]);
-          a[4 * g + 3] = fmaf(-xm, l.w, a[4 * g + 3]);
+      for (int q = 0; q < XV; ++q)
+        xn[q] = cb > 0 ? *reinterpret_cast<const float4*>(xr + 4 * q)
+                       : make_float4(0.f, 0.f, 0.f, 0.f);
+      for (int m0 = 0; m0 < c0; m0 += 4 * XV) {  // the solved columns
+        float xc[4 * XV];
+#pragma unroll
+        for (int q = 0; q < XV; ++q) {
+          xc[4 * q] = xn[q].x;
+          xc[4 * q + 1] = xn[q].y;
+          xc[4 * q + 2] = xn[q].z;
+          xc[4 * q + 3] = xn[q].w;
+        }
+        if (m0 + 4 * XV < c0) {
+#pragma unroll
+          for (int q = 0; q < XV; ++q)
+            xn[q] = *reinterpret_cast<const float4*>(xr + m0 + 4 * XV + 4 * q);
+        }
+#pragma unroll
+        for (int m = 0; m < 4 * XV; ++m) {
+          const float xm = xc[m];
+#pragma unroll
+          for (int g = 0; g < PB / 4; ++g) {
+            const float4 l = *reinterpret_cast<const float4*>(LT + (m0 + m) * LDT + c0 + 4 * g);
+            a[4 * g] = fmaf(-xm, l.x, a[4 * g]);
+            a[4 * g + 1] = fmaf(-xm, l.y, a[4 * g + 1]);
+            a[4 * g + 2] = fmaf(-xm, l.z, a[4 * g + 2]);
+            a[4 * g + 3] = fmaf(-xm, l.w, a[4 * g + 3]);
+          }
         }
       }
 #pragma unroll
@@ -805,7 +863,7 @@ __device__ void chol_inv(const Slot& S, int ld, int np, int* info, float* smem) 
     float* Lp = S.L + (int64_t)(o + TT) * ld + o;
     panel_solve(S.A + (int64_t)(o + TT) * ld + o, Lp, ld, R, smem);
     __syncthreads();
-    track_rows(S.L, ld, o + TT, R, o, TT, S.dtrack);
+    track_rows(S.L, ld, o + TT, R, o, S.dtrack);
   }
   constexpr int DEPTH = 8;  // np <= 4096: at most 6 levels
   int so[DEPTH], ss[DEPTH], sst[DEPTH];
@@ -967,57 +1025,145 @@ __device__ __forceinline__ void ff_add_b(float& hi, float& lo, float a) {
   hi = s;
 }
 
+// f(kind, dim): both compile-time, dim the input dimension rounded up to a
+// multiple of 4 (BDM at most).
+template <class F>
+__device__ __forceinline__ void with_kind_dim(int kind, int d, F f) {
+  static_assert(BDM == 16, "the dimensions below");
+  with_kind(kind, [&](auto kind_c) {
+    if (d <= 4)
+      f(kind_c, std::integral_constant<int, 4>{});
+    else if (d <= 8)
+      f(kind_c, std::integral_constant<int, 8>{});
+    else if (d <= 12)
+      f(kind_c, std::integral_constant<int, 12>{});
+    else
+      f(kind_c, std::integral_constant<int, 16>{});
+  });
+}
+
 // r = diff - Sigma alpha for rows < n (zeros past n) into rres (float64),
 // Sigma regenerated from the scaled inputs, products summed in float-float.
 // ah / al: alpha split into float hi / lo parts (shared memory).  The
 // columns go by chunks of RCH inputs staged in shared memory (gx, odd row
-// stride); a warp takes a row, its lanes the chunk's columns, and each
-// row's chunk sums add up in float64 in rres.
+// stride); a warp takes four rows, its lanes the chunk's columns, and each
+// row's chunk sums add up in float64 in rres.  Four rows share each column's
+// loads and their float-float chains run side by side (with the Gram blocks
+// below: 33.4 to 32.4 ms for the 512-instance batch).
 constexpr int RCH = 512;
 __device__ __noinline__ void residual(const BatchInst& I, const Slot& S, int np, float s2, float ka,
                          double noise_diag, const float* ah, const float* al, double* rres,
                          float* gx) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n = I.n, d = I.d, sd = d | 1;
+  constexpr int RB = 4;  // rows of a warp at a time
   for (int i = threadIdx.x; i < np; i += BNT) rres[i] = 0.0;
-  with_kind(I.kind, [&](auto kind_c) {
-    constexpr int KIND = decltype(kind_c)::value;
+  with_kind_dim(I.kind, d, [&](auto kind_c, auto dim_c) {
+    constexpr int KIND = decltype(kind_c)::value, DC = decltype(dim_c)::value;
     for (int c0 = 0; c0 < n; c0 += RCH) {
       const int cn = min(RCH, n - c0);
       __syncthreads();  // the previous chunk is done with gx (and rres is zeroed)
       for (int e = threadIdx.x; e < cn * d; e += BNT)
         gx[(e / d) * sd + e % d] = S.xs[c0 * d + e];
       __syncthreads();
-      for (int i = warp; i < n; i += BNT / 32) {
-        float xi[BDM];
+      for (int i0 = warp * RB; i0 < n; i0 += (BNT / 32) * RB) {
+        float xi[RB][DC], sh[RB], sl[RB];
 #pragma unroll
-        for (int k = 0; k < BDM; ++k) xi[k] = k < d ? S.xs[i * d + k] : 0.f;
-        float sh = 0.f, sl = 0.f;
+        for (int q = 0; q < RB; ++q) {
+          const int i = min(i0 + q, n - 1);  // (rows past n repeat the last, not kept)
+          sh[q] = sl[q] = 0.f;
+#pragma unroll
+          for (int k = 0; k < DC; ++k) xi[q][k] = k < d ? S.xs[i * d + k] : 0.f;
+        }
         for (int jl = lane; jl < cn; jl += 32) {
           const float* xj = gx + jl * sd;
-          float sq = 0.f;
+          float sq[RB];
 #pragma unroll
-          for (int k = 0; k < BDM; ++k) {
+          for (int q = 0; q < RB; ++q) sq[q] = 0.f;
+#pragma unroll
+          for (int k = 0; k < DC; ++k) {
             if (k < d) {
-              const float df = xi[k] - xj[k];
-              sq = fmaf(df, df, sq);
+              const float x = xj[k];
+#pragma unroll
+              for (int q = 0; q < RB; ++q) {
+                const float df = xi[q][k] - x;
+                sq[q] = fmaf(df, df, sq[q]);
+              }
             }
           }
-          const float kv = kval<float>(KIND, sq, s2, ka);
-          const int j = c0 + jl;
-          const float p = kv * ah[j];
-          const float pe = fmaf(kv, ah[j], -p);
-          ff_add_b(sh, sl, p);
-          sl = fmaf(kv, al[j], sl + pe);
+          const float h = ah[c0 + jl], l = al[c0 + jl];
+#pragma unroll
+          for (int q = 0; q < RB; ++q) {
+            const float kv = kval<float>(KIND, sq[q], s2, ka);
+            const float p = kv * h;
+            const float pe = fmaf(kv, h, -p);
+            ff_add_b(sh[q], sl[q], p);
+            sl[q] = fmaf(kv, l, sl[q] + pe);
+          }
         }
-        const double t = warp_sum((double)sh + (double)sl);
-        if (lane == 0) rres[i] += t;
+        double v[RB];
+#pragma unroll
+        for (int q = 0; q < RB; ++q) v[q] = (double)sh[q] + (double)sl[q];
+        const double t = warp_sums<RB>(v, lane);
+        const int i = i0 + lane / (32 / RB);
+        if (lane % (32 / RB) == 0 && i < n) rres[i] += t;
       }
     }
   });
   __syncthreads();
   for (int i = threadIdx.x; i < np; i += BNT)
     rres[i] = i < n ? S.diff[i] - (rres[i] + noise_diag * S.alpha[i]) : 0.0;
+}
+
+// The Gram matrix's lower 128-blocks (diagonal blocks in full), identity past
+// n.  A thread keeps one column's inputs in registers and takes every fourth
+// row of the block, whose inputs a warp reads from shared memory by
+// broadcast (gx: 128 rows of 16).
+__device__ __noinline__ void gram_blocks(const BatchInst& I, const Slot& S, int np, float s2,
+                                         float ka, double noise_diag, float* gx) {
+  const int n = I.n, d = I.d, ld = np;
+  const int nb = np / TT, nt = nb * (nb + 1) / 2;
+  const int jl = threadIdx.x % TT;
+  with_kind_dim(I.kind, d, [&](auto kind_c, auto dim_c) {
+    constexpr int KIND = decltype(kind_c)::value, DC = decltype(dim_c)::value;
+    for (int t = 0; t < nt; ++t) {
+      int bi, bj;
+      tri_index(t, bi, bj);
+      if (t == 0 || bj == 0) {  // a new block row
+        __syncthreads();
+        for (int e = threadIdx.x; e < TT * DC; e += BNT) {
+          const int r = e / DC, k = e % DC, i = bi * TT + r;
+          gx[e] = i < n && k < d ? S.xs[i * d + k] : 0.f;
+        }
+        __syncthreads();
+      }
+      const int j = bj * TT + jl;
+      float xj[DC];
+#pragma unroll
+      for (int k = 0; k < DC; ++k) xj[k] = j < n && k < d ? S.xs[j * d + k] : 0.f;
+#pragma unroll 4
+      for (int il = threadIdx.x / TT; il < TT; il += BNT / TT) {
+        const int i = bi * TT + il;
+        float sq = 0.f;
+#pragma unroll
+        for (int k = 0; k < DC; k += 4) {
+          const float4 x = *reinterpret_cast<const float4*>(gx + il * DC + k);
+          float df = x.x - xj[k];
+          sq = fmaf(df, df, sq);
+          df = x.y - xj[k + 1];
+          sq = fmaf(df, df, sq);
+          df = x.z - xj[k + 2];
+          sq = fmaf(df, df, sq);
+          df = x.w - xj[k + 3];
+          sq = fmaf(df, df, sq);
+        }
+        float v = kval<float>(KIND, sq, s2, ka);
+        if (i == j) v = (float)((double)v + noise_diag);
+        if (i >= n || j >= n) v = i == j ? 1.f : 0.f;
+        S.A[(int64_t)i * ld + j] = v;
+      }
+    }
+  });
 }
 
 // One W tile (shared memory, row stride WLD) contracted against dK/dtheta:
@@ -1059,15 +1205,25 @@ __device__ __forceinline__ void adj_tile(int i0, int j0, int n, int d, float ka,
     for (int kp = 0; kp < DP; ++kp) pl2[kp] = f2_fma(cc2, dsq2[kp], pl2[kp]);
     if (gi == gj) pnoise += fmaf(sai[r], sai[r], -w);
   }
-  for (int s = 0; s < d + 2; ++s) {
-    float v = s == d ? pvar : pnoise;
+  // slots: lengthscale k at k, then the variance at d and the noise at d + 1
+  constexpr int V = DP == 2 ? 8 : 16;
 #pragma unroll
-    for (int kp = 0; kp < DP; ++kp) {  // (pairs past d hold the zero padding)
-      if (s < d && 2 * kp == s) v = f2_lo(pl2[kp]);
-      if (s < d && 2 * kp + 1 == s) v = f2_hi(pl2[kp]);
+  for (int b = 0; b < 2 * DP + 2; b += V) {
+    if (b < d + 2) {
+      double v[V];
+#pragma unroll
+      for (int q = 0; q < V; ++q) {
+        const int s = b + q;  // pairs past d hold the zero padding
+        float f = 0.f;
+        if (s < 2 * DP) f = (s & 1) ? f2_hi(pl2[s / 2 < DP ? s / 2 : 0]) : f2_lo(pl2[s / 2 < DP ? s / 2 : 0]);
+        if (s == d) f = pvar;
+        if (s == d + 1) f = pnoise;
+        v[q] = (double)f;
+      }
+      const double t = warp_sums<V>(v, lane);
+      const int s = b + lane / (32 / V);
+      if (lane % (32 / V) == 0 && s < d + 2) wred[s * NW + warp] += t;
     }
-    const double t = warp_sum((double)v);
-    if (lane == 0) wred[s * NW + warp] += t;
   }
 }
 
@@ -1201,47 +1357,7 @@ __device__ bool instance_front(const BatchArgs& a, const BatchInst& I, const Slo
     S.M[(int64_t)i * ld + (i / TT) * TT + c] = 0.f;
   }
   __syncthreads();
-  // Gram: lower 128-blocks (diagonal blocks in full), identity past n.  The
-  // block's row and column inputs are staged in shared memory with an odd
-  // row stride (a warp reads 32 consecutive columns' coordinates without
-  // bank conflicts); the kernel kind is resolved outside the loops.
-  {
-    const int nb = np / TT, nt = nb * (nb + 1) / 2;
-    const int sd = d | 1;
-    float* gxi = smem;              // [TT][sd]
-    float* gxj = smem + TT * (BDM + 1);
-    with_kind(I.kind, [&](auto kind_c) {
-      constexpr int KIND = decltype(kind_c)::value;
-      for (int t = 0; t < nt; ++t) {
-        int bi, bj;
-        tri_index(t, bi, bj);
-        for (int e = threadIdx.x; e < TT * d; e += BNT) {
-          const int r = e / d, k = e % d;
-          gxi[r * sd + k] = bi * TT + r < n ? S.xs[(bi * TT + r) * d + k] : 0.f;
-          gxj[r * sd + k] = bj * TT + r < n ? S.xs[(bj * TT + r) * d + k] : 0.f;
-        }
-        __syncthreads();
-        for (int e = threadIdx.x; e < TT * TT; e += BNT) {
-          const int il = e / TT, jl = e % TT;
-          const int i = bi * TT + il, j = bj * TT + jl;
-          float v;
-          if (i >= n || j >= n) {
-            v = i == j ? 1.f : 0.f;
-          } else {
-            float sq = 0.f;
-            for (int k = 0; k < d; ++k) {
-              const float df = gxi[il * sd + k] - gxj[jl * sd + k];
-              sq = fmaf(df, df, sq);
-            }
-            v = kval<float>(KIND, sq, s2, ka);
-            if (i == j) v = (float)((double)v + noise_diag);
-          }
-          S.A[(int64_t)i * ld + j] = v;
-        }
-        __syncthreads();
-      }
-    });
-  }
+  gram_blocks(I, S, np, s2, ka, noise_diag, smem);
   __syncthreads();
   chol_inv<BK>(S, ld, np, I.info, smem);
   __syncthreads();
