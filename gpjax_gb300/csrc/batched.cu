@@ -224,7 +224,7 @@ __device__ __forceinline__ int tile_col(int v) { return (threadIdx.x & 31) * 4 +
 // of two raw stages (32 KB each, two slices in flight), then split into TF32
 // hi / lo by all 512 threads and stored into the 128B-swizzled K-major layout
 // the MMA reads (one split stage of A_hi, A_lo, B_hi, B_lo, 64 KB, 1024-byte
-// aligned).  Thread 0 issues the slice's 3 products (A_lo B_hi, A_hi B_lo,
+// aligned).  An elected lane of the converged warp 0 issues the slice's 3 products (A_lo B_hi, A_hi B_lo,
 // then A_hi B_hi) x 4 K steps of tcgen05.mma kind::tf32 into one of two TMEM
 // accumulators and commits to that accumulator's mbarrier; while they run,
 // every thread adds the previous slice's accumulator (its 32 columns) to
@@ -392,15 +392,16 @@ __device__ void tc_setup(long long stall) {
 }
 
 // Kernel end (every thread): after a timeout (when later waits were skipped
-// and the counters no longer tell which MMAs were seen to complete), thread
-// 0, which issued every MMA, commits once more to `fin` -- it arrives when
-// all of them have completed -- and waits for that (bounded) before the TMEM
-// columns are released.
+// and the counters no longer tell which MMAs were seen to complete), the
+// lane that issued every MMA commits once more to `fin` -- it arrives when
+// all of them have completed -- and its warp waits for that (bounded) before
+// the TMEM columns are released.
 __device__ void tc_teardown() {
   TcState& st = tc_state();
   __syncthreads();
-  if (threadIdx.x == 0 && st.err && (st.issued[0] | st.issued[1])) {
-    tc::mma_commit(&st.fin);
+  if (threadIdx.x < 32 && st.err && (st.issued[0] | st.issued[1])) {
+    if (tc::elect_one()) tc::mma_commit(&st.fin);  // the lane that issued the MMAs
+    __syncwarp();
     tc::mbar_wait_own(&st.fin, 0u, kTcWait);
   }
   tc::tc_fence_before();
@@ -428,6 +429,7 @@ __device__ void tile_mma_tc(const float* __restrict__ A, int lda, const float* _
   // completions consumed per accumulator (the same in every thread; two
   // scalars, not an array indexed at run time, which would live in memory)
   uint32_t nb0 = st.n[0], nb1 = st.n[1];
+  const uint32_t tm = __shfl_sync(0xffffffffu, st.tmem, 0);
   float c32[32];
   if constexpr (ACC_IN) {  // the incoming accumulator (fragment layout) to the row layout
     float* Cs = reinterpret_cast<float*>(base);
@@ -487,27 +489,34 @@ __device__ void tile_mma_tc(const float* __restrict__ A, int lda, const float* _
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     tc::tc_fence_before();
     __syncthreads();  // the split stage is written; raw stage sl & 1 is free
-    copy(sl + 2);
-    if (threadIdx.x == 0) {
+    // The MMAs before the copies, and by an elected lane of the converged
+    // warp: from a thread picked by its index each MMA's descriptors cost ~80
+    // clocks of register moves, 1000 a slice, before the copies' 370 (512
+    // instances: 31.4 to 29.5 ms).
+    if (warp == 0) {
       tc::tc_fence_after();
       const uint32_t a = tc::smem_u32(sp);
       const uint64_t ahi = tc::sdesc<128>(a), alo = tc::sdesc<128>(a + 16384);
       const uint64_t bhi = tc::sdesc<128>(a + 32768), blo = tc::sdesc<128>(a + 49152);
-      const uint32_t tacc = st.tmem + (uint32_t)((sl & 1) * 128);
+      const uint32_t tacc = tm + (uint32_t)((sl & 1) * 128);
       constexpr uint32_t idesc = tc::idesc_tf32(128, 128);
-      // the small cross products first, the hi x hi products last: the
-      // accumulator's roundings at the size of the result happen 4 times
-      // per slice instead of 12
+      if (tc::elect_one()) {
+        // the small cross products first, the hi x hi products last: the
+        // accumulator's roundings at the size of the result happen 4 times
+        // per slice instead of 12
 #pragma unroll
-      for (int ks = 0; ks < 4; ++ks)
-        tc::mma_tf32(tacc, alo + 2 * ks, bhi + 2 * ks, idesc, ks ? 1u : 0u);
+        for (int ks = 0; ks < 4; ++ks)
+          tc::mma_tf32(tacc, alo + 2 * ks, bhi + 2 * ks, idesc, ks ? 1u : 0u);
 #pragma unroll
-      for (int ks = 0; ks < 4; ++ks) tc::mma_tf32(tacc, ahi + 2 * ks, blo + 2 * ks, idesc, 1u);
+        for (int ks = 0; ks < 4; ++ks) tc::mma_tf32(tacc, ahi + 2 * ks, blo + 2 * ks, idesc, 1u);
 #pragma unroll
-      for (int ks = 0; ks < 4; ++ks) tc::mma_tf32(tacc, ahi + 2 * ks, bhi + 2 * ks, idesc, 1u);
-      tc::mma_commit(&st.bar[sl & 1]);
-      st.issued[sl & 1] += 1;
+        for (int ks = 0; ks < 4; ++ks) tc::mma_tf32(tacc, ahi + 2 * ks, bhi + 2 * ks, idesc, 1u);
+        tc::mma_commit(&st.bar[sl & 1]);
+        st.issued[sl & 1] += 1;
+      }
+      __syncwarp();
     }
+    copy(sl + 2);
     if (sl > 0) {  // slice sl - 1's accumulator, complete since the wait above
       drain((sl - 1) & 1);
       if ((sl - 1) & 1) ++nb1; else ++nb0;
