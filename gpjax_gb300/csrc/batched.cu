@@ -224,8 +224,8 @@ __device__ __forceinline__ int tile_col(int v) { return (threadIdx.x & 31) * 4 +
 // of two raw stages (32 KB each, two slices in flight), then split into TF32
 // hi / lo by all 512 threads and stored into the 128B-swizzled K-major layout
 // the MMA reads (one split stage of A_hi, A_lo, B_hi, B_lo, 64 KB, 1024-byte
-// aligned).  An elected lane of the converged warp 0 issues the slice's 3 products (A_lo B_hi, A_hi B_lo,
-// then A_hi B_hi) x 4 K steps of tcgen05.mma kind::tf32 into one of two TMEM
+// aligned).  An elected lane of the converged warp 0 issues the slice's 3
+// products (A_lo B_hi, A_hi B_lo, then A_hi B_hi) x 4 K steps of tcgen05.mma kind::tf32 into one of two TMEM
 // accumulators and commits to that accumulator's mbarrier; while they run,
 // every thread adds the previous slice's accumulator (its 32 columns) to
 // float32 registers (round to nearest: 12 MMAs per TMEM accumulation) and
@@ -343,6 +343,7 @@ __device__ __forceinline__ void tc_split(const float* raw, char* hi, char* lo) {
 // still waited for, so none is in flight when the CTA moves on.
 __device__ __forceinline__ void tc_wait(int b, uint32_t n) {
   TcState& st = tc_state();
+  if (st.stall <= 0 && tc::mbar_try_wait(&st.bar[b], n & 1u)) return;
   if (*(volatile int*)&st.err) return;
   if (st.stall > 0 && !*(volatile int*)&st.stalled) {
     if (!tc::mbar_wait_own(&st.never, 0u, st.stall)) st.stalled = 1;
@@ -460,16 +461,38 @@ __device__ void tile_mma_tc(const float* __restrict__ A, int lda, const float* _
     }
     cp_async_commit();
   };
-  auto drain = [&](int b) {  // accumulator b, complete, into c32
-    const uint32_t ta =
-        st.tmem + ((uint32_t)(32 * (warp & 3)) << 16) + (uint32_t)(b * 128 + 32 * (warp >> 2));
+  auto drain16 = [&](int b, int h) {  // 16 columns of accumulator b, complete, into c32
+    uint32_t v[16];
+    tc::tmem_ld16_nowait(tm + ((uint32_t)(32 * (warp & 3)) << 16) +
+                             (uint32_t)(b * 128 + 32 * (warp >> 2) + 16 * h),
+                         v);
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {  // two 16-column loads: fewer live registers
-      uint32_t v[16];
-      tc::tmem_ld16_nowait(ta + 16 * h, v);
-      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+    for (int k = 0; k < 16; ++k) c32[16 * h + k] += __uint_as_float(v[k]);
+  };
+  // Product `part` of the slice in the split stage (warp 0): A_lo B_hi,
+  // A_hi B_lo, A_hi B_hi.  The small cross products first, the hi x hi
+  // products last: the accumulator's roundings at the size of the result
+  // happen 4 times per slice instead of 12.
+  const uint32_t sp32 = tc::smem_u32(sp);
+  const uint64_t ahi = tc::sdesc<128>(sp32), alo = tc::sdesc<128>(sp32 + 16384);
+  const uint64_t bhi = tc::sdesc<128>(sp32 + 32768), blo = tc::sdesc<128>(sp32 + 49152);
+  auto issue = [&](int sl, auto part) {
+    constexpr int P = decltype(part)::value;
+    constexpr uint32_t idesc = tc::idesc_tf32(128, 128);
+    if (warp == 0) {
+      if (tc::elect_one()) {
+        const uint32_t tacc = tm + (uint32_t)((sl & 1) * 128);
+        const uint64_t a = P == 0 ? alo : ahi, b = P == 1 ? blo : bhi;
 #pragma unroll
-      for (int k = 0; k < 16; ++k) c32[16 * h + k] += __uint_as_float(v[k]);
+        for (int ks = 0; ks < 4; ++ks)
+          tc::mma_tf32(tacc, a + 2 * ks, b + 2 * ks, idesc, P || ks ? 1u : 0u);
+        if (P == 2) {
+          tc::mma_commit(&st.bar[sl & 1]);
+          st.issued[sl & 1] += 1;
+        }
+      }
+      __syncwarp();
     }
   };
   if (nsl > 0) {
@@ -489,36 +512,19 @@ __device__ void tile_mma_tc(const float* __restrict__ A, int lda, const float* _
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     tc::tc_fence_before();
     __syncthreads();  // the split stage is written; raw stage sl & 1 is free
-    // The MMAs before the copies, and by an elected lane of the converged
-    // warp: from a thread picked by its index each MMA's descriptors cost ~80
-    // clocks of register moves, 1000 a slice, before the copies' 370 (512
-    // instances: 31.4 to 29.5 ms).
-    if (warp == 0) {
-      tc::tc_fence_after();
-      const uint32_t a = tc::smem_u32(sp);
-      const uint64_t ahi = tc::sdesc<128>(a), alo = tc::sdesc<128>(a + 16384);
-      const uint64_t bhi = tc::sdesc<128>(a + 32768), blo = tc::sdesc<128>(a + 49152);
-      const uint32_t tacc = tm + (uint32_t)((sl & 1) * 128);
-      constexpr uint32_t idesc = tc::idesc_tf32(128, 128);
-      if (tc::elect_one()) {
-        // the small cross products first, the hi x hi products last: the
-        // accumulator's roundings at the size of the result happen 4 times
-        // per slice instead of 12
-#pragma unroll
-        for (int ks = 0; ks < 4; ++ks)
-          tc::mma_tf32(tacc, alo + 2 * ks, bhi + 2 * ks, idesc, ks ? 1u : 0u);
-#pragma unroll
-        for (int ks = 0; ks < 4; ++ks) tc::mma_tf32(tacc, ahi + 2 * ks, blo + 2 * ks, idesc, 1u);
-#pragma unroll
-        for (int ks = 0; ks < 4; ++ks) tc::mma_tf32(tacc, ahi + 2 * ks, bhi + 2 * ks, idesc, 1u);
-        tc::mma_commit(&st.bar[sl & 1]);
-        st.issued[sl & 1] += 1;
-      }
-      __syncwarp();
-    }
+    // By an elected lane of the converged warp: from a thread picked by its
+    // index each MMA's descriptors cost ~80 clocks of register moves.  The
+    // tensor pipe takes the next MMA when an earlier one is done, so the 12
+    // of a slice keep their warp for 900 clocks; its share of the copies and
+    // of the previous slice's accumulator goes in between the products.
+    tc::tc_fence_after();
+    issue(sl, std::integral_constant<int, 0>{});
     copy(sl + 2);
-    if (sl > 0) {  // slice sl - 1's accumulator, complete since the wait above
-      drain((sl - 1) & 1);
+    issue(sl, std::integral_constant<int, 1>{});
+    if (sl > 0) drain16((sl - 1) & 1, 0);  // complete since the wait above
+    issue(sl, std::integral_constant<int, 2>{});
+    if (sl > 0) {
+      drain16((sl - 1) & 1, 1);
       if ((sl - 1) & 1) ++nb1; else ++nb0;
       tc::tc_fence_before();  // ordered before the next barrier, after which it is rewritten
     }
@@ -528,7 +534,8 @@ __device__ void tile_mma_tc(const float* __restrict__ A, int lda, const float* _
     const int b = (nsl - 1) & 1;
     tc_wait(b, b ? nb1 : nb0);
     tc::tc_fence_after();
-    drain(b);
+    drain16(b, 0);
+    drain16(b, 1);
     if (b) ++nb1; else ++nb0;
     tc::tc_fence_before();
   }
@@ -1138,12 +1145,16 @@ __device__ __noinline__ void residual(const BatchInst& I, const Slot& S, int np,
 // The Gram matrix's lower 128-blocks (diagonal blocks in full), identity past
 // n.  A thread keeps one column's inputs in registers and takes every fourth
 // row of the block, whose inputs a warp reads from shared memory by
-// broadcast (gx: 128 rows of 16).
+// broadcast (gx: 128 rows of 16).  The noise is added to the diagonal of a
+// finished block: tested for at each element, its float64 addition and two
+// conversions went through the float64 pipe for all of them, 28k clocks a
+// block.
 __device__ __noinline__ void gram_blocks(const BatchInst& I, const Slot& S, int np, float s2,
                                          float ka, double noise_diag, float* gx) {
   const int n = I.n, d = I.d, ld = np;
   const int nb = np / TT, nt = nb * (nb + 1) / 2;
   const int jl = threadIdx.x % TT;
+  float* A = S.A;
   with_kind_dim(I.kind, d, [&](auto kind_c, auto dim_c) {
     constexpr int KIND = decltype(kind_c)::value, DC = decltype(dim_c)::value;
     for (int t = 0; t < nt; ++t) {
@@ -1178,9 +1189,15 @@ __device__ __noinline__ void gram_blocks(const BatchInst& I, const Slot& S, int 
           sq = fmaf(df, df, sq);
         }
         float v = kval<float>(KIND, sq, s2, ka);
-        if (i == j) v = (float)((double)v + noise_diag);
         if (i >= n || j >= n) v = i == j ? 1.f : 0.f;
-        S.A[(int64_t)i * ld + j] = v;
+        A[(int64_t)i * ld + j] = v;
+      }
+      if (bi == bj) {
+        __syncthreads();
+        if (threadIdx.x < TT && j < n) {
+          float* a = A + (int64_t)j * ld + j;
+          *a = (float)((double)*a + noise_diag);
+        }
       }
     }
   });
