@@ -1,0 +1,134 @@
+"""GPU: the float64 form where its kernels and their dispatch change shape --
+the 64-wide fixed-point Cholesky blocks and their panels, the tile edges of the
+gradient reduction and of the cross-covariance cotangents, the column blocks
+of the collapsed bound, and the range of the integer exp and sqrt."""
+import numpy as np
+import pytest
+import torch
+
+import gpjax_gb300 as gpx
+from gpjax_gb300 import linalg
+from oracle import gp_oracle as O
+from tests._gpu_helpers import KINDS, grads_of, make_posterior, to_cuda_params
+from tests.test_sgpr_gpu import _oracle as elbo_oracle, _run as elbo_run
+
+pytestmark = pytest.mark.gpu
+
+U = 2.0 ** -53
+
+
+# |A - L L^T| <= (n + 1) u |L| |L|^T <= (n + 1) u sqrt(a_ii a_jj) for any order
+# of a float64 Cholesky's sums; the fixed-point block rounds an entry at 2^-60
+# of a scale below 2 sqrt(a_ii), well inside u.  A factor of 4 covers the panel
+# and update products' own scales (powers of two above a row's largest entry).
+@pytest.mark.parametrize("n", [1, 2, 63, 64, 65, 127, 128, 129, 200, 513, 900])
+@pytest.mark.parametrize("spread", [0.0, 40.0])
+def test_cholesky_blocks(cuda_lib, n, spread):
+    rng = np.random.default_rng(n)
+    b = rng.standard_normal((n, n + 3))
+    s = np.exp(rng.uniform(-spread, spread, n))
+    a = (b @ b.T + 0.01 * np.eye(n)) * s[:, None] * s[None, :]
+    a = np.tril(a) + np.tril(a, -1).T
+    low = linalg.lower_cholesky(linalg.Dense(torch.as_tensor(a, device="cuda"))).to_dense()
+    low = np.tril(low.cpu().numpy()).astype(np.longdouble)
+    size = np.sqrt(np.diag(a))
+    err = np.abs((low @ low.T - a) / (size[:, None] * size[None, :]).astype(np.longdouble))
+    assert float(err.max()) <= 4 * (n + 1) * U, float(err.max()) / U
+
+
+# Same bounds as the float64 parity test of the marginal likelihood, at the
+# sizes on either side of each tile edge of the gradient reduction.
+@pytest.mark.parametrize("kind,n,d", [(0, 128, 3), (1, 130, 5), (2, 384, 2), (0, 385, 9),
+                                      (1, 1536, 4), (2, 1537, 3)])
+def test_mll_tile_edges(cuda_lib, kind, n, d):
+    rng = np.random.default_rng(n + d)
+    x = rng.uniform(-2, 2, size=(n, d))
+    y = np.sin(x).sum(1, keepdims=True) + 0.1 * rng.standard_normal((n, 1))
+    ls = np.exp(rng.uniform(np.log(0.5), np.log(2.0), d))
+    post = to_cuda_params(make_posterior(kind, ls, 1.2, 0.3, 0.1))
+    val = gpx.objectives.conjugate_mll(post, gpx.Dataset(X=x, y=y), precision="fp64")
+    val.backward()
+    got = grads_of(post)
+    ref = O.conjugate_mll(kind, x, y, ls, 1.2, 0.3, 0.1)
+    _, g = O.conjugate_mll_torch(kind, x, y, ls, 1.2, 0.3, 0.1, lu=False)
+    gref = np.concatenate([np.atleast_1d(g["lengthscale"]),
+                           [g["variance"], g["obs_stddev"], g["constant"]]])
+    assert abs(float(val) - ref) <= 1e-10 * max(1.0, abs(ref))
+    assert np.allclose(got, gref, rtol=1e-7, atol=1e-8 * max(1.0, np.abs(gref).max()))
+
+
+# 16-, 32- and 64-wide tiles with ragged last tiles, and d on both sides of the
+# 64-wide form's bound.  Sums of at most n terms of mixed sign, each with a few
+# roundings and an exp whose argument is below 100: 1e-12 of the sum of the
+# terms' sizes is 4e3 times u n at n = 2.
+@pytest.mark.parametrize("kind,n,m,d", [(0, 15, 17, 3), (1, 1, 40, 1), (2, 385, 417, 5),
+                                        (0, 1121, 1217, 16), (1, 1121, 1217, 17)])
+def test_cross_covariance_cotangent_tiles(cuda_lib, kind, n, m, d):
+    rng = np.random.default_rng(n + m + d)
+    x, z = rng.uniform(-2, 2, (n, d)), rng.uniform(-2, 2, (m, d))
+    G, ls = rng.standard_normal((n, m)), np.exp(rng.uniform(0.0, 1.0, d))
+    k = KINDS[kind](lengthscale=ls, variance=1.3)
+    for p in (k.lengthscale, k.variance):
+        p.to("cuda").requires_grad_(True)
+    xt, zt = (torch.as_tensor(v, device="cuda").requires_grad_(True) for v in (x, z))
+    K = k.cross_covariance(xt, zt)
+    got = torch.autograd.grad(K, [k.lengthscale.value, k.variance.value, xt, zt],
+                              torch.as_tensor(G, device="cuda"))
+    xr, zr, lr, vr = (torch.as_tensor(v, dtype=torch.float64).requires_grad_(True)
+                      for v in (x, z, ls, 1.3))
+    sq = (((xr[:, None] - zr[None]) / lr) ** 2).sum(-1)
+    t = torch.sqrt(sq)
+    Kr = vr * [torch.exp(-0.5 * sq), (1 + 3 ** 0.5 * t) * torch.exp(-3 ** 0.5 * t),
+               (1 + 5 ** 0.5 * t + 5.0 / 3.0 * sq) * torch.exp(-5 ** 0.5 * t)][kind]
+    ref = torch.autograd.grad(Kr, [lr, vr, xr, zr], torch.as_tensor(G))
+    assert torch.allclose(K.detach().cpu(), Kr.detach(), rtol=1e-12, atol=0)
+    # sizes of the terms: |G| times bounds of |dK/d.|, at most 4 K-sized factors
+    for g, r, terms in zip(got, ref, (n * m, n * m, m, n)):
+        assert float((g.cpu() - r).abs().max()) <= 1e-12 * 4 * 1.3 * 4 * terms
+
+
+# Columns on both sides of a 65536-wide block; the bounds of the parity test of
+# the collapsed bound (the inducing points are spread: K is well conditioned).
+@pytest.mark.parametrize("n,m", [(65536, 33), (65537, 150)])
+def test_elbo_column_blocks(cuda_lib, n, m):
+    rng = np.random.default_rng(n)
+    x = rng.uniform(-2, 2, size=(n, 2))
+    y = np.sin(x).sum(1, keepdims=True) + 0.1 * rng.standard_normal((n, 1))
+    Z, ls = rng.uniform(-2, 2, (m, 2)), np.array([0.3, 0.4])
+    val, g, gz = elbo_run(1, x, y, Z, ls, 1.2, 0.3, 0.1)
+    ref, gref, gzref = elbo_oracle(1, x, y, Z, ls, 1.2, 0.3, 0.1)
+    cond = np.linalg.cond(O.gram(1, Z, ls, 1.2) + 1e-6 * np.eye(m))
+    tol = max(1e-9, 1e-12 * cond)
+    assert abs(val - ref) <= tol * abs(ref)
+    assert np.allclose(g, gref, rtol=max(1e-6, 10 * tol), atol=1e-7 * np.abs(gref).max())
+    assert np.allclose(gz, gzref, rtol=max(1e-6, 10 * tol), atol=1e-7 * np.abs(gzref).max())
+
+
+# exp(-a) with a formed in float64 from t = sqrt(sq): a is off by at most 4 u a
+# (square, sqrt, constant, product), so the value by (4 a + 6) u plus the
+# functions' own last bit; past 708 the results are below 2^-1021, where one
+# step of the subnormal range (2^-1074) is allowed as well.
+@pytest.mark.parametrize("kind", [0, 1, 2])
+def test_kernel_values_over_range(cuda_lib, kind):
+    r = np.concatenate([[0.0], np.exp(np.linspace(np.log(1e-9), np.log(400.0), 3000)),
+                        np.linspace(30.0, 45.0, 500)])
+    k = KINDS[kind](lengthscale=1.0, variance=1.0)
+    k.lengthscale.to("cuda")
+    k.variance.to("cuda")
+    got = k.cross_covariance(torch.as_tensor(r[:, None], device="cuda"),
+                             torch.zeros(1, 1, dtype=torch.float64, device="cuda"))
+    got = got.detach().cpu().numpy()[:, 0]
+    q = r.astype(np.longdouble)
+    t = np.maximum(q, np.longdouble(1e-18))  # the kernels' floor of sq, 1e-36
+    if kind == 0:
+        a, f = q * q / 2, 1
+    elif kind == 1:
+        a = np.sqrt(np.longdouble(3)) * t
+        f = 1 + a
+    else:
+        a = np.sqrt(np.longdouble(5)) * t
+        f = 1 + a + a * a / 3
+    ref = f * np.exp(-a)
+    tol = (4 * a + 12) * U * ref + np.longdouble(2.0) ** -1074 * (1 + f)
+    tol = np.where(ref < 2.0 ** -1021, np.maximum(tol, ref), tol)
+    assert np.all(np.abs(got - ref) <= tol)
