@@ -1,8 +1,10 @@
-// CUDA-core (SIMT) dense linear algebra for the float64 form and for the
-// parts of the mixed form that stay off the tensor cores: a batched NT GEMM
-// with triangular operand masks, the blocked right-looking Cholesky
-// (diagonal block in shared memory, row-substitution panel solve, SYRK
-// trailing update), the recursive triangular inverse and triangular GEMVs.
+// Dense linear algebra of the float64 form and of the parts of the mixed form
+// that stay off the tensor-core GEMM: a batched NT GEMM on CUDA cores with
+// triangular operand masks, the blocked Cholesky (64-wide diagonal blocks and
+// their panels in fixed point for float64, fixed64.cuh; trailing updates by
+// the split GEMM of xgemm.cuh where the product is large enough and scratch
+// for its digit planes was given, else by the CUDA-core GEMM), the recursive
+// triangular inverse and triangular GEMVs.
 //
 // The reference reaches the same arithmetic through XLA: jnp.linalg.cholesky
 // (gpjax/linalg/operations.py:54-55), jsp.linalg.solve_triangular
@@ -720,7 +722,7 @@ __global__ void __launch_bounds__(NB) trtri_diag_kernel(const T* L, int64_t ldl,
 // The float64 leaf: right-looking forward substitution on the identity, all
 // threads on every step (row k final, the rows below lose L[i, k] / L[k, k]
 // times it).  One thread per column, as above, is a chain of dependent
-// products: 130 us; this one issues each product once: TRTRI64_US.
+// products: 130 us; this one issues each product once: 35 us.
 template <int NB>
 __global__ void __launch_bounds__(256)
     trtri_diag64_kernel(const double* L, int64_t ldl, int n, double* M, int64_t ldm, double* V,

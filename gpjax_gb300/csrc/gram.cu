@@ -6,9 +6,9 @@
 // (computations/base.py:56-72).  Each pointwise kernel divides both inputs by
 // the lengthscale before taking the squared distance
 // (kernels/stationary/rbf.py:41-43, matern32.py:46-47, matern52.py:45-46).
-// Here the inputs are scaled once (xs = x / l), then each CTA stages a
-// 64-row panel of each side in shared memory and every thread produces a
-// column strip of the output tile.
+// Here the inputs are scaled once (xs = x / l, or once per tile), then each
+// CTA stages a panel of each side in shared memory and every thread produces
+// a column strip of the output tile.
 #include "gpk_internal.cuh"
 #include "simt_tile.cuh"
 

@@ -12,8 +12,8 @@
 //   d loocv / d mean = sum_i u_i,
 // so the kernel-hyperparameter gradient is the cross-covariance VJP of G and the
 // noise gradient 2 obs_stddev tr(G).  Everything is float64: Sigma's Cholesky
-// factor, its triangular inverse, W = L^-T L^-1 and W diag(a) W as SIMT GEMMs,
-// alpha refined once against a float64 residual.
+// factor, its triangular inverse, W = L^-T L^-1 and W diag(a) W as split or
+// CUDA-core GEMMs by size (xgemm.cuh), alpha refined once against a float64 residual.
 #include <algorithm>
 #include <climits>
 #include "gpk_internal.cuh"

@@ -14,8 +14,9 @@
 // from the scaled inputs; the reference differentiates the same sequence
 // with JAX reverse mode.
 //
-// The m x n work has two forms.  Plain (float64): Phi, P, c and the fused
-// H Phi adjoint on CUDA cores.  Mixed: Phi is generated once in float32 and
+// The m x n work has two forms.  Plain (float64): Phi by blocks of columns, P
+// and H Phi by the split float64 GEMM where it is large enough (xgemm.cuh),
+// else on CUDA cores.  Mixed: Phi is generated once in float32 and
 // stored as TF32 hi/lo pairs in both layouts (m x n for P, n x m for the
 // adjoint); P = Phi Phi^T per n-chunk and G = H Phi run on the tensor cores
 // (split-TF32 tcgen05 GEMM), with G reduced against dPhi/dtheta, dPhi/dZ in

@@ -8,7 +8,7 @@
 // same split in float16 instead (same 11-bit significand, twice the MMA rate,
 // half the operand bytes), on operands whose rows were scaled by powers of
 // two into float16's range; the epilogue undoes the scales exactly.  Operands
-// are staged by TMA (swizzled) into a shared-memory ring, one elected thread
+// are staged by TMA (swizzled) into a shared-memory ring, one elected lane
 // issues tcgen05.mma into float32 accumulators in tensor memory, and eight
 // epilogue warps read them back with tcgen05.ld and apply a fused epilogue
 // (trailing update, split store with optional transpose, the MLL adjoint

@@ -21,16 +21,31 @@ struct VjpShape {
   int te, tn, strips, per;  // tile edge, column tiles, strips of row tiles, row tiles per strip
 };
 
-// 64-wide tiles once they fill the chip twice (d <= 16: registers), 32-wide from
-// one wave, else 16.
+// 64-wide tiles from 256 of them (d <= 16: registers): 165 us against 187 with
+// 32-wide ones at 1024 x 1024, d = 5, and 144 against 150 (d = 12), 92 against
+// 89 (d = 5) at 640 x 640; 16-wide ones are no faster at any size (97 against
+// 84 us at 384 x 384).  The row tiles are cut into strips that fill whole
+// waves of the blocks an SM holds (by registers 3, 2 or 1), a block costing
+// its tiles and about 0.15 of one more: 3000 x 1100, d = 5 took 539 us in 432
+// blocks of two tiles, one wave and a 0.4, and 439 in 288 of three.
 VjpShape vjp_shape(int64_t n, int64_t m, int d) {
-  VjpShape s;
-  s.te = d <= 16 && cdiv(n, 64) * cdiv(m, 64) >= 304 ? 64 : cdiv(n, 32) * cdiv(m, 32) >= 152 ? 32 : 16;
-  const int64_t tm = cdiv(n, s.te);
+  VjpShape s{};
+  s.te = d <= 16 && cdiv(n, 64) * cdiv(m, 64) >= 256 ? 64 : 32;
+  const int64_t tm = cdiv(n, s.te), slots = 152 * (d <= 4 ? 3 : d <= 8 ? 2 : 1);
   s.tn = (int)cdiv(m, s.te);
-  const int64_t want = s.tn ? std::min<int64_t>(tm, std::max<int64_t>(1, cdiv(608, s.tn))) : 0;
-  s.per = want ? (int)cdiv(tm, want) : 0;
-  s.strips = s.per ? (int)cdiv(tm, s.per) : 0;
+  if (!s.tn) return s;
+  double best = 0.0;
+  // at most about 8 waves (bounded partial sums)
+  for (int64_t per = std::min(tm, cdiv(tm * s.tn, 8 * slots)); per > 0 && per <= tm; ++per) {
+    const int64_t strips = cdiv(tm, per);
+    const double cost = (double)cdiv(strips * s.tn, slots) * ((double)per + 0.15);
+    if (!s.per || cost < best) {
+      best = cost;
+      s.per = (int)per;
+      s.strips = (int)strips;
+    }
+    if (strips * s.tn <= slots) break;  // one wave: longer strips only cost more
+  }
   return s;
 }
 
@@ -255,10 +270,7 @@ cudaError_t cross_cov_vjp(int kind, int n, int m, int d, const double* x, int64_
   if (n > 0 && m > 0) {
     auto run = [&](auto dim) {
       constexpr int D = decltype(dim)::value;
-      constexpr int BIG = D <= 16 ? 64 : 32;
-      auto* f = s.te == 64   ? vjp_launch<D, BIG>
-                : s.te == 32 ? vjp_launch<D, 32>
-                             : vjp_launch<D, 16>;
+      auto* f = s.te == 64 ? vjp_launch<D, D <= 16 ? 64 : 32> : vjp_launch<D, 32>;
       return f(kind, n, m, d, s, x, ldx, y, ldy, theta, n_ls, G, ldg, b, stream);
     };
     const cudaError_t e = d <= 4    ? run(std::integral_constant<int, 4>{})

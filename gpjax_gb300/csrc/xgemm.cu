@@ -20,7 +20,12 @@ constexpr int XTHREADS = 320;     // w0 TMA, w1 MMA + TMEM, w2..w9 epilogue
 constexpr int XEPI_WARPS = 8, XEPI_THREADS = XEPI_WARPS * 32;
 constexpr int XHC = XN / 2;       // accumulator columns of one epilogue thread
 constexpr int XTLD = XN + 1;      // staged tile row stride (doubles)
-constexpr double XMIN_MULTS = 5e5;  // below, a CUDA-core product is as quick as the split
+// Multiply-adds from which a product whose operands are split first beats the
+// CUDA-core tiles: 7e6 (192^3) 39 us against 23, 8.4e6 34 against 45 (512 x 128
+// x 128) and 63 against 53 (128 x 128 x 512), 1.7e7 (256^3) 43 against 86.
+// Marginal likelihood with the line at 5e5 / 8e6 / 1.6e7 / 3.2e7: n = 384
+// 860 / 757 / 745 / 816 us, n = 1024 1979 / 1930 / 1955 / 1955 us.
+constexpr double XMIN_MULTS = 8e6;
 constexpr int XMAX_K = 1 << 18;   // the drained 64-bit sums stay below K * 2^41
 
 // K slices summed by one accumulator before it is drained: a group holds up to
