@@ -197,6 +197,13 @@ __device__ __forceinline__ float tf32_round(float x) {
   return __uint_as_float(r);
 }
 
+// The same rounding (to nearest, ties away) in two integer instructions of
+// the ALU pipe instead of a conversion.  A NaN's bits may wrap to a number:
+// for the hi part of a split only, whose lo part then carries the NaN.
+__device__ __forceinline__ float tf32_hi(float x) {
+  return __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xffffe000u);
+}
+
 // warp / block reductions
 template <typename T>
 __device__ __forceinline__ T warp_sum(T v) {

@@ -289,6 +289,10 @@ __device__ __forceinline__ void ff_acc(float& hi, float& lo, float a) {
 // the block's columns summed in float-float (d split into float hi + lo) into
 // cpart[block column][c (m) | Phi 1 (m)].  The grid covers npad columns (a
 // multiple of KCHUNK; PG_X * PG_SUB divides KCHUNK).
+// Instruction issue bounds it, ahead of the 16 bytes written per element: the
+// kernel kind is resolved outside the loops, four coordinates are read at a
+// time and the hi parts rounded by integers (n = 1e6, m = 1024, d = 8: 4.3 ms
+// before, 3.8 after; the bound's whole evaluation 25.0 -> 24.5 ms).
 template <int D>
 __global__ void __launch_bounds__(256)
     sg_phi_gen(int kind, int m, int n, int64_t npad, int d, const float* __restrict__ zs,
@@ -298,12 +302,12 @@ __global__ void __launch_bounds__(256)
                double* __restrict__ cpart) {
   static_assert(KCHUNK % (PG_X * PG_SUB) == 0, "generation blocks must not straddle chunks");
   __shared__ __align__(16) float tile[PG_I][PG_X + 1];
-  __shared__ float sz[PG_I][D + 1];
+  __shared__ __align__(16) float sz[PG_I][D];  // read by broadcast
   __shared__ float sxp[PG_X][D + 1];
   __shared__ float sdh[PG_X], sdl[PG_X];
   const int i0 = blockIdx.y * PG_I;
   const int64_t xb0 = (int64_t)blockIdx.x * PG_X * PG_SUB;
-  const float s2 = (float)theta[n_ls];
+  const float s2 = (float)theta[n_ls], ka = kshape<float>(kind, theta, n_ls);
   const int t = threadIdx.x;
   for (int e = t; e < PG_I * D; e += 256) {
     const int r = e / D, k = e % D;
@@ -333,21 +337,32 @@ __global__ void __launch_bounds__(256)
       float xr[D];
 #pragma unroll
       for (int k = 0; k < D; ++k) xr[k] = sxp[a][k];
-      for (int r = t >> 7; r < PG_I; r += 2) {
-        float sq = 0.f;
+      with_kind(kind, [&](auto kind_c) {
+        constexpr int KIND = decltype(kind_c)::value;
+#pragma unroll 2
+        for (int r = t >> 7; r < PG_I; r += 2) {
+          float sq = 0.f;
 #pragma unroll
-        for (int k = 0; k < D; ++k) {
-          const float df = sz[r][k] - xr[k];
-          sq = fmaf(df, df, sq);
+          for (int k = 0; k < D; k += 4) {
+            const float4 z = *reinterpret_cast<const float4*>(&sz[r][k]);
+            float df = z.x - xr[k];
+            sq = fmaf(df, df, sq);
+            df = z.y - xr[k + 1];
+            sq = fmaf(df, df, sq);
+            df = z.z - xr[k + 2];
+            sq = fmaf(df, df, sq);
+            df = z.w - xr[k + 3];
+            sq = fmaf(df, df, sq);
+          }
+          const float v = gx < n ? kval<float>(KIND, sq, s2, ka) : 0.f;
+          tile[r][a] = v;
+          if (i0 + r < m) {
+            const float h = tf32_hi(v);
+            Phh[cbase + (int64_t)(i0 + r) * KCHUNK] = h;
+            Phl[cbase + (int64_t)(i0 + r) * KCHUNK] = tf32_round(v - h);
+          }
         }
-        const float v = gx < n ? kval<float>(kind, sq, s2, kshape<float>(kind, theta, n_ls)) : 0.f;
-        tile[r][a] = v;
-        if (i0 + r < m) {
-          const float h = tf32_round(v);
-          Phh[cbase + (int64_t)(i0 + r) * KCHUNK] = h;
-          Phl[cbase + (int64_t)(i0 + r) * KCHUNK] = tf32_round(v - h);
-        }
-      }
+      });
     }
     __syncthreads();
     if (i0 + bi < m) {  // transposed pass and the c / Phi 1 sums
@@ -355,7 +370,7 @@ __global__ void __launch_bounds__(256)
         const int64_t gx = x0 + c;
         if (gx >= n) break;
         const float v = tile[bi][c];
-        const float h = tf32_round(v);
+        const float h = tf32_hi(v);
         PTh[gx * ldt + i0 + bi] = h;
         PTl[gx * ldt + i0 + bi] = tf32_round(v - h);
         const float p = __fmul_rn(v, sdh[c]);
