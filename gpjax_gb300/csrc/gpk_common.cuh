@@ -212,6 +212,31 @@ __device__ __forceinline__ T warp_sum(T v) {
   return v;
 }
 
+// V values per lane summed over the warp at once: lane l returns the sum of
+// value l / (32 / V).  At offset 16 the halves of the warp exchange halves of
+// the values, and so on: V - 1 additions and then log2(32 / V) instead of
+// 5 V, in the pairing of warp_sum (x + y and y + x round alike), so each sum
+// is the one warp_sum gives.  The float64 pipe takes 19 clocks a warp
+// instruction, which is what the sums at the end of a tile wait for.
+template <int V>
+__device__ __forceinline__ double warp_sums(double (&v)[V], int lane) {
+  static_assert(V >= 2 && V <= 32 && (V & (V - 1)) == 0, "a power of two");
+  int off = 16;
+#pragma unroll
+  for (int h = V / 2; h > 0; h /= 2, off /= 2) {
+    const bool up = lane & off;
+#pragma unroll
+    for (int q = 0; q < h; ++q) {
+      const double send = up ? v[q] : v[q + h];
+      const double keep = up ? v[q + h] : v[q];
+      v[q] = keep + __shfl_xor_sync(0xffffffffu, send, off);
+    }
+  }
+#pragma unroll
+  for (int o = 16 / V; o > 0; o /= 2) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+  return v[0];
+}
+
 // Sums v over the block into *out with one atomicAdd per warp.
 __device__ __forceinline__ void block_atomic_add(double* out, double v) {
   v = warp_sum(v);

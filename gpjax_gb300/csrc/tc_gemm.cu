@@ -102,6 +102,24 @@ struct SmemCtl {
 constexpr int EPI_WARPS = 8;   // epilogue warps: two per TMEM lane quarter
 constexpr int EPI_THREADS = EPI_WARPS * 32;
 
+// A warp's sums of d lengthscale terms (float-float), the variance term and the
+// noise term into the first `slots` of gred[0], gred[EPI_WARPS], ...  The float64
+// pipe (19 clocks a warp instruction) bounds this end of a tile: the terms are
+// picked by fixed indices (a search over k for each slot converted all of them
+// again) and summed together.
+template <int DM>
+__device__ __forceinline__ void warp_slots(const float (&lh)[DM], const float (&ll)[DM], float vh,
+                                           float vl, double noise, int d, int slots, int lane,
+                                           double* gred) {
+  double v[DM], u[2] = {(double)vh + (double)vl, noise};
+#pragma unroll
+  for (int k = 0; k < DM; ++k) v[k] = (double)lh[k] + (double)ll[k];
+  const double tv = warp_sums<DM>(v, lane), tu = warp_sums<2>(u, lane);
+  const int k = lane / (32 / DM), s = d + lane / 16;
+  if (lane % (32 / DM) == 0 && k < d) gred[k * EPI_WARPS] = tv;
+  if (lane % 16 == 0 && s < slots) gred[s * EPI_WARPS] = tu;
+}
+
 // MODE: epilogue.  TS: tile shape (Tile<TS>).  DM: bound on the input
 // dimension of the MODE_GRAD epilogue (registers scale with it).
 template <int MODE, int TS, int DM>
@@ -596,21 +614,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
       }
       // reduce over the 4 epilogue warps into gpart[tile]
       const int slots = p.d + 2;
-      for (int sidx = 0; sidx < slots; ++sidx) {
-        double val;
-        if (sidx < p.d) {
-          val = 0.0;
-#pragma unroll
-          for (int kk = 0; kk < DM; ++kk)
-            if (kk == sidx) val = (double)glh[kk] + (double)gll[kk];
-        } else if (sidx == p.d) {
-          val = (double)gvh + (double)gvl;
-        } else {
-          val = gnoise;
-        }
-        val = warp_sum(val);
-        if (lane == 0) gred[sidx * EPI_WARPS + ew] = val;
-      }
+      warp_slots<DM>(glh, gll, gvh, gvl, gnoise, p.d, slots, lane, gred + ew);
       asm volatile("bar.sync 1, %0;" ::"r"(EPI_THREADS) : "memory");
       const int tile_id = blockIdx.x + (int)gridDim.x * z;
       for (int sidx = et; sidx < slots; sidx += EPI_THREADS) {
@@ -695,17 +699,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
       }
       // theta partials: reduce over the epilogue warps into gpart[tile]
       const int slots = p.d + 1;
-      for (int sidx = 0; sidx < slots; ++sidx) {
-        double val = (double)gvh + (double)gvl;
-        if (sidx < p.d) {
-          val = 0.0;
-#pragma unroll
-          for (int kk = 0; kk < DM; ++kk)
-            if (kk == sidx) val = (double)glh[kk] + (double)gll[kk];
-        }
-        val = warp_sum(val);
-        if (lane == 0) gred[sidx * EPI_WARPS + ew] = val;
-      }
+      warp_slots<DM>(glh, gll, gvh, gvl, 0.0, p.d, slots, lane, gred + ew);
       asm volatile("bar.sync 1, %0;" ::"r"(EPI_THREADS) : "memory");
       if (hcol == 0 && gi < p.M) {
         double* zp = p.zpart + ((int64_t)z * p.tiles_n + J) * (int64_t)p.M * p.d + (int64_t)gi * p.d;
