@@ -650,6 +650,8 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
         f32x2 zi2[DP];
 #pragma unroll
         for (int kp = 0; kp < DP; ++kp) zi2[kp] = f2_pack(zi[2 * kp], zi[2 * kp + 1]);
+      auto cols = [&](auto full_c) {
+      constexpr bool FULL = decltype(full_c)::value;
 #pragma unroll 1
       for (int cb = 0; cb < HC / 32; ++cb) {
         f32x2 pl2[DP], pz2[DP];
@@ -659,7 +661,7 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
 #pragma unroll 4
         for (int k = 0; k < 32; ++k) {
           const int c = hcol + cb * 32 + k;
-          if (!row_ok || j0 + c >= p.n_true) continue;
+          if (!FULL && (!row_ok || j0 + c >= p.n_true)) continue;
           const float g = fmaf(ai, ga[c], otile[r * GLD + c]);
           const f32x2* gx2 = reinterpret_cast<const f32x2*>(gx + c * DM);
           f32x2 df2[DP];
@@ -691,6 +693,12 @@ __global__ void __launch_bounds__(NUM_THREADS, 1)
         }
         ff_add(gvh, gvl, pvar);
       }
+      };
+      // a warp whose elements all exist runs without the test of each
+      if (__all_sync(0xffffffffu, row_ok) && j0 + BN <= p.n_true)
+        cols(std::integral_constant<bool, true>{});
+      else
+        cols(std::integral_constant<bool, false>{});
       });
       // per-row z partials: the two threads of a row combine in a fixed order
       if (hcol != 0) {
