@@ -568,6 +568,88 @@ static cudaError_t potrf_block64(double* A, int64_t lda, int n, int o, double* l
   return launch_status();
 }
 
+// Panel solve, float64 form: TRSM_ROWS rows per CTA (so that a short panel
+// still spreads over many SMs: float64 throughput per SM is low), eliminated
+// column by column by all threads: after column j is final, every later
+// column c of every row takes x[c] -= (x[j] / L[j, j]) L[c, j].  The columns
+// stay unscaled until the end (one barrier per column).
+constexpr int TRSM_ROWS = 32;
+template <typename T, int NB>
+__global__ void __launch_bounds__(256) trsm_rows_kernel(T* A, int64_t lda, int n, int k0) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  constexpr int LD = NB + 1;
+  T* Ls = reinterpret_cast<T*>(smem_raw);
+  T* Xs = Ls + NB * LD;
+  T* rinv = Xs + TRSM_ROWS * LD;
+  const int nb = min(NB, n - k0);
+  const int r0 = k0 + nb + blockIdx.x * TRSM_ROWS;
+  const int rows = min(TRSM_ROWS, n - r0);
+  if (rows <= 0) return;
+  for (int e = threadIdx.x; e < nb * nb; e += blockDim.x) {
+    int i = e / nb, j = e % nb;
+    Ls[i * LD + j] = (j <= i) ? A[(int64_t)(k0 + i) * lda + k0 + j] : T(0);
+  }
+  for (int e = threadIdx.x; e < rows * nb; e += blockDim.x) {
+    int r = e / nb, c = e % nb;
+    Xs[r * LD + c] = A[(int64_t)(r0 + r) * lda + k0 + c];
+  }
+  __syncthreads();
+  for (int j = threadIdx.x; j < nb; j += blockDim.x) rinv[j] = T(1) / Ls[j * LD + j];
+  __syncthreads();
+  for (int j = 0; j + 1 < nb; ++j) {
+    const int w = nb - 1 - j;  // columns j+1 .. nb-1
+    const T rj = rinv[j];
+    for (int e = threadIdx.x; e < rows * w; e += blockDim.x) {
+      const int r = e / w, c = j + 1 + e % w;
+      Xs[r * LD + c] -= (Xs[r * LD + j] * rj) * Ls[c * LD + j];
+    }
+    __syncthreads();
+  }
+  for (int e = threadIdx.x; e < rows * nb; e += blockDim.x) {
+    int r = e / nb, c = e % nb;
+    A[(int64_t)(r0 + r) * lda + k0 + c] = Xs[r * LD + c] * rinv[c];
+  }
+}
+
+// The factor in native float64 throughout (right-looking, CUDA-core updates).
+cudaError_t potrf_lower_native(double* A, int64_t lda, int n, double* logdiag, int* info,
+                               bool zero_upper, cudaStream_t s) {
+  constexpr int NB = Blk<double>::NB;
+  const size_t smem_diag = (size_t)(NB * (NB + 1) + 5 * NB) * sizeof(double);
+  const size_t smem_trsm = (size_t)(NB * (NB + 1) + TRSM_ROWS * (NB + 1) + NB) * sizeof(double);
+  cudaFuncSetAttribute(potrf_diag_kernel<double, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)smem_diag);
+  cudaFuncSetAttribute(trsm_rows_kernel<double, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                       (int)smem_trsm);
+  if (zero_upper && n > NB) {
+    zero_upper_kernel<double><<<(int)cdiv((int64_t)n * n, 256), 256, 0, s>>>(A, lda, n, NB);
+    cudaError_t e = launch_status();
+    if (e != cudaSuccess) return e;
+  }
+  for (int k0 = 0; k0 < n; k0 += NB) {
+    const int nb = min(NB, n - k0), rest = n - k0 - nb;
+    potrf_diag_kernel<double, NB><<<1, 512, smem_diag, s>>>(A, lda, n, k0, logdiag, info, nullptr);
+    cudaError_t e = launch_status();
+    if (e != cudaSuccess || rest <= 0) return e;
+    trsm_rows_kernel<double, NB><<<(rest + TRSM_ROWS - 1) / TRSM_ROWS, 256, smem_trsm, s>>>(
+        A, lda, n, k0);
+    e = launch_status();
+    if (e != cudaSuccess) return e;
+    GemmProb<double> p{};
+    p.A = p.B = A + (int64_t)(k0 + nb) * lda + k0;
+    p.C = A + (int64_t)(k0 + nb) * lda + k0 + nb;
+    p.lda = p.ldb = p.ldc = lda;
+    p.M = p.N = rest;
+    p.K = nb;
+    p.c_lower = 1;
+    p.alpha = -1.0;
+    p.beta = 1.0;
+    e = gemm_nt<double>(p, 1, s);
+    if (e != cudaSuccess) return e;
+  }
+  return cudaSuccess;
+}
+
 template <typename T>
 cudaError_t potrf_lower(T* A, int64_t lda, int n, double* logdiag, int* info, double* dtrack,
                         bool zero_upper, cudaStream_t s, bool keep_upper) {
@@ -818,14 +900,15 @@ static cudaError_t trtri_merge(const T* L, int64_t ldl, T* M, int64_t ldm, T* V,
 
 template <typename T>
 cudaError_t trtri_lower(const T* L, int64_t ldl, int n, T* M, int64_t ldm, T* V, int64_t ldv,
-                        T* scratch, const XRoom& x, cudaStream_t s) {
+                        T* scratch, const XRoom& x, cudaStream_t s, bool native) {
   constexpr int NB = Blk<T>::NB;
   const size_t smem = (size_t)(2 * NB * (NB + 1) + NB) * sizeof(T);
   const int nblk = (n + NB - 1) / NB;
-  if constexpr (sizeof(T) == 8) {
+  if (sizeof(T) == 8 && !native) {
     cudaFuncSetAttribute(trtri_diag64_kernel<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)smem);
-    trtri_diag64_kernel<NB><<<nblk, 256, smem, s>>>(L, ldl, n, M, ldm, V, ldv);
+    trtri_diag64_kernel<NB><<<nblk, 256, smem, s>>>((const double*)L, ldl, n, (double*)M, ldm,
+                                                    (double*)V, ldv);
   } else {
     cudaFuncSetAttribute(trtri_diag_kernel<T, NB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                          (int)smem);
@@ -910,7 +993,7 @@ cudaError_t gemv_dense(const T* A, int64_t ld, int rows, int cols, const double*
   template cudaError_t potrf_lower<T>(T*, int64_t, int, double*, int*, double*, bool,          \
                                       cudaStream_t, bool);                                           \
   template cudaError_t trtri_lower<T>(const T*, int64_t, int, T*, int64_t, T*, int64_t, T*,     \
-                                      const XRoom&, cudaStream_t);                                            \
+                                      const XRoom&, cudaStream_t, bool);                        \
   template cudaError_t gemv_tri<T>(const T*, int64_t, int, bool, const double*, double*, double, \
                                    bool, cudaStream_t);                                         \
   template cudaError_t gemv_dense<T>(const T*, int64_t, int, int, const double*, double*,      \

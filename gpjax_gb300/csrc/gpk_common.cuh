@@ -96,6 +96,20 @@ __device__ __forceinline__ T kval(int kind, T sq, T s2, T ka = T(1)) {
   return s2 * (T(1) + r5 * t + T(5.0 / 3.0) * (t * t)) * d_exp(-r5 * t);
 }
 
+// The same by the math library's exp and sqrt.
+__device__ __forceinline__ double kval_lib(int kind, double sq, double s2, double ka) {
+  if (kind == GPK_RBF) return s2 * exp(-0.5 * sq);
+  if (kind == GPK_RATIONAL_QUADRATIC) return s2 * exp(-ka * log1p(sq / (2.0 * ka)));
+  const double t = sqrt(sq > Consts<double>::floor_() ? sq : Consts<double>::floor_());
+  if (kind == GPK_MATERN12) return s2 * exp(-t);
+  if (kind == GPK_MATERN32) {
+    const double r3 = 1.7320508075688772;
+    return s2 * (1.0 + r3 * t) * exp(-r3 * t);
+  }
+  const double r5 = 2.23606797749979;
+  return s2 * (1.0 + r5 * t + (5.0 / 3.0) * (t * t)) * exp(-r5 * t);
+}
+
 // value and derivative coefficient together (one exp)
 template <typename T>
 __device__ __forceinline__ void kval_dcoef(int kind, T sq, T s2, T& k, T& c, T ka = T(1)) {

@@ -36,7 +36,7 @@ cudaError_t scale_inputs(const double* x, int64_t ldx, int n, int d, const doubl
 constexpr int GT = 64;  // output tile edge
 
 // D bounds the input dimension (coordinates past d are zero and add nothing).
-template <typename T, typename TO, int D>
+template <typename T, typename TO, int D, bool LIB = false>
 __global__ void __launch_bounds__(256)
     cross_cov_kernel(int kind, int n, int m, int d, const T* __restrict__ xs,
                      const T* __restrict__ ys, const double* __restrict__ theta, int n_ls, int mode,
@@ -81,7 +81,11 @@ __global__ void __launch_bounds__(256)
         T df = sx[r][k] - yv[k];
         sq = fma(df, df, sq);
       }
-      T kv = kval<T>(kind, sq, s2, kshape<T>(kind, theta, n_ls));
+      T kv;
+      if constexpr (LIB)
+        kv = kval_lib(kind, sq, s2, kshape<T>(kind, theta, n_ls));
+      else
+        kv = kval<T>(kind, sq, s2, kshape<T>(kind, theta, n_ls));
       if (mode == 1 && gi == gj) {
         // (K + I*jitter) + I*obs_stddev^2 (objectives.py:100-103)
         double dv = ((double)kv + jitter) + sd * sd;
@@ -201,6 +205,25 @@ template cudaError_t scale_inputs<double>(const double*, int64_t, int, int, cons
                                           double*, cudaStream_t);
 template cudaError_t scale_inputs<float>(const double*, int64_t, int, int, const double*, int,
                                          float*, cudaStream_t);
+cudaError_t cross_cov_lib(int kind, int n, int m, int d, const double* xs, const double* ys,
+                          const double* theta, int n_ls, int mode, double jitter, double* out,
+                          int64_t ldo, cudaStream_t s) {
+  if (n <= 0 || m <= 0) return cudaSuccess;
+  if (d > GPK_MAX_D) return cudaErrorInvalidValue;
+  const dim3 grid((unsigned)cdiv(m, GT), (unsigned)cdiv(n, GT));
+  auto run = [&](auto dim) {
+    cross_cov_kernel<double, double, decltype(dim)::value, true><<<grid, 256, 0, s>>>(
+        kind, n, m, d, xs, ys, theta, n_ls, mode, jitter, out, ldo);
+  };
+  if (d <= 8)
+    run(std::integral_constant<int, 8>{});
+  else if (d <= 16)
+    run(std::integral_constant<int, 16>{});
+  else
+    run(std::integral_constant<int, 32>{});
+  return launch_status();
+}
+
 template cudaError_t cross_cov_scaled<double, double>(int, int, int, int, const double*,
                                                       const double*, const double*, int, int,
                                                       double, double*, int64_t, cudaStream_t);

@@ -175,7 +175,12 @@ size_t sgpr_layout(int64_t n, int64_t m, int d, void* ws, SgprBuf<T>& b) {
   b.gzs = a.take<double>((size_t)m * d);
   b.ddds = a.take<double>(2);
   b.err = a.take<int>(1);
-  const size_t small = m <= 128 ? 0 : std::max(xroom_factor_bytes(m), 2 * xsplit_bytes(m, m));
+  // The mixed form's m x m algebra stays in native float64: at m near 1024 the
+  // condition of Kzz + jitter carries the last bit of its entries and products
+  // to 4e-7 of the gradient of Z, and the form's results are to be the same
+  // from one version to the next (with the split products and fixed-point
+  // blocks a bound at n = 1e6 took 23.1 ms).
+  const size_t small = mixed || m <= 128 ? 0 : std::max(xroom_factor_bytes(m), 2 * xsplit_bytes(m, m));
   size_t want = small;
   if (!mixed) {
     // P's partials go through the room in groups of at most 2 GB of digits
@@ -784,13 +789,17 @@ gpk_status sgpr_run(int kind, int n, int m, int d, const double* x, int64_t ldx,
   const unsigned mgrid = (unsigned)cdiv((int64_t)m * m, 256);
   GPK_CUDA_TRY(cudaEventRecord(side->fork, s));
   GPK_CUDA_TRY(cudaStreamWaitEvent(ss, side->fork, 0));
-  GPK_CUDA_TRY(cross_cov_scaled<double, double>(kind, m, m, d, b.zs64, b.zs64, theta, n_ls, 0, 0.0,
-                                                b.Kf, ldm, ss));
-  GPK_CUDA_TRY(cross_cov_scaled<double, double>(kind, m, m, d, b.zs64, b.zs64, theta, n_ls, 2,
-                                                jitter, b.Lz, ldm, ss));
-  GPK_CUDA_TRY(potrf_lower_x(b.Lz, ldm, m, b.ldK, info, false,
-                             planes_in(b.xk, b.Mz, b.Kinv), ss));
-  GPK_CUDA_TRY(trtri_lower<double>(b.Lz, ldm, m, b.Mz, ldm, b.Vz, ldm, b.scr, b.xk, ss));
+  auto kzz = [&](int mode, double jit, double* out) {
+    return mixed ? cross_cov_lib(kind, m, m, d, b.zs64, b.zs64, theta, n_ls, mode, jit, out, ldm, ss)
+                 : cross_cov_scaled<double, double>(kind, m, m, d, b.zs64, b.zs64, theta, n_ls,
+                                                    mode, jit, out, ldm, ss);
+  };
+  GPK_CUDA_TRY(kzz(0, 0.0, b.Kf));
+  GPK_CUDA_TRY(kzz(2, jitter, b.Lz));
+  GPK_CUDA_TRY(mixed ? potrf_lower_native(b.Lz, ldm, m, b.ldK, info, false, ss)
+                     : potrf_lower_x(b.Lz, ldm, m, b.ldK, info, false,
+                                     planes_in(b.xk, b.Mz, b.Kinv), ss));
+  GPK_CUDA_TRY(trtri_lower<double>(b.Lz, ldm, m, b.Mz, ldm, b.Vz, ldm, b.scr, b.xk, ss, mixed));
   {
     GemmProb<double> p{};
     p.A = b.Vz;
@@ -890,9 +899,10 @@ gpk_status sgpr_run(int kind, int n, int m, int d, const double* x, int64_t ldx,
                                                          b.Su);
     GPK_LAUNCH_CHECK();
   }
-  GPK_CUDA_TRY(potrf_lower_x(b.Su, ldm, m, b.ldU, info, true, planes_in(b.xu, b.Mu, b.Suinv),
-                             s));
-  GPK_CUDA_TRY(trtri_lower<double>(b.Su, ldm, m, b.Mu, ldm, b.Vu, ldm, b.scr, b.xu, s));
+  GPK_CUDA_TRY(mixed ? potrf_lower_native(b.Su, ldm, m, b.ldU, info, true, s)
+                     : potrf_lower_x(b.Su, ldm, m, b.ldU, info, true,
+                                     planes_in(b.xu, b.Mu, b.Suinv), s));
+  GPK_CUDA_TRY(trtri_lower<double>(b.Su, ldm, m, b.Mu, ldm, b.Vu, ldm, b.scr, b.xu, s, mixed));
   {  // Su^-1 = Vu Vu^T (lower triangle, then mirrored)
     GemmProb<double> p{};
     p.A = b.Vu;
