@@ -568,7 +568,7 @@ static cudaError_t potrf_block64(double* A, int64_t lda, int n, int o, double* l
   return launch_status();
 }
 
-// Panel solve, float64 form: TRSM_ROWS rows per CTA (so that a short panel
+// Panel solve, native float64: TRSM_ROWS rows per CTA (so that a short panel
 // still spreads over many SMs: float64 throughput per SM is low), eliminated
 // column by column by all threads: after column j is final, every later
 // column c of every row takes x[c] -= (x[j] / L[j, j]) L[c, j].  The columns
@@ -611,7 +611,8 @@ __global__ void __launch_bounds__(256) trsm_rows_kernel(T* A, int64_t lda, int n
   }
 }
 
-// The factor in native float64 throughout (right-looking, CUDA-core updates).
+// The factor in native float64 throughout (right-looking, CUDA-core updates),
+// 72 us a diagonal block: for the mixed collapsed bound alone (sgpr.cu).
 cudaError_t potrf_lower_native(double* A, int64_t lda, int n, double* logdiag, int* info,
                                bool zero_upper, cudaStream_t s) {
   constexpr int NB = Blk<double>::NB;

@@ -21,7 +21,8 @@
 // adjoint); P = Phi Phi^T per n-chunk and G = H Phi run on the tensor cores
 // (split-TF32 tcgen05 GEMM), with G reduced against dPhi/dtheta, dPhi/dZ in
 // the GEMM epilogue; c = Phi d and Phi 1 are summed in float-float during
-// generation.  The m x m algebra always runs in float64.  Reductions go
+// generation.  The m x m algebra always runs in float64
+// (split products and fixed-point blocks in the plain form, native in the mixed).  Reductions go
 // through per-block partials summed in a fixed order.
 #include <algorithm>
 #include <climits>
@@ -179,7 +180,7 @@ size_t sgpr_layout(int64_t n, int64_t m, int d, void* ws, SgprBuf<T>& b) {
   // condition of Kzz + jitter carries the last bit of its entries and products
   // to 4e-7 of the gradient of Z, and the form's results are to be the same
   // from one version to the next (with the split products and fixed-point
-  // blocks a bound at n = 1e6 took 23.1 ms).
+  // blocks a bound at n = 1e6 took 23.1 ms instead of 29.2).
   const size_t small = mixed || m <= 128 ? 0 : std::max(xroom_factor_bytes(m), 2 * xsplit_bytes(m, m));
   size_t want = small;
   if (!mixed) {
@@ -899,6 +900,33 @@ gpk_status sgpr_run(int kind, int n, int m, int d, const double* x, int64_t ldx,
                                                          b.Su);
     GPK_LAUNCH_CHECK();
   }
+  lock.lock();  // not held across the exchange above, which waits for other callers
+  GPK_CUDA_TRY(cudaEventRecord(side->fork, s));
+  GPK_CUDA_TRY(cudaStreamWaitEvent(ss, side->fork, 0));
+  {
+    // T1 = K^-1 P ; KPK = T1 K^-1 (symmetric operands: NT form; KPK is
+    // symmetric, so its lower triangle is formed and mirrored), on the side
+    // stream beside the chain of Su: one after the other they took 1.4 ms more
+    // at m = 1024 in the mixed form (30.6 against 29.2).
+    GemmProb<double> q{};
+    q.A = b.Kinv;
+    q.B = b.P64;
+    q.lda = q.ldb = ldm;
+    q.C = b.T1;
+    q.ldc = ldm;
+    q.M = q.N = q.K = m;
+    q.alpha = 1.0;
+    q.beta = 0.0;
+    GPK_CUDA_TRY(gemm_nt_x(q, 1, b.xk, ss));
+    q.A = b.T1;
+    q.B = b.Kinv;
+    q.C = b.KPK;
+    q.c_lower = 1;
+    GPK_CUDA_TRY(gemm_nt_x(q, 1, b.xk, ss));
+    sg_mirror<<<mgrid, 256, 0, ss>>>(m, ldm, b.KPK);
+    GPK_LAUNCH_CHECK();
+  }
+  GPK_CUDA_TRY(cudaEventRecord(side->join, ss));
   GPK_CUDA_TRY(mixed ? potrf_lower_native(b.Su, ldm, m, b.ldU, info, true, s)
                      : potrf_lower_x(b.Su, ldm, m, b.ldU, info, true,
                                      planes_in(b.xu, b.Mu, b.Suinv), s));
@@ -918,26 +946,9 @@ gpk_status sgpr_run(int kind, int n, int m, int d, const double* x, int64_t ldx,
     GPK_CUDA_TRY(gemm_nt_x(p, 1, b.xu, s));
     sg_mirror<<<mgrid, 256, 0, s>>>(m, ldm, b.Suinv);
     GPK_LAUNCH_CHECK();
-    // T1 = K^-1 P ; KPK = T1 K^-1 (symmetric operands: NT form; KPK is
-    // symmetric, so its lower triangle is formed and mirrored)
-    GemmProb<double> q{};
-    q.A = b.Kinv;
-    q.B = b.P64;
-    q.lda = q.ldb = ldm;
-    q.C = b.T1;
-    q.ldc = ldm;
-    q.M = q.N = q.K = m;
-    q.alpha = 1.0;
-    q.beta = 0.0;
-    GPK_CUDA_TRY(gemm_nt_x(q, 1, b.xu, s));
-    q.A = b.T1;
-    q.B = b.Kinv;
-    q.C = b.KPK;
-    q.c_lower = 1;
-    GPK_CUDA_TRY(gemm_nt_x(q, 1, b.xu, s));
-    sg_mirror<<<mgrid, 256, 0, s>>>(m, ldm, b.KPK);
-    GPK_LAUNCH_CHECK();
   }
+  GPK_CUDA_TRY(cudaStreamWaitEvent(s, side->join, 0));
+  lock.unlock();
   GPK_CUDA_TRY(gemv_dense<double>(b.Suinv, ldm, m, m, b.cv, b.gam, s));
   GPK_CUDA_TRY(gemv_dense<double>(b.P64, ldm, m, m, b.gam, b.pgam, s));
   sg_combine<T><<<256, 256, 0, s>>>(m, ldm, b.Kinv, b.Suinv, b.KPK, b.P64, b.gam, theta, n_ls,
