@@ -225,8 +225,9 @@ __device__ __forceinline__ int tile_col(int v) { return (threadIdx.x & 31) * 4 +
 // hi / lo by all 512 threads and stored into the 128B-swizzled K-major layout
 // the MMA reads (one split stage of A_hi, A_lo, B_hi, B_lo, 64 KB, 1024-byte
 // aligned).  An elected lane of the converged warp 0 issues the slice's 3
-// products (A_lo B_hi, A_hi B_lo, then A_hi B_hi) x 4 K steps of tcgen05.mma kind::tf32 into one of two TMEM
-// accumulators and commits to that accumulator's mbarrier; while they run,
+// products (A_lo B_hi, A_hi B_lo, then A_hi B_hi) x 4 K steps of tcgen05.mma
+// kind::tf32 into one of two TMEM accumulators and commits to that
+// accumulator's mbarrier; while they run,
 // every thread adds the previous slice's accumulator (its 32 columns) to
 // float32 registers (round to nearest: 12 MMAs per TMEM accumulation) and
 // the next raw slice lands.  The finished tile goes through shared memory
