@@ -328,9 +328,10 @@ class BatchPlan:
     and its gradient per instance) evaluated by ONE persistent kernel launch per
     :meth:`execute`: the plan sorts the instances by n into a device queue, and
     one CTA per SM pulls instances from it and runs each to completion
-    (``gpk_batch_plan_*`` in include/gpk.h).  With ``autotune`` the plan times
-    the library's tile configurations on its own instances for every padded n
-    not tuned before in this process.
+    (``gpk_batch_plan_*`` in include/gpk.h).  With ``autotune`` the plan tries
+    its own instances of every padded n not tried before in this process and
+    keeps the first of the library's tile configurations (tensor cores first)
+    that fails the fewest of them.
 
     kinds: kernel codes; xs: [n_i, d_i] float64 CUDA tensors (n_i <= 4096,
     d_i <= 16); ys: [n_i]; thetas: the theta layout ``[lengthscale (n_ls[i]),

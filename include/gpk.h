@@ -290,10 +290,11 @@ gpk_status gpk_conjugate_mll_batched(int count, const int* kind, const int64_t* 
  * gpk_batch_plan_create records the instances (same arguments and result
  * locations as gpk_conjugate_mll_batched; the device arrays are read at each
  * execution, so their contents may change between executions), sorts them
- * by n (largest first) into a device queue and, when autotune != 0, times the
- * tile configurations on the plan's own instances for every n_pad not yet
- * tuned on this device and keeps the fastest of those that fail the fewest
- * of the trial's instances (results kept for the process).  It allocates a few
+ * by n (largest first) into a device queue and, when autotune != 0, runs the
+ * plan's own instances of every n_pad not yet tried on this device and keeps
+ * the first of configurations 2, 0, 1 that fails the fewest of them (kept for
+ * the process; no timing takes part, so equal programs get equal results, and
+ * without autotune an n_pad never tried runs configuration 1).  It allocates a few
  * bytes per instance of device memory and synchronises the device: call it
  * outside stream capture.  gpk_batch_plan_execute zeroes the queue head and
  * launches ONE persistent kernel (one CTA per SM pulls instances from the

@@ -9,6 +9,8 @@ float32 rounding of Sigma's entries alone moves the log-determinant of the
 Matern-5/2 n = 2048, d = 4 case (condition number 1.6e5) by 4.8e-5 of the MLL
 (LAPACK's float32 Cholesky of the same matrix).  The same bounds hold for every
 tile configuration (CUDA-core and tcgen05 split-TF32) forced in turn."""
+import shutil
+
 import numpy as np
 import pytest
 import torch
@@ -233,3 +235,27 @@ def test_tensor_core_wait_timeout_is_reported(cuda_lib):
     with pytest.raises(_lib.GPKError):
         plan.selftest_stall(-1)
     plan.close()
+
+
+def test_configuration_does_not_depend_on_timing(cuda_lib, tmp_path, monkeypatch):
+    """Plans in fresh processes (here: fresh copies of the library, whose tables
+    are per copy) run the same configurations and give the same bits.  At
+    n_pad = 128 the configurations take equally long, so a choice by their times
+    falls differently in about one of ten processes."""
+    specs = [((_lib.RBF, _lib.MATERN32)[k % 2], 16 + k % 112, 2 + k % 9, False)
+             for k in range(300)]
+    insts = [_instance(s, 500 + k) for k, s in enumerate(specs)]
+    path, seen = _lib.LIB_PATH, set()
+    for k in range(60):
+        copy = tmp_path / f"copy{k}.so"
+        shutil.copy(path, copy)
+        monkeypatch.setattr(_lib, "LIB_PATH", str(copy))
+        monkeypatch.setattr(_lib, "_LIB", None)
+        plan = _plan(insts)
+        mll, grads, info = plan.execute()
+        torch.cuda.synchronize()
+        assert not info.any()
+        seen.add((plan.config(128), tuple(mll.tolist()), tuple(torch.cat(grads).tolist())))
+        plan.close()
+        copy.unlink()
+    assert [s[0] for s in seen] == [2]  # the first choice: no instance fails it
