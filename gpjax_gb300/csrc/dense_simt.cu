@@ -525,9 +525,11 @@ __global__ void __launch_bounds__(FX_NT)
   // the first panel (updates only lower a diagonal entry and with it the scale)
   if (planes.planes) {
     const int r = threadIdx.x >> 4, c = (threadIdx.x & 15) * 4;
-    if (r < rows) {
-      int* expo = planes.expo + r0 + r;
-      const int e0 = k0 == 0 ? ei[r] : *expo - 1022;
+    const bool in = r < rows;  // a warp's second row may be past the last
+    int* expo = planes.expo + r0 + r;
+    const int e0 = !in ? 0 : k0 == 0 ? ei[r] : *expo - 1022;
+    __syncwarp();  // the row's 16 lanes have read its exponent
+    if (in) {
       const bool ok = !sbad[r] && ei[r] <= e0;
       const int sh = min(62, FRAC - 55 + (ok ? e0 - ei[r] : 0));
       long long q[4];
@@ -536,7 +538,6 @@ __global__ void __launch_bounds__(FX_NT)
       x_store_digits4(q,
                       static_cast<__half*>(planes.planes) + (int64_t)(r0 + r) * planes.ldk + k0 + c,
                       (int64_t)planes.rows * planes.ldk);
-      __syncwarp();  // the row's 16 lanes have read its exponent
       if (c == 0 && (k0 == 0 || !ok)) *expo = ok ? e0 + 1022 : XNAN;
     }
   }

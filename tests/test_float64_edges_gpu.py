@@ -57,6 +57,26 @@ def test_mll_tile_edges(cuda_lib, kind, n, d):
     assert np.allclose(got, gref, rtol=1e-7, atol=1e-8 * max(1.0, np.abs(gref).max()))
 
 
+# Odd row counts below a panel that writes digit planes: the last warp of the
+# last block then holds one row, whose exponent its lanes read before one of
+# them replaces it.  Bounds and repeatability as above; equal bits each time.
+@pytest.mark.parametrize("n", [129, 195, 323, 577])
+def test_mll_odd_panels(cuda_lib, n):
+    rng = np.random.default_rng(n)
+    x = rng.uniform(-2, 2, size=(n, 2))
+    y = np.sin(x).sum(1, keepdims=True) + 0.1 * rng.standard_normal((n, 1))
+    ls = np.array([0.7, 1.3])
+    runs = []
+    for _ in range(4):
+        post = to_cuda_params(make_posterior(1, ls, 1.2, 0.3, 0.1))
+        val = gpx.objectives.conjugate_mll(post, gpx.Dataset(X=x, y=y), precision="fp64")
+        val.backward()
+        runs.append(np.concatenate([[val.item()], grads_of(post)]))
+    assert all(np.array_equal(runs[0], r) for r in runs[1:])
+    ref = O.conjugate_mll(1, x, y, ls, 1.2, 0.3, 0.1)
+    assert abs(runs[0][0] - ref) <= 1e-10 * max(1.0, abs(ref))
+
+
 # 16-, 32- and 64-wide tiles with ragged last tiles, and d on both sides of the
 # 64-wide form's bound.  Sums of at most n terms of mixed sign, each with a few
 # roundings and an exp whose argument is below 100: 1e-12 of the sum of the
