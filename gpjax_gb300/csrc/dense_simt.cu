@@ -297,7 +297,10 @@ __global__ void __launch_bounds__(FX_NT)
     if (bad) sbad[r] = 1;
   }
   __syncthreads();
-  // column k loses the eight columns of a group
+  // column k loses the eight columns of a group.  A diagonal entry only falls,
+  // by at most 4 in either half, so its sign is seen before it can leave the
+  // range of [-8, 8): negative once, the row's pivot has failed whatever the
+  // entry wraps to later.
   auto update = [&](const Limbs (&l)[FX_G][FX_NB], int k) {
     if (k >= nb || i < k) return;
     Acc a0, a1;
@@ -306,7 +309,9 @@ __global__ void __launch_bounds__(FX_NT)
       a0.add(l[q][i], l[q][k]);
       a1.add(l[q + 1][i], l[q + 1][k]);
     }
-    S[i][k] -= a0.value() + a1.value();
+    const long long t0 = S[i][k] - a0.value(), t1 = t0 - a1.value();
+    if (i == k && (t0 < 0 || t1 < 0)) sbad[i] = 1;
+    S[i][k] = t1;
   };
   for (int c0 = 0; c0 < nb; c0 += FX_G) {
     Limbs(&cur)[FX_G][FX_NB] = lim[(c0 / FX_G) & 1];
@@ -335,7 +340,7 @@ __global__ void __launch_bounds__(FX_NT)
         lv = limbs(v);
         cur[q][i] = lv;
         if (bad) sbad[i] = 1;
-        if (!good && i == j) {  // the rest of this group's columns mean nothing
+        if ((!good || bad) && i == j) {  // the rest of this group's columns mean nothing
           atomicMin(info, k0 + j + 1);
           sdead = 1;
         }
@@ -470,6 +475,11 @@ __global__ void __launch_bounds__(FX_NT)
   }
   __syncthreads();
   long long* x = X + lane * FX_XLD;
+  // The squared norm of the row's solved entries: below 1 in a definite matrix
+  // (its scale is that of its diagonal entry).  An entry can leave the range of
+  // [-8, 8) and come back as another number only in a row of norm 6 and more,
+  // which is marked before.
+  float norm = 0.f;
   auto solve = [&](int c0) {  // one warp: the group's four columns
     Limbs* out = LX + ((c0 / FX_TG) & 1) * FX_TG * FX_ROWS;
     long long t[FX_TG];
@@ -480,6 +490,8 @@ __global__ void __launch_bounds__(FX_NT)
     for (int q = 0; q < FX_TG; ++q) {
       t[q] = times_rsqrt(t[q], ry[c0 + q], rs[c0 + q], bad);
       const Limbs l = limbs(t[q]);
+      const float f = (float)l.h * 0x1p-28f;
+      norm = fmaf(f, f, norm);
       out[q * FX_ROWS + lane] = l;
 #pragma unroll
       for (int u = q + 1; u < FX_TG; ++u) {
@@ -490,7 +502,7 @@ __global__ void __launch_bounds__(FX_NT)
     }
 #pragma unroll
     for (int q = 0; q < FX_TG; ++q) x[c0 + q] = t[q];
-    if (bad) sbad[lane] = 1;
+    if (bad || norm > 2.f) sbad[lane] = 1;
   };
   auto update = [&](const Limbs (&lx)[FX_TG], int c0, int k) {  // column k loses the group at c0
     Acc acc;

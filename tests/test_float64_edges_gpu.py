@@ -36,6 +36,38 @@ def test_cholesky_blocks(cuda_lib, n, spread):
     assert float(err.max()) <= 4 * (n + 1) * U, float(err.max()) / U
 
 
+# Indefinite matrices whose last pivot, 1 - (n - 1) c^2, lies far below the range
+# [-8, 8) of a fixed-point entry: in all of them the leading minors before the
+# last are positive, so the order that fails is n.
+@pytest.mark.parametrize("n", [64, 65, 200])
+@pytest.mark.parametrize("c", [0.3, 0.5, 0.7, 0.75, 0.8, 0.85, 0.9, 0.95, 1.0])
+def test_cholesky_indefinite_arrow(cuda_lib, n, c):
+    a = np.eye(n)
+    a[-1, :-1] = a[:-1, -1] = c
+    low, info = linalg.cholesky_dense(torch.as_tensor(a, device="cuda"))
+    assert int(info.item()) == n
+    assert np.isnan(low[-1, -1].item())
+
+
+# The same through the marginal likelihood: 63 points at distance r from the
+# last (kernel value c there), sqrt(2) r or 2 r from one another (c^2, c^4), and
+# a negative jitter that leaves D on Sigma's diagonal.  The leading minors are
+# positive (D > 2 c^2), the last pivot is far below -D.
+@pytest.mark.parametrize("D", [0.035, 0.04, 0.05, 0.06])
+@pytest.mark.parametrize("ratio", [17.0, 20.0, 25.0, 30.0])
+def test_mll_indefinite_sigma(cuda_lib, D, ratio):
+    r = np.sqrt(np.log(ratio / D))
+    x = np.concatenate([r * np.eye(32), -r * np.eye(32)[:31], np.zeros((1, 32))])
+    sigma = O.gram(0, x, np.ones(32), 1.0)
+    sigma[np.diag_indices(64)] = D
+    assert np.linalg.eigvalsh(sigma[:63, :63])[0] > 0.5 * D
+    assert sigma[63, :63] @ np.linalg.solve(sigma[:63, :63], sigma[63, :63]) > 8 * D
+    post = to_cuda_params(make_posterior(0, np.ones(32), 1.0, 1e-3, 0.0, jitter=D - 1.0 - 1e-6))
+    val = gpx.objectives.conjugate_mll(
+        post, gpx.Dataset(X=x, y=np.sin(np.arange(64.0))[:, None]), precision="fp64")
+    assert np.isnan(val.item()) and int(val.grad_fn.info.item()) == 64
+
+
 # Same bounds as the float64 parity test of the marginal likelihood, at the
 # sizes on either side of each tile edge of the gradient reduction.
 @pytest.mark.parametrize("kind,n,d", [(0, 128, 3), (1, 130, 5), (2, 384, 2), (0, 385, 9),
