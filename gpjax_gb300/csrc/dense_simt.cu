@@ -19,7 +19,9 @@ namespace gpk {
 // ---------------------------------------------------------------------------
 // Batched NT GEMM, register-tiled.
 // ---------------------------------------------------------------------------
-template <typename T, typename Cfg>
+// BLOCKED (float64): sums of 16 products added in pairs up to 128, those in
+// order: an error of about 20 + K / 128 roundings instead of K.
+template <typename T, typename Cfg, bool BLOCKED = false>
 __global__ void __launch_bounds__((Cfg::BM / Cfg::TM) * (Cfg::BN / Cfg::TN))
     gemm_nt_kernel(GemmProb<T> p) {
   constexpr int BM = Cfg::BM, BN = Cfg::BN, BK = Cfg::BK;
@@ -53,8 +55,45 @@ __global__ void __launch_bounds__((Cfg::BM / Cfg::TM) * (Cfg::BN / Cfg::TN))
   for (int a = 0; a < TM; ++a)
 #pragma unroll
     for (int b = 0; b < TN; ++b) acc[a][b] = T(0);
-  simt_tile_mma<T, Cfg>(A, p.lda, p.M, p.a_tri, B, p.ldb, p.N, p.b_tri, i0, j0, klo, khi, sm,
-                        acc);
+  if constexpr (BLOCKED) {
+    double l0[TM][TN], l1[TM][TN], l2[TM][TN], total[TM][TN];  // waiting sums of 16, 32, 64
+#pragma unroll
+    for (int a = 0; a < TM; ++a)
+#pragma unroll
+      for (int b = 0; b < TN; ++b) l0[a][b] = l1[a][b] = l2[a][b] = total[a][b] = 0.0;
+    int blocks = 0;
+    auto each = [&](auto f) {
+#pragma unroll
+      for (int a = 0; a < TM; ++a)
+#pragma unroll
+        for (int b = 0; b < TN; ++b) f(acc[a][b], l0[a][b], l1[a][b], l2[a][b], total[a][b]);
+    };
+    typedef double& R;
+    simt_tile_mma<T, Cfg>(A, p.lda, p.M, p.a_tri, B, p.ldb, p.N, p.b_tri, i0, j0, klo, khi, sm, acc,
+                          [&]() {
+                            const int q = blocks++;
+                            if (!(q & 1))
+                              each([](R v, R w, R, R, R) { w = v, v = 0.0; });
+                            else if (!(q & 2))
+                              each([](R v, R w0, R w, R, R) { w = w0 + v, v = 0.0; });
+                            else if (!(q & 4))
+                              each([](R v, R w0, R w1, R w, R) { w = w1 + (w0 + v), v = 0.0; });
+                            else
+                              each([](R v, R w0, R w1, R w2, R t) {
+                                t += w2 + (w1 + (w0 + v)), v = 0.0;
+                              });
+                          });
+    const int q = blocks;  // what is left waiting, the small sums first
+    each([q](R v, R w0, R w1, R w2, R t) {
+      v = q & 1 ? w0 : 0.0;
+      if (q & 2) v += w1;
+      if (q & 4) v += w2;
+      v += t;
+    });
+  } else {
+    simt_tile_mma<T, Cfg>(A, p.lda, p.M, p.a_tri, B, p.ldb, p.N, p.b_tri, i0, j0, klo, khi, sm,
+                          acc);
+  }
 
   const int tx = threadIdx.x % NTX, ty = threadIdx.x / NTX;
 #pragma unroll
@@ -82,29 +121,41 @@ static int gemm_tiles(const GemmProb<T>& p) {
   return p.c_lower ? tilesM * (tilesM + 1) / 2 : tilesM * tilesN;
 }
 
-template <typename T, typename Cfg>
+template <typename T, typename Cfg, bool BLOCKED>
 static cudaError_t gemm_nt_cfg(const GemmProb<T>& p, int batch, cudaStream_t s) {
   constexpr int NT = (Cfg::BM / Cfg::TM) * (Cfg::BN / Cfg::TN);
   dim3 grid(gemm_tiles<T, Cfg>(p), 1, batch);
-  gemm_nt_kernel<T, Cfg><<<grid, NT, 0, s>>>(p);
+  gemm_nt_kernel<T, Cfg, BLOCKED><<<grid, NT, 0, s>>>(p);
   return launch_status();
 }
 
 constexpr int SIMT_SMALL_BELOW = 152;  // CTAs of the full-size grid (one wave)
 
-template <typename T>
-cudaError_t gemm_nt(const GemmProb<T>& p, int batch, cudaStream_t s) {
+template <typename T, bool BLOCKED>
+static cudaError_t gemm_nt_tiles(const GemmProb<T>& p, int batch, cudaStream_t s) {
   if (p.M <= 0 || p.N <= 0 || batch <= 0) return cudaSuccess;
   // float64 only: the float32 form runs many independent GPs side by side
-  // (batched MLL), where total work rather than one launch's latency counts
-  if (sizeof(T) == 8 && (int64_t)gemm_tiles<T, GemmCfg<T>>(p) * batch < SIMT_SMALL_BELOW) {
+  // (batched MLL), where total work rather than one launch's latency counts.
+  // Products in blocks always: their waiting sums take the registers that 64 x 64
+  // tiles would need (2048^3: 18.3 ms with those, 15.1 with 32 x 32).
+  if (BLOCKED ||
+      (sizeof(T) == 8 && (int64_t)gemm_tiles<T, GemmCfg<T>>(p) * batch < SIMT_SMALL_BELOW)) {
     // tiles of 16 once four times as many 32 x 32 tiles still fit one wave (a
     // 36 x 36 x 64 update: 27 us with 32 x 32 tiles, 9 with 16 x 16)
     if ((int64_t)gemm_tiles<T, GemmCfgSmall<T>>(p) * batch * 4 <= SIMT_SMALL_BELOW)
-      return gemm_nt_cfg<T, GemmCfgTiny<T>>(p, batch, s);
-    return gemm_nt_cfg<T, GemmCfgSmall<T>>(p, batch, s);
+      return gemm_nt_cfg<T, GemmCfgTiny<T>, BLOCKED>(p, batch, s);
+    return gemm_nt_cfg<T, GemmCfgSmall<T>, BLOCKED>(p, batch, s);
   }
-  return gemm_nt_cfg<T, GemmCfg<T>>(p, batch, s);
+  return gemm_nt_cfg<T, GemmCfg<T>, BLOCKED>(p, batch, s);
+}
+
+template <typename T>
+cudaError_t gemm_nt(const GemmProb<T>& p, int batch, cudaStream_t s) {
+  return gemm_nt_tiles<T, false>(p, batch, s);
+}
+
+cudaError_t gemm_nt_blocked(const GemmProb<double>& p, cudaStream_t s) {
+  return gemm_nt_tiles<double, true>(p, 1, s);
 }
 
 // ---------------------------------------------------------------------------

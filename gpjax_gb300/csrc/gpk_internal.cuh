@@ -32,6 +32,8 @@ template <> struct Blk<float> { static constexpr int NB = 128; };
 
 template <typename T>
 cudaError_t gemm_nt(const GemmProb<T>& p, int batch, cudaStream_t s);
+// The float64 product with the sums over K in blocks of 16, added in pairs.
+cudaError_t gemm_nt_blocked(const GemmProb<double>& p, cudaStream_t s);
 
 // Lower Cholesky in place (row-major, lda).  logdiag[n] (may be null)
 // receives log(L_ii) in float64; info gets the first failing order.

@@ -67,11 +67,17 @@ struct SimtSmem {
   T Bs[Cfg::BK][Cfg::BN + 4];
 };
 
-template <typename T, typename Cfg = GemmCfg<T>>
+// fold() after every 16 K elements (the sums in acc may be taken over there).
+struct NoFold {
+  __device__ __forceinline__ void operator()() const {}
+};
+
+template <typename T, typename Cfg = GemmCfg<T>, typename Fold = NoFold>
 __device__ __forceinline__ void simt_tile_mma(const T* A, int64_t lda, int M, int a_tri, const T* B,
                                               int64_t ldb, int N, int b_tri, int i0, int j0,
                                               int klo, int khi, SimtSmem<T, Cfg>& sm,
-                                              T (&acc)[Cfg::TM][Cfg::TN]) {
+                                              T (&acc)[Cfg::TM][Cfg::TN],
+                                              const Fold& fold = Fold()) {
   constexpr int BM = Cfg::BM, BN = Cfg::BN, BK = Cfg::BK;
   constexpr int TM = Cfg::TM, TN = Cfg::TN;
   constexpr int NTX = BN / TN, NTY = BM / TM, NT = NTX * NTY;
@@ -97,6 +103,7 @@ __device__ __forceinline__ void simt_tile_mma(const T* A, int64_t lda, int M, in
       for (int a = 0; a < TM; ++a)
 #pragma unroll
         for (int b = 0; b < TN; ++b) acc[a][b] = fma(av[a], bv[b], acc[a][b]);
+      if (kk % 16 == 15) fold();
     }
     __syncthreads();
   }

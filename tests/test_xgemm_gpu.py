@@ -50,3 +50,63 @@ def test_split_product_non_finite(cuda_lib):
     bad = torch.zeros(300, 170, dtype=torch.bool, device="cuda")
     bad[3], bad[140], bad[:, 9] = True, True, True
     assert torch.equal(torch.isfinite(c), ~bad)
+
+
+# The product's error bound for any order of the sum, K u sum_k |a_ik| |b_jk|,
+# plus the rounding of the result: it knows nothing of the range along K.
+# Sizes on both sides of 8e6 multiply-adds.
+@pytest.mark.parametrize("size", [180, 256])
+@pytest.mark.parametrize("r", [1e6, 1e12, 1e16, 2.0 ** 60])
+def test_product_range_along_k(cuda_lib, size, r):
+    rng = np.random.default_rng(size)
+    a, b = rng.standard_normal((size, size)), rng.standard_normal((size, size))
+    if r == 2.0 ** 60:  # large entries against zeros
+        a[:, 0], b[:, 0] = r, 0.0
+    else:  # a column of A larger by r, the matching column of B smaller by r
+        a[:, 0] *= r
+        b[:, 0] /= r
+    got = linalg.matmul(torch.as_tensor(a, device="cuda"), torch.as_tensor(b, device="cuda"),
+                        transb=True).cpu().numpy()
+    ref = a.astype(np.longdouble) @ b.astype(np.longdouble).T
+    tol = 2.0 ** -53 * (np.abs(ref) + size * (np.abs(a) @ np.abs(b).T))
+    assert np.all(np.abs(got - ref) <= tol)
+
+
+def test_product_infinity(cuda_lib):
+    """An infinity in a row gives an infinity where the sum has one."""
+    rng = np.random.default_rng(3)
+    a, b = rng.standard_normal((260, 300)), np.abs(rng.standard_normal((250, 300))) + 0.1
+    a[3, 5], a[7, 2] = np.inf, -np.inf
+    c = linalg.matmul(torch.as_tensor(a, device="cuda"), torch.as_tensor(b, device="cuda"),
+                      transb=True).cpu().numpy()
+    assert np.all(c[3] == np.inf) and np.all(c[7] == -np.inf)
+    assert np.isfinite(np.delete(c, [3, 7], 0)).all()
+
+
+# X = M B through the inverse M of L: componentwise within a few n u |M| |L| |M| |B|
+# (each product's error is n u of the products of the absolute values), which
+# scaled rows or columns of L leave as it is.
+@pytest.mark.parametrize("axis", ["rows", "columns"])
+@pytest.mark.parametrize("spread", [0, 7, 14, 20])
+def test_triangular_solve_graded(cuda_lib, axis, spread):
+    n, rng = 512, np.random.default_rng(spread)
+    g = rng.standard_normal((n, n + 8))
+    low = np.linalg.cholesky(g @ g.T / n)
+    s = np.exp(rng.uniform(-spread, spread, n))
+    scaled = low * (s[:, None] if axis == "rows" else s[None, :])
+    b = scaled @ rng.standard_normal((n, 300))
+    x = linalg.solve_triangular(torch.as_tensor(scaled, device="cuda"),
+                                torch.as_tensor(b, device="cuda")).cpu().numpy()
+    m = np.linalg.inv(low)  # scaling L scales M exactly as well: sizes only
+    m = np.abs(m / s[None, :] if axis == "rows" else m / s[:, None])
+    res = scaled.astype(np.longdouble) @ x.astype(np.longdouble) - b
+    bound = np.abs(scaled) @ (m @ (np.abs(scaled) @ (m @ np.abs(b))))
+    assert np.all(np.abs(res) <= 4 * n * 2.0 ** -53 * bound)
+
+
+def test_triangular_solve_range_of_right_side(cuda_lib):
+    b = np.ones((256, 256))
+    b[0] = 1e20
+    x = linalg.solve_triangular(torch.eye(256, dtype=torch.float64, device="cuda"),
+                                torch.as_tensor(b, device="cuda")).cpu().numpy()
+    assert np.array_equal(x, b)
