@@ -676,7 +676,8 @@ __global__ void __launch_bounds__(256) trsm_rows_kernel(T* A, int64_t lda, int n
 }
 
 // The factor in native float64 throughout (right-looking, CUDA-core updates),
-// 72 us a diagonal block: for the mixed collapsed bound alone (sgpr.cu).
+// 72 us a diagonal block: for a caller's matrix (gpk_lower_cholesky) and the
+// mixed collapsed bound (sgpr.cu).
 cudaError_t potrf_lower_native(double* A, int64_t lda, int n, double* logdiag, int* info,
                                bool zero_upper, cudaStream_t s) {
   constexpr int NB = Blk<double>::NB;

@@ -49,6 +49,37 @@ def test_cholesky_indefinite_arrow(cuda_lib, n, c):
     assert np.isnan(low[-1, -1].item())
 
 
+# An entry of the factor is good relative to itself, however small beside its
+# row's diagonal: here each one is a_ij / l_jj but for products below 1e-25 of it
+# (two roundings, one of the reciprocal).
+@pytest.mark.parametrize("n", [2, 64, 130, 200])
+def test_cholesky_small_entries(cuda_lib, n):
+    rng = np.random.default_rng(n)
+    d = np.exp(rng.uniform(-3, 3, n))
+    a = np.tril(rng.standard_normal((n, n)) * 10.0 ** rng.uniform(-31, -30, (n, n)), -1)
+    a = a + np.diag(d)
+    low, info = linalg.cholesky_dense(torch.as_tensor(a + np.tril(a, -1).T, device="cuda"))
+    ref = np.tril(a, -1) / np.sqrt(d)[None, :] + np.diag(np.sqrt(d))
+    assert int(info.item()) == 0
+    assert np.all(np.abs(np.tril(low.cpu().numpy()) - ref) <= 4 * U * np.abs(ref))
+
+
+# The columns before the order that fails hold the factor, all entries of the
+# lower triangle from there on are NaN.
+@pytest.mark.parametrize("n,k", [(60, 7), (200, 70), (200, 128), (130, 129)])
+def test_cholesky_failed_factor(cuda_lib, n, k):
+    rng = np.random.default_rng(k)
+    g = rng.standard_normal((n, n + 5))
+    a = g @ g.T
+    ref = np.linalg.cholesky(a)
+    a[k, k] = -1.0
+    low, info = linalg.cholesky_dense(torch.as_tensor(a, device="cuda"))
+    low = np.tril(low.cpu().numpy())
+    assert int(info.item()) == k + 1
+    assert np.abs(low[:k, :k] - ref[:k, :k]).max() <= 1e-10 * np.abs(ref).max()
+    assert np.isnan(low[k:, k:][np.tril_indices(n - k)]).all()
+
+
 # The same through the marginal likelihood: 63 points at distance r from the
 # last (kernel value c there), sqrt(2) r or 2 r from one another (c^2, c^4), and
 # a negative jitter that leaves D on Sigma's diagonal.  The leading minors are
