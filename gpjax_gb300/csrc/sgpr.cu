@@ -560,7 +560,11 @@ __global__ void __launch_bounds__(256)
   __shared__ double red[4][AB][D + 1];
   const int il = threadIdx.x & (AB - 1), ph = threadIdx.x >> 6;
   const int i = blockIdx.x * AB + il, split = blockIdx.y;
-  const double inv = 1.0 / theta[n_ls], ka = kshape<double>(kind, theta, n_ls);
+  // The RBF's value is its own coefficient and stands in Phi, times the variance;
+  // a variance of zero or far from one (its inverse or the products may leave the
+  // range) has it evaluated again, as the other kernels have.
+  const double s2 = theta[n_ls], inv = 1.0 / s2, ka = kshape<double>(kind, theta, n_ls);
+  const bool stored = kind == GPK_RBF && s2 >= 1e-6 && s2 <= 1e6;
   double zi[D], al[D], az[D], av = 0.0;
 #pragma unroll
   for (int k = 0; k < D; ++k) {
@@ -579,8 +583,8 @@ __global__ void __launch_bounds__(256)
         sq = fma(dz[k], dz[k], sq);
       }
       double k1, c1;
-      if (kind == GPK_RBF)
-        k1 = c1 = PhiT[(int64_t)j * ldm + i] * inv;  // the value is its own coefficient
+      if (stored)
+        k1 = c1 = PhiT[(int64_t)j * ldm + i] * inv;
       else
         kval_dcoef<double>(kind, sq, 1.0, k1, c1, ka);
       av = fma(g, k1, av);

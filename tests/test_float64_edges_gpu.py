@@ -187,6 +187,22 @@ def test_elbo_column_blocks(cuda_lib, n, m):
     assert np.allclose(gz, gzref, rtol=max(1e-6, 10 * tol), atol=1e-7 * np.abs(gzref).max())
 
 
+# Variances where 1 / variance is no number or Phi holds nothing: the bounds of
+# the parity test for a well conditioned K.
+@pytest.mark.parametrize("kind", [0, 1])
+@pytest.mark.parametrize("var", [0.0, 1e-310, 1e-7, 30.0])
+def test_elbo_small_variance(cuda_lib, kind, var):
+    rng = np.random.default_rng(5)
+    x = rng.uniform(-2, 2, size=(400, 2))
+    y = np.sin(x).sum(1, keepdims=True) + 0.1 * rng.standard_normal((400, 1))
+    Z, ls = x[:12], np.array([0.3, 0.4])
+    val, g, gz = elbo_run(kind, x, y, Z, ls, var, 0.3, 0.1)
+    ref, gref, gzref = elbo_oracle(kind, x, y, Z, ls, var, 0.3, 0.1)
+    assert abs(val - ref) <= 1e-9 * abs(ref)
+    assert np.allclose(g, gref, rtol=1e-6, atol=1e-7 * np.abs(gref).max())
+    assert np.allclose(gz, gzref, rtol=1e-6, atol=1e-7 * np.abs(gzref).max())
+
+
 # exp(-a) with a formed in float64 from t = sqrt(sq): a is off by at most 4 u a
 # (square, sqrt, constant, product), so the value by (4 a + 6) u plus the
 # functions' own last bit; past 708 the results are below 2^-1021, where one
