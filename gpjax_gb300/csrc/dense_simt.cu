@@ -325,7 +325,7 @@ __global__ void __launch_bounds__(FX_NT)
   pdl_trigger();
   __shared__ long long S[FX_NB][FX_NB + 1];
   __shared__ Limbs lim[2][FX_G][FX_NB];  // this group's columns and the last one's
-  __shared__ int ex[FX_NB], sbad[FX_NB], sdead;
+  __shared__ int ex[FX_NB], sbad[FX_NB], sinf[FX_NB], sdead;
   const int nb = min(FX_NB, n - k0);
   const int i = threadIdx.x & 63, g = threadIdx.x >> 6;
   double av[FX_EL];  // every load in flight at once
@@ -335,8 +335,12 @@ __global__ void __launch_bounds__(FX_NT)
     av[u] = r < nb && c <= r ? A[(int64_t)(k0 + r) * lda + k0 + c] : 0.0;
   }
   if (threadIdx.x < FX_NB) {
-    ex[i] = i < nb ? scale_of(A[(int64_t)(k0 + i) * lda + k0 + i]) : 0;
+    const double a = i < nb ? A[(int64_t)(k0 + i) * lda + k0 + i] : 1.0;
+    ex[i] = scale_of(a);
     sbad[i] = 0;
+    // an infinite variance (a noise whose square overflows) is no failure: its
+    // pivot is infinite and the rest of its row and column zero
+    sinf[i] = __double_as_longlong(a) == 0x7ff0000000000000LL;
     if (i == 0) sdead = 0;
   }
   __syncthreads();
@@ -344,7 +348,10 @@ __global__ void __launch_bounds__(FX_NT)
   for (int u = 0; u < FX_EL; ++u) {
     const int e = threadIdx.x + u * FX_NT, r = e >> 6, c = e & 63;
     bool bad = false;
-    S[r][c] = r < nb || r != c ? to_fixed(av[u], ex[r] + ex[c], bad) : ONE;  // identity past nb
+    if (r >= nb || sinf[r] || sinf[c])
+      S[r][c] = r == c ? ONE : 0;  // identity past nb
+    else
+      S[r][c] = to_fixed(av[u], ex[r] + ex[c], bad);
     if (bad) sbad[r] = 1;
   }
   __syncthreads();
@@ -416,15 +423,16 @@ __global__ void __launch_bounds__(FX_NT)
   }
   const bool dead = sdead != 0;  // a pivot failed
   const double nan = __longlong_as_double(0x7ff8000000000000ULL);
+  const double inf = __longlong_as_double(0x7ff0000000000000ULL);
 #pragma unroll 4
   for (int u = 0; u < FX_EL; ++u) {
     const int e = threadIdx.x + u * FX_NT, r = e >> 6, c = e & 63;
     if (r < nb && c < nb && !(keep_upper && c > r))
       A[(int64_t)(k0 + r) * lda + k0 + c] =
-          c > r ? 0.0 : dead ? nan : to_double(S[r][c], ex[r]);
+          c > r ? 0.0 : dead ? nan : c == r && sinf[r] ? inf : to_double(S[r][c], ex[r]);
   }
   if (logdiag && threadIdx.x < nb)
-    logdiag[k0 + i] = dead ? nan : log(to_double(S[i][i], ex[i]));
+    logdiag[k0 + i] = dead ? nan : sinf[i] ? inf : log(to_double(S[i][i], ex[i]));
 }
 
 // Panel solve X L^T = A for 32 rows per CTA: lane = row.  One warp substitutes

@@ -140,6 +140,19 @@ def test_mll_odd_panels(cuda_lib, n):
     assert abs(runs[0][0] - ref) <= 1e-10 * max(1.0, abs(ref))
 
 
+# A noise whose square is infinite: Sigma's diagonal is infinite, its inverse
+# zero, the predictive variance the prior's, and no order fails.
+@pytest.mark.parametrize("n", [30, 100, 400])
+def test_infinite_noise(cuda_lib, n):
+    rng = np.random.default_rng(n)
+    x = rng.uniform(-2, 2, size=(n, 2))
+    post = to_cuda_params(make_posterior(0, np.ones(2), 1.0, 1e200, 0.1))
+    dist = post.predict(torch.as_tensor(x[:5], device="cuda"),
+                        gpx.Dataset(X=x, y=np.sin(x[:, :1])), precision="fp64")
+    assert int(dist.info.item()) == 0
+    assert np.allclose(dist.variance.cpu().numpy(), 1.0 + 1e-6, rtol=1e-15, atol=0)
+
+
 # 16-, 32- and 64-wide tiles with ragged last tiles, and d on both sides of the
 # 64-wide form's bound.  Sums of at most n terms of mixed sign, each with a few
 # roundings and an exp whose argument is below 100: 1e-12 of the sum of the
