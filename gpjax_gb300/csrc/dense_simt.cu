@@ -807,7 +807,7 @@ static cudaError_t potrf_rec(double* A, int64_t lda, int n, int o, int w, double
   XSplit x = planes;
   x.row0 = o + h;
   x.col0 = o;
-  e = xgemm_run(p, x, x, 1, s, true);
+  e = xgemm_run(p, x, x, 1, info, s, true);
   if (e != cudaSuccess) return e;
   return potrf_rec(A, lda, n, o + h, w - h, logdiag, info, keep_upper, planes, s);
 }

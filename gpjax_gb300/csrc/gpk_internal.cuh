@@ -52,6 +52,7 @@ cudaError_t potrf_lower(T* A, int64_t lda, int n, double* logdiag, int* info, do
 struct XRoom {
   void* mem = nullptr;
   size_t bytes = 0;
+  int* info = nullptr;  // the call's info, where a wait that runs out reports
 };
 
 // The float64 factor with products on the tensor cores where `planes` holds the
@@ -64,7 +65,7 @@ cudaError_t potrf_lower_x(double* A, int64_t lda, int n, double* logdiag, int* i
 // CUDA cores.
 inline XRoom planes_in(const XRoom& x, double* from, double* to) {
   if (!x.bytes) return XRoom();
-  return XRoom{from, (size_t)(reinterpret_cast<char*>(to) - reinterpret_cast<char*>(from))};
+  return XRoom{from, (size_t)(reinterpret_cast<char*>(to) - reinterpret_cast<char*>(from)), x.info};
 }
 
 // M = L^-1 (lower, row-major) and V = L^-T (upper, row-major) from the factor L.

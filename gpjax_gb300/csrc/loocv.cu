@@ -172,6 +172,7 @@ extern "C" gpk_status gpk_conjugate_loocv(int kind, int64_t n, int d, const doub
   loocv_layout(n, d, workspace, b);
   const int64_t ld = b.ld;
   const int g1 = (int)cdiv(nn, 256), g2 = (int)cdiv((int64_t)nn * nn, 256);
+  b.x.info = info;
   loocv_init_kernel<<<1, 1, 0, s>>>(info, b.red);
   GPK_LAUNCH_CHECK();
   GPK_CUDA_TRY(scale_inputs<double>(x, ldx, nn, d, theta, n_ls, b.xs, s));

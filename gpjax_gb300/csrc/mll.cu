@@ -239,6 +239,7 @@ static gpk_status mll_run(int kind, int n, int d, const double* x, int64_t ldx, 
                           cudaStream_t s, bool room = true) {
   MllBuffers<T> b;
   mll_layout<T>(n, d, ws, b, room);
+  b.x.info = info;
   prof_mark(0, s);
   init_info_kernel<<<1, 1, 0, s>>>(info);
   GPK_LAUNCH_CHECK();

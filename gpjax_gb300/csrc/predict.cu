@@ -153,6 +153,7 @@ gpk_status predict_run(int kind, int n, int t, int d, const double* x, int64_t l
                        cudaStream_t s) {
   PredBuffers<T> b;
   pred_layout<T>(n, t, d, cov != nullptr, ws, b);
+  b.x.info = info;
   pred_init_kernel<<<1, 1, 0, s>>>(info);
   GPK_LAUNCH_CHECK();
   GPK_CUDA_TRY(scale_inputs<T>(x, ldx, n, d, theta, n_ls, b.xs, s));

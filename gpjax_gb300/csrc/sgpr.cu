@@ -778,6 +778,7 @@ gpk_status sgpr_run(int kind, int n, int m, int d, const double* x, int64_t ldx,
   sgpr_layout<T>(n, m, d, ws, b);
   const int64_t ldm = b.ldm;
   if (n_total < 0) n_total = n;
+  b.xk.info = b.xu.info = info;
   sg_init<<<b.nb, 256, 0, s>>>(info, b.err, y, theta, n_ls, n, b.dv, b.ddpart);
   GPK_LAUNCH_CHECK();
   sg_zero<<<1, 64, 0, s>>>(b.red, 64);

@@ -50,6 +50,9 @@ struct XParams {
   int64_t ldc, ldct, sC, sCt;
   double alpha, beta;
   int alpha_mode, beta_mode;  // 0: general; 1: alpha 1 / beta 0; 2: alpha -1 / beta 1
+  int* info;                  // a wait that ran out makes it -1 (may be null)
+  long long wait_cycles;      // bound of every wait
+  int test_stall;             // self-test: the MMA warp waits on a barrier nothing arrives at
 };
 
 // (hi * 2^32 + lo) * 2^e rounded to float64, in integer arithmetic (this
@@ -148,6 +151,7 @@ __global__ void __launch_bounds__(XTHREADS, 1)
   pdl_wait();
   pdl_trigger();
   const uint32_t tmem = ctl->tmem;
+  const long long wlim = p.wait_cycles;
   volatile int* abort_flag = &ctl->abort_flag;
 
   if (warp == 0) {
@@ -156,7 +160,7 @@ __global__ void __launch_bounds__(XTHREADS, 1)
       for (int kc = 0; kc < nk; ++kc) {
         const int s = kc % XSTAGES;
         if (kc >= XSTAGES &&
-            !mbar_wait(&ctl->empty[s], ((kc / XSTAGES) - 1) & 1, abort_flag, nullptr, kWaitCycles))
+            !mbar_wait(&ctl->empty[s], ((kc / XSTAGES) - 1) & 1, abort_flag, nullptr, wlim))
           break;
         uint8_t* st = ring + s * XSTAGE_BYTES;
         mbar_expect_tx(&ctl->full[s], XSTAGE_BYTES);
@@ -166,7 +170,7 @@ __global__ void __launch_bounds__(XTHREADS, 1)
         ++issued;
       }
       for (int kc = max(0, issued - XSTAGES); kc < issued; ++kc)
-        mbar_wait_own(&ctl->full[kc % XSTAGES], (kc / XSTAGES) & 1, kWaitCycles);
+        mbar_wait_own(&ctl->full[kc % XSTAGES], (kc / XSTAGES) & 1, wlim);
     }
   } else if (warp == 1) {
     // The whole warp runs this loop and an elected lane issues: with the
@@ -177,9 +181,11 @@ __global__ void __launch_bounds__(XTHREADS, 1)
     const uint32_t tm = __shfl_sync(0xffffffffu, tmem, 0);
     const bool leader = elect_one();
     bool ok = true, issued_mma = false;
+    if (p.test_stall)
+      ok = __all_sync(0xffffffffu, mbar_wait(&ctl->mdone, 0, abort_flag, nullptr, wlim));
     auto chunk = [&](int kc, const int s) {
       ok = __all_sync(0xffffffffu, mbar_wait(&ctl->full[s], (kc / XSTAGES) & 1, abort_flag,
-                                             nullptr, kWaitCycles));
+                                             nullptr, wlim));
       if (!ok) return;
       tc_fence_after();
       const uint32_t sb = smem_u32(ring) + (uint32_t)s * XSTAGE_BYTES;
@@ -191,8 +197,8 @@ __global__ void __launch_bounds__(XTHREADS, 1)
       for (int pr = 0; pr < XG / 2; ++pr) {
         if (first && kc > 0) {
           const uint32_t ph = ((kc / XPER) - 1) & 1;
-          ok = mbar_wait(&ctl->tempty[2 * pr], ph, abort_flag, nullptr, kWaitCycles) &&
-               mbar_wait(&ctl->tempty[2 * pr + 1], ph, abort_flag, nullptr, kWaitCycles);
+          ok = mbar_wait(&ctl->tempty[2 * pr], ph, abort_flag, nullptr, wlim) &&
+               mbar_wait(&ctl->tempty[2 * pr + 1], ph, abort_flag, nullptr, wlim);
           ok = __all_sync(0xffffffffu, ok);
           if (!ok) return;
           tc_fence_after();
@@ -227,7 +233,7 @@ __global__ void __launch_bounds__(XTHREADS, 1)
     }
     if (!ok && issued_mma) {  // MMAs already issued finish before TMEM is freed
       if (leader) mma_commit(&ctl->mdone);
-      mbar_wait_own(&ctl->mdone, 0, kWaitCycles);
+      mbar_wait_own(&ctl->mdone, 0, wlim);
     }
     __syncwarp();
   } else {
@@ -247,7 +253,7 @@ __global__ void __launch_bounds__(XTHREADS, 1)
         constexpr int per = XPER;
         if (!have || !(kc % per == per - 1 || kc == nk - 1)) continue;
         have = __all_sync(0xffffffffu, mbar_wait(&ctl->tfull[g], (kc / per) & 1, abort_flag,
-                                                 nullptr, kWaitCycles));
+                                                 nullptr, wlim));
         if (!have) continue;
         tc_fence_after();
         const uint32_t tg = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(g * XN + hcol);
@@ -286,10 +292,22 @@ __global__ void __launch_bounds__(XTHREADS, 1)
       return gi < p.M && gj < p.N && !(p.c_lower && gj > gi);
     };
     asm volatile("bar.sync 1, %0;" ::"r"(XEPI_THREADS) : "memory");  // ring free, eb staged
+    // A wait that ran out (its flag is set ahead of the barrier, and with every
+    // sum drained no wait is left to run out): the tile is NaN, straight from the
+    // registers, for copies and MMAs may still be at work in the ring.
+    const bool failed = *abort_flag != 0;
+    if (failed) {
+      for (int c = 0; c < XHC; ++c) {
+        if (!inside(r, hcol + c)) continue;
+        if (C) C[(int64_t)gi0 * p.ldc + j0 + hcol + c] = nan;
+        if (Ct) Ct[(int64_t)(j0 + hcol + c) * p.ldct + gi0] = nan;
+      }
+      if (et == 0 && p.info) atomicMin(p.info, -1);
+    }
     // the old C tile comes into the other half of the ring while the sums are
     // rounded (2.5 us of loads otherwise)
     double* ctile = otile + BM * XTLD;
-    if (C && bm != 1) {
+    if (C && bm != 1 && !failed) {
 #pragma unroll 4
       for (int e = et; e < BM * XN; e += XEPI_THREADS) {
         const int rr = e / XN, cc = e % XN;
@@ -302,8 +320,9 @@ __global__ void __launch_bounds__(XTHREADS, 1)
 #pragma unroll
     for (int c = 0; c < XHC; ++c) {
       const int eb = ctl->eb[hcol + c];
-      const bool bad = !have || ea == XNAN || eb == XNAN;
-      otile[r * XTLD + hcol + c] = bad ? nan : x_round(hi[c], lo[c], ea + eb - 2 * 1022 - 70);
+      const bool bad = ea == XNAN || eb == XNAN;
+      const double v = bad ? nan : x_round(hi[c], lo[c], ea + eb - 2 * 1022 - 70);
+      if (!failed) otile[r * XTLD + hcol + c] = v;
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
     asm volatile("bar.sync 1, %0;" ::"r"(XEPI_THREADS) : "memory");
@@ -315,7 +334,7 @@ __global__ void __launch_bounds__(XTHREADS, 1)
         return __longlong_as_double(__double_as_longlong(v) ^ (long long)0x8000000000000000ULL);
       return alpha * v;
     };
-    if (C) {
+    if (C && !failed) {
 #pragma unroll 8
       for (int e = et; e < BM * XN; e += XEPI_THREADS) {
         const int rr = e / XN, cc = e % XN;
@@ -328,7 +347,7 @@ __global__ void __launch_bounds__(XTHREADS, 1)
         C[(int64_t)(i0 + rr) * p.ldc + j0 + cc] = v;
       }
     }
-    if (Ct) {
+    if (Ct && !failed) {
       for (int e = et; e < BM * XN; e += XEPI_THREADS) {
         const int cc = e / BM, rr = e % BM;
         if (inside(rr, cc)) Ct[(int64_t)(j0 + cc) * p.ldct + i0 + rr] = scaled(otile[rr * XTLD + cc]);
@@ -475,7 +494,8 @@ cudaError_t xsplit_run(const double* src, int64_t ld, int64_t stride, int rows, 
 }
 
 cudaError_t xgemm_run(const GemmProb<double>& p, const XSplit& A, const XSplit& B, int batch,
-                      cudaStream_t s, bool pdl) {
+                      int* info, cudaStream_t s, bool pdl, long long wait_cycles,
+                      int test_stall) {
   if (p.M <= 0 || p.N <= 0 || batch <= 0) return cudaSuccess;
   if (p.K > XMAX_K) return cudaErrorInvalidValue;
   CUtensorMap ma, mb;
@@ -505,6 +525,9 @@ cudaError_t xgemm_run(const GemmProb<double>& p, const XSplit& A, const XSplit& 
   q.beta = p.beta;
   q.alpha_mode = p.alpha == 1.0 ? 1 : p.alpha == -1.0 ? 2 : 0;
   q.beta_mode = p.beta == 0.0 ? 1 : p.beta == 1.0 ? 2 : 0;
+  q.info = info;
+  q.wait_cycles = wait_cycles ? wait_cycles : kWaitCycles;
+  q.test_stall = test_stall;
   const size_t smem = 1024 + (size_t)XSTAGES * XSTAGE_BYTES + sizeof(XCtl);
   cudaFuncSetAttribute(xgemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   const PdlAttr attr(pdl);
@@ -540,7 +563,7 @@ cudaError_t gemm_nt_x(const GemmProb<double>& p, int batch, const XRoom& x, cuda
     e = xsplit_run(p.B, p.ldb, p.sB, p.N, p.K, p.b_tri, batch, B, s);
     if (e != cudaSuccess) return e;
   }
-  return xgemm_run(p, A, B, batch, s, true);  // follows a split kernel
+  return xgemm_run(p, A, B, batch, x.info, s, true);  // follows a split kernel
 }
 
 size_t xroom_factor_bytes(int64_t n) {
@@ -557,3 +580,38 @@ size_t xroom_fit(size_t base, size_t want) {
 }
 
 }  // namespace gpk
+
+// ---------------------------------------------------------------------------
+// Self-test of the bounded waits: one product whose MMA warp waits 20M cycles
+// on a barrier that nothing arrives on.
+// ---------------------------------------------------------------------------
+using namespace gpk;
+
+constexpr int kSelfTestN = 256, kSelfTestK = 128;
+
+extern "C" size_t gpk_selftest_split_wait_timeout_workspace_bytes(void) {
+  return (size_t)kSelfTestN * kSelfTestK * sizeof(double) + 512 +
+         xsplit_bytes(kSelfTestN, kSelfTestK);
+}
+
+extern "C" gpk_status gpk_selftest_split_wait_timeout(double* C, int* info, void* workspace,
+                                                      size_t workspace_bytes,
+                                                      cudaStream_t stream) {
+  if (!C || !info || !workspace ||
+      workspace_bytes < gpk_selftest_split_wait_timeout_workspace_bytes())
+    return GPK_ERR_BAD_ARG;
+  const uintptr_t base = (reinterpret_cast<uintptr_t>(workspace) + 255) & ~uintptr_t(255);
+  double* A = reinterpret_cast<double*>(base);
+  const size_t bytes = (size_t)kSelfTestN * kSelfTestK * sizeof(double);
+  GPK_CUDA_TRY(cudaMemsetAsync(A, 0, bytes, stream));
+  const XSplit x = xsplit_at(reinterpret_cast<void*>(base + bytes), kSelfTestN, kSelfTestK);
+  GPK_CUDA_TRY(xsplit_run(A, kSelfTestK, 0, kSelfTestN, kSelfTestK, TRI_NONE, 1, x, stream));
+  GemmProb<double> p{};
+  p.C = C;
+  p.ldc = kSelfTestN;
+  p.M = p.N = kSelfTestN;
+  p.K = kSelfTestK;
+  p.alpha = 1.0;
+  GPK_CUDA_TRY(xgemm_run(p, x, x, 1, info, stream, false, 20000000LL, 1));
+  return GPK_OK;
+}

@@ -77,10 +77,12 @@ cudaError_t xsplit_run(const double* src, int64_t ld, int64_t stride, int rows, 
 
 // The product of two split operands with p's shape, triangles, outputs, alpha
 // and beta (p.A, p.B and their strides are not read).  Operand rows of batch z
-// start at z * p.M in A and z * p.N in B.  pdl: launched as a programmatic
-// dependent of the kernel before it in the stream.
+// start at z * p.M in A and z * p.N in B.  A wait that runs out makes its tile
+// NaN and *info -1.  pdl: launched as a programmatic dependent of the kernel
+// before it in the stream.  (The last two arguments are the self-test's.)
 cudaError_t xgemm_run(const GemmProb<double>& p, const XSplit& A, const XSplit& B, int batch,
-                      cudaStream_t s, bool pdl = false);
+                      int* info, cudaStream_t s, bool pdl = false, long long wait_cycles = 0,
+                      int test_stall = 0);
 
 // gemm_nt<double> with room for the split form: splits A and B (once when B is
 // the front of A's rows) and multiplies on the tensor cores where that is the

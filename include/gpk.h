@@ -372,6 +372,13 @@ size_t gpk_selftest_wait_timeout_workspace_bytes(void);
 gpk_status gpk_selftest_wait_timeout(int* err_flag, void* workspace, size_t workspace_bytes,
                                      cudaStream_t stream);
 
+/* The same of the split float64 product, whose waits report through the info of
+ * the calls that use it: *info (device, set to 0 by the caller) becomes -1 and
+ * C [256, 256] NaN. */
+size_t gpk_selftest_split_wait_timeout_workspace_bytes(void);
+gpk_status gpk_selftest_split_wait_timeout(double* C, int* info, void* workspace,
+                                           size_t workspace_bytes, cudaStream_t stream);
+
 #ifdef __cplusplus
 }
 #endif

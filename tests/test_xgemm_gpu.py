@@ -10,7 +10,7 @@ import numpy as np
 import pytest
 import torch
 
-from gpjax_gb300 import linalg
+from gpjax_gb300 import _lib, linalg
 
 pytestmark = pytest.mark.gpu
 
@@ -110,3 +110,20 @@ def test_triangular_solve_range_of_right_side(cuda_lib):
     x = linalg.solve_triangular(torch.eye(256, dtype=torch.float64, device="cuda"),
                                 torch.as_tensor(b, device="cuda")).cpu().numpy()
     assert np.array_equal(x, b)
+
+
+def test_split_product_wait_timeout_is_reported(cuda_lib):
+    """A bounded wait that runs out (the self-test's MMA warp waits 20M cycles on
+    a barrier nothing arrives on) gives info = -1 and a NaN result; the context
+    stays usable."""
+    dev = torch.device("cuda")
+    info = torch.zeros(1, dtype=torch.int32, device=dev)
+    c = torch.zeros(256, 256, dtype=torch.float64, device=dev)
+    ws = _lib.workspace(cuda_lib.gpk_selftest_split_wait_timeout_workspace_bytes(), dev)
+    _lib.call("gpk_selftest_split_wait_timeout", c.data_ptr(), info.data_ptr(), ws.data_ptr(),
+              ws.numel(), _lib.stream_ptr())
+    torch.cuda.synchronize()
+    assert int(info.item()) == -1
+    assert torch.isnan(c).all()
+    a = torch.eye(300, dtype=torch.float64, device=dev)
+    assert torch.equal(linalg.matmul(a, a), a)
