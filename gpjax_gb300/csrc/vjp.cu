@@ -8,8 +8,10 @@
 // element's kernel is evaluated once and the inputs are scaled once per tile: a
 // block holds a column tile and walks a strip of row tiles; column sums (d y,
 // theta) stay in registers, and the elements' coefficients pass through shared
-// memory to the threads that sum rows (d x).  All partial sums are added in a
-// fixed order.  Two passes that scaled and evaluated every element twice, and
+// memory to the threads that sum rows (d x).  Each column tile leaves n d partial
+// row sums; past 128 MB of them the columns go in groups, whose sums are taken
+// before the next begins (all at once they would be as large as G at d = 32).
+// All partial sums are added in a fixed order.  Two passes that scaled and evaluated every element twice, and
 // a finalisation in one block, took 1.82 ms at 3000 x 1100, d = 5.
 #include <algorithm>
 #include "gpk_internal.cuh"
@@ -18,8 +20,11 @@ namespace gpk {
 namespace {
 
 struct VjpShape {
-  int te, tn, strips, per;  // tile edge, column tiles, strips of row tiles, row tiles per strip
+  int te, tn;             // tile edge, column tiles
+  int group;              // column tiles at a time
+  int strips, per;        // strips of row tiles, row tiles per strip
 };
+constexpr int64_t VJP_ROW_BYTES = (int64_t)128 << 20;  // partial row sums held at a time
 
 // 64-wide tiles from 256 of them (d <= 16: registers): 165 us against 187 with
 // 32-wide ones at 1024 x 1024, d = 5, and 144 against 150 (d = 12), 92 against
@@ -28,33 +33,39 @@ struct VjpShape {
 // waves of the blocks an SM holds (by registers 3, 2 or 1), a block costing
 // its tiles and about 0.15 of one more: 3000 x 1100, d = 5 took 539 us in 432
 // blocks of two tiles, one wave and a 0.4, and 439 in 288 of three.
-VjpShape vjp_shape(int64_t n, int64_t m, int d) {
+VjpShape vjp_shape(int64_t n, int64_t m, int d, bool need_x) {
   VjpShape s{};
   s.te = d <= 16 && cdiv(n, 64) * cdiv(m, 64) >= 256 ? 64 : 32;
   const int64_t tm = cdiv(n, s.te), slots = 152 * (d <= 4 ? 3 : d <= 8 ? 2 : 1);
   s.tn = (int)cdiv(m, s.te);
   if (!s.tn) return s;
+  s.group = s.tn;
+  if (need_x)
+    s.group = (int)std::max<int64_t>(
+        1, std::min<int64_t>(s.tn, VJP_ROW_BYTES / std::max<int64_t>(1, n * d * 8)));
   double best = 0.0;
   // at most about 8 waves (bounded partial sums)
-  for (int64_t per = std::min(tm, cdiv(tm * s.tn, 8 * slots)); per > 0 && per <= tm; ++per) {
+  for (int64_t per = std::min(tm, cdiv(tm * s.group, 8 * slots)); per > 0 && per <= tm; ++per) {
     const int64_t strips = cdiv(tm, per);
-    const double cost = (double)cdiv(strips * s.tn, slots) * ((double)per + 0.15);
+    const double cost = (double)cdiv(strips * s.group, slots) * ((double)per + 0.15);
     if (!s.per || cost < best) {
       best = cost;
       s.per = (int)per;
       s.strips = (int)strips;
     }
-    if (strips * s.tn <= slots) break;  // one wave: longer strips only cost more
+    if (strips * s.group <= slots) break;  // one wave: longer strips only cost more
   }
   return s;
 }
 
 struct VjpBuf {
-  double *rpart, *cpart, *tpart;  // [tn][n][d], [strips][m][d], [strips * tn][d + 1]
+  // one group's: [group][n][d], [strips][its columns][d], [strips * group][d + 1];
+  // theta's sums over the groups before, [d + 1]
+  double *rpart, *cpart, *tpart, *tsum;
 };
 
 size_t vjp_layout(int64_t n, int64_t m, int d, bool need_x, bool need_y, void* ws, VjpBuf& b) {
-  const VjpShape s = vjp_shape(n, m, d);
+  const VjpShape s = vjp_shape(n, m, d, need_x);
   double* p = static_cast<double*>(ws);
   size_t off = 0;
   auto take = [&](size_t count) {
@@ -62,9 +73,11 @@ size_t vjp_layout(int64_t n, int64_t m, int d, bool need_x, bool need_y, void* w
     off += count;
     return q;
   };
-  b.rpart = need_x ? take((size_t)s.tn * n * d) : nullptr;
-  b.cpart = need_y ? take((size_t)s.strips * m * d) : nullptr;
-  b.tpart = take((size_t)s.strips * s.tn * (d + 1));
+  const int64_t cols = std::min<int64_t>(m, (int64_t)s.group * s.te);
+  b.rpart = need_x ? take((size_t)s.group * n * d) : nullptr;
+  b.cpart = need_y ? take((size_t)s.strips * cols * d) : nullptr;
+  b.tpart = take((size_t)s.strips * s.group * (d + 1));
+  b.tsum = take((size_t)d + 1);
   return off * sizeof(double) + 512;
 }
 
@@ -77,7 +90,8 @@ __host__ __device__ constexpr size_t vjp_smem() {
 
 template <int D, int TE>
 __global__ void __launch_bounds__(256)
-    vjp_tile_kernel(int kind, int n, int m, int d, int per, const double* __restrict__ x,
+    vjp_tile_kernel(int kind, int n, int m, int d, int per, int J0, int cols,
+                    const double* __restrict__ x,
                     int64_t ldx, const double* __restrict__ y, int64_t ldy,
                     const double* __restrict__ theta, int n_ls, const double* __restrict__ G,
                     int64_t ldg, double* __restrict__ rpart, double* __restrict__ cpart,
@@ -88,7 +102,7 @@ __global__ void __launch_bounds__(256)
   double* sy = sx + TE * (D + 1);        // [TE][D + 1]
   double* st = sy + TE * (D + 1);        // [TE][TE + 4]
   double* red = vjp_sm + vjp_smem<D, TE>() / 8 - 8 * (D + 1);
-  const int J = blockIdx.x, j0 = J * TE;
+  const int J = blockIdx.x, j0 = (J0 + J) * TE;  // J: within the group
   const int c = threadIdx.x % TE, ph = threadIdx.x / TE, gj = j0 + c;
   const double ka = kshape<double>(kind, theta, n_ls);
   auto scale = [&](double* out, const double* p, int64_t ld, int o, int rows) {
@@ -172,7 +186,7 @@ __global__ void __launch_bounds__(256)
       const int r = e / d, k = e % d;
       double v = 0.0;
       for (int p = 0; p < PH; ++p) v += st[(p * TE + r) * D + k];
-      if (j0 + r < m) cpart[((int64_t)blockIdx.y * m + j0 + r) * d + k] = v;
+      if (j0 + r < m) cpart[((int64_t)blockIdx.y * cols + J * TE + r) * d + k] = v;
     }
   }
   const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
@@ -192,11 +206,14 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// Block 0: theta, one warp a slot; the others: one output coordinate a thread.
+// The sums of one group of tn column tiles (`cols` columns).  Block 0: theta, one
+// warp a slot; the others: one output coordinate a thread.  Between groups tsum
+// and gx hold the sums so far.
 __global__ void __launch_bounds__(256)
-    vjp_finalize_kernel(int n, int m, int d, int tn, int strips, const double* __restrict__ theta,
-                        int n_ls, const double* __restrict__ rpart,
-                        const double* __restrict__ cpart, const double* __restrict__ tpart,
+    vjp_finalize_kernel(int n, int cols, int d, int tn, int strips, int first_group,
+                        int last_group, const double* __restrict__ theta, int n_ls,
+                        const double* __restrict__ rpart, const double* __restrict__ cpart,
+                        const double* __restrict__ tpart, double* __restrict__ tsum,
                         double* __restrict__ gtheta, double* __restrict__ gx,
                         double* __restrict__ gy) {
   const double s2 = theta[n_ls];
@@ -207,9 +224,13 @@ __global__ void __launch_bounds__(256)
       double t = 0.0;
       for (int q = l; q < tn * strips; q += 32) t += tpart[(int64_t)q * (d + 1) + k];
       t = warp_sum(t);
-      if (l == 0) sl[k] = t;
+      if (l == 0) {
+        if (!first_group) t += tsum[k];
+        sl[k] = tsum[k] = t;
+      }
     }
     __syncthreads();
+    if (!last_group) return;
     if (n_ls > 1 && threadIdx.x < d) gtheta[threadIdx.x] = s2 * sl[threadIdx.x] / theta[threadIdx.x];
     if (threadIdx.x == 0) {
       if (n_ls == 1) {
@@ -224,32 +245,34 @@ __global__ void __launch_bounds__(256)
     return;
   }
   int64_t e = (int64_t)(blockIdx.x - 1) * 256 + threadIdx.x;
-  const int64_t nd = gx ? (int64_t)n * d : 0, md = gy ? (int64_t)m * d : 0;
+  const int64_t nd = gx ? (int64_t)n * d : 0, md = gy ? (int64_t)cols * d : 0;
   const bool first = e < nd;
   if (!first) e -= nd;
   if (!first && e >= md) return;
   const double* p = first ? rpart : cpart;
-  const int64_t stride = (int64_t)(first ? n : m) * d;
+  const int64_t stride = (int64_t)(first ? n : cols) * d;
   const int parts = first ? tn : strips;
-  double t = 0.0;
+  double t = first && !first_group ? gx[e] : 0.0;
 #pragma unroll 8
   for (int q = 0; q < parts; ++q) t += p[q * stride + e];
   const double v = s2 * t / theta[n_ls == 1 ? 0 : (int)(e % d)];
   if (first)
-    gx[e] = -v;
+    gx[e] = last_group ? -v : t;
   else
     gy[e] = v;
 }
 
 template <int D, int TE>
-cudaError_t vjp_launch(int kind, int n, int m, int d, const VjpShape& s, const double* x,
-                       int64_t ldx, const double* y, int64_t ldy, const double* theta, int n_ls,
-                       const double* G, int64_t ldg, const VjpBuf& b, cudaStream_t stream) {
+cudaError_t vjp_launch(int kind, int n, int m, int d, const VjpShape& s, int J0, int tiles,
+                       int cols, const double* x, int64_t ldx, const double* y, int64_t ldy,
+                       const double* theta, int n_ls, const double* G, int64_t ldg,
+                       const VjpBuf& b, cudaStream_t stream) {
   constexpr size_t smem = vjp_smem<D, TE>();
   cudaFuncSetAttribute(vjp_tile_kernel<D, TE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                        (int)smem);
-  vjp_tile_kernel<D, TE><<<dim3(s.tn, s.strips), 256, smem, stream>>>(
-      kind, n, m, d, s.per, x, ldx, y, ldy, theta, n_ls, G, ldg, b.rpart, b.cpart, b.tpart);
+  vjp_tile_kernel<D, TE><<<dim3(tiles, s.strips), 256, smem, stream>>>(
+      kind, n, m, d, s.per, J0, cols, x, ldx, y, ldy, theta, n_ls, G, ldg, b.rpart, b.cpart,
+      b.tpart);
   return launch_status();
 }
 
@@ -264,25 +287,33 @@ cudaError_t cross_cov_vjp(int kind, int n, int m, int d, const double* x, int64_
                           const double* y, int64_t ldy, const double* theta, int n_ls,
                           const double* G, int64_t ldg, double* gtheta, double* gx, double* gy,
                           void* ws, cudaStream_t stream) {
-  const VjpShape s = vjp_shape(n, m, d);
+  const VjpShape s = vjp_shape(n, m, d, gx != nullptr);
   VjpBuf b;
   vjp_layout(n, m, d, gx != nullptr, gy != nullptr, ws, b);
-  if (n > 0 && m > 0) {
-    auto run = [&](auto dim) {
-      constexpr int D = decltype(dim)::value;
-      auto* f = s.te == 64 ? vjp_launch<D, D <= 16 ? 64 : 32> : vjp_launch<D, 32>;
-      return f(kind, n, m, d, s, x, ldx, y, ldy, theta, n_ls, G, ldg, b, stream);
-    };
-    const cudaError_t e = d <= 4    ? run(std::integral_constant<int, 4>{})
-                          : d <= 8  ? run(std::integral_constant<int, 8>{})
-                          : d <= 16 ? run(std::integral_constant<int, 16>{})
-                                    : run(std::integral_constant<int, 32>{});
+  const int groups = s.group ? (int)cdiv(s.tn, s.group) : 1;  // 1 with nothing in it for m = 0
+  for (int g = 0; g < groups; ++g) {
+    const int J0 = g * s.group, tiles = std::min(s.group, s.tn - J0), col0 = J0 * s.te;
+    const int cols = std::min(m - col0, s.group * s.te);
+    if (n > 0 && m > 0) {
+      auto run = [&](auto dim) {
+        constexpr int D = decltype(dim)::value;
+        auto* f = s.te == 64 ? vjp_launch<D, D <= 16 ? 64 : 32> : vjp_launch<D, 32>;
+        return f(kind, n, m, d, s, J0, tiles, cols, x, ldx, y, ldy, theta, n_ls, G, ldg, b, stream);
+      };
+      const cudaError_t e = d <= 4    ? run(std::integral_constant<int, 4>{})
+                            : d <= 8  ? run(std::integral_constant<int, 8>{})
+                            : d <= 16 ? run(std::integral_constant<int, 16>{})
+                                      : run(std::integral_constant<int, 32>{});
+      if (e != cudaSuccess) return e;
+    }
+    const int64_t outs = (gx ? (int64_t)n * d : 0) + (gy ? (int64_t)cols * d : 0);
+    vjp_finalize_kernel<<<(unsigned)(1 + cdiv(outs, 256)), 256, 0, stream>>>(
+        n, cols, d, tiles, s.strips, g == 0, g == groups - 1, theta, n_ls, b.rpart, b.cpart,
+        b.tpart, b.tsum, gtheta, gx, gy ? gy + (int64_t)col0 * d : nullptr);
+    const cudaError_t e = launch_status();
     if (e != cudaSuccess) return e;
   }
-  const int64_t outs = (gx ? (int64_t)n * d : 0) + (gy ? (int64_t)m * d : 0);
-  vjp_finalize_kernel<<<(unsigned)(1 + cdiv(outs, 256)), 256, 0, stream>>>(
-      n, m, d, s.tn, s.strips, theta, n_ls, b.rpart, b.cpart, b.tpart, gtheta, gx, gy);
-  return launch_status();
+  return cudaSuccess;
 }
 
 }  // namespace gpk
@@ -291,7 +322,9 @@ using namespace gpk;
 
 extern "C" size_t gpk_cross_covariance_vjp_workspace_bytes(int64_t n, int64_t m, int d) {
   if (n < 0 || m < 0 || d <= 0) return 256;
-  return cross_cov_vjp_bytes(n, m, d, true, true);
+  // (without the x cotangents the columns go in one group: more strips' partials)
+  return std::max(cross_cov_vjp_bytes(n, m, d, true, true),
+                  cross_cov_vjp_bytes(n, m, d, false, true));
 }
 
 extern "C" gpk_status gpk_cross_covariance_vjp(int kind, int64_t n, int64_t m, int d,

@@ -329,3 +329,13 @@ def test_workspace_queries_grow_with_the_problem(built_lib):
     # the float16 copies of the wide nodes: present from n_pad = 4096 (halves of 2048)
     mixed = {n: lib.gpk_conjugate_mll_workspace_bytes(n, 8, _lib.PREC_MIXED) for n in (3968, 4096)}
     assert mixed[4096] - mixed[3968] > 16 * 2048 * 2048
+
+
+@pytest.mark.parametrize("n,m,d", [(50000, 50000, 32), (65536, 65536, 16), (200000, 20000, 8),
+                                   (1000000, 1000, 4)])
+def test_cross_covariance_cotangent_scratch_is_bounded(built_lib, n, m, d):
+    """The partial sums of the cotangents do not grow with n m: 128 MB of row
+    sums (or one column tile's n d), and columns and theta by at most 8 waves."""
+    from gpjax_gb300 import _lib
+    got = _lib.lib().gpk_cross_covariance_vjp_workspace_bytes(n, m, d)
+    assert got <= max(128 << 20, 8 * n * d) + (32 << 20)

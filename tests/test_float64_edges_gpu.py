@@ -183,6 +183,33 @@ def test_cross_covariance_cotangent_tiles(cuda_lib, kind, n, m, d):
         assert float((g.cpu() - r).abs().max()) <= 1e-12 * 4 * 1.3 * 4 * terms
 
 
+# 128 MB of partial row sums hold 69 of these 79 column tiles: two groups.  Against
+# the same sums in torch; bounds as above.
+def test_cross_covariance_cotangent_groups(cuda_lib):
+    n, m, d = 30000, 5003, 8
+    g = torch.Generator(device="cuda").manual_seed(1)
+    x, z, G = (torch.randn(*s, dtype=torch.float64, device="cuda", generator=g)
+               for s in ((n, d), (m, d), (n, m)))
+    ls = torch.linspace(0.7, 2.0, d, dtype=torch.float64)
+    th = torch.cat([ls, torch.tensor([1.3, 0.0, 0.0], dtype=torch.float64)]).cuda()
+    from gpjax_gb300.objectives import cross_covariance_vjp
+    gth, gx, gz = cross_covariance_vjp(0, d, th, x, z, G, need_x=True, need_y=True)
+    rx, rz, rl = torch.zeros_like(x), torch.zeros_like(z), torch.zeros(d + 1).to(x)
+    xs, zs = x / ls.cuda(), z / ls.cuda()
+    for lo in range(0, m, 500):
+        k = torch.exp(-0.5 * sum((xs[:, None, q] - zs[None, lo:lo + 500, q]) ** 2
+                                 for q in range(d)))
+        c = G[:, lo:lo + 500] * k
+        rl[d] += c.sum()
+        for q in range(d):
+            df = xs[:, None, q] - zs[None, lo:lo + 500, q]
+            rx[:, q] -= 1.3 * (c * df).sum(1) / ls[q]
+            rz[lo:lo + 500, q] = 1.3 * (c * df).sum(0) / ls[q]
+            rl[q] += 1.3 * (c * df * df).sum() / ls[q]
+    for got, ref, terms in ((gth[:d + 1], rl, n * m), (gx, rx, m), (gz, rz, n)):
+        assert float((got - ref).abs().max()) <= 1e-12 * 4 * 1.3 * 4 * terms
+
+
 # Columns on both sides of a 65536-wide block; the bounds of the parity test of
 # the collapsed bound (the inducing points are spread: K is well conditioned).
 @pytest.mark.parametrize("n,m", [(65536, 33), (65537, 150)])
