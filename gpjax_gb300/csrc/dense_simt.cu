@@ -162,7 +162,8 @@ cudaError_t gemm_nt_blocked(const GemmProb<double>& p, cudaStream_t s) {
 // Diagonal-block Cholesky: one CTA factors the nb x nb block at (k0, k0) in
 // shared memory (unblocked right-looking, two barriers per column).  Each
 // pivot's square root and reciprocal are taken once, by the thread that
-// finishes that diagonal entry.  Float32 form; the float64 one is below.
+// finishes that diagonal entry.  The float32 form's, and the native float64
+// factor's (potrf_lower_native); the float64 objectives' block is below.
 // ---------------------------------------------------------------------------
 template <typename T, int NB>
 __global__ void __launch_bounds__(512) potrf_diag_kernel(T* A, int64_t lda, int n, int k0,

@@ -5,7 +5,8 @@
 // units per warp (measured), and evaluating a kernel function cost more than
 // its distance.  The same functions from 32-bit multiplies take 25 and 20.
 // Accuracy before the final rounding: sqrt 2^-58.9, exp 2^-56 up to x = 32 and
-// 2^-53.2 up to 708 (exhaustive sampling against 60-digit arithmetic).
+// 2^-52.9 up to 512 (sampling against 60-digit arithmetic); from 512 on the
+// library's exp is called.
 #pragma once
 #include <cuda_runtime.h>
 #include <math.h>

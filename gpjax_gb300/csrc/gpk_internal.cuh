@@ -68,15 +68,17 @@ inline XRoom planes_in(const XRoom& x, double* from, double* to) {
   return XRoom{from, (size_t)(reinterpret_cast<char*>(to) - reinterpret_cast<char*>(from)), x.info};
 }
 
-// M = L^-1 (lower, row-major) and V = L^-T (upper, row-major) from the factor L.
-// scratch: n*n/2 elements of T.
-// Native float64 throughout (no fixed point, no split products, the math
-// library's exp and sqrt): where the caller's results amplify the last bit.
+// Native float64 throughout (no fixed point, no split products; the kernel
+// values by the math library's exp and sqrt): a caller's own matrix, and the
+// m x m chain of the mixed collapsed bound.
 cudaError_t potrf_lower_native(double* A, int64_t lda, int n, double* logdiag, int* info,
                                bool zero_upper, cudaStream_t s);
 cudaError_t cross_cov_lib(int kind, int n, int m, int d, const double* xs, const double* ys,
                           const double* theta, int n_ls, int mode, double jitter, double* out,
                           int64_t ldo, cudaStream_t s);
+// M = L^-1 (lower, row-major) and V = L^-T (upper, row-major) from the factor L.
+// scratch: n*n/2 elements of T.  native (float64): the leaves by columns, for
+// the mixed collapsed bound.
 template <typename T>
 cudaError_t trtri_lower(const T* L, int64_t ldl, int n, T* M, int64_t ldm, T* V, int64_t ldv,
                         T* scratch, const XRoom& x, cudaStream_t s,

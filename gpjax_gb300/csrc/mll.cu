@@ -82,8 +82,9 @@ static size_t mll_layout(int64_t n, int d, void* ws, MllBuffers<T>& b, bool room
   b.alpha = a.take<double>(n);
   b.r = a.take<double>(n);
   b.logdiag = a.take<double>(n);
-  b.dtrack = a.take<double>(n);
-  b.rpart = a.take<double>(residual_scratch_doubles((int)n));
+  // float32: pivots and residual partials (float64 has both in the matrix itself)
+  b.dtrack = sizeof(T) == 8 ? nullptr : a.take<double>(n);
+  b.rpart = sizeof(T) == 8 ? nullptr : a.take<double>(residual_scratch_doubles((int)n));
   b.gpart = a.take<double>((size_t)lauum_grad_tiles<T>((int)n) * (d + 2));
   b.fin = a.take<double>(mll_finalize_scratch_doubles(d));
   return a.off + 256;

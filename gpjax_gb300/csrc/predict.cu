@@ -66,8 +66,9 @@ size_t pred_layout(int64_t n, int64_t t, int d, bool want_cov, void* ws, PredBuf
   b.alpha = a.take<double>(n);
   b.r = a.take<double>(n);
   b.logdiag = a.take<double>(n);
-  b.dtrack = a.take<double>(n);
-  b.rpart = a.take<double>(residual_scratch_doubles((int)n));
+  // float32: pivots and residual partials (float64 has both in the matrix itself)
+  b.dtrack = sizeof(T) == 8 ? nullptr : a.take<double>(n);
+  b.rpart = sizeof(T) == 8 ? nullptr : a.take<double>(residual_scratch_doubles((int)n));
   if (sizeof(T) == 8) {
     // the factor's products; then Ktx beside M, and Q^T alone
     const size_t want = n <= 128 && t <= 128 ? 0

@@ -176,11 +176,12 @@ size_t sgpr_layout(int64_t n, int64_t m, int d, void* ws, SgprBuf<T>& b) {
   b.gzs = a.take<double>((size_t)m * d);
   b.ddds = a.take<double>(2);
   b.err = a.take<int>(1);
-  // The mixed form's m x m algebra stays in native float64: at m near 1024 the
-  // condition of Kzz + jitter carries the last bit of its entries and products
-  // to 4e-7 of the gradient of Z, and the form's results are to be the same
-  // from one version to the next (with the split products and fixed-point
-  // blocks a bound at n = 1e6 took 23.1 ms instead of 29.2).
+  // The mixed form's m x m algebra is in native float64: at m near 1024 the
+  // condition of Kzz + jitter carries a last bit of its entries and products to
+  // 4e-7 of the gradient of Z.  That is less than the form's own distance from
+  // float64 (2e-6 to 1e-4); the split products and fixed-point blocks, no farther
+  // from extended precision in the plain form, took 23.1 ms at n = 1e6 instead
+  // of 29.2.
   const size_t small = mixed || m <= 128 ? 0 : std::max(xroom_factor_bytes(m), 2 * xsplit_bytes(m, m));
   size_t want = small;
   if (!mixed) {
