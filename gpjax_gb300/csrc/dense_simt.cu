@@ -326,7 +326,7 @@ __global__ void __launch_bounds__(FX_NT)
   pdl_trigger();
   __shared__ long long S[FX_NB][FX_NB + 1];
   __shared__ Limbs lim[2][FX_G][FX_NB];  // this group's columns and the last one's
-  __shared__ int ex[FX_NB], sbad[FX_NB], sinf[FX_NB], sdead;
+  __shared__ int ex[FX_NB], sbad[FX_NB], sinf[FX_NB], sdead, sany;
   const int nb = min(FX_NB, n - k0);
   const int i = threadIdx.x & 63, g = threadIdx.x >> 6;
   double av[FX_EL];  // every load in flight at once
@@ -339,27 +339,30 @@ __global__ void __launch_bounds__(FX_NT)
     const double a = i < nb ? A[(int64_t)(k0 + i) * lda + k0 + i] : 1.0;
     ex[i] = scale_of(a);
     sbad[i] = 0;
-    // an infinite variance (a noise whose square overflows) is no failure: its
-    // pivot is infinite and the rest of its row and column zero
     sinf[i] = __double_as_longlong(a) == 0x7ff0000000000000LL;
-    if (i == 0) sdead = 0;
+    if (i == 0) sdead = sany = 0;
   }
   __syncthreads();
+  if (threadIdx.x < FX_NB && sinf[i]) sany = 1;
 #pragma unroll
   for (int u = 0; u < FX_EL; ++u) {
     const int e = threadIdx.x + u * FX_NT, r = e >> 6, c = e & 63;
     bool bad = false;
-    if (r >= nb || sinf[r] || sinf[c])
-      S[r][c] = r == c ? ONE : 0;  // identity past nb
-    else
-      S[r][c] = to_fixed(av[u], ex[r] + ex[c], bad);
-    if (bad) sbad[r] = 1;
+    S[r][c] = r < nb || r != c ? to_fixed(av[u], ex[r] + ex[c], bad) : ONE;  // identity past nb
+    if (bad && !(r == c && sinf[r])) sbad[r] = 1;
   }
   __syncthreads();
-  // column k loses the eight columns of a group.  A diagonal entry only falls,
-  // by at most 4 in either half, so its sign is seen before it can leave the
-  // range of [-8, 8): negative once, the row's pivot has failed whatever the
-  // entry wraps to later.
+  // an infinite variance (a noise whose square overflows) is no failure: its
+  // pivot is infinite and the rest of its row and column zero
+  const bool any = sany;
+  if (any) {
+    for (int e = threadIdx.x; e < FX_NB * FX_NB; e += FX_NT) {
+      const int r = e >> 6, c = e & 63;
+      if (sinf[r] || sinf[c]) S[r][c] = r == c ? ONE : 0;
+    }
+    __syncthreads();
+  }
+  // column k loses the eight columns of a group
   auto update = [&](const Limbs (&l)[FX_G][FX_NB], int k) {
     if (k >= nb || i < k) return;
     Acc a0, a1;
@@ -368,10 +371,14 @@ __global__ void __launch_bounds__(FX_NT)
       a0.add(l[q][i], l[q][k]);
       a1.add(l[q + 1][i], l[q + 1][k]);
     }
-    const long long t0 = S[i][k] - a0.value(), t1 = t0 - a1.value();
-    if (i == k && (t0 < 0 || t1 < 0)) sbad[i] = 1;
-    S[i][k] = t1;
+    S[i][k] -= a0.value() + a1.value();
   };
+  // The squared norm of this row of the factor (last 64 threads): in a definite
+  // matrix at most its diagonal entry, which the scale puts below 1.  A diagonal
+  // entry can leave the range of [-8, 8) and come back as another number, but
+  // not between two groups' looks at the norm: the row is marked before its
+  // pivot's turn.
+  float norm = 0.f;
   for (int c0 = 0; c0 < nb; c0 += FX_G) {
     Limbs(&cur)[FX_G][FX_NB] = lim[(c0 / FX_G) & 1];
     Limbs(&prev)[FX_G][FX_NB] = lim[((c0 / FX_G) & 1) ^ 1];
@@ -418,6 +425,14 @@ __global__ void __launch_bounds__(FX_NT)
     }
     if (sdead) break;
     update(cur, c0 + FX_G + g);  // the next group's columns
+    if (g == FX_G - 1) {
+#pragma unroll
+      for (int q = 0; q < FX_G; ++q) {
+        const float f = (float)cur[q][i].h * 0x1p-28f;
+        norm = fmaf(f, f, norm);
+      }
+      if (norm > 1.5f) sbad[i] = 1;
+    }
     const Limbs l = cur[g][i];
     S[i][c0 + g] = ((long long)l.h << 32) + l.l;
     __syncthreads();
@@ -430,10 +445,10 @@ __global__ void __launch_bounds__(FX_NT)
     const int e = threadIdx.x + u * FX_NT, r = e >> 6, c = e & 63;
     if (r < nb && c < nb && !(keep_upper && c > r))
       A[(int64_t)(k0 + r) * lda + k0 + c] =
-          c > r ? 0.0 : dead ? nan : c == r && sinf[r] ? inf : to_double(S[r][c], ex[r]);
+          c > r ? 0.0 : dead ? nan : any && c == r && sinf[r] ? inf : to_double(S[r][c], ex[r]);
   }
   if (logdiag && threadIdx.x < nb)
-    logdiag[k0 + i] = dead ? nan : sinf[i] ? inf : log(to_double(S[i][i], ex[i]));
+    logdiag[k0 + i] = dead ? nan : any && sinf[i] ? inf : log(to_double(S[i][i], ex[i]));
 }
 
 // Panel solve X L^T = A for 32 rows per CTA: lane = row.  One warp substitutes

@@ -10,11 +10,11 @@
 // row's size), split into signed 32-bit halves v = vh 2^32 + vl for the
 // products: three 32 x 32 + 64 multiply-adds and the high half of a fourth.
 //
-// A row whose entry leaves [-1, 1], or whose diagonal entry turns negative
-// after some columns, belongs to a matrix that is not positive definite; it is
-// marked, which makes the pivot of its order fail.  The marks are needed beside
-// the pivots' own signs: 63 columns can take 63 from a diagonal entry, which in
-// 64 bits (a range of [-8, 8)) wraps to a positive number.
+// A row whose entry leaves [-1, 1], or whose norm does, belongs to a matrix that
+// is not positive definite; it is marked, which makes the pivot of its order
+// fail.  The marks are needed beside the pivots' own signs: 63 columns can take
+// 63 from a diagonal entry, which in 64 bits (a range of [-8, 8)) wraps to a
+// positive number.
 #pragma once
 #include "gpk_common.cuh"
 

@@ -51,8 +51,8 @@ struct XParams {
   double alpha, beta;
   int alpha_mode, beta_mode;  // 0: general; 1: alpha 1 / beta 0; 2: alpha -1 / beta 1
   int* info;                  // a wait that ran out makes it -1 (may be null)
-  long long wait_cycles;      // bound of every wait
-  int test_stall;             // self-test: the MMA warp waits on a barrier nothing arrives at
+  long long test_stall;       // self-test (0: off): cycles that the MMA warp first waits on a
+                              // barrier nothing arrives at
 };
 
 // (hi * 2^32 + lo) * 2^e rounded to float64, in integer arithmetic (this
@@ -151,7 +151,6 @@ __global__ void __launch_bounds__(XTHREADS, 1)
   pdl_wait();
   pdl_trigger();
   const uint32_t tmem = ctl->tmem;
-  const long long wlim = p.wait_cycles;
   volatile int* abort_flag = &ctl->abort_flag;
 
   if (warp == 0) {
@@ -160,7 +159,7 @@ __global__ void __launch_bounds__(XTHREADS, 1)
       for (int kc = 0; kc < nk; ++kc) {
         const int s = kc % XSTAGES;
         if (kc >= XSTAGES &&
-            !mbar_wait(&ctl->empty[s], ((kc / XSTAGES) - 1) & 1, abort_flag, nullptr, wlim))
+            !mbar_wait(&ctl->empty[s], ((kc / XSTAGES) - 1) & 1, abort_flag, nullptr, kWaitCycles))
           break;
         uint8_t* st = ring + s * XSTAGE_BYTES;
         mbar_expect_tx(&ctl->full[s], XSTAGE_BYTES);
@@ -170,7 +169,7 @@ __global__ void __launch_bounds__(XTHREADS, 1)
         ++issued;
       }
       for (int kc = max(0, issued - XSTAGES); kc < issued; ++kc)
-        mbar_wait_own(&ctl->full[kc % XSTAGES], (kc / XSTAGES) & 1, wlim);
+        mbar_wait_own(&ctl->full[kc % XSTAGES], (kc / XSTAGES) & 1, kWaitCycles);
     }
   } else if (warp == 1) {
     // The whole warp runs this loop and an elected lane issues: with the
@@ -182,10 +181,10 @@ __global__ void __launch_bounds__(XTHREADS, 1)
     const bool leader = elect_one();
     bool ok = true, issued_mma = false;
     if (p.test_stall)
-      ok = __all_sync(0xffffffffu, mbar_wait(&ctl->mdone, 0, abort_flag, nullptr, wlim));
+      ok = __all_sync(0xffffffffu, mbar_wait(&ctl->mdone, 0, abort_flag, nullptr, p.test_stall));
     auto chunk = [&](int kc, const int s) {
       ok = __all_sync(0xffffffffu, mbar_wait(&ctl->full[s], (kc / XSTAGES) & 1, abort_flag,
-                                             nullptr, wlim));
+                                             nullptr, kWaitCycles));
       if (!ok) return;
       tc_fence_after();
       const uint32_t sb = smem_u32(ring) + (uint32_t)s * XSTAGE_BYTES;
@@ -197,8 +196,8 @@ __global__ void __launch_bounds__(XTHREADS, 1)
       for (int pr = 0; pr < XG / 2; ++pr) {
         if (first && kc > 0) {
           const uint32_t ph = ((kc / XPER) - 1) & 1;
-          ok = mbar_wait(&ctl->tempty[2 * pr], ph, abort_flag, nullptr, wlim) &&
-               mbar_wait(&ctl->tempty[2 * pr + 1], ph, abort_flag, nullptr, wlim);
+          ok = mbar_wait(&ctl->tempty[2 * pr], ph, abort_flag, nullptr, kWaitCycles) &&
+               mbar_wait(&ctl->tempty[2 * pr + 1], ph, abort_flag, nullptr, kWaitCycles);
           ok = __all_sync(0xffffffffu, ok);
           if (!ok) return;
           tc_fence_after();
@@ -233,7 +232,7 @@ __global__ void __launch_bounds__(XTHREADS, 1)
     }
     if (!ok && issued_mma) {  // MMAs already issued finish before TMEM is freed
       if (leader) mma_commit(&ctl->mdone);
-      mbar_wait_own(&ctl->mdone, 0, wlim);
+      mbar_wait_own(&ctl->mdone, 0, kWaitCycles);
     }
     __syncwarp();
   } else {
@@ -253,7 +252,7 @@ __global__ void __launch_bounds__(XTHREADS, 1)
         constexpr int per = XPER;
         if (!have || !(kc % per == per - 1 || kc == nk - 1)) continue;
         have = __all_sync(0xffffffffu, mbar_wait(&ctl->tfull[g], (kc / per) & 1, abort_flag,
-                                                 nullptr, wlim));
+                                                 nullptr, kWaitCycles));
         if (!have) continue;
         tc_fence_after();
         const uint32_t tg = tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(g * XN + hcol);
@@ -284,7 +283,7 @@ __global__ void __launch_bounds__(XTHREADS, 1)
     }
     const double nan = __longlong_as_double(0x7ff8000000000000ULL);
     const double beta = p.beta;
-    const int am = p.alpha_mode, bm = p.beta_mode;
+    const int bm = p.beta_mode;
     double* C = p.C ? p.C + (int64_t)z * p.sC : nullptr;
     double* Ct = p.Ct ? p.Ct + (int64_t)z * p.sCt : nullptr;
     auto inside = [&](int rr, int cc) {
@@ -293,21 +292,16 @@ __global__ void __launch_bounds__(XTHREADS, 1)
     };
     asm volatile("bar.sync 1, %0;" ::"r"(XEPI_THREADS) : "memory");  // ring free, eb staged
     // A wait that ran out (its flag is set ahead of the barrier, and with every
-    // sum drained no wait is left to run out): the tile is NaN, straight from the
-    // registers, for copies and MMAs may still be at work in the ring.
+    // sum drained no wait is left to run out): the tile is NaN through alpha, for
+    // copies still under way may land on what is staged below.
     const bool failed = *abort_flag != 0;
-    if (failed) {
-      for (int c = 0; c < XHC; ++c) {
-        if (!inside(r, hcol + c)) continue;
-        if (C) C[(int64_t)gi0 * p.ldc + j0 + hcol + c] = nan;
-        if (Ct) Ct[(int64_t)(j0 + hcol + c) * p.ldct + gi0] = nan;
-      }
-      if (et == 0 && p.info) atomicMin(p.info, -1);
-    }
+    const int am = failed ? 0 : p.alpha_mode;
+    const double alpha = failed ? nan : p.alpha;
+    if (failed && et == 0 && p.info) atomicMin(p.info, -1);
     // the old C tile comes into the other half of the ring while the sums are
     // rounded (2.5 us of loads otherwise)
     double* ctile = otile + BM * XTLD;
-    if (C && bm != 1 && !failed) {
+    if (C && bm != 1) {
 #pragma unroll 4
       for (int e = et; e < BM * XN; e += XEPI_THREADS) {
         const int rr = e / XN, cc = e % XN;
@@ -321,20 +315,18 @@ __global__ void __launch_bounds__(XTHREADS, 1)
     for (int c = 0; c < XHC; ++c) {
       const int eb = ctl->eb[hcol + c];
       const bool bad = ea == XNAN || eb == XNAN;
-      const double v = bad ? nan : x_round(hi[c], lo[c], ea + eb - 2 * 1022 - 70);
-      if (!failed) otile[r * XTLD + hcol + c] = v;
+      otile[r * XTLD + hcol + c] = bad ? nan : x_round(hi[c], lo[c], ea + eb - 2 * 1022 - 70);
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
     asm volatile("bar.sync 1, %0;" ::"r"(XEPI_THREADS) : "memory");
     // integer modes: a float64 comparison per element runs at the float64 rate
-    const double alpha = p.alpha;
     auto scaled = [&](double v) {
       if (am == 1) return v;
       if (am == 2)
         return __longlong_as_double(__double_as_longlong(v) ^ (long long)0x8000000000000000ULL);
       return alpha * v;
     };
-    if (C && !failed) {
+    if (C) {
 #pragma unroll 8
       for (int e = et; e < BM * XN; e += XEPI_THREADS) {
         const int rr = e / XN, cc = e % XN;
@@ -347,7 +339,7 @@ __global__ void __launch_bounds__(XTHREADS, 1)
         C[(int64_t)(i0 + rr) * p.ldc + j0 + cc] = v;
       }
     }
-    if (Ct && !failed) {
+    if (Ct) {
       for (int e = et; e < BM * XN; e += XEPI_THREADS) {
         const int cc = e / BM, rr = e % BM;
         if (inside(rr, cc)) Ct[(int64_t)(j0 + cc) * p.ldct + i0 + rr] = scaled(otile[rr * XTLD + cc]);
@@ -494,8 +486,7 @@ cudaError_t xsplit_run(const double* src, int64_t ld, int64_t stride, int rows, 
 }
 
 cudaError_t xgemm_run(const GemmProb<double>& p, const XSplit& A, const XSplit& B, int batch,
-                      int* info, cudaStream_t s, bool pdl, long long wait_cycles,
-                      int test_stall) {
+                      int* info, cudaStream_t s, bool pdl, long long test_stall) {
   if (p.M <= 0 || p.N <= 0 || batch <= 0) return cudaSuccess;
   if (p.K > XMAX_K) return cudaErrorInvalidValue;
   CUtensorMap ma, mb;
@@ -526,7 +517,6 @@ cudaError_t xgemm_run(const GemmProb<double>& p, const XSplit& A, const XSplit& 
   q.alpha_mode = p.alpha == 1.0 ? 1 : p.alpha == -1.0 ? 2 : 0;
   q.beta_mode = p.beta == 0.0 ? 1 : p.beta == 1.0 ? 2 : 0;
   q.info = info;
-  q.wait_cycles = wait_cycles ? wait_cycles : kWaitCycles;
   q.test_stall = test_stall;
   const size_t smem = 1024 + (size_t)XSTAGES * XSTAGE_BYTES + sizeof(XCtl);
   cudaFuncSetAttribute(xgemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
@@ -612,6 +602,6 @@ extern "C" gpk_status gpk_selftest_split_wait_timeout(double* C, int* info, void
   p.M = p.N = kSelfTestN;
   p.K = kSelfTestK;
   p.alpha = 1.0;
-  GPK_CUDA_TRY(xgemm_run(p, x, x, 1, info, stream, false, 20000000LL, 1));
+  GPK_CUDA_TRY(xgemm_run(p, x, x, 1, info, stream, false, 20000000LL));
   return GPK_OK;
 }

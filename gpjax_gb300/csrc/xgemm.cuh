@@ -79,10 +79,9 @@ cudaError_t xsplit_run(const double* src, int64_t ld, int64_t stride, int rows, 
 // and beta (p.A, p.B and their strides are not read).  Operand rows of batch z
 // start at z * p.M in A and z * p.N in B.  A wait that runs out makes its tile
 // NaN and *info -1.  pdl: launched as a programmatic dependent of the kernel
-// before it in the stream.  (The last two arguments are the self-test's.)
+// before it in the stream.  (test_stall: the self-test's.)
 cudaError_t xgemm_run(const GemmProb<double>& p, const XSplit& A, const XSplit& B, int batch,
-                      int* info, cudaStream_t s, bool pdl = false, long long wait_cycles = 0,
-                      int test_stall = 0);
+                      int* info, cudaStream_t s, bool pdl = false, long long test_stall = 0);
 
 // gemm_nt<double> with room for the split form: splits A and B (once when B is
 // the front of A's rows) and multiplies on the tensor cores where that is the
