@@ -29,7 +29,8 @@ constexpr double XMIN_MULTS = 8e6;
 constexpr int XMAX_K = 1 << 18;   // the drained 64-bit sums stay below K * 2^41
 
 // K slices summed by one accumulator before it is drained: a group holds up to
-// 7 products of digits up to 128 x 128, and 7 * (4 * 32) * 2^14 < 2^24.
+// 7 products of digits up to 128 x 128, two of them with a top digit, which in
+// the factor's planes reaches 182: (4 * 32) (5 * 128^2 + 2 * 182 * 128) < 2^24.
 constexpr int XPER = 4;
 
 struct XCtl {

@@ -13,10 +13,12 @@
 // the finished sum is rounded to float64 once.  What is left out is the
 // rounding of an element below 2^-56 of its row's scale and the digit products
 // with p + q > 9, below 2^-62 of the two scales each; a float64 loop over k
-// rounds at every step.  Measured largest error over |a_i| |b_j|, against
-// extended precision: 1.8e-17 (a float64 library GEMM 2.1e-16) at K = 512,
-// 7.4e-18 (1.1e-16) at K = 4000 on normal data, 6e-17 (1.2e-14) on constant
-// rows at K = 2048.
+// rounds at every step.  Measured largest error over the product of the two
+// rows' norms, against extended precision: 1.8e-17 (a float64 library GEMM
+// 2.1e-16) at K = 512, 7.4e-18 (1.1e-16) at K = 4000 on normal data, 6e-17
+// (1.2e-14) on constant rows at K = 2048.  It is a bound of norms: an element 2^-56 below its row's
+// largest is lost, which the objectives' operands bear and a caller's need not
+// (gpk_gemm_f64 and gpk_solve_triangular therefore run native float64).
 //
 // This part has 1.7 float64 multiply-adds per clock and SM (measured: a warp
 // instruction every 19 clocks); the 34 float16 products this takes run at
@@ -41,7 +43,7 @@ constexpr int XNAN = 0x7ff;  // row exponent of a row with a NaN or an infinity
 
 // The digits of four elements (integers of 55 fraction bits at the row's
 // scale), one 8-byte store of float16s per plane.  An integer d in [-128, 128]
-// becomes a float16 through the bit pattern of 1536 + d (unit spacing there),
+// (the top digit of the factor's planes: [-182, 182]) becomes a float16 through the bit pattern of 1536 + d (unit spacing there),
 // less 1536: no conversion instruction.
 __device__ __forceinline__ void x_store_digits4(long long (&q)[4], __half* dst, int64_t plane) {
   const __half2 base = __halves2half2(__ushort_as_half(0x6600), __ushort_as_half(0x6600));

@@ -271,3 +271,61 @@ def test_kernel_values_over_range(cuda_lib, kind):
     tol = (4 * a + 12) * U * ref + np.longdouble(2.0) ** -1074 * (1 + f)
     tol = np.where(ref < 2.0 ** -1021, np.maximum(tol, ref), tol)
     assert np.all(np.abs(got - ref) <= tol)
+
+
+# d mll / d obs_stddev in 80-bit arithmetic (float64 and remainder): RBF of unit
+# lengthscale and variance, noise 0.01, n = 1000, d = 4, inputs as below
+NOISE_GRADIENTS = [
+    (-531.36525574425, 1.0825e-14), (-739.6165996968416, 2.0428e-14),
+    (-557.9018744831025, 1.1824e-14), (-482.77064718635705, -7.7161e-15),
+    (-663.4948325301002, -2.2093e-14), (-634.2266094538219, -3.0476e-14),
+    (-645.4184764004425, 1.9429e-15), (-505.19895390241936, -2.6701e-14),
+    (-559.6680332924761, -1.2434e-14), (-559.0717053337254, 4.4797e-14),
+    (-692.2731405473314, -1.6209e-14), (-496.50009117651143, -3.0531e-16),
+    (-582.2574271196455, 2.9476e-14), (-646.1361506316309, 3.0809e-14),
+    (-613.6955398755817, 1.5543e-14), (-557.0100501669929, 9.6589e-15)]
+
+
+def test_noise_gradient_error(cuda_lib):
+    """The factor's split products keep the accuracy of a native float64 factor,
+    whose median error on these inputs is 7.6e-15 (a diagonal of 1.01 puts the
+    digits' row scale, a power of two, at twice the row's bound)."""
+    errors = []
+    for seed, (hi, lo) in enumerate(NOISE_GRADIENTS):
+        rng = np.random.default_rng(seed)
+        x = rng.uniform(-3.0, 3.0, (1000, 4))
+        y = x[:, 0] * x[:, 1] / 4 - x[:, 2] / 2 + 0.2 * rng.uniform(-1.0, 1.0, 1000)
+        kern = gpx.kernels.RBF(lengthscale=1.0, variance=1.0)
+        post = gpx.gps.Prior(kernel=kern) * gpx.likelihoods.Gaussian(1000, obs_stddev=0.1)
+        for p in (kern.lengthscale, kern.variance, post.likelihood.obs_stddev):
+            p.to("cuda")
+        _, g = gpx.objectives.value_and_grad(gpx.objectives.conjugate_mll, post,
+                                             gpx.Dataset(X=x, y=y[:, None]), precision="fp64")
+        errors.append(abs((float(g["likelihood.obs_stddev"]) - hi) - lo) / abs(hi))
+    assert np.median(errors) <= 7.6e-15, sorted(errors)
+
+
+@pytest.mark.parametrize("n", [65, 129, 200, 321])
+@pytest.mark.parametrize("diag", [1.01, 1.99, 2.01, 3.99, 7.9])
+def test_mll_row_scales(cuda_lib, n, diag):
+    """Equal inputs make Sigma c 1 1^T + s I, with everything known in closed
+    form: diagonals around the powers of two and four at which the factor's digit
+    planes change their scale, at the largest top digits."""
+    s, y = 0.01, np.cos(np.arange(n))
+    c = diag - s
+    kern = gpx.kernels.RBF(lengthscale=1.0, variance=c)
+    post = gpx.gps.Prior(kernel=kern, jitter=0.0) * gpx.likelihoods.Gaussian(n, obs_stddev=0.1)
+    for p in (kern.lengthscale, kern.variance, post.likelihood.obs_stddev):
+        p.to("cuda")
+    val, g = gpx.objectives.value_and_grad(gpx.objectives.conjugate_mll, post,
+                                           gpx.Dataset(X=np.zeros((n, 2)), y=y[:, None]),
+                                           precision="fp64")
+    t = s + n * c
+    alpha = (y - c * y.sum() / t) / s
+    ref = -0.5 * (y @ alpha + (n - 1) * np.log(s) + np.log(t) + n * np.log(2 * np.pi))
+    total = y.sum() / t  # of alpha
+    gv = 0.5 * (total ** 2 - n / t)
+    gs = 0.1 * (alpha @ alpha - ((n - 1) / s + 1 / t))
+    assert abs(float(val) - ref) <= 1e-10 * abs(ref)
+    assert abs(float(g["prior.kernel.variance"]) - gv) <= 0.5e-7 * (total ** 2 + n / t)
+    assert abs(float(g["likelihood.obs_stddev"]) - gs) <= 1e-7 * abs(gs)
