@@ -373,7 +373,7 @@ class BatchPlan:
                                      dtype=torch.uint8, device=dev)
 
     def config(self, n: int) -> int:
-        """Tile configuration the autotuner chose for instances of size n."""
+        """Tile configuration chosen for instances of size n."""
         return int(_lib.lib().gpk_batch_plan_config(self._handle, int(n)))
 
     @staticmethod
